@@ -1,4 +1,4 @@
-"""ctypes binding of ``libbrainpylib_b200.so`` and the one call path every operator uses.
+"""ctypes binding of ``libbrainpylib_b200.so``, and the loader of the ``_native`` module that calls it without Python.
 
 The library's entry points are XLA legacy custom-call targets
 ``void f(cudaStream_t, void** buffers, const char* opaque, size_t opaque_len)``;
@@ -15,6 +15,7 @@ from .errors import GPUOperatorNotFound
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, 'libbrainpylib_b200.so')
 _lib = None
+fast = None      # the `_native` module once load_fast() has run
 _targets = {}
 _TARGET_TYPE = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p), ctypes.c_char_p,
                                 ctypes.c_size_t)
@@ -39,6 +40,22 @@ def lib():
     _lib.bpl_workspace_bytes.restype = ctypes.c_size_t
     _lib.bpl_workspace_bytes.argtypes = [ctypes.c_char_p, ctypes.c_char_p, ctypes.c_size_t]
   return _lib
+
+
+def load_fast():
+  """The native host path (``csrc/native.cc``): every operator tries it first.  Missing module = hard error."""
+  global fast
+  if fast is None:
+    lib()
+    try:
+      from . import _native
+    except ImportError as e:
+      raise GPUOperatorNotFound(f'_native ({e})') from e
+    from . import event_ops, sparse_ops
+    _native.register(event_ops.ColumnBlockedCSR, event_ops.backward_rule, sparse_ops.backward_rule,
+                     sparse_ops.outer_backward_rule)
+    fast = _native
+  return fast
 
 
 def target(name):

@@ -1,5 +1,7 @@
 """Compile the CUDA sources under ``csrc/`` into ``libbrainpylib_b200.so`` (in-tree).
 
+and the operators' host path ``csrc/native.cc`` into the extension module ``_native`` (g++, against torch's headers).
+
 Usage: ``python -m brainpylib_b200.build [--force] [--verbose]``
 
 sm_100a only; no fast-math (the just-in-time-connectivity kernels must reproduce the
@@ -10,6 +12,7 @@ import concurrent.futures
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, 'csrc')
@@ -21,6 +24,11 @@ HEADERS = ['abi.h', 'common.cuh', 'spike_scan.cuh', 'row_scatter.cuh', 'cb_scatt
 NVCC = os.environ.get('NVCC', 'nvcc')
 FLAGS = ['-O3', '-std=c++17', '-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo',
          '-Xcompiler', '-fPIC', '-Xptxas', '-v', '-Xcudafe', '--diag_suppress=68']
+
+
+NATIVE_SOURCE = os.path.join(CSRC, 'native.cc')
+NATIVE = os.path.join(HERE, '_native' + sysconfig.get_config_var('EXT_SUFFIX'))
+CXX = os.environ.get('CXX', 'g++')
 
 
 def _sources():
@@ -48,12 +56,47 @@ def _compile(src, verbose):
   return obj, p.stdout
 
 
+def _native_command():
+  import torch
+  from torch.utils import cpp_extension
+  includes = cpp_extension.include_paths('cuda') + [sysconfig.get_path('include')]
+  libs = cpp_extension.library_paths('cuda')
+  return ([CXX, '-O2', '-std=c++17', '-shared', '-fPIC', '-fvisibility=hidden', '-w',
+           f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}'] + [f'-I{d}' for d in includes] +
+          [NATIVE_SOURCE, '-o', NATIVE] + [f'-L{d}' for d in libs] +
+          ['-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch', '-ltorch_python', f'-L{HERE}', '-lbrainpylib_b200',
+           '-Wl,-rpath,$ORIGIN'])
+
+
+def _build_native(force, verbose):
+  """The extension module.  Its text depends on the C ABI only, so it is linked again when the headers change and not
+  when a kernel does.  The object goes to a temporary name first: a reader never sees half a file."""
+  deps = [NATIVE_SOURCE, os.path.join(CSRC, 'abi.h'), os.path.join(CSRC, HEADERS[-1]), os.path.abspath(__file__)]
+  if not force and not _stale(NATIVE, deps):
+    return
+  cmd = _native_command()
+  out = NATIVE + '.tmp'
+  cmd[cmd.index(NATIVE)] = out
+  if verbose:
+    print(' '.join(cmd), flush=True)
+  p = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+  if p.returncode != 0:
+    raise RuntimeError(f'{CXX} failed on native.cc:\n{p.stdout}')
+  os.replace(out, NATIVE)
+
+
 def build(force=False, verbose=False):
-  """Build the shared library if any source is newer than it.  Returns its path."""
+  """Build the shared library and the extension module if any source is newer.  Returns the library's path."""
+  _build_library(force, verbose)
+  _build_native(force, verbose)
+  return LIB
+
+
+def _build_library(force, verbose):
   srcs = _sources()
   all_inputs = [os.path.join(CSRC, f) for f in srcs + HEADERS] + [os.path.abspath(__file__)]
   if not force and not _stale(LIB, all_inputs):
-    return LIB
+    return
   os.makedirs(BUILD_DIR, exist_ok=True)
   if force:
     for s in srcs:
@@ -79,7 +122,6 @@ def build(force=False, verbose=False):
     if verbose:
       print(' '.join(cmd), flush=True)
     subprocess.check_call(cmd)
-  return LIB
 
 
 if __name__ == '__main__':

@@ -63,6 +63,15 @@ __device__ __forceinline__ void red_add(double *p, double v) {
     asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" :: "l"(p), "d"(v) : "memory");
 }
 
+// 4 consecutive values to a 16-byte aligned address
+__device__ __forceinline__ void store_quad(float *p, float a, float b, float c, float d) {
+    *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void store_quad(double *p, double a, double b, double c, double d) {
+    *reinterpret_cast<double2 *>(p) = make_double2(a, b);
+    *reinterpret_cast<double2 *>(p + 2) = make_double2(c, d);
+}
+
 template<typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

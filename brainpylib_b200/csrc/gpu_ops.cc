@@ -66,9 +66,6 @@ using namespace bpl;
 
 extern "C" {
 
-size_t bpl_event_csr_workspace_bytes(uint32_t n_row, int transpose);   // csr_kernels.cu
-size_t bpl_nonzero_workspace_bytes(uint32_t batch_size);               // event_info_kernels.cu
-
 void bpl_profile_scatter_events(void *before, void *after) {
     g_profile_before = static_cast<cudaEvent_t>(before);
     g_profile_after = static_cast<cudaEvent_t>(after);

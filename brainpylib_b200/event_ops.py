@@ -88,22 +88,9 @@ class _EventCSRMatvec(torch.autograd.Function):
   # transforms the tangents and cotangents arrive wrapped, and only `apply` knows how to unwrap them.
   @staticmethod
   def backward(ctx, ct):
-    from .sparse_ops import _CSRMatvec, csr_to_coo
     data, indices, indptr, events = ctx.saved_tensors
-    shape, transpose = ctx.shape, ctx.transpose
-    ct = contiguous(ct)
-    g_data = g_events = None
-    if ctx.needs_input_grad[0]:
-      if data.shape[0] == 1:
-        ones = torch.ones(1, dtype=data.dtype, device=data.device)
-        r = _EventCSRMatvec.apply(ones, indices, indptr, events, shape, transpose)
-        g_data = torch.dot(ct, r).reshape(1)
-      else:
-        row, col = csr_to_coo(indices, indptr)
-        ev = events.to(data.dtype)
-        g_data = ev[row] * ct[col] if transpose else ev[col] * ct[row]
-    if ctx.needs_input_grad[3]:
-      g_events = _CSRMatvec.apply(data, indices, indptr, ct, shape, not transpose, 'vector')
+    g_data, g_events = backward_rule(data, indices, indptr, events, ct, *ctx.shape, ctx.transpose,
+                                     ctx.needs_input_grad[0], ctx.needs_input_grad[3])
     return g_data, None, None, g_events, None, None
 
   @staticmethod
@@ -122,6 +109,24 @@ class _EventCSRMatvec(torch.autograd.Function):
   @staticmethod
   def vmap(info, in_dims, data, indices, indptr, events, shape, transpose):
     return loop_vmap(_EventCSRMatvec.apply, info, in_dims, (data, indices, indptr, events, shape, transpose))
+
+
+def backward_rule(data, indices, indptr, events, ct, n_row, n_col, transpose, need_data, need_events):
+  """Gradients of the event product w.r.t. its weights and its events (``None`` where not needed)."""
+  from .sparse_ops import _CSRMatvec, weight_gradient
+  shape = (n_row, n_col)
+  ct = contiguous(ct)
+  g_data = g_events = None
+  if need_data:
+    if data.shape[0] == 1:
+      ones = torch.ones(1, dtype=data.dtype, device=data.device)
+      r = _EventCSRMatvec.apply(ones, indices, indptr, events, shape, transpose)
+      g_data = torch.dot(ct, r).reshape(1)
+    else:
+      g_data = weight_gradient(indices, indptr, events.to(data.dtype), ct, transpose)
+  if need_events:
+    g_events = _CSRMatvec.apply(data, indices, indptr, ct, shape, not transpose, 'vector')
+  return g_data, g_events
 
 
 def event_csr_matvec(
@@ -163,6 +168,9 @@ def event_csr_matvec(
   y : tensor
     The array of shape ``(shape[1] if transpose else shape[0],)``.
   """
+  y = (_lib.fast or _lib.load_fast()).event_csr_matvec(data, indices, indptr, events, shape, transpose, prepared)
+  if y is not None:
+    return y
   device = device_of(data, indices, indptr, events)
   data = torch.atleast_1d(as_tensor(data, device))
   if not data.dtype.is_floating_point:
@@ -231,6 +239,9 @@ def event_info(events: torch.Tensor):
     (same shape as ``events``), and their count (shape ``()`` or ``(batch,)``).  The reference's
     GPU kernel returns the same set of indices in an arbitrary order.
   """
+  r = (_lib.fast or _lib.load_fast()).event_info(events)
+  if r is not None:
+    return r
   events = as_tensor(events, device_of(events))
   if events.ndim not in (1, 2):
     raise TypeError('Only support 1D boolean vector.')

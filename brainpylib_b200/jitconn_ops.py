@@ -11,6 +11,7 @@ As in the reference, ``transpose`` is consumed here by swapping the two dimensio
 input length.  The GPU kernels receive ``log(1 - conn_prob)`` rounded to float32
 (matvec.py:346-349 with lib/kernel_helper_descriptor.cu:34-38).
 """
+import functools
 from typing import Optional, Tuple
 
 import numpy as np
@@ -29,7 +30,23 @@ __all__ = [
 
 
 def _log_p(conn_prob):
+  return _log_p_of_float(conn_prob) if type(conn_prob) is float else _log_p_of(conn_prob)
+
+
+def _log_p_of(conn_prob):
   return float(np.log((1 - conn_prob) if conn_prob < 1 else 1e-40))
+
+
+_log_p_of_float = functools.lru_cache(maxsize=256)(_log_p_of)
+_HOMO, _UNIFORM, _NORMAL = 0, 1, 2     # the native module's names of the weight kinds
+
+
+def _fast_matvec(vector, events, kind, weight, w1, w2, conn_prob, shape, seed, transpose, outdim_parallel, version):
+  """The native call of a matvec / event-matvec, or ``None`` when it is not the plain case."""
+  if version != 'v2':
+    return None
+  return (_lib.fast or _lib.load_fast()).jit_matvec(vector, events, kind, weight, w1, w2, _log_p(conn_prob), shape, seed,
+                                                    transpose, outdim_parallel)
 
 
 def _descriptor(kind, n_row, n_col, seed, conn_prob, w1, w2):
@@ -309,6 +326,10 @@ def matvec_prob_conn_homo_weight(
     Generate along the output dimension (one stream per output, no atomics) or along
     the input dimension (one stream per input, scattered with atomics).
   """
+  seed = _seed(seed)
+  r = _fast_matvec(vector, False, _HOMO, weight, 0., 0., conn_prob, shape, seed, transpose, outdim_parallel, version)
+  if r is not None:
+    return r
   r = _matvec(vector, 'homo', 0., 0., conn_prob, shape, seed, transpose, outdim_parallel, version)
   weight = as_tensor(weight, r.device, r.dtype)
   return r * weight
@@ -329,6 +350,10 @@ def matvec_prob_conn_uniform_weight(
   r"""Perform :math:`y = M @ v` with connection values drawn uniformly from
   ``[w_low, w_high)``.  See :func:`matvec_prob_conn_homo_weight` for the other arguments."""
   assert w_high > w_low
+  seed = _seed(seed)
+  r = _fast_matvec(vector, False, _UNIFORM, 1., w_low, w_high - w_low, conn_prob, shape, seed, transpose, outdim_parallel, version)
+  if r is not None:
+    return r
   return _matvec(vector, 'uniform', w_low, w_high - w_low, conn_prob, shape, seed, transpose, outdim_parallel,
                  version)
 
@@ -347,6 +372,10 @@ def matvec_prob_conn_normal_weight(
 ) -> torch.Tensor:
   r"""Perform :math:`y = M @ v` with connection values drawn from ``N(w_mu, w_sigma)``.
   See :func:`matvec_prob_conn_homo_weight` for the other arguments."""
+  seed = _seed(seed)
+  r = _fast_matvec(vector, False, _NORMAL, 1., w_mu, w_sigma, conn_prob, shape, seed, transpose, outdim_parallel, version)
+  if r is not None:
+    return r
   return _matvec(vector, 'normal', w_mu, w_sigma, conn_prob, shape, seed, transpose, outdim_parallel, version)
 
 
@@ -365,6 +394,10 @@ def event_matvec_prob_conn_homo_weight(
   connection.  ``events`` is bool or floating point (its non-zero entries are the events).
   ``version='v1'`` (not reachable from the reference's Python layer) uses the counter-based generator of
   lib/kernel_helpers_random.cuh: another random matrix, defined entry by entry by ``(seed, row, column)``."""
+  seed = _seed(seed)
+  r = _fast_matvec(events, True, _HOMO, weight, 0., 0., conn_prob, shape, seed, transpose, outdim_parallel, version)
+  if r is not None:
+    return r
   r = _event_matvec(events, 'homo', 0., 0., conn_prob, shape, seed, transpose, outdim_parallel, version)
   weight = as_tensor(weight, r.device, r.dtype)
   return r * weight
@@ -385,6 +418,10 @@ def event_matvec_prob_conn_uniform_weight(
   r"""Event-driven product with connection values drawn uniformly from ``[w_low, w_high)``.
   ``version``: see :func:`event_matvec_prob_conn_homo_weight`."""
   assert w_high > w_low
+  seed = _seed(seed)
+  r = _fast_matvec(events, True, _UNIFORM, 1., w_low, w_high - w_low, conn_prob, shape, seed, transpose, outdim_parallel, version)
+  if r is not None:
+    return r
   return _event_matvec(events, 'uniform', w_low, w_high - w_low, conn_prob, shape, seed, transpose,
                        outdim_parallel, version)
 
@@ -403,10 +440,19 @@ def event_matvec_prob_conn_normal_weight(
 ) -> torch.Tensor:
   r"""Event-driven product with connection values drawn from ``N(w_mu, w_sigma)``.
   ``version``: see :func:`event_matvec_prob_conn_homo_weight`."""
+  seed = _seed(seed)
+  r = _fast_matvec(events, True, _NORMAL, 1., w_mu, w_sigma, conn_prob, shape, seed, transpose, outdim_parallel, version)
+  if r is not None:
+    return r
   return _event_matvec(events, 'normal', w_mu, w_sigma, conn_prob, shape, seed, transpose, outdim_parallel, version)
 
 
 def _matmat(matrix, kind, w1, w2, conn_prob, shape, seed, version, what):
+  if version == 'v1':
+    r = (_lib.fast or _lib.load_fast()).jit_matmat(matrix, _UNIFORM if kind == 'uniform' else _NORMAL, w1, w2,
+                                                   _log_p(conn_prob), shape, seed)
+    if r is not None:
+      return r
   matrix = as_tensor(matrix, device_of(matrix))
   if matrix.ndim != 2:
     raise ValueError(what)

@@ -85,6 +85,9 @@ def lif_exp_step(y: torch.Tensor, g: torch.Tensor, V: torch.Tensor, t_last: torc
   that the next list-driven product can accumulate into it) and conductances.  ``V``, ``t_last``: float32 ``(n,)``.
   Returns ``(spikes, spike_list)``: float32 0/1 ``(n,)`` and the uint8 buffer holding the compacted spike list
   (``spike_list_bytes(n)`` bytes) for :func:`event_csr_matvec_from_list`; both are allocated when not given."""
+  done = (_lib.fast or _lib.load_fast()).lif_exp_step(y, g, V, t_last, params, t, spikes, spike_list)
+  if done is not None:
+    return done
   n = V.shape[0]
   k = params.n_channels
   if V.device.type != 'cuda':
@@ -107,6 +110,8 @@ def event_csr_matvec_from_list(data, indices, indptr, spike_list, y, *, shape, p
   """``y += A^T spikes`` from the compacted spike list of :func:`lif_exp_step` (``y`` float32 ``(shape[1],)``, already
   zero: ``lif_exp_step`` leaves it so).  With ``prepared`` (see ``prepare_event_csr``) the product runs on the
   column-blocked layout and the CSR operands may be ``None``."""
+  if (_lib.fast or _lib.load_fast()).list_matvec(data, indices, indptr, spike_list, y, shape, prepared):
+    return y
   from .event_ops import _cb_descriptor, ColumnBlockedCSR
   n_row, n_col = int(shape[0]), int(shape[1])
   if y.dtype != torch.float32 or y.numel() != n_col or not y.is_contiguous():

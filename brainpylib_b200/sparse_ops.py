@@ -61,6 +61,71 @@ def csr_to_dense(data, indices, indptr, *, shape):
   return dense
 
 
+class _CSROuter(torch.autograd.Function):
+  """``g[e] = row_vector[row of entry e] * col_vector[indices[e]]`` over the stored entries: the derivative of a CSR
+  product with respect to its weights.  Bilinear; its own transposes are CSR products with the matrix of cotangents."""
+
+  @staticmethod
+  def forward(row_vector, col_vector, indices, indptr):
+    return _lib.load_fast().csr_outer(row_vector, col_vector, indices, indptr)
+
+  @staticmethod
+  def setup_context(ctx, inputs, output):
+    ctx.save_for_backward(*inputs)
+    ctx.save_for_forward(*inputs)
+
+  @staticmethod
+  def backward(ctx, g):
+    row, col, indices, indptr = ctx.saved_tensors
+    need_row, need_col = ctx.needs_input_grad[:2]
+    g_row, g_col = outer_backward_rule(row, col, indices, indptr, g, row.shape[0], col.shape[0], False, need_row, need_col)
+    return g_row, g_col, None, None
+
+  @staticmethod
+  def jvp(ctx, row_dot, col_dot, _indices, _indptr):
+    row, col, indices, indptr = ctx.saved_tensors
+    tangent = None
+    if row_dot is not None:
+      tangent = _CSROuter.apply(contiguous(row_dot), col, indices, indptr)
+    if col_dot is not None:
+      t = _CSROuter.apply(row, contiguous(col_dot), indices, indptr)
+      tangent = t if tangent is None else tangent + t
+    return tangent
+
+  @staticmethod
+  def vmap(info, in_dims, row_vector, col_vector, indices, indptr):
+    return loop_vmap(_CSROuter.apply, info, in_dims, (row_vector, col_vector, indices, indptr))
+
+
+def outer_backward_rule(row, col, indices, indptr, g, n_row, n_col, _transpose, need_row, need_col):
+  shape = (n_row, n_col)
+  g = contiguous(g)
+  return (_CSRMatvec.apply(g, indices, indptr, col, shape, False, 'vector') if need_row else None,
+          _CSRMatvec.apply(g, indices, indptr, row, shape, True, 'vector') if need_col else None)
+
+
+def weight_gradient(indices, indptr, x, ct, transpose):
+  """``x[row] * ct[col]`` of every stored entry if ``transpose`` else ``x[col] * ct[row]``."""
+  row_vector, col_vector = (x, ct) if transpose else (ct, x)
+  return _CSROuter.apply(row_vector, col_vector, indices, indptr)
+
+
+def backward_rule(data, indices, indptr, vector, ct, n_row, n_col, transpose, need_data, need_vector):
+  """Gradients of a CSR product w.r.t. its weights and its vector (``None`` where not needed)."""
+  shape = (n_row, n_col)
+  ct = contiguous(ct)
+  g_data = g_vec = None
+  if need_data:
+    if data.shape[0] == 1:
+      ones = torch.ones(1, dtype=data.dtype, device=data.device)
+      g_data = torch.dot(ct, _CSRMatvec.apply(ones, indices, indptr, vector, shape, transpose, 'vector')).reshape(1)
+    else:
+      g_data = weight_gradient(indices, indptr, vector, ct, transpose)
+  if need_vector:
+    g_vec = _CSRMatvec.apply(data, indices, indptr, ct, shape, not transpose, 'vector')
+  return g_data, g_vec
+
+
 class _CSRMatvec(torch.autograd.Function):
   """Differentiation and batching rules of brainpylib/_src/sparse_ops/cusparse_matvec.py:281-307.
   Reverse mode: w.r.t. the vector the same product with ``not transpose``; w.r.t. homogeneous data
@@ -81,18 +146,8 @@ class _CSRMatvec(torch.autograd.Function):
   @staticmethod
   def backward(ctx, ct):
     data, indices, indptr, vector = ctx.saved_tensors
-    shape, transpose = ctx.shape, ctx.transpose
-    ct = contiguous(ct)
-    g_data = g_vec = None
-    if ctx.needs_input_grad[0]:
-      if data.shape[0] == 1:
-        ones = torch.ones(1, dtype=data.dtype, device=data.device)
-        g_data = torch.dot(ct, _CSRMatvec.apply(ones, indices, indptr, vector, shape, transpose, 'vector')).reshape(1)
-      else:
-        row, col = csr_to_coo(indices, indptr)
-        g_data = vector[row] * ct[col] if transpose else vector[col] * ct[row]
-    if ctx.needs_input_grad[3]:
-      g_vec = _CSRMatvec.apply(data, indices, indptr, ct, shape, not transpose, 'vector')
+    g_data, g_vec = backward_rule(data, indices, indptr, vector, ct, *ctx.shape, ctx.transpose, ctx.needs_input_grad[0],
+                                  ctx.needs_input_grad[3])
     return g_data, None, None, g_vec, None, None, None
 
   # (through `apply`, not the raw kernels: under torch.func transforms tangents arrive wrapped)
@@ -228,6 +283,9 @@ def csr_matvec(
   if method not in ['scalar', 'vector', 'adaptive']:
     raise ValueError('Only support methods: scalar, vector, and adaptive. '
                      f'But we got {method}.')
+  y = (_lib.fast or _lib.load_fast()).csr_matvec(data, indices, indptr, vector, shape, transpose, prepared)
+  if y is not None:
+    return y
   _, data, indices, indptr, vector = _prepare(data, indices, indptr, vector)
   if data.dtype not in [torch.float32, torch.float64]:
     raise TypeError(f'Only support float32 and float64. But we got {data.dtype}.')
@@ -259,6 +317,9 @@ def cusparse_csr_matvec(
 ) -> torch.Tensor:
   """Product of CSR sparse matrix and a dense vector (the op the reference's
   differentiation rules call; same arguments as ``csr_matvec`` without ``method``)."""
+  y = (_lib.fast or _lib.load_fast()).csr_matvec(data, indices, indptr, vector, shape, transpose, None)
+  if y is not None:
+    return y
   _, data, indices, indptr, vector = _prepare(data, indices, indptr, vector)
   if len(shape) != 2:
     raise ValueError(f'shape should be a tuple of int denoting (n_row, n_col). Got {shape}.')

@@ -270,6 +270,17 @@ void bpl_profile_scatter_events(void *before, void *after);
 BPL_FOR_EACH_TARGET(BPL_DECLARE_ONE)
 #undef BPL_DECLARE_ONE
 
+/* ---- helpers of the operator layer ------------------------------------------------------------
+ * Workspace sizes without the name look-up of bpl_workspace_bytes: event_csr_matvec_* / event_cbcsr_matvec_* (also the
+ * size of a spike list of n_row neurons) and nonzero_*.
+ * bpl_csr_outer: g[e] = row_vector[row of entry e] * col_vector[indices[e]] for the nse stored entries of a CSR matrix
+ * (float32, or float64 with is_double): the gradient of a CSR product with respect to its weights
+ * (brainpylib/_src/sparse_ops/cusparse_matvec.py:292-304). */
+size_t bpl_event_csr_workspace_bytes(uint32_t n_row, int transpose);
+size_t bpl_nonzero_workspace_bytes(uint32_t batch_size);
+void bpl_csr_outer(bpl_stream_t stream, const void *row_vector, const void *col_vector, const void *indices,
+                   const void *indptr, void *out, uint32_t n_row, uint32_t nse, int is_double);
+
 /* ---- builder of the column-blocked format (takes the place of the host-side layout code of
  *      brainpylib/_src/sparse_ops/utils.py:21-51 for the one layout this library adds) ---------
  * From a CSR matrix (float32 weights, one shared weight when `homogeneous`; uint32 ids) on the device.

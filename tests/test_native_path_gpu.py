@@ -1,0 +1,55 @@
+"""The native host path: its gradients (C++ nodes, weight gradient in one kernel) against index arithmetic in float64, on
+row lengths around the kernel's units of 4 entries and 4..32 lanes, and its second-order gradients."""
+import numpy as np
+import pytest
+import torch
+
+import cases
+import brainpylib_b200 as bpl
+from brainpylib_b200 import sparse_ops
+
+pytestmark = pytest.mark.gpu
+
+ROWS = {'mixed': [0, 1, 3, 4, 5, 0, 31, 32, 33, 127, 64, 2], 'short': [1] * 70, 'long': [700, 1, 1024, 513], 'empty': [0, 0]}
+
+
+def _expected(data, indices, indptr, x, ct, shape, transpose):
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  d, x, ct = data.detach().double(), x.detach().double(), ct.double()
+  g_data = x[row] * ct[col] if transpose else x[col] * ct[row]
+  g_x = torch.zeros(x.shape[0], dtype=torch.float64, device=x.device)
+  g_x.index_add_(0, row if transpose else col, d * (ct[col] if transpose else ct[row]))
+  return g_data, g_x
+
+
+@pytest.mark.parametrize('event', [False, True])
+@pytest.mark.parametrize('transpose', [False, True])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('rows', sorted(ROWS))
+@pytest.mark.parametrize('offset', [0, 1])     # 1: index array not 16-byte aligned
+def test_gradients_of_weights_and_vector(cuda, rows, dtype, transpose, event, offset):
+  n_col = 900
+  data, indices, indptr, rng = cases.ragged_csr(ROWS[rows], n_col, 3)
+  shape = (len(ROWS[rows]), n_col)
+  indices = torch.as_tensor(np.concatenate([np.zeros(offset, np.int32), indices])).to(cuda)[offset:]
+  indptr = torch.as_tensor(indptr).to(cuda)
+  data = torch.as_tensor(data).to(cuda, dtype).requires_grad_(True)
+  n_in, n_out = shape if transpose else shape[::-1]
+  x = torch.as_tensor(rng.standard_normal(n_in) * (rng.random(n_in) < 0.5)).to(cuda, dtype).requires_grad_(True)
+  ct = torch.as_tensor(rng.standard_normal(n_out)).to(cuda, dtype)
+  op = bpl.event_csr_matvec if event else bpl.csr_matvec
+  y = op(data, indices, indptr, x, shape=shape, transpose=transpose)
+  got = torch.autograd.grad(y, (data, x), ct)
+  tol = dict(rtol=1e-5, atol=1e-4) if dtype == torch.float32 else dict(rtol=1e-12, atol=1e-11)
+  for g, want in zip(got, _expected(data, indices, indptr, x, ct, shape, transpose)):
+    torch.testing.assert_close(g.double(), want, **tol)
+
+
+@pytest.mark.parametrize('transpose', [False, True])
+def test_second_order_gradients(cuda, transpose):
+  data, indices, indptr, rng = cases.csr_case((30, 40), 0.3, 11, dtype=np.float64)
+  w = torch.as_tensor(data).to(cuda).requires_grad_(True)
+  indices, indptr = torch.as_tensor(indices).to(cuda), torch.as_tensor(indptr).to(cuda)
+  x = torch.as_tensor(rng.standard_normal(30 if transpose else 40)).to(cuda).requires_grad_(True)
+  op = lambda w, x: bpl.csr_matvec(w, indices, indptr, x, shape=(30, 40), transpose=transpose)
+  assert torch.autograd.gradcheck(op, (w, x)) and torch.autograd.gradgradcheck(op, (w, x))
