@@ -99,11 +99,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template<int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
-__device__ __forceinline__ void red_add_v4(float *p, float a, float b, float c, float d) {
-    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                 :: "l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 struct CbGroup { uint4 wa, wb, cc; };
 
 template<bool FIXED>

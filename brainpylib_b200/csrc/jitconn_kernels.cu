@@ -4,159 +4,19 @@
 //   gpu_event_matvec{,_atomic}_prob_*_v2  replaces lib/gpu_jitconn_event_matvec{,_atomic}.cu
 //   gpu_matmat_prob_prob_*_v1             replaces lib/gpu_jitconn_matmat.cu
 //
-// Generator scheme (must stay bit-identical to the reference, whose sampled connectivity is
-// the contract): cuRAND XORWOW, `curand_init(seed + i, 0, 0)`; position of the next synapse
-//     pos += (int) ceil( log(curand_uniform(&st)) / log_p )
-// with a float `log`, a float/double division carried out in double, `ceil`, and a
-// conversion to int (lib/gpu_jitconn_matvec.cu:99-106).  The weight of a synapse is drawn
-// after its position and before the next gap: uniform `(T)(u * w_range + w_min)`,
-// normal `(T)(n * w_sigma + w_mu)`, both evaluated in double (lib/gpu_jitconn_matvec.cu:243,386).
-// The same cuRAND device functions and the same expressions are used here, compiled
-// without fast-math, so the bits agree.
-#include <curand_kernel.h>
+// The generator scheme and the walk along a stream: jit_stream.cuh.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
 
 #include "abi.h"
 #include "common.cuh"
+#include "jit_stream.cuh"
 
 namespace bpl {
 namespace {
 
-enum { W_HOMO = 0, W_UNIFORM = 1, W_NORMAL = 2 };
-
-struct Stream {
-    curandState st;
-    double log_p;
-    float inv_log_p;   // float(1 / log_p)
-    float tol_k;       // |inv_log_p| * 2^-20; negative when the shortcuts are switched off
-
-    __device__ __forceinline__ Stream(unsigned int stream_seed, double lp) : log_p(lp) {
-        curand_init(stream_seed, 0, 0, &st);
-        inv_log_p = (float) (1.0 / lp);
-        // log(u) lies in [-22.9, 0]; the shortcuts need 0 <= q = log(u) / log_p < 2^20
-        const bool ok = inv_log_p < 0.0f && inv_log_p > -45000.0f;
-        tol_k = ok ? -inv_log_p * 9.5367432e-7f : -1.0f;
-    }
-
-    // The reference's gap is (int) ceil(log(u) / log_p): float log, double division, ceil.
-    // It is reproduced exactly in up to three stages, each falling through to the next when it
-    // cannot prove the result:
-    //  (1) q = __logf(u) * float(1 / log_p).  __logf is within 2^-21.41 (absolute, u in [0.5, 2])
-    //      or 3 ulp of the true logarithm and logf within 1 ulp; with the float rounding of the
-    //      product (2^-23 q) q is within |1 / log_p| * max(2^-21.19 + 2^-23 |log u|, 1.25 * 2^-21 |log u|)
-    //      of the reference's quotient.  The test distance |1 / log_p| * 2^-20 * (1 + 1.5 |log u|) is
-    //      more than 2.2x that bound everywhere, so when q is farther than it from the nearest
-    //      integer the reference's quotient lies strictly between the same two integers: same ceil.
-    //  (2) the same test with the accurate logf (the value the reference uses): error < 2^-22.9 q,
-    //      margin 2^-21 q.
-    //  (3) the reference's own expression.
-    // rint(q) and its integer value come from adding 1.5 * 2^23, exact for 0 <= q < 2^22.
-    // At a mean gap of 1000 about 1 draw in 200 leaves stage 1 and 1 in 1000 stage 2.
-    __device__ __forceinline__ int gap() {
-        const float u = curand_uniform(&st);
-        if (tol_k > 0.0f) {
-            const float a = __logf(u);
-            const float q = a * inv_log_p;
-            const float t = q + 12582912.0f;
-            const float frac = q - (t - 12582912.0f);
-            if (fabsf(frac) > fmaf(fabsf(a), 1.5f * tol_k, tol_k))
-                return (__float_as_int(t) - 0x4B400000) + (frac > 0.0f ? 1 : 0);
-            const float lg = log(u);
-            const float q2 = lg * inv_log_p;
-            const float t2 = q2 + 12582912.0f;
-            const float frac2 = q2 - (t2 - 12582912.0f);
-            if (fabsf(frac2) > q2 * 4.8e-7f)
-                return (__float_as_int(t2) - 0x4B400000) + (frac2 > 0.0f ? 1 : 0);
-            return (int) ceil(lg / log_p);
-        }
-        return (int) ceil(log(u) / log_p);
-    }
-    // the matmat kernels of the reference hold positions as `unsigned int` (lib/gpu_jitconn_matmat.cu:252);
-    // the shortcuts only return non-negative values, for which both conversions agree
-    __device__ __forceinline__ unsigned int ugap() {
-        const float u = curand_uniform(&st);
-        if (tol_k > 0.0f) {
-            const float a = __logf(u);
-            const float q = a * inv_log_p;
-            const float t = q + 12582912.0f;
-            const float frac = q - (t - 12582912.0f);
-            if (fabsf(frac) > fmaf(fabsf(a), 1.5f * tol_k, tol_k))
-                return (unsigned int) ((__float_as_int(t) - 0x4B400000) + (frac > 0.0f ? 1 : 0));
-            const float lg = log(u);
-            const float q2 = lg * inv_log_p;
-            const float t2 = q2 + 12582912.0f;
-            const float frac2 = q2 - (t2 - 12582912.0f);
-            if (fabsf(frac2) > q2 * 4.8e-7f)
-                return (unsigned int) ((__float_as_int(t2) - 0x4B400000) + (frac2 > 0.0f ? 1 : 0));
-            return (unsigned int) ceil(lg / log_p);
-        }
-        return (unsigned int) ceil(log(u) / log_p);
-    }
-    template<typename T, int KIND>
-    __device__ __forceinline__ T weight(double w1, double w2) {
-        if (KIND == W_UNIFORM) return (T) (curand_uniform(&st) * w2 + w1);
-        if (KIND == W_NORMAL) return (T) (curand_normal(&st) * w2 + w1);
-        return T(1);
-    }
-};
-
-// A synapse weight whose raw draws are taken immediately (the stream must advance exactly as in
-// the reference) but whose value is only computed when asked for.  Event products ask for it on
-// a hit only, which skips the conversions, the double multiply-add and (normal) the Box-Muller
-// transform for every silent input.  The value is produced by cuRAND's own conversion functions
-// on the same raw draws, in the same pairing as curand_normal (two draws on odd calls, the
-// second half of the pair on even calls), so it is bit-identical.
-template<typename T, int KIND>
-struct LazyWeight {
-    unsigned int x, y;
-    int second;   // normal: 1 when the current value is the second half of the pair
-    int have;     // normal: 1 when an unused second half is pending
-
-    __device__ __forceinline__ LazyWeight() : x(0), y(0), second(0), have(0) {}
-    __device__ __forceinline__ void draw(curandState *st) {
-        if (KIND == W_UNIFORM) {
-            x = curand(st);
-        } else if (KIND == W_NORMAL) {
-            if (!have) { x = curand(st); y = curand(st); have = 1; second = 0; }
-            else { have = 0; second = 1; }
-        }
-    }
-    __device__ __forceinline__ T value(double w1, double w2) const {
-        if (KIND == W_UNIFORM) return (T) (_curand_uniform(x) * w2 + w1);
-        if (KIND == W_NORMAL) {
-            const float2 v = _curand_box_muller(x, y);
-            return (T) ((second ? v.y : v.x) * w2 + w1);
-        }
-        return T(1);
-    }
-};
-
 constexpr int JIT_THREADS = 256;
-
-// ------------------------------------------------------------------------------------------
-// Row-parallel (outdim_parallel = True): one thread owns one output row.
-// ------------------------------------------------------------------------------------------
-// Dense input: lib/gpu_jitconn_matvec.cu:84-112, :220-251, :363-394.
-template<typename T, int KIND>
-__global__ void __launch_bounds__(JIT_THREADS)
-jit_rows_dense_kernel(const T *__restrict__ vector, const unsigned int seed, const double log_p,
-                      const double w1, const double w2, const unsigned int num_row,
-                      const unsigned int num_col, T *__restrict__ out) {
-    const unsigned int row_i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row_i >= num_row) return;
-    Stream s(seed + row_i, log_p);
-    T sum = 0;
-    int pos = s.gap();
-    while (pos < num_col) {
-        if (KIND == W_HOMO) {
-            sum += vector[pos];
-        } else {
-            const T rand = s.template weight<T, KIND>(w1, w2);
-            sum += (vector[pos] * rand);
-        }
-        pos += s.gap();
-    }
-    out[row_i] = sum;
-}
 
 // Version 'v1' of the dense-vector product: a Bernoulli test per (row, column) instead of the
 // geometric skip, `conn_prob` being the raw probability (lib/gpu_jitconn_matvec.cu:10-54, :141-187,
@@ -190,131 +50,286 @@ jit_rows_dense_v1_kernel(const T *__restrict__ vector, const unsigned int seed, 
     if (row_i < num_row) out[row_i] = sum;
 }
 
-// Event input read straight from global memory: lib/gpu_jitconn_event_matvec.cu:81-108
-// (homogeneous: adds the event VALUE), :217-248, :365-396 (weight drawn for every synapse,
-// added when the event is truthy).
-template<typename T, typename E, int KIND>
-__global__ void __launch_bounds__(JIT_THREADS)
-jit_rows_event_kernel(const E *__restrict__ events, const unsigned int seed, const double log_p,
-                      const double w1, const double w2, const unsigned int num_row,
-                      const unsigned int num_col, T *__restrict__ out) {
-    const unsigned int row_i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row_i >= num_row) return;
-    Stream s(seed + row_i, log_p);
-    LazyWeight<T, KIND> lw;
-    T sum = 0;
-    int pos = s.gap();
-    while (pos < num_col) {
-        if (KIND == W_HOMO) {
-            sum += events[pos];
-        } else {
-            lw.draw(&s.st);
-            if (events[pos]) sum += lw.value(w1, w2);
-        }
-        pos += s.gap();
+// ------------------------------------------------------------------------------------------
+// Row-parallel (outdim_parallel = True): one thread walks the stream of one output row.
+// ------------------------------------------------------------------------------------------
+// Dense input: `sum += vector[pos] (* weight)`, lib/gpu_jitconn_matvec.cu:84-112, :220-251, :363-394.  Event input:
+// lib/gpu_jitconn_event_matvec.cu:81-108 (homogeneous: adds the event VALUE), :217-248, :365-396 (the weight is added
+// when the event is truthy; it is drawn always, its value computed on a hit only).
+//
+// Where the input is read decides the rate once the walk itself is cheap (1e6 x 1e6, 1e9 connections, all rows):
+//   FROM_GLOBAL  a gather through L1: one 128-byte line per clock and SM whatever is used of it, 3.2 ms
+//   FROM_MASK    events as one bit each in shared memory (1e6 inputs = 125 KB): truthiness is all that is needed.  A hit
+//                leaves its raw draws in a queue of its thread (shared memory); the weights are computed when a queue is
+//                full, by all threads of the warp together, instead of by one thread at a time where it hits
+//   FROM_TILES   the vector in shared memory, in as few tiles as fit (58,000 floats each).  Positions ascend along a
+//                stream, so all streams of a block cross one tile together; a batch that straddles the end of a tile is
+//                simply looked at again in the next one, where the other positions fall into range.
+enum { FROM_GLOBAL = 0, FROM_MASK = 1, FROM_TILES = 2 };
+
+constexpr int WALK_THREADS = 1024;                          // per block with shared memory, one block per SM
+constexpr int GATHER_THREADS = 256;                         // at most, per block without
+constexpr unsigned int WALK_SMEM = 227u * 1024u;            // all that a block can have
+constexpr unsigned int MASK_MAX_BITS = 200u * 1024u * 8u;   // the rest of it: the queues of hits
+
+// The rows (columns) of a block: equal shares, so that no SM is left with a last wave of its own.
+struct Share {
+    unsigned int begin, end;
+    __device__ __forceinline__ explicit Share(unsigned int n) {
+        begin = static_cast<unsigned int>(static_cast<unsigned long long>(n) * blockIdx.x / gridDim.x);
+        end = static_cast<unsigned int>(static_cast<unsigned long long>(n) * (blockIdx.x + 1ull) / gridDim.x);
     }
-    out[row_i] = sum;
+};
+
+// Elements [first, first + count) of `src` into shared memory, by the whole block.
+template<typename T>
+__device__ __forceinline__ void load_tile(T *tile, const T *__restrict__ src, const unsigned int first, const unsigned int count) {
+    constexpr unsigned int PER = 16 / sizeof(T);
+    const T *p = src + first;
+    const unsigned int n_vec = (reinterpret_cast<uintptr_t>(p) & 15u) == 0 ? count / PER : 0u;
+#pragma unroll 4
+    for (unsigned int i = threadIdx.x; i < n_vec; i += blockDim.x)
+        reinterpret_cast<uint4 *>(tile)[i] = reinterpret_cast<const uint4 *>(p)[i];
+    for (unsigned int i = n_vec * PER + threadIdx.x; i < count; i += blockDim.x) tile[i] = p[i];
 }
 
-// Event input held as a bitmask in shared memory (one bit per input neuron).  Used when only
-// the truthiness of an event matters (bool events, or weighted variants) and the mask fits:
-// 1e6 inputs = 125 KB.  One persistent block per SM packs the events once and then walks rows
-// `block + k * grid`; a random 1-byte gather from L2 per synapse becomes a shared-memory read.
-constexpr int MASK_THREADS = 1024;
-constexpr unsigned int MASK_MAX_BITS = 200u * 1024u * 8u;   // 200 KB of shared memory
+template<typename T, typename E, int KIND, bool EVENT, int FROM, bool QUICK>
+__global__ void __launch_bounds__(FROM == FROM_GLOBAL ? GATHER_THREADS : WALK_THREADS)
+jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapParams gp, const double w1, const double w2,
+                const unsigned int num_row, const unsigned int num_col, const unsigned int tile_len, const unsigned int slots,
+                const T scale, T *__restrict__ out) {
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    uint32_t *mask = reinterpret_cast<uint32_t *>(walk_smem);
+    uint32_t *queue = mask + ((num_col + 31u) >> 5) + threadIdx.x;     // slot i of this thread: queue[i * blockDim.x]
+    E *tile = reinterpret_cast<E *>(walk_smem);
+    constexpr int N = Batch<KIND, QUICK>::N;
+    const Share share(num_row);
+    const bool one_tile = tile_len >= num_col;
 
-template<typename T, typename E, int KIND>
-__global__ void __launch_bounds__(MASK_THREADS, 1)
-jit_rows_event_mask_kernel(const E *__restrict__ events, const unsigned int seed, const double log_p,
-                           const double w1, const double w2, const unsigned int num_row,
-                           const unsigned int num_col, T *__restrict__ out) {
-    extern __shared__ uint32_t mask[];
-    pack_event_mask(events, num_col, mask);
-    __syncthreads();
-
-    for (unsigned int row_i = blockIdx.x * MASK_THREADS + threadIdx.x; row_i < num_row;
-         row_i += gridDim.x * MASK_THREADS) {
-        Stream s(seed + row_i, log_p);
-        LazyWeight<T, KIND> lw;
+    if (FROM == FROM_MASK) {
+        pack_event_mask(in, num_col, mask);
+        __syncthreads();
+        // the first event of a word in its top bit: one shift by the position brings an event into the sign bit
+        for (unsigned int i = threadIdx.x; i < ((num_col + 31u) >> 5); i += blockDim.x) mask[i] = __brev(mask[i]);
+        __syncthreads();
+    } else if (FROM == FROM_TILES && one_tile) {
+        load_tile(tile, in, 0, num_col);
+        __syncthreads();
+    }
+    for (unsigned int row0 = share.begin; row0 < share.end; row0 += blockDim.x) {
+        const unsigned int row = row0 + threadIdx.x;
+        const bool live = row < share.end;
+        if (FROM == FROM_GLOBAL && !live) break;
+        if (FROM == FROM_MASK && !__any_sync(FULL_MASK, live)) break;
+        Xorwow s;
+        s.seed(seed + row);
+        Batch<KIND, QUICK> b;
+        unsigned int at = 0;
         T sum = 0;
-        unsigned int hits = 0;   // homogeneous: events are 0 or 1, their float sum is the exact count (< 2^24)
-        int pos = s.gap();
-        while (pos < num_col) {
-            const unsigned int hit = (mask[pos >> 5] >> (pos & 31)) & 1u;
-            if (KIND == W_HOMO) {
-                hits += hit;
-            } else {
-                lw.draw(&s.st);
-                if (hit) sum += lw.value(w1, w2);
+        if (FROM == FROM_TILES) {
+            if (live) b.draw(s, at, num_col, gp);
+            for (unsigned int t0 = 0; t0 < num_col; t0 += tile_len) {
+                const unsigned int len = min(tile_len, num_col - t0);
+                if (!one_tile) {
+                    __syncthreads();                       // everyone is done with the tile before
+                    load_tile(tile, in, t0, len);
+                    __syncthreads();
+                }
+                while (live) {
+                    T w[N];
+                    b.weights(w, w1, w2);
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        const unsigned int i = b.pos[j] - t0;
+                        if (i < len) {
+                            if (KIND == W_HOMO) sum += static_cast<T>(tile[i]);
+                            else sum += (static_cast<T>(tile[i]) * w[j]);
+                        }
+                    }
+                    if (at - t0 >= len) break;             // the batch ends behind this tile
+                    b.draw(s, at, num_col, gp);
+                }
             }
-            pos += s.gap();
-        }
-        if (KIND == W_HOMO) sum = (T) hits;
-        out[row_i] = sum;
-    }
-}
-
-// ------------------------------------------------------------------------------------------
-// Column-parallel (outdim_parallel = False): one thread owns one input column and scatters.
-// ------------------------------------------------------------------------------------------
-// Dense input: lib/gpu_jitconn_matvec_atomic.cu:27-52, :82-110, :143-171.
-template<typename T, int KIND>
-__global__ void __launch_bounds__(JIT_THREADS)
-jit_cols_dense_kernel(const T *__restrict__ vector, const unsigned int seed, const double log_p,
-                      const double w1, const double w2, const unsigned int num_row,
-                      const unsigned int num_col, T *__restrict__ out) {
-    const unsigned int col_i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col_i >= num_col) return;
-    Stream s(seed + col_i, log_p);
-    const T v = vector[col_i];
-    int row_i = s.gap();
-    while (row_i < num_row) {
-        if (KIND == W_HOMO) {
-            atomicAdd(&out[row_i], v);
+        } else if (FROM == FROM_MASK) {
+            // all lanes of the warp stay in the loop until the last is done: what a lane draws behind its end is no hit
+            unsigned int hits = 0;                         // homogeneous: the float sum of 0/1 events is the exact count
+            unsigned int queued = 0, seconds = 0;
+            if (!live) at = num_col;                       // draws behind the end from the start
+            auto drain = [&]() {
+                const unsigned int most = __reduce_max_sync(FULL_MASK, queued);
+                for (unsigned int i = 0; i < most; ++i) {
+                    if (i < queued) {
+                        if (KIND == W_UNIFORM) sum += uniform_weight<T>(queue[i * blockDim.x], w1, w2);
+                        if (KIND == W_NORMAL)
+                            sum += normal_weight<T>(queue[2 * i * blockDim.x], queue[(2 * i + 1) * blockDim.x],
+                                                    (seconds >> i) & 1u, w1, w2);
+                    }
+                }
+                queued = seconds = 0;
+            };
+            // checked: positions may lie behind the end
+            auto look = [&](auto checked) {
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    uint32_t word = 0;                     // 24 bits of the position hold it: the mask has at most 2^21
+                    if (!checked.value || (b.pos[j] & 0xffffffu) < num_col)
+                        word = *reinterpret_cast<const uint32_t *>(walk_smem + ((b.pos[j] >> 3) & 0x1ffffcu));
+                    const uint32_t hit = __funnelshift_l(0u, word, b.pos[j]) >> 31;
+                    if (KIND == W_HOMO) {
+                        hits += hit;
+                    } else {
+                        if (KIND == W_UNIFORM) store_shared_if(hit, queue + queued * blockDim.x, b.raw[j]);
+                        if (KIND == W_NORMAL) {
+                            store_shared_if(hit, queue + 2 * queued * blockDim.x, b.raw[j & ~1]);
+                            store_shared_if(hit, queue + (2 * queued + 1) * blockDim.x, b.raw[j | 1]);
+                            if (j & 1) seconds |= hit << queued;
+                        }
+                        queued += hit;
+                    }
+                }
+                if (KIND != W_HOMO && __any_sync(FULL_MASK, queued + N > slots)) drain();
+            };
+            b.template draw<true>(s, at, num_col, gp);
+            while (__all_sync(FULL_MASK, at < num_col)) {
+                look(std::false_type());
+                b.template draw<true>(s, at, num_col, gp);
+            }
+            look(std::true_type());
+            while (__any_sync(FULL_MASK, at < num_col)) {
+                b.template draw<true>(s, at, num_col, gp);
+                look(std::true_type());
+            }
+            if (KIND == W_HOMO) sum = static_cast<T>(hits);
+            else drain();
         } else {
-            const T rand = s.template weight<T, KIND>(w1, w2);
-            atomicAdd(&out[row_i], v * rand);
+            do {
+                b.draw(s, at, num_col, gp);
+                E v[N];
+#pragma unroll
+                for (int j = 0; j < N; ++j) v[j] = b.pos[j] < num_col ? in[b.pos[j]] : E(0);
+                T w[N];
+                if (!EVENT) b.weights(w, w1, w2);
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    if (b.pos[j] >= num_col) continue;
+                    if (KIND == W_HOMO) sum += static_cast<T>(v[j]);
+                    else if (!EVENT) sum += (static_cast<T>(v[j]) * w[j]);
+                    else if (is_event(v[j])) {
+                        if (KIND == W_UNIFORM) sum += uniform_weight<T>(b.raw[j], w1, w2);
+                        if (KIND == W_NORMAL) sum += normal_weight<T>(b.raw[j & ~1], b.raw[j | 1], j & 1, w1, w2);
+                    }
+                }
+            } while (at < num_col);
         }
-        row_i += s.gap();
+        if (live) out[row] = KIND == W_HOMO ? sum * scale : sum;
     }
 }
 
-// Event input: lib/gpu_jitconn_event_matvec_atomic.cu:30-58, :88-117, :150-178.  There every
-// column walks its stream and only the atomicAdd is conditional; a silent column therefore
-// contributes nothing and its stream is private, so it is skipped here.  Each block compacts
-// the firing columns of its chunk into shared memory and gives one thread to each of them.
-constexpr int COL_CHUNK = JIT_THREADS * 8;
+// ------------------------------------------------------------------------------------------
+// Column-parallel (outdim_parallel = False): one thread walks the stream of one input column and scatters.
+// ------------------------------------------------------------------------------------------
+// Dense input: lib/gpu_jitconn_matvec_atomic.cu:27-52, :82-110, :143-171.  The L2 of a B200 retires about 155 G scattered
+// reductions per second (0.55 per clock and SM); an addition in shared memory runs six times faster.  TILES: a tile of the
+// output lives in shared memory while all columns of the block cross it (positions ascend along a stream), and is then
+// added to the zero-filled output with 16-byte reductions.
+template<typename T>
+__device__ __forceinline__ void flush_tile(const T *tile, T *__restrict__ out, const unsigned int count) {
+    const bool vec = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    const unsigned int n4 = vec ? count / 4 : 0u;
+    for (unsigned int i = threadIdx.x; i < n4; i += blockDim.x) {
+        const float4 v = reinterpret_cast<const float4 *>(tile)[i];
+        if (v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f)
+            red_add_v4(reinterpret_cast<float *>(out) + 4u * i, v.x, v.y, v.z, v.w);
+    }
+    for (unsigned int i = 4u * n4 + threadIdx.x; i < count; i += blockDim.x)
+        if (tile[i] != T(0)) red_add(out + i, tile[i]);
+}
 
-template<typename T, typename E, int KIND>
-__global__ void __launch_bounds__(JIT_THREADS)
-jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, const double log_p,
-                      const double w1, const double w2, const unsigned int num_row,
-                      const unsigned int num_col, T *__restrict__ out) {
+template<typename T, int KIND, bool TILES, bool QUICK>
+__global__ void __launch_bounds__(TILES ? WALK_THREADS : GATHER_THREADS)
+jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const GapParams gp, const double w1, const double w2,
+                const unsigned int num_row, const unsigned int num_col, const unsigned int tile_len, const T scale,
+                T *__restrict__ out) {
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    T *tile = reinterpret_cast<T *>(walk_smem);
+    constexpr int N = Batch<KIND, QUICK>::N;
+    const Share share(num_col);
+    for (unsigned int col0 = share.begin; col0 < share.end; col0 += blockDim.x) {
+        const unsigned int col = col0 + threadIdx.x;
+        const bool live = col < share.end;
+        if (!TILES && !live) break;
+        Xorwow s;
+        s.seed(seed + col);
+        Batch<KIND, QUICK> b;
+        unsigned int at = 0;
+        T v = live ? vector[col] : T(0);
+        if (KIND == W_HOMO) v = v * scale;
+        if (live) b.draw(s, at, num_row, gp);
+        for (unsigned int t0 = 0; t0 < num_row; t0 += tile_len) {
+            const unsigned int len = min(tile_len, num_row - t0);
+            if (TILES) {
+                for (unsigned int i = threadIdx.x; i < len; i += blockDim.x) tile[i] = T(0);
+                __syncthreads();
+            }
+            while (live) {
+                T w[N];
+                b.weights(w, w1, w2);
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    const unsigned int i = b.pos[j] - t0;
+                    if (i < len) {
+                        const T add = KIND == W_HOMO ? v : v * w[j];
+                        if (TILES) atomicAdd(tile + i, add);
+                        else red_add(out + i, add);
+                    }
+                }
+                if (at - t0 >= len) break;
+                b.draw(s, at, num_row, gp);
+            }
+            if (TILES) {
+                __syncthreads();
+                flush_tile(tile, out + t0, len);
+                __syncthreads();
+            }
+        }
+    }
+}
+
+// Event input: lib/gpu_jitconn_event_matvec_atomic.cu:30-58, :88-117, :150-178.  There every column walks its stream and
+// only the atomicAdd is conditional; a silent column contributes nothing and its stream is private, so it is skipped
+// here.  Each block compacts the firing columns of its chunk into shared memory and gives one thread to each of them.
+constexpr int COL_CHUNK = GATHER_THREADS * 8;
+
+template<typename T, typename E, int KIND, bool QUICK>
+__global__ void __launch_bounds__(GATHER_THREADS)
+jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, const GapParams gp, const double w1,
+                      const double w2, const unsigned int num_row, const unsigned int num_col, T *__restrict__ out) {
     __shared__ unsigned int active[COL_CHUNK];
     __shared__ unsigned int n_active;
+    constexpr int N = Batch<KIND, QUICK>::N;
     if (threadIdx.x == 0) n_active = 0;
     __syncthreads();
     const unsigned long long base = static_cast<unsigned long long>(blockIdx.x) * COL_CHUNK;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const unsigned long long c = base + k * JIT_THREADS + threadIdx.x;
+        const unsigned long long c = base + k * GATHER_THREADS + threadIdx.x;
         if (c < num_col && is_event(events[c])) active[atomicAdd(&n_active, 1u)] = static_cast<unsigned int>(c);
     }
     __syncthreads();
     const unsigned int n = n_active;
-    for (unsigned int i = threadIdx.x; i < n; i += JIT_THREADS) {
-        const unsigned int col_i = active[i];
-        Stream s(seed + col_i, log_p);
-        int row_i = s.gap();
-        while (row_i < num_row) {
-            if (KIND == W_HOMO) {
-                atomicAdd(&out[row_i], T(1));
-            } else {
-                const T weight = s.template weight<T, KIND>(w1, w2);
-                atomicAdd(&out[row_i], weight);
-            }
-            row_i += s.gap();
-        }
+    for (unsigned int i = threadIdx.x; i < n; i += GATHER_THREADS) {
+        Xorwow s;
+        s.seed(seed + active[i]);
+        Batch<KIND, QUICK> b;
+        unsigned int at = 0;
+        do {
+            b.draw(s, at, num_row, gp);
+            T w[N];
+            b.weights(w, w1, w2);
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                if (b.pos[j] < num_row) red_add(out + b.pos[j], KIND == W_HOMO ? T(1) : w[j]);
+        } while (at < num_row);
     }
 }
 
@@ -367,7 +382,7 @@ __device__ __forceinline__ void mm_stage_tile(T *tile, const T *__restrict__ X, 
 
 template<typename T, int KIND>
 __global__ void __launch_bounds__(MM_THREADS, (sizeof(T) == 8 ? 1 : 2))     // 32 double sums: more than 64 registers
-jit_matmat_kernel(const T *__restrict__ X, const unsigned int seed, const double log_p, const double w1,
+jit_matmat_kernel(const T *__restrict__ X, const unsigned int seed, const GapParams gp, const double w1,
                   const double w2, const unsigned int m, const unsigned int k, const unsigned int n,
                   T *__restrict__ Y, const unsigned int col0 = 0, const unsigned int *__restrict__ cnt = nullptr,
                   const unsigned int cap = 0, const unsigned int *__restrict__ n_over = nullptr) {
@@ -390,9 +405,9 @@ jit_matmat_kernel(const T *__restrict__ X, const unsigned int seed, const double
     const unsigned int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool vec_ok = (k % (16 / sizeof(T)) == 0) && ((reinterpret_cast<uintptr_t>(X) & 15u) == 0);
 
-    Stream s(seed + n_i, log_p);
-    curandState &st = s.st;
-    unsigned int pos = live ? s.ugap() : 0xffffffffu;
+    curandState st;
+    curand_init(seed + n_i, 0, 0, &st);
+    unsigned int pos = live ? next_position(0u, curand(&st), gp) : 0xffffffffu;
     T sum[MM_ROWS];
 #pragma unroll
     for (int i = 0; i < MM_ROWS; ++i) sum[i] = 0;
@@ -422,7 +437,7 @@ jit_matmat_kernel(const T *__restrict__ X, const unsigned int seed, const double
                     sum[c * 2 + 1] += (x.y * rand);
                 }
             }
-            pos += s.ugap();
+            pos = next_position(pos, curand(&st), gp);
         }
         __syncthreads();
     }
@@ -465,48 +480,38 @@ template<typename T> struct __align__(16) MMEntryPair { MMEntry<T> a, b; };
 // slots per column: the entries, the terminating entry, rounded up to whole pairs
 __host__ __device__ inline unsigned int mm_list_stride(unsigned int cap) { return (cap + 2u) & ~1u; }
 
-template<typename T, int KIND>
+// One thread per column: bound by the latency of its chain (C5: 14 warps per SM), hence the batches (jit_stream.cuh).
+template<typename T, int KIND, bool QUICK>
 __global__ void __launch_bounds__(256)
-jit_matmat_fill_kernel(const unsigned int seed, const double log_p, const double w1, const double w2,
+jit_matmat_fill_kernel(const unsigned int seed, const GapParams gp, const double w1, const double w2,
                        const unsigned int k, const unsigned int n, const unsigned int col0, const unsigned int cap,
                        unsigned int *__restrict__ cnt, MMEntry<T> *__restrict__ entries,
                        unsigned int *__restrict__ n_over) {
     const unsigned int c = blockIdx.x * 256u + threadIdx.x;     // column within the chunk
     const unsigned long long n_i64 = static_cast<unsigned long long>(col0) + c;
     if (n_i64 >= n) return;
-    Stream s(seed + static_cast<unsigned int>(n_i64), log_p);
-    curandState &st = s.st;
+    Xorwow s;
+    s.seed(seed + static_cast<unsigned int>(n_i64));
     MMEntry<T> *mine = entries + static_cast<size_t>(c) * mm_list_stride(cap);
-    unsigned int count = 0;
-    unsigned int pos = s.ugap();
-    // The stream is a chain (state -> draw -> logarithm -> position -> loop test) and a column is one thread, so the
-    // walk is bound by latency, not by issue slots.  The draws of the next FOUR connections (weight, gap, weight, gap,
-    // ... in the stream's order) are therefore taken ahead of the loop test: only the cheap state update chains them,
-    // their logarithms and normal transforms overlap.  Draws behind the last connection of the column are thrown away;
-    // nobody else reads this column's stream.
-    while (pos < k) {
-        T w4[4];
-        unsigned int g4[4];
+    Batch<KIND, QUICK> b;
+    unsigned int count = 0, at = 0;
+    do {
+        b.draw(s, at, k, gp);
+        T w[Batch<KIND, QUICK>::N];
+        b.weights(w, w1, w2);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (KIND == W_NORMAL) w4[u] = (T) (curand_normal(&st) * w2 + w1);
-            else w4[u] = (T) (curand_uniform(&st) * w2 + w1);
-            g4[u] = s.ugap();
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (pos < k) {
+        for (int j = 0; j < b.N; ++j) {
+            if (b.pos[j] < k) {
                 if (count < cap) {
                     MMEntry<T> e;
-                    e.pos = pos;
-                    e.w = w4[u];
+                    e.pos = b.pos[j];
+                    e.w = w[j];
                     mine[count] = e;
                 }
                 ++count;
-                pos += g4[u];
             }
         }
-    }
+    } while (at < k);
     cnt[c] = count;
     // the list ends with a position no tile contains; a list that overflowed reads as empty
     MMEntry<T> last;
@@ -698,26 +703,154 @@ inline unsigned int blocks_for(unsigned int n, unsigned int per_block) {
     return static_cast<unsigned int>((static_cast<unsigned long long>(n) + per_block - 1) / per_block);
 }
 
-template<typename T, int KIND, bool ROWS>
-void jit_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len) {
+template<typename T, typename E>
+struct JitCall {
+    cudaStream_t stream;
+    const E *in;
+    T *out;
     JitArgs a;
-    if (!unpack_jit<KIND>(opaque, opaque_len, a)) return;
-    const T *vector = static_cast<const T *>(buffers[0]);
-    T *y = static_cast<T *>(buffers[1]);
-    if (a.n_row == 0) return;
-    if (ROWS) {
-        jit_rows_dense_kernel<T, KIND><<<blocks_for(a.n_row, JIT_THREADS), JIT_THREADS, 0, stream>>>(
-            vector, a.seed, a.log_p, a.w1, a.w2, a.n_row, a.n_col, y);
-    } else {
-        if (cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(a.n_row), stream) != cudaSuccess) {
+    T scale;       // homogeneous weights: factor of the sums (rows) or of the input (columns)
+};
+
+// Lets a kernel take WALK_SMEM bytes of dynamic shared memory on the current device.
+template<auto KERNEL>
+bool allow_walk_smem() {
+    static thread_local int configured_device = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured_device != dev) {
+        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(WALK_SMEM)) != cudaSuccess) {
+            launch_ok();
+            return false;
+        }
+        configured_device = dev;
+    }
+    return true;
+}
+
+// One block per SM (fewer when there is not a warp of streams for each) and the threads that split its streams into
+// equal waves.
+struct WalkGrid {
+    unsigned int blocks, waves, threads;
+    WalkGrid(unsigned int n, unsigned int at_least) {
+        blocks = std::min(static_cast<unsigned int>(sm_count()), blocks_for(n, 32));
+        const unsigned int per_block = blocks_for(n, blocks);
+        waves = blocks_for(per_block, WALK_THREADS);
+        threads = std::max(blocks_for(blocks_for(per_block, waves), 32) * 32u, at_least);
+    }
+};
+
+// Tiles of equal length, a multiple of 32 elements, as few as fit.
+inline unsigned int tile_length(unsigned int n, size_t elem) {
+    const unsigned int tiles = std::max(1u, blocks_for(n, static_cast<unsigned int>(WALK_SMEM / elem) & ~31u));
+    return blocks_for(blocks_for(n, tiles), 32) * 32u;
+}
+
+// Rules in clocks of one SM.  A gather through L1 takes one clock per connection.  Filling shared memory reads the whole
+// input per block, at about 32 bytes per clock, after a start of some 2000 clocks; a vector in several tiles is read
+// again for every wave of streams.
+template<typename T, typename E, int KIND, bool EVENT>
+void jit_rows(const JitCall<T, E> &c) {
+    const JitArgs &a = c.a;
+    const GapParams gp = gap_params(a.log_p, a.n_col);
+    const double gathers = static_cast<double>(a.n_row) * a.n_col * -std::expm1(a.log_p) / sm_count();
+    constexpr bool TRUTH_ONLY = EVENT && (KIND != W_HOMO || sizeof(E) == 1);
+    WalkGrid g(a.n_row, 512);
+    // (n_col + 5 * 23 mean gaps stay below 2^24)
+    if (gp.quick && TRUTH_ONLY && a.n_col <= MASK_MAX_BITS && -1.0 / a.log_p < 130000.0) {
+        if (gathers > static_cast<double>(a.n_col) * sizeof(E) / 32 + 2000) {
+            constexpr auto kernel = jit_rows_kernel<T, E, KIND, EVENT, TRUTH_ONLY ? FROM_MASK : FROM_GLOBAL, true>;
+            if (!allow_walk_smem<kernel>()) return;
+            // what the mask leaves holds the queues of hits, up to 16 slots per thread (`seconds` has 32 bits); beside a
+            // mask of the largest size only those of 512 threads fit
+            const unsigned int mask_bytes = blocks_for(a.n_col, 32) * 4u, slot_bytes = KIND == W_HOMO ? 0u : KIND == W_UNIFORM ? 4u : 8u;
+            unsigned int slots = 0;
+            if (slot_bytes != 0) {
+                slots = (WALK_SMEM - mask_bytes) / (slot_bytes * g.threads);
+                if (slots < 6u) {
+                    g.threads = 512;
+                    slots = (WALK_SMEM - mask_bytes) / (slot_bytes * g.threads);
+                }
+                slots = std::min(slots, 16u);
+            }
+            kernel<<<g.blocks, g.threads, static_cast<size_t>(mask_bytes) + slots * slot_bytes * g.threads, c.stream>>>(
+                c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, 0, slots, c.scale, c.out);
             launch_ok();
             return;
         }
-        if (a.n_col == 0) return;
-        jit_cols_dense_kernel<T, KIND><<<blocks_for(a.n_col, JIT_THREADS), JIT_THREADS, 0, stream>>>(
-            vector, a.seed, a.log_p, a.w1, a.w2, a.n_row, a.n_col, y);
+    } else if (gp.quick && !TRUTH_ONLY && (KIND == W_HOMO || !EVENT)) {
+        const unsigned int len = tile_length(a.n_col, sizeof(E));
+        const double loads = static_cast<double>(a.n_col) * sizeof(E) / 32 * (len >= a.n_col ? 1 : g.waves);
+        if (0.75 * gathers > loads + 2000) {
+            constexpr auto kernel = jit_rows_kernel<T, E, KIND, EVENT, TRUTH_ONLY ? FROM_GLOBAL : FROM_TILES, true>;
+            if (!allow_walk_smem<kernel>()) return;
+            kernel<<<g.blocks, g.threads, static_cast<size_t>(len) * sizeof(E), c.stream>>>(
+                c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, len, 0, c.scale, c.out);
+            launch_ok();
+            return;
+        }
     }
+    // blocks small enough that every SM gets one
+    const unsigned int threads = std::min(static_cast<unsigned int>(GATHER_THREADS), blocks_for(blocks_for(a.n_row, sm_count()), 32) * 32u);
+    const unsigned int blocks = blocks_for(a.n_row, threads);
+    if (gp.quick)
+        jit_rows_kernel<T, E, KIND, EVENT, FROM_GLOBAL, true><<<blocks, threads, 0, c.stream>>>(
+            c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, a.n_col, 0, c.scale, c.out);
+    else
+        jit_rows_kernel<T, E, KIND, EVENT, FROM_GLOBAL, false><<<blocks, threads, 0, c.stream>>>(
+            c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, a.n_col, 0, c.scale, c.out);
     launch_ok();
+}
+
+// In clocks of one SM: a scattered reduction into L2 takes 1.8, an addition in shared memory 0.3; a tile costs about 0.7
+// per element to clear and to flush, once per wave of columns.
+template<typename T, int KIND>
+void jit_cols(const JitCall<T, T> &c) {
+    const JitArgs &a = c.a;
+    if (cudaMemsetAsync(c.out, 0, sizeof(T) * static_cast<size_t>(a.n_row), c.stream) != cudaSuccess) {
+        launch_ok();
+        return;
+    }
+    if (a.n_col == 0) return;
+    const GapParams gp = gap_params(a.log_p, a.n_row);
+    const double additions = static_cast<double>(a.n_row) * a.n_col * -std::expm1(a.log_p) / sm_count();
+    const WalkGrid g(a.n_col, 512);
+    if (gp.quick && 1.8 * additions > 0.3 * additions + 0.7 * (sizeof(T) / 4) * a.n_row * g.waves + 5000) {
+        const unsigned int len = tile_length(a.n_row, sizeof(T));
+        constexpr auto kernel = jit_cols_kernel<T, KIND, true, true>;
+        if (!allow_walk_smem<kernel>()) return;
+        kernel<<<g.blocks, g.threads, static_cast<size_t>(len) * sizeof(T), c.stream>>>(
+            c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, len, c.scale, c.out);
+        launch_ok();
+        return;
+    }
+    const unsigned int threads = std::min(static_cast<unsigned int>(GATHER_THREADS), blocks_for(blocks_for(a.n_col, sm_count()), 32) * 32u);
+    const unsigned int blocks = blocks_for(a.n_col, threads);
+    (gp.quick ? jit_cols_kernel<T, KIND, false, true> : jit_cols_kernel<T, KIND, false, false>)<<<blocks, threads, 0, c.stream>>>(
+        c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, a.n_row, c.scale, c.out);
+    launch_ok();
+}
+
+template<typename T, typename E, int KIND>
+void jit_cols_event(const JitCall<T, E> &c) {
+    const JitArgs &a = c.a;
+    if (cudaMemsetAsync(c.out, 0, sizeof(T) * static_cast<size_t>(a.n_row), c.stream) != cudaSuccess) {
+        launch_ok();
+        return;
+    }
+    if (a.n_col == 0) return;
+    const GapParams gp = gap_params(a.log_p, a.n_row);
+    (gp.quick ? jit_cols_event_kernel<T, E, KIND, true> : jit_cols_event_kernel<T, E, KIND, false>)<<<
+        blocks_for(a.n_col, COL_CHUNK), GATHER_THREADS, 0, c.stream>>>(c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, c.out);
+    launch_ok();
+}
+
+template<typename T, int KIND, bool ROWS>
+void jit_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len) {
+    JitCall<T, T> c{stream, static_cast<const T *>(buffers[0]), static_cast<T *>(buffers[1]), {}, T(1)};
+    if (!unpack_jit<KIND>(opaque, opaque_len, c.a) || c.a.n_row == 0) return;
+    if (ROWS) jit_rows<T, T, KIND, false>(c);
+    else jit_cols<T, KIND>(c);
 }
 
 template<typename T, int KIND>
@@ -731,55 +864,12 @@ void jit_matvec_v1_impl(cudaStream_t stream, void **buffers, const char *opaque,
     launch_ok();
 }
 
-template<typename T, typename E, int KIND>
-bool enable_mask_kernel(size_t bytes) {
-    static thread_local int configured_device = -1;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (configured_device != dev) {
-        if (cudaFuncSetAttribute(jit_rows_event_mask_kernel<T, E, KIND>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(MASK_MAX_BITS / 8)) != cudaSuccess) {
-            launch_ok();
-            return false;
-        }
-        configured_device = dev;
-    }
-    (void) bytes;
-    return true;
-}
-
 template<typename T, typename E, int KIND, bool ROWS>
 void jit_event_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len) {
-    JitArgs a;
-    if (!unpack_jit<KIND>(opaque, opaque_len, a)) return;
-    const E *events = static_cast<const E *>(buffers[0]);
-    T *y = static_cast<T *>(buffers[1]);
-    if (a.n_row == 0) return;
-    if (ROWS) {
-        // the bitmask holds truthiness only: enough unless a homogeneous product must add float event values
-        const bool truth_only = (KIND != W_HOMO) || (sizeof(E) == 1);
-        const bool big_enough = static_cast<unsigned long long>(a.n_row) >= 4ull * MASK_THREADS;
-        if (truth_only && big_enough && a.n_col <= MASK_MAX_BITS) {
-            const size_t bytes = static_cast<size_t>((a.n_col + 31u) >> 5) * 4;
-            if (!enable_mask_kernel<T, E, KIND>(bytes)) return;
-            const unsigned int grid = min(static_cast<unsigned int>(sm_count()), blocks_for(a.n_row, MASK_THREADS));
-            jit_rows_event_mask_kernel<T, E, KIND><<<grid, MASK_THREADS, bytes, stream>>>(
-                events, a.seed, a.log_p, a.w1, a.w2, a.n_row, a.n_col, y);
-        } else {
-            jit_rows_event_kernel<T, E, KIND><<<blocks_for(a.n_row, JIT_THREADS), JIT_THREADS, 0, stream>>>(
-                events, a.seed, a.log_p, a.w1, a.w2, a.n_row, a.n_col, y);
-        }
-    } else {
-        if (cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(a.n_row), stream) != cudaSuccess) {
-            launch_ok();
-            return;
-        }
-        if (a.n_col == 0) return;
-        jit_cols_event_kernel<T, E, KIND><<<blocks_for(a.n_col, COL_CHUNK), JIT_THREADS, 0, stream>>>(
-            events, a.seed, a.log_p, a.w1, a.w2, a.n_row, a.n_col, y);
-    }
-    launch_ok();
+    JitCall<T, E> c{stream, static_cast<const E *>(buffers[0]), static_cast<T *>(buffers[1]), {}, T(1)};
+    if (!unpack_jit<KIND>(opaque, opaque_len, c.a) || c.a.n_row == 0) return;
+    if (ROWS) jit_rows<T, E, KIND, true>(c);
+    else jit_cols_event<T, E, KIND>(c);
 }
 
 template<typename T, int KIND>
@@ -808,7 +898,7 @@ void jit_matmat_impl(cudaStream_t stream, void **buffers, const char *opaque, si
     }
     const dim3 grid(blocks_for(d->n, MM_THREADS), gy);
     jit_matmat_kernel<T, KIND><<<grid, MM_THREADS, smem, stream>>>(
-        X, d->seed, d->log_p, d->w1, d->w2, d->m, d->k, d->n, Y);
+        X, d->seed, gap_params(d->log_p, d->k), d->w1, d->w2, d->m, d->k, d->n, Y);
     launch_ok();
 }
 
@@ -890,6 +980,7 @@ void jit_matmat_list_impl(cudaStream_t stream, void **buffers, const char *opaqu
     unsigned int *cnt = reinterpret_cast<unsigned int *>(ws + p.cnt_off);
     MMEntry<T> *entries = reinterpret_cast<MMEntry<T> *>(ws + p.entries_off);
     T *Xt = reinterpret_cast<T *>(ws + p.xt_off);
+    const GapParams gp = gap_params(d->log_p, d->k);
     const unsigned int sms = static_cast<unsigned int>(sm_count());
     jit_matmat_transpose_kernel<T><<<dim3(blocks_for(d->k, 32), p.m_pad / 32), dim3(32, 8), 0, stream>>>(
         X, d->m, d->k, p.m_pad, Xt);
@@ -901,8 +992,8 @@ void jit_matmat_list_impl(cudaStream_t stream, void **buffers, const char *opaqu
             launch_ok();
             return;
         }
-        jit_matmat_fill_kernel<T, KIND><<<blocks_for(cols, 256), 256, 0, stream>>>(
-            d->seed, d->log_p, d->w1, d->w2, d->k, d->n, c0, p.cap, cnt, entries, n_over);
+        (gp.quick ? jit_matmat_fill_kernel<T, KIND, true> : jit_matmat_fill_kernel<T, KIND, false>)<<<
+            blocks_for(cols, 256), 256, 0, stream>>>(d->seed, gp, d->w1, d->w2, d->k, d->n, c0, p.cap, cnt, entries, n_over);
         const dim3 grid(blocks_for(cols, MM_THREADS), gy);
         // threads per block (= columns per block): the size whose last wave of blocks, one per SM, wastes least
         unsigned int threads = 128, best_cost = 0xffffffffu;
@@ -919,7 +1010,7 @@ void jit_matmat_list_impl(cudaStream_t stream, void **buffers, const char *opaqu
         jit_matmat_apply_kernel<T><<<grid_apply, threads, smem_apply, stream>>>(Xt, d->m, p.m_pad, d->k, d->n, c0, cols,
                                                                                p.cap, cnt, entries, Y);
         jit_matmat_kernel<T, KIND><<<grid, MM_THREADS, smem_inline, stream>>>(
-            X, d->seed, d->log_p, d->w1, d->w2, d->m, d->k, d->n, Y, c0, cnt, p.cap, n_over);
+            X, d->seed, gp, d->w1, d->w2, d->m, d->k, d->n, Y, c0, cnt, p.cap, n_over);
     }
     launch_ok();
 }
