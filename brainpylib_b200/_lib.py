@@ -51,9 +51,9 @@ def load_fast():
       from . import _native
     except ImportError as e:
       raise GPUOperatorNotFound(f'_native ({e})') from e
-    from . import event_ops, sparse_ops
+    from . import event_ops, jitconn_ops, sparse_ops
     _native.register(event_ops.ColumnBlockedCSR, event_ops.backward_rule, sparse_ops.backward_rule,
-                     sparse_ops.outer_backward_rule)
+                     sparse_ops.outer_backward_rule, jitconn_ops.backward_rule)
     fast = _native
   return fast
 

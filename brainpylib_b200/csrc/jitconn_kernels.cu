@@ -853,6 +853,20 @@ void jit_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, si
     else jit_cols<T, KIND>(c);
 }
 
+// The same without a descriptor, for the operator layer.
+template<typename T, int KIND>
+void jit_dense_call(cudaStream_t stream, const void *in, void *out, const JitArgs &a, bool rows, double scale) {
+    const JitCall<T, T> c{stream, static_cast<const T *>(in), static_cast<T *>(out), a, static_cast<T>(scale)};
+    if (rows) jit_rows<T, T, KIND, false>(c);
+    else jit_cols<T, KIND>(c);
+}
+template<typename T, typename E, int KIND>
+void jit_event_call(cudaStream_t stream, const void *in, void *out, const JitArgs &a, bool rows, double scale) {
+    const JitCall<T, E> c{stream, static_cast<const E *>(in), static_cast<T *>(out), a, static_cast<T>(scale)};
+    if (rows) jit_rows<T, E, KIND, true>(c);
+    else jit_cols_event<T, E, KIND>(c);
+}
+
 template<typename T, int KIND>
 void jit_matvec_v1_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len) {
     JitArgs a;
@@ -1029,6 +1043,25 @@ size_t matmat_list_workspace_bytes(const char *opaque, size_t opaque_len, size_t
 using namespace bpl;
 
 extern "C" {
+
+void bpl_jit_matvec(bpl_stream_t stream, const void *in, void *out, int in_type, int events, int kind, int rows,
+                    uint32_t n_row, uint32_t n_col, uint32_t seed, float log_p, float w1, float w2, double scale) {
+    using Call = void (*)(cudaStream_t, const void *, void *, const JitArgs &, bool, double);
+    static const Call dense[2][3] = {{jit_dense_call<float, W_HOMO>, jit_dense_call<float, W_UNIFORM>, jit_dense_call<float, W_NORMAL>},
+                                     {jit_dense_call<double, W_HOMO>, jit_dense_call<double, W_UNIFORM>, jit_dense_call<double, W_NORMAL>}};
+    static const Call event[3][3] = {
+        {jit_event_call<float, bool, W_HOMO>, jit_event_call<float, bool, W_UNIFORM>, jit_event_call<float, bool, W_NORMAL>},
+        {jit_event_call<float, float, W_HOMO>, jit_event_call<float, float, W_UNIFORM>, jit_event_call<float, float, W_NORMAL>},
+        {jit_event_call<double, double, W_HOMO>, jit_event_call<double, double, W_UNIFORM>, jit_event_call<double, double, W_NORMAL>}};
+    if (in_type < 0 || in_type > 2 || kind < 0 || kind > 2 || (!events && in_type == 0)) {
+        set_status(BPL_ERR_ARGUMENT, "bpl_jit_matvec: unknown type or kind");
+        return;
+    }
+    if (n_row == 0) return;
+    const JitArgs a{n_row, n_col, seed, log_p, kind == W_HOMO ? 0.0 : static_cast<double>(w1),
+                    kind == W_HOMO ? 0.0 : static_cast<double>(w2)};
+    (events ? event[in_type] : dense[in_type - 1])[kind](stream, in, out, a, rows != 0, scale);
+}
 
 #define JIT_MATVEC(name, T, KIND, ROWS) \
     void name(bpl_stream_t s, void **b, const char *o, size_t n) { jit_matvec_impl<T, KIND, ROWS>(s, b, o, n); }

@@ -480,63 +480,61 @@ struct JitArgs {
     double w1, w2, log_p;
     int64_t n_out, n_in, seed;
     bool rows;                  // one stream per output (outdim_parallel) or per input
+
+    // the transposed product walks the same streams from the other side
+    JitArgs transposed() const {
+        JitArgs t = *this;
+        std::swap(t.n_out, t.n_in);
+        t.rows = !rows;
+        return t;
+    }
 };
 
-// the descriptor's real fields are float32-rounded, as bpl_build_jitconn_prob_*_descriptor does it
-size_t jit_descriptor(const JitArgs &a, char (&opaque)[64]) {
-    const uint32_t n_row = static_cast<uint32_t>(a.n_out), n_col = static_cast<uint32_t>(a.n_in),
-                   seed = static_cast<uint32_t>(a.seed);
-    const float p = static_cast<float>(a.log_p), w1 = static_cast<float>(a.w1), w2 = static_cast<float>(a.w2);
-    if (a.kind == 0) return bpl_build_jitconn_prob_homo_descriptor(n_row, n_col, seed, p, opaque, sizeof(opaque));
-    if (a.kind == 1) return bpl_build_jitconn_prob_uniform_descriptor(n_row, n_col, seed, p, w1, w2, opaque, sizeof(opaque));
-    return bpl_build_jitconn_prob_normal_descriptor(n_row, n_col, seed, p, w1, w2, opaque, sizeof(opaque));
-}
-
-Tensor jit_product(const Tensor &vector, const JitArgs &a) {
-    static const Target targets[2][3][2] = {   // [rows][kind][double]
-        {{gpu_matvec_atomic_prob_homo_v2_float, gpu_matvec_atomic_prob_homo_v2_double},
-         {gpu_matvec_atomic_prob_uniform_v2_float, gpu_matvec_atomic_prob_uniform_v2_double},
-         {gpu_matvec_atomic_prob_normal_v2_float, gpu_matvec_atomic_prob_normal_v2_double}},
-        {{gpu_matvec_prob_homo_v2_float, gpu_matvec_prob_homo_v2_double},
-         {gpu_matvec_prob_uniform_v2_float, gpu_matvec_prob_uniform_v2_double},
-         {gpu_matvec_prob_normal_v2_float, gpu_matvec_prob_normal_v2_double}}};
-    OnDevice on(vector);
-    Tensor out = new_tensor({a.n_out}, vector.scalar_type(), vector.device());
-    char opaque[64];
-    const size_t len = jit_descriptor(a, opaque);
-    void *buffers[2] = {ptr(vector), ptr(out)};
-    targets[a.rows][a.kind][is_double(vector)](on.stream, buffers, opaque, len);
+// The descriptor's real fields are float32-rounded, here as in bpl_build_jitconn_prob_*_descriptor.
+Tensor jit_product(const Tensor &x, const JitArgs &a, const bool events) {
+    OnDevice on(x);
+    const bool b = x.scalar_type() == at::kBool;
+    Tensor out = new_tensor({a.n_out}, b ? at::kFloat : x.scalar_type(), x.device());
+    bpl_jit_matvec(on.stream, ptr(x), ptr(out), b ? 0 : is_double(x) ? 2 : 1, events, static_cast<int>(a.kind), a.rows,
+                   static_cast<uint32_t>(a.n_out), static_cast<uint32_t>(a.n_in), static_cast<uint32_t>(a.seed),
+                   static_cast<float>(a.log_p), static_cast<float>(a.w1), static_cast<float>(a.w2), a.weight);
     check_status();
+    // homogeneous event sums over columns are counts: scaled once, like the counts of rows
+    if (events && !a.rows && a.kind == 0) out.mul_(a.weight);
     return out;
 }
 
-Tensor jit_event_product(const Tensor &events, const JitArgs &a) {
-    static const Target targets[2][3][3] = {   // [rows][kind][bool, float, double events]
-        {{gpu_event_matvec_atomic_prob_homo_v2_float_bool, gpu_event_matvec_atomic_prob_homo_v2_float_float,
-          gpu_event_matvec_atomic_prob_homo_v2_double_double},
-         {gpu_event_matvec_atomic_prob_uniform_v2_float_bool, gpu_event_matvec_atomic_prob_uniform_v2_float_float,
-          gpu_event_matvec_atomic_prob_uniform_v2_double_double},
-         {gpu_event_matvec_atomic_prob_normal_v2_float_bool, gpu_event_matvec_atomic_prob_normal_v2_float_float,
-          gpu_event_matvec_atomic_prob_normal_v2_double_double}},
-        {{gpu_event_matvec_prob_homo_v2_float_bool, gpu_event_matvec_prob_homo_v2_float_float,
-          gpu_event_matvec_prob_homo_v2_double_double},
-         {gpu_event_matvec_prob_uniform_v2_float_bool, gpu_event_matvec_prob_uniform_v2_float_float,
-          gpu_event_matvec_prob_uniform_v2_double_double},
-         {gpu_event_matvec_prob_normal_v2_float_bool, gpu_event_matvec_prob_normal_v2_float_float,
-          gpu_event_matvec_prob_normal_v2_double_double}}};
-    OnDevice on(events);
-    const bool b = events.scalar_type() == at::kBool;
-    Tensor out = new_tensor({a.n_out}, b ? at::kFloat : events.scalar_type(), events.device());
-    char opaque[64];
-    const size_t len = jit_descriptor(a, opaque);
-    void *buffers[2] = {ptr(events), ptr(out)};
-    targets[a.rows][a.kind][b ? 0 : is_double(events) ? 2 : 1](on.stream, buffers, opaque, len);
-    check_status();
-    return out;
-}
+PyObject *g_jit_backward = nullptr;     // jitconn_ops.backward_rule
+
+struct JitFn : public torch::autograd::Function<JitFn> {
+    static Tensor forward(AutogradContext *ctx, const Tensor &x, const JitArgs &a, bool events) {
+        ctx->saved_data["i"] = std::vector<int64_t>{a.kind, a.n_out, a.n_in, a.seed, a.rows ? 1 : 0};
+        ctx->saved_data["f"] = std::vector<double>{a.weight, a.w1, a.w2, a.log_p};
+        return jit_product(x, a, events);
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        const auto i = ctx->saved_data["i"].toIntVector();
+        const auto f = ctx->saved_data["f"].toDoubleVector();
+        const JitArgs a{i[0], f[0], f[1], f[2], f[3], i[1], i[2], i[3], i[4] != 0};
+        const JitArgs t = a.transposed();
+        const Tensor ct = grads[0].contiguous();
+        Tensor g;
+        if (plain_cotangent(ct)) g = JitFn::apply(ct, t, false);
+        else g = python_jit_rule(ct, t);
+        return {g, Tensor(), Tensor()};
+    }
+    // backward_rule(ct, kind, weight, w1, w2, log_p, n_out, n_in, seed, rows)
+    static Tensor python_jit_rule(const Tensor &ct, const JitArgs &t) {
+        pybind11::gil_scoped_acquire gil;
+        const auto c = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(ct));
+        const auto r = pybind11::reinterpret_borrow<pybind11::object>(g_jit_backward)(
+            c, t.kind, t.weight, t.w1, t.w2, t.log_p, t.n_out, t.n_in, t.seed, t.rows);
+        return THPVariable_Unpack(r.ptr());
+    }
+};
 
 // jit_matvec(vector, events, kind, weight, w1, w2, log_p, shape, seed, transpose, outdim_parallel)
-//   events: whether `vector` is an event vector.  A vector that needs a gradient goes the Python way.
+//   events: whether `vector` is an event vector
 PyObject *py_jit_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     NONE_UNLESS(nargs == 11 && plain_thread());
@@ -544,12 +542,11 @@ PyObject *py_jit_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     const bool events = args[1] == Py_True;
     JitArgs a;
     int64_t s0, s1;
-    double kind, seed;
-    NONE_UNLESS(x && x->dim() == 1 && (float_like(*x) || (events && x->scalar_type() == at::kBool)) && !wants_grad(*x));
+    double kind;
+    NONE_UNLESS(x && x->dim() == 1 && (float_like(*x) || (events && x->scalar_type() == at::kBool)));
     NONE_UNLESS(number_of(args[2], kind) && number_of(args[3], a.weight) && number_of(args[4], a.w1) &&
                 number_of(args[5], a.w2) && number_of(args[6], a.log_p) && shape_of(args[7], s0, s1) &&
                 PyLong_CheckExact(args[8]));
-    (void) seed;
     const int t = PyObject_IsTrue(args[9]), rows = PyObject_IsTrue(args[10]);
     if (t < 0 || rows < 0) return nullptr;
     a.kind = static_cast<int64_t>(kind);
@@ -558,9 +555,7 @@ PyObject *py_jit_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     a.n_in = t ? s0 : s1;
     a.rows = rows != 0;
     NONE_UNLESS(x->size(0) == a.n_in);
-    Tensor out = events ? jit_event_product(*x, a) : jit_product(*x, a);
-    if (a.kind == 0) out.mul_(a.weight);
-    return THPVariable_Wrap(std::move(out));
+    return THPVariable_Wrap(wants_grad(*x) ? JitFn::apply(*x, a, events) : jit_product(*x, a, events));
     END_HANDLE_TH_ERRORS
 }
 
@@ -747,14 +742,14 @@ PyObject *py_csr_outer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
-// register(blocked_type, event_csr_backward, csr_backward, csr_outer_backward)
+// register(blocked_type, event_csr_backward, csr_backward, csr_outer_backward, jit_backward)
 PyObject *py_register(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 4) {
-        PyErr_SetString(PyExc_TypeError, "register takes 4 arguments");
+    if (nargs != 5) {
+        PyErr_SetString(PyExc_TypeError, "register takes 5 arguments");
         return nullptr;
     }
-    PyObject **slots[4] = {&g_blocked_type, &g_event_csr_backward, &g_csr_backward, &g_csr_outer};
-    for (int i = 0; i < 4; ++i) {
+    PyObject **slots[5] = {&g_blocked_type, &g_event_csr_backward, &g_csr_backward, &g_csr_outer, &g_jit_backward};
+    for (int i = 0; i < 5; ++i) {
         Py_INCREF(args[i]);
         Py_XSETREF(*slots[i], args[i]);
     }

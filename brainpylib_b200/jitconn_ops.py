@@ -49,8 +49,8 @@ def _fast_matvec(vector, events, kind, weight, w1, w2, conn_prob, shape, seed, t
                                                     transpose, outdim_parallel)
 
 
-def _descriptor(kind, n_row, n_col, seed, conn_prob, w1, w2):
-  p = _log_p(conn_prob)
+def _descriptor(kind, n_row, n_col, seed, conn_prob, w1, w2, log_p=None):
+  p = _log_p(conn_prob) if log_p is None else log_p
   if kind == 'homo':
     return gpu_ops.build_jitconn_prob_homo_descriptor(n_row, n_col, seed, p)
   if kind == 'uniform':
@@ -59,7 +59,7 @@ def _descriptor(kind, n_row, n_col, seed, conn_prob, w1, w2):
 
 
 def matvec_raw(vector, *, kind, w1=0., w2=0., conn_prob, shape, seed, transpose, outdim_parallel, version='v2',
-               out=None):
+               out=None, log_p=None):
   """Primitive ``matvec_prob_{homo,uniform,normal}``: dense input vector.
   ``w1, w2`` = ``(w_low, w_high - w_low)`` or ``(w_mu, w_sigma)``.  ``version='v1'`` passes the raw
   probability in the descriptor (matvec.py:338-343) and exists row-parallel only, as in the reference."""
@@ -74,7 +74,7 @@ def matvec_raw(vector, *, kind, w1=0., w2=0., conn_prob, shape, seed, transpose,
     else:
       opaque = gpu_ops.build_jitconn_prob_normal_descriptor(n_row, n_col, seed, conn_prob, w1, w2)
   else:
-    opaque = _descriptor(kind, n_row, n_col, seed, conn_prob, w1, w2)
+    opaque = _descriptor(kind, n_row, n_col, seed, conn_prob, w1, w2, log_p)
   name = ('gpu_matvec_prob_' if outdim_parallel else 'gpu_matvec_atomic_prob_') + kind + '_' + version + \
          float_suffix(vector.dtype)
   if out is None:
@@ -161,6 +161,13 @@ class _Matvec(torch.autograd.Function):
   @staticmethod
   def vmap(info, in_dims, vector, kw):
     return loop_vmap(_Matvec.apply, info, in_dims, (vector, kw))
+
+
+def backward_rule(ct, kind, weight, w1, w2, log_p, n_out, n_in, seed, rows):
+  """The transposed dense product for a cotangent that is not a plain tensor (called from the native nodes)."""
+  r = _Matvec.apply(contiguous(ct), dict(kind=('homo', 'uniform', 'normal')[kind], w1=w1, w2=w2, log_p=log_p, conn_prob=None,
+                                         shape=(n_out, n_in), seed=seed, transpose=False, outdim_parallel=rows))
+  return r * weight if kind == _HOMO else r
 
 
 class _EventMatvec(torch.autograd.Function):

@@ -1,0 +1,80 @@
+"""The ways a just-in-time product reads its input and gathers its sums (global memory, event bits, tiles of the vector,
+tiles of the output) against the CPU oracle, at sizes around the edges of tiles and of the rules that choose.  The
+oracle's logarithm may move single connections (it counts them); so many outputs may differ."""
+import numpy as np
+import pytest
+import torch
+
+import brainpylib_b200 as bpl
+from oracle import cpu
+
+pytestmark = pytest.mark.gpu
+
+KINDS = {'homo': (cpu.W_HOMO, 0., 0.), 'uniform': (cpu.W_UNIFORM, -0.1, 0.2), 'normal': (cpu.W_NORMAL, 0., 0.01)}
+
+
+def _call(x, kind, prob, shape, rows, event, seed=77):
+  kw = dict(conn_prob=prob, shape=shape, seed=seed, outdim_parallel=rows)
+  name = ('event_' if event else '') + f'matvec_prob_conn_{kind}_weight'
+  op = getattr(bpl, name)
+  if kind == 'homo':
+    return op(x, 1., **kw)
+  return op(x, w_low=-0.1, w_high=0.1, **kw) if kind == 'uniform' else op(x, w_mu=0., w_sigma=0.01, **kw)
+
+
+def _compare(cuda, x, kind, prob, shape, rows, event):
+  k, w1, w2 = KINDS[kind]
+  got = _call(torch.as_tensor(x).to(cuda), kind, prob, shape, rows, event).cpu().numpy()
+  oracle = cpu.jitconn_event_matvec if event else cpu.jitconn_matvec
+  want, info = oracle(x, kind=k, w1=w1, w2=w2, conn_prob=prob, shape=shape, seed=77, outdim_parallel=rows, return_info=True)
+  scale = float(np.abs(want).max())
+  bad = ~np.isclose(got, want, rtol=2e-5, atol=2e-5 * scale)
+  assert bad.sum() <= 2 * info['fragile'], (int(bad.sum()), info['fragile'])
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [np.float32, np.float64])
+# one tile, exactly two tiles, one element more than a tile of either type, few rows (read from global memory)
+@pytest.mark.parametrize('shape,prob', [((3000, 901), 0.3), ((4000, 58113), 0.01), ((2500, 29057), 0.02), ((70, 40000), 0.01)])
+def test_dense_rows(cuda, shape, prob, dtype, kind):
+  x = np.random.default_rng(1).standard_normal(shape[1]).astype(dtype)
+  _compare(cuda, x, kind, prob, shape, True, False)
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('shape,prob', [((901, 3000), 0.3), ((58113, 4000), 0.01), ((29057, 2500), 0.02)])
+def test_dense_columns(cuda, shape, prob, dtype, kind):
+  """Sums in tiles of the output against the same streams (seed + column) a few columns at a time, which are too few for
+  tiles.  (One connection that the oracle moves would shift all that follow in its stream.)"""
+  x = torch.randn(shape[1], dtype=dtype, generator=torch.Generator().manual_seed(2)).to(cuda)
+  got = _call(x, kind, prob, shape, False, False).double()
+  want = torch.zeros(shape[0], dtype=torch.float64, device=cuda)
+  for lo in range(0, shape[1], 50):
+    part = x[lo:lo + 50].contiguous()
+    want += _call(part, kind, prob, (shape[0], part.shape[0]), False, False, seed=77 + lo).double()
+  torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+def test_dense_columns_against_the_oracle(cuda, kind):
+  _compare(cuda, np.random.default_rng(2).standard_normal(400), kind, 0.4, (501, 400), False, False)
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [np.bool_, np.float32])
+# every input fires (full queues), ragged last word, more rows than threads, a mask of the largest size
+@pytest.mark.parametrize('shape,prob,rate', [((5000, 1000), 0.1, 1.0), ((2111, 4097), 0.2, 0.1), ((160000, 333), 0.1, 0.02),
+                                             ((12000, 1_638_400), 0.0004, 0.3), ((50, 3000), 0.1, 0.2)])
+def test_event_rows(cuda, shape, prob, rate, dtype, kind):
+  x = (np.random.default_rng(3).random(shape[1]) < rate).astype(dtype)
+  _compare(cuda, x, kind, prob, shape, True, True)
+
+
+@pytest.mark.parametrize('prob', [6e-6, 2e-5, 1.0])      # outside the quick test's range, sparse, every position
+def test_probabilities_at_the_ends_of_the_range(cuda, prob):
+  shape = (600, 200) if prob == 1.0 else (600, 300_000)
+  ev = np.random.default_rng(4).random(shape[1]) < 0.5
+  for kind in KINDS:
+    _compare(cuda, ev, kind, prob, shape, True, True)
+    _compare(cuda, ev.astype(np.float32), kind, prob, shape, True, False)
