@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "spike_scan.cuh"
 #include "row_scatter.cuh"
+#include "csr_shared.h"
 
 namespace bpl {
 namespace {
@@ -290,16 +291,8 @@ void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaq
 }
 
 template<typename T, bool HOMO>
-void csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len,
-                     bool transpose, int vector_slot) {
-    const DoubleSizeDescriptor *d = unpack<DoubleSizeDescriptor>(opaque, opaque_len);
-    if (!d) return;
-    const uint32_t n_row = d->size_x, n_col = d->size_y;
-    const T *data = static_cast<const T *>(buffers[0]);
-    const uint32_t *indices = static_cast<const uint32_t *>(buffers[1]);
-    const uint32_t *indptr = static_cast<const uint32_t *>(buffers[2]);
-    const T *x = static_cast<const T *>(buffers[vector_slot]);
-    T *y = static_cast<T *>(buffers[vector_slot + 1]);
+void csr_matvec_call(cudaStream_t stream, const T *data, const uint32_t *indices, const uint32_t *indptr, const T *x, T *y,
+                     const uint32_t n_row, const uint32_t n_col, const bool transpose) {
     const bool vec = aligned16(indices) && (HOMO || aligned16(data));
 
     if (transpose) {
@@ -331,13 +324,36 @@ void csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, si
     launch_ok();
 }
 
+template<typename T, bool HOMO>
+void csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len,
+                     bool transpose, int vector_slot) {
+    const DoubleSizeDescriptor *d = unpack<DoubleSizeDescriptor>(opaque, opaque_len);
+    if (!d) return;
+    csr_matvec_call<T, HOMO>(stream, static_cast<const T *>(buffers[0]), static_cast<const uint32_t *>(buffers[1]),
+                             static_cast<const uint32_t *>(buffers[2]), static_cast<const T *>(buffers[vector_slot]),
+                             static_cast<T *>(buffers[vector_slot + 1]), d->size_x, d->size_y, transpose);
+}
+
+// With the number of stored entries known: the kernels that hold the vector in shared memory where they are faster.
+template<typename T>
+void csr_matvec_known(cudaStream_t stream, const void *data, const uint32_t *indices, const uint32_t *indptr, const void *x,
+                      void *y, uint32_t n_row, uint32_t n_col, uint32_t nse, bool homo, bool transpose) {
+    const T *d = static_cast<const T *>(data), *v = static_cast<const T *>(x);
+    T *out = static_cast<T *>(y);
+    const CsrMatrix<T> m{indices, indptr, d, n_row, n_col, nse, homo};
+    if (transpose ? scatter_shared(stream, m, v, out) : gather_shared(stream, m, v, out)) return;
+    if (homo) csr_matvec_call<T, true>(stream, d, indices, indptr, v, out, n_row, n_col, transpose);
+    else csr_matvec_call<T, false>(stream, d, indices, indptr, v, out, n_row, n_col, transpose);
+}
+
 template<typename T>
 void csr_outer_impl(cudaStream_t stream, const void *row_vector, const void *col_vector, const uint32_t *indices,
-                    const uint32_t *indptr, void *out, uint32_t n_row, uint32_t nse) {
+                    const uint32_t *indptr, void *out, uint32_t n_row, uint32_t n_col, uint32_t nse) {
     if (n_row == 0 || nse == 0) return;
     const int grid = persistent_blocks(8, n_row);
     const T *r = static_cast<const T *>(row_vector), *c = static_cast<const T *>(col_vector);
     T *g = static_cast<T *>(out);
+    if (outer_shared(stream, CsrMatrix<T>{indices, indptr, nullptr, n_row, n_col, nse, false}, r, c, g)) return;
     if (aligned16(indices) && aligned16(out))
         csr_outer_kernel<T, true><<<grid, ROW_THREADS, 0, stream>>>(r, c, indices, indptr, g, n_row, nse);
     else
@@ -353,10 +369,17 @@ using namespace bpl;
 extern "C" {
 
 void bpl_csr_outer(bpl_stream_t stream, const void *row_vector, const void *col_vector, const void *indices,
-                   const void *indptr, void *out, uint32_t n_row, uint32_t nse, int is_double) {
+                   const void *indptr, void *out, uint32_t n_row, uint32_t n_col, uint32_t nse, int is_double) {
     const uint32_t *ix = static_cast<const uint32_t *>(indices), *ip = static_cast<const uint32_t *>(indptr);
-    if (is_double) csr_outer_impl<double>(stream, row_vector, col_vector, ix, ip, out, n_row, nse);
-    else csr_outer_impl<float>(stream, row_vector, col_vector, ix, ip, out, n_row, nse);
+    if (is_double) csr_outer_impl<double>(stream, row_vector, col_vector, ix, ip, out, n_row, n_col, nse);
+    else csr_outer_impl<float>(stream, row_vector, col_vector, ix, ip, out, n_row, n_col, nse);
+}
+
+void bpl_csr_matvec(bpl_stream_t stream, const void *data, const void *indices, const void *indptr, const void *vector,
+                    void *out, uint32_t n_row, uint32_t n_col, uint32_t nse, int homo, int is_double, int transpose) {
+    const uint32_t *ix = static_cast<const uint32_t *>(indices), *ip = static_cast<const uint32_t *>(indptr);
+    (is_double ? csr_matvec_known<double> : csr_matvec_known<float>)(stream, data, ix, ip, vector, out, n_row, n_col, nse,
+                                                                    homo != 0, transpose != 0);
 }
 
 size_t bpl_event_csr_workspace_bytes(uint32_t n_row, int transpose) {

@@ -1,0 +1,345 @@
+// CSR products on whole matrices with the dense vector (or the sums) in shared memory, for matrices whose number of
+// stored entries the caller knows and whose vector fits.
+//
+// What bounds the plain kernels (csr_kernels.cu): a gather of x through L1 takes one clock per entry and SM whatever it
+// hits (1e7 entries: 35 us, three times their memory time), a scattered reduction into L2 1.8 clocks (more on few
+// columns: 1.9e7 entries into 2185 sums took 853 us, here 46).  A lookup in shared memory takes a tenth of a clock, an
+// addition there 0.3.  So one block per SM holds the whole vector.
+//
+// Longer vectors stay with the plain kernels.  What shared memory takes from the 256 KB of an SM is missing for the
+// entries in flight, which pass through L1: 1e7 float entries, 80 MB, take 18.6 us with up to 132 KB of x, 19.9 with
+// 160 KB, 23 with 195 KB, 31 with 226 KB.  For that reason neither the first 160 KB of a longer vector here and the rest
+// by the plain ways (100,000 columns: gather 44 us against 39, scatter 78 against 65), nor slices of it in several blocks
+// that read the same rows side by side (58 us) paid; and reading a neighbour's slice out of its shared memory moves 0.33
+// random words per clock and SM.
+#include <algorithm>
+
+#include "abi.h"
+#include "common.cuh"
+#include "csr_shared.h"
+#include "row_scatter.cuh"
+
+namespace bpl {
+namespace {
+
+constexpr int SHARED_THREADS = 768;                  // one block per SM
+constexpr uint32_t SHARED_WARPS = SHARED_THREADS / 32;
+constexpr uint32_t SHARED_SMEM = 226u * 1024u;       // the longest vector
+
+// The rows of one block, in one walk that all three products share.
+//
+// A warp takes 32 / lpr rows at a time, lpr lanes each: a lane takes 4 consecutive entries per 128-bit load and U such
+// loads per step, so that an average row takes one step.  Row groups are dealt out to the blocks in turn: neither a run of
+// empty rows nor a run of long ones falls to one SM.  Two things held the first form at half the memory rate: a branch per
+// entry (30 instructions each; the entries of a quad go through predicates now, and whether any lane's quad crosses the
+// ends of its row is asked once per quad and warp), and a warp that waited for a step's entries before it asked for the
+// next.  The entries of the next step, of this row or the next, are therefore requested before a step is worked on.
+struct Deal {
+    uint32_t lpr, rows_per_warp;
+    __device__ __forceinline__ Deal(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
+        const uint32_t want = (nse / n_row + per_step - 1u) / per_step;
+        lpr = want <= 4u ? 4u : want <= 8u ? 8u : want <= 16u ? 16u : 32u;
+        rows_per_warp = 32u / lpr;
+    }
+    __device__ __forceinline__ uint32_t row(const uint32_t local_group, const uint32_t sub) const {
+        return (local_group * gridDim.x + blockIdx.x) * rows_per_warp + sub;
+    }
+};
+
+// `visit` has
+//   fetch(row)                            what is needed of a row besides its entries (requested one row ahead)
+//   quad<FULL>(base, c[4], w[4], lo, hi)  entries base .. base + 3, of which lo <= e < hi belong to the row (FULL: all)
+//   entry(pos, c, w)                      one entry (the ragged end of the arrays)
+//   begin(fetched), end(row, lead)        around a row; lead: this lane speaks for it
+// `ready` runs before the first entry is visited, behind the first loads: it fills shared memory and ends with a barrier.
+template<typename T, bool WEIGHTS, int U, typename Visit, typename Ready>
+__device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
+                                          const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
+                                          const Deal deal, Visit &visit, Ready ready) {
+    const uint32_t lane = threadIdx.x & 31, lpr = deal.lpr;
+    const uint32_t sub = lane / lpr, sl = lane % lpr;
+    const uint32_t g_full = nse >> 2;
+    using Fetched = decltype(visit.fetch(0u));
+    struct Step {
+        uint4 ix[U];
+        Quad<T> w[WEIGHTS ? U : 1];
+        uint32_t g0;                                       // the lane's first quad
+    };
+    struct Row {
+        uint32_t start, end;
+        Fetched fetched;
+    };
+    auto pointers = [&](const uint32_t group) {
+        const uint32_t row = deal.row(group, sub);
+        Row r{0u, 0u, visit.fetch(row)};
+        if (row < n_row) { r.start = indptr[row]; r.end = indptr[row + 1]; }
+        return r;
+    };
+    auto load = [&](Step &s, const Row &r) {
+        const uint32_t g_stop = min((r.end + 3u) >> 2, g_full);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t g = s.g0 + u * lpr;
+            if (g < g_stop) {
+                s.ix[u] = ldg_stream_u4(indices + 4ull * g);
+                if (WEIGHTS) load_quad(data + 4ull * g, s.w[u]);
+            }
+        }
+    };
+    uint32_t group = threadIdx.x >> 5;
+    Row row = pointers(group), next = pointers(group + SHARED_WARPS);
+    // one step: request what comes after it (`after`), then work on it
+    auto step = [&](Step &now, Step &after) {
+        const uint32_t g_stop = min((row.end + 3u) >> 2, g_full);
+        const bool more = __any_sync(FULL_MASK, now.g0 + U * lpr < g_stop);
+        after.g0 = more ? now.g0 + U * lpr : (next.start >> 2) + sl;
+        load(after, more ? row : next);
+        Row later{0u, 0u, Fetched()};
+        if (!more) later = pointers(group + 2 * SHARED_WARPS);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t base = 4u * (now.g0 + u * lpr);
+            const bool here = now.g0 + u * lpr < g_stop;
+            if (!__any_sync(FULL_MASK, here)) continue;
+            const uint32_t c[4] = {now.ix[u].x, now.ix[u].y, now.ix[u].z, now.ix[u].w};
+            const T *v = now.w[WEIGHTS ? u : 0].v;
+            const int lo = static_cast<int>(row.start) - static_cast<int>(base), hi = static_cast<int>(row.end) - static_cast<int>(base);
+            if (__all_sync(FULL_MASK, here && lo <= 0 && hi >= 4)) visit.template quad<true>(base, c, v, lo, hi);
+            else visit.template quad<false>(base, c, v, lo, here ? hi : 0);
+        }
+        if (more) return;
+        if (sl == 0)
+            for (uint32_t pos = max(4u * g_full, row.start); pos < row.end; ++pos)
+                visit.entry(pos, indices[pos], WEIGHTS ? data[pos] : T(0));
+        visit.end(deal.row(group, sub), sl == 0 && deal.row(group, sub) < n_row);
+        group += SHARED_WARPS;
+        row = next;
+        next = later;
+        visit.begin(row.fetched);
+    };
+    Step a, b;
+#pragma unroll
+    for (int u = 0; u < U; ++u) a.ix[u] = b.ix[u] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < (WEIGHTS ? U : 1); ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a.w[u].v[e] = b.w[u].v[e] = T(0);
+    a.g0 = (row.start >> 2) + sl;
+    load(a, row);
+    ready();
+    visit.begin(row.fetched);
+    while (deal.row(group, 0) < n_row) {
+        step(a, b);
+        if (deal.row(group, 0) >= n_row) break;
+        step(b, a);
+    }
+}
+
+// The first `count` elements of x into shared memory, by the whole block.
+template<typename T>
+__device__ __forceinline__ void fill_shared(T *shared, const T *__restrict__ p, const uint32_t count) {
+    constexpr uint32_t PER = 16 / sizeof(T);
+    const uint32_t n_vec = aligned16_device(p) ? count / PER : 0u;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < n_vec; i += SHARED_THREADS)
+        reinterpret_cast<uint4 *>(shared)[i] = __ldg(reinterpret_cast<const uint4 *>(p) + i);
+    for (uint32_t i = n_vec * PER + threadIdx.x; i < count; i += SHARED_THREADS) shared[i] = __ldg(p + i);
+}
+
+// y = A x
+template<typename T, bool HOMO>
+struct GatherVisit {
+    const T *xs;
+    uint32_t lpr;
+    T homo_w, *y;
+    T acc;
+    __device__ __forceinline__ int fetch(uint32_t) const { return 0; }
+    __device__ __forceinline__ void begin(int) { acc = T(0); }
+    template<bool FULL>
+    __device__ __forceinline__ void quad(uint32_t, const uint32_t (&c)[4], const T *w, const int lo, const int hi) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (FULL || (e >= lo && e < hi)) acc += (HOMO ? homo_w : w[e]) * xs[c[e]];
+    }
+    __device__ __forceinline__ void entry(uint32_t, const uint32_t c, const T w) { acc += (HOMO ? homo_w : w) * xs[c]; }
+    __device__ __forceinline__ void end(const uint32_t row, const bool lead) {
+        acc = group_sum(acc, static_cast<int>(lpr));
+        if (lead) y[row] = acc;
+    }
+};
+
+template<typename T, bool HOMO, int U>
+__global__ void __launch_bounds__(SHARED_THREADS, 1)
+gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
+                     const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col) {
+    extern __shared__ __align__(16) unsigned char shared_vector[];
+    T *xs = reinterpret_cast<T *>(shared_vector);
+    const Deal deal(nse, n_row, 4 * U);
+    GatherVisit<T, HOMO> visit{xs, deal.lpr, HOMO ? data[0] : T(0), y, T(0)};
+    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
+        fill_shared(xs, x, n_col);
+        __syncthreads();
+    });
+}
+
+// y += A^T x: sums in shared memory, added to the zero-filled y at the end
+template<typename T, bool HOMO>
+struct ScatterVisit {
+    T *sums;
+    uint32_t n_row;
+    const T *x;
+    T homo_w, scale;
+    __device__ __forceinline__ T fetch(const uint32_t row) const { return row < n_row ? x[row] : T(0); }
+    __device__ __forceinline__ void begin(const T s) { scale = s; }
+    template<bool FULL>
+    __device__ __forceinline__ void quad(uint32_t, const uint32_t (&c)[4], const T *w, const int lo, const int hi) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (FULL || (e >= lo && e < hi)) atomicAdd(sums + c[e], (HOMO ? homo_w : w[e]) * scale);
+    }
+    __device__ __forceinline__ void entry(uint32_t, const uint32_t c, const T w) { atomicAdd(sums + c, (HOMO ? homo_w : w) * scale); }
+    __device__ __forceinline__ void end(uint32_t, bool) {}
+};
+
+template<typename T, bool HOMO, int U>
+__global__ void __launch_bounds__(SHARED_THREADS, 1)
+scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
+                      const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse,
+                      const uint32_t n_col) {
+    extern __shared__ __align__(16) unsigned char shared_vector[];
+    T *sums = reinterpret_cast<T *>(shared_vector);
+    const Deal deal(nse, n_row, 4 * U);
+    ScatterVisit<T, HOMO> visit{sums, n_row, x, HOMO ? data[0] : T(0), T(0)};
+    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
+        for (uint32_t i = threadIdx.x; i < n_col; i += SHARED_THREADS) sums[i] = T(0);
+        __syncthreads();
+    });
+    __syncthreads();
+    add_sums(sums, y, n_col, blockIdx.x, gridDim.x);
+}
+
+// g[e] = row_vector[row] * col_vector[column]
+template<typename T>
+struct OuterVisit {
+    const T *xs, *row_vector;
+    T *g;
+    uint32_t n_row;
+    T r;
+    __device__ __forceinline__ T fetch(const uint32_t row) const { return row < n_row ? row_vector[row] : T(0); }
+    __device__ __forceinline__ void begin(const T v) { r = v; }
+    template<bool FULL>
+    __device__ __forceinline__ void quad(const uint32_t base, const uint32_t (&c)[4], const T *, const int lo, const int hi) {
+        if (FULL) {
+            store_quad(g + base, r * xs[c[0]], r * xs[c[1]], r * xs[c[2]], r * xs[c[3]]);
+        } else if (lo <= 0 && hi >= 4) {
+            store_quad(g + base, r * xs[c[0]], r * xs[c[1]], r * xs[c[2]], r * xs[c[3]]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (e >= lo && e < hi) g[base + e] = r * xs[c[e]];
+        }
+    }
+    __device__ __forceinline__ void entry(const uint32_t pos, const uint32_t c, T) { g[pos] = r * xs[c]; }
+    __device__ __forceinline__ void end(uint32_t, bool) {}
+};
+
+template<typename T, int U>
+__global__ void __launch_bounds__(SHARED_THREADS, 1)
+outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
+                    const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g,
+                    const uint32_t n_row, const uint32_t nse, const uint32_t n_col) {
+    extern __shared__ __align__(16) unsigned char shared_vector[];
+    T *xs = reinterpret_cast<T *>(shared_vector);
+    const Deal deal(nse, n_row, 4 * U);
+    OuterVisit<T> visit{xs, row_vector, g, n_row, T(0)};
+    walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, deal, visit, [&]() {
+        fill_shared(xs, col_vector, n_col);
+        __syncthreads();
+    });
+}
+
+// ---- host side: the rules, in clocks of one SM (1.9 GHz) ----
+template<typename T>
+struct Plan {
+    double per;                 // stored entries per SM
+    double entry;               // clocks to stream an entry, by what is left for entries in flight (see above)
+    double fill;                // clocks to start and to fill or clear the vector, 56 bytes per clock
+
+    Plan(const CsrMatrix<T> &m, const bool values) {
+        const double kb = static_cast<double>(m.n_col) * sizeof(T) / 1024.0;
+        per = static_cast<double>(m.nse) / sm_count();
+        entry = (4.0 + (values ? sizeof(T) : 0)) / (kb <= 131 ? 15.0 : kb <= 163 ? 14.0 : kb <= 195 ? 11.7 : 9.0);
+        fill = 3000 + kb * 1024 / 56;
+    }
+};
+
+template<typename T>
+bool usable(const CsrMatrix<T> &m, const bool weights) {
+    return m.n_row != 0 && m.n_col != 0 && m.nse != 0 && m.n_col <= SHARED_SMEM / sizeof(T) && aligned16(m.indices) &&
+           (!weights || aligned16(m.data));
+}
+
+template<typename T, bool HOMO>
+bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
+    constexpr auto kernel = gather_shared_kernel<T, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    if (!usable(m, !HOMO)) return false;
+    const Plan<T> p(m, !HOMO);
+    if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
+    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, m.data, x, y,
+                                                                                             m.n_row, m.nse, m.n_col);
+    launch_ok();
+    return true;
+}
+
+template<typename T, bool HOMO>
+bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
+    constexpr auto kernel = scatter_shared_kernel<T, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    if (!usable(m, !HOMO)) return false;
+    const Plan<T> p(m, !HOMO);
+    // a reduction into L2: slower the fewer columns share them (20,000 columns 3.1 clocks, 2000 columns 13), and in double
+    const double words = sizeof(T) / 4, reduction = (1.85 + 25000.0 / m.n_col) * (sizeof(T) == 8 ? 1.25 : 1.0);
+    if (p.fill + 0.3 * words * m.n_col + p.per * (p.entry + 0.3 * words) > 0.95 * (reduction * p.per + 1500)) return false;
+    if (cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(m.n_col), stream) != cudaSuccess) return launch_ok(), true;
+    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, m.data, x, y,
+                                                                                             m.n_row, m.nse, m.n_col);
+    launch_ok();
+    return true;
+}
+
+template<typename T>
+bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g) {
+    constexpr auto kernel = outer_shared_kernel<T, 2>;
+    if (!usable(m, false) || !aligned16(g)) return false;
+    const Plan<T> p(m, true);                // one index in, one value out
+    if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
+    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, row_vector,
+                                                                                             col_vector, g, m.n_row, m.nse, m.n_col);
+    launch_ok();
+    return true;
+}
+
+}  // namespace
+
+bool gather_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *x, float *y) {
+    return m.homo ? gather_impl<float, true>(stream, m, x, y) : gather_impl<float, false>(stream, m, x, y);
+}
+bool gather_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *x, double *y) {
+    return m.homo ? gather_impl<double, true>(stream, m, x, y) : gather_impl<double, false>(stream, m, x, y);
+}
+bool scatter_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *x, float *y) {
+    return m.homo ? scatter_impl<float, true>(stream, m, x, y) : scatter_impl<float, false>(stream, m, x, y);
+}
+bool scatter_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *x, double *y) {
+    return m.homo ? scatter_impl<double, true>(stream, m, x, y) : scatter_impl<double, false>(stream, m, x, y);
+}
+bool outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *r, const float *c, float *g) {
+    return outer_impl<float>(stream, m, r, c, g);
+}
+bool outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *r, const double *c, double *g) {
+    return outer_impl<double>(stream, m, r, c, g);
+}
+
+}  // namespace bpl

@@ -232,19 +232,6 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
 // reductions per second (0.55 per clock and SM); an addition in shared memory runs six times faster.  TILES: a tile of the
 // output lives in shared memory while all columns of the block cross it (positions ascend along a stream), and is then
 // added to the zero-filled output with 16-byte reductions.
-template<typename T>
-__device__ __forceinline__ void flush_tile(const T *tile, T *__restrict__ out, const unsigned int count) {
-    const bool vec = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-    const unsigned int n4 = vec ? count / 4 : 0u;
-    for (unsigned int i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 v = reinterpret_cast<const float4 *>(tile)[i];
-        if (v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f)
-            red_add_v4(reinterpret_cast<float *>(out) + 4u * i, v.x, v.y, v.z, v.w);
-    }
-    for (unsigned int i = 4u * n4 + threadIdx.x; i < count; i += blockDim.x)
-        if (tile[i] != T(0)) red_add(out + i, tile[i]);
-}
-
 template<typename T, int KIND, bool TILES, bool QUICK>
 __global__ void __launch_bounds__(TILES ? WALK_THREADS : GATHER_THREADS)
 jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const GapParams gp, const double w1, const double w2,
@@ -288,7 +275,7 @@ jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const Gap
             }
             if (TILES) {
                 __syncthreads();
-                flush_tile(tile, out + t0, len);
+                add_sums(tile, out + t0, len, blockIdx.x, gridDim.x);
                 __syncthreads();
             }
         }
@@ -712,22 +699,6 @@ struct JitCall {
     T scale;       // homogeneous weights: factor of the sums (rows) or of the input (columns)
 };
 
-// Lets a kernel take WALK_SMEM bytes of dynamic shared memory on the current device.
-template<auto KERNEL>
-bool allow_walk_smem() {
-    static thread_local int configured_device = -1;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (configured_device != dev) {
-        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(WALK_SMEM)) != cudaSuccess) {
-            launch_ok();
-            return false;
-        }
-        configured_device = dev;
-    }
-    return true;
-}
-
 // One block per SM (fewer when there is not a warp of streams for each) and the threads that split its streams into
 // equal waves.
 struct WalkGrid {
@@ -747,7 +718,7 @@ inline unsigned int tile_length(unsigned int n, size_t elem) {
 }
 
 // Rules in clocks of one SM.  A gather through L1 takes one clock per connection.  Filling shared memory reads the whole
-// input per block, at about 32 bytes per clock, after a start of some 2000 clocks; a vector in several tiles is read
+// input per block, at about 56 bytes per clock, after a start of some 2000 clocks; a vector in several tiles is read
 // again for every wave of streams.
 template<typename T, typename E, int KIND, bool EVENT>
 void jit_rows(const JitCall<T, E> &c) {
@@ -758,9 +729,12 @@ void jit_rows(const JitCall<T, E> &c) {
     WalkGrid g(a.n_row, 512);
     // (n_col + 5 * 23 mean gaps stay below 2^24)
     if (gp.quick && TRUTH_ONLY && a.n_col <= MASK_MAX_BITS && -1.0 / a.log_p < 130000.0) {
-        if (gathers > static_cast<double>(a.n_col) * sizeof(E) / 32 + 2000) {
+        if (gathers > static_cast<double>(a.n_col) * sizeof(E) / 56 + 2000) {
             constexpr auto kernel = jit_rows_kernel<T, E, KIND, EVENT, TRUTH_ONLY ? FROM_MASK : FROM_GLOBAL, true>;
-            if (!allow_walk_smem<kernel>()) return;
+            if (!allow_shared<kernel>(WALK_SMEM)) {
+                launch_ok();
+                return;
+            }
             // what the mask leaves holds the queues of hits, up to 16 slots per thread (`seconds` has 32 bits); beside a
             // mask of the largest size only those of 512 threads fit
             const unsigned int mask_bytes = blocks_for(a.n_col, 32) * 4u, slot_bytes = KIND == W_HOMO ? 0u : KIND == W_UNIFORM ? 4u : 8u;
@@ -780,10 +754,13 @@ void jit_rows(const JitCall<T, E> &c) {
         }
     } else if (gp.quick && !TRUTH_ONLY && (KIND == W_HOMO || !EVENT)) {
         const unsigned int len = tile_length(a.n_col, sizeof(E));
-        const double loads = static_cast<double>(a.n_col) * sizeof(E) / 32 * (len >= a.n_col ? 1 : g.waves);
+        const double loads = static_cast<double>(a.n_col) * sizeof(E) / 56 * (len >= a.n_col ? 1 : g.waves);
         if (0.75 * gathers > loads + 2000) {
             constexpr auto kernel = jit_rows_kernel<T, E, KIND, EVENT, TRUTH_ONLY ? FROM_GLOBAL : FROM_TILES, true>;
-            if (!allow_walk_smem<kernel>()) return;
+            if (!allow_shared<kernel>(WALK_SMEM)) {
+                launch_ok();
+                return;
+            }
             kernel<<<g.blocks, g.threads, static_cast<size_t>(len) * sizeof(E), c.stream>>>(
                 c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, len, 0, c.scale, c.out);
             launch_ok();
@@ -802,7 +779,7 @@ void jit_rows(const JitCall<T, E> &c) {
     launch_ok();
 }
 
-// In clocks of one SM: a scattered reduction into L2 takes 1.8, an addition in shared memory 0.3; a tile costs about 0.7
+// In clocks of one SM: a scattered reduction into L2 takes 1.8, an addition in shared memory 0.3; a tile costs about 0.4
 // per element to clear and to flush, once per wave of columns.
 template<typename T, int KIND>
 void jit_cols(const JitCall<T, T> &c) {
@@ -815,10 +792,13 @@ void jit_cols(const JitCall<T, T> &c) {
     const GapParams gp = gap_params(a.log_p, a.n_row);
     const double additions = static_cast<double>(a.n_row) * a.n_col * -std::expm1(a.log_p) / sm_count();
     const WalkGrid g(a.n_col, 512);
-    if (gp.quick && 1.8 * additions > 0.3 * additions + 0.7 * (sizeof(T) / 4) * a.n_row * g.waves + 5000) {
+    if (gp.quick && 1.8 * additions > 0.3 * (sizeof(T) / 4) * additions + 0.4 * (sizeof(T) / 4) * a.n_row * g.waves + 5000) {
         const unsigned int len = tile_length(a.n_row, sizeof(T));
         constexpr auto kernel = jit_cols_kernel<T, KIND, true, true>;
-        if (!allow_walk_smem<kernel>()) return;
+        if (!allow_shared<kernel>(WALK_SMEM)) {
+                launch_ok();
+                return;
+            }
         kernel<<<g.blocks, g.threads, static_cast<size_t>(len) * sizeof(T), c.stream>>>(
             c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, len, c.scale, c.out);
         launch_ok();

@@ -145,16 +145,11 @@ void *ptr(const Tensor &t) { return const_cast<void *>(t.const_data_ptr()); }
 // ---------------------------------------------------------------------------------------------------------
 Tensor csr_product(const Tensor &data, const Tensor &indices, const Tensor &indptr, const Tensor &vector, int64_t n_row,
                    int64_t n_col, bool transpose) {
-    static const Target targets[2][2][2] = {   // [transpose][double][homo]
-        {{csr_matvec_heter_vector_float, csr_matvec_homo_vector_float},
-         {csr_matvec_heter_vector_double, csr_matvec_homo_vector_double}},
-        {{csr_matvec_transpose_heter_float, csr_matvec_transpose_homo_float},
-         {csr_matvec_transpose_heter_double, csr_matvec_transpose_homo_double}}};
     OnDevice on(data);
     Tensor out = new_tensor({transpose ? n_col : n_row}, data.scalar_type(), data.device());
-    const bpl::DoubleSizeDescriptor d{static_cast<unsigned>(n_row), static_cast<unsigned>(n_col)};
-    void *buffers[5] = {ptr(data), ptr(indices), ptr(indptr), ptr(vector), ptr(out)};
-    targets[transpose][is_double(data)][data.size(0) == 1](on.stream, buffers, reinterpret_cast<const char *>(&d), sizeof(d));
+    bpl_csr_matvec(on.stream, ptr(data), ptr(indices), ptr(indptr), ptr(vector), ptr(out), static_cast<uint32_t>(n_row),
+                   static_cast<uint32_t>(n_col), static_cast<uint32_t>(indices.size(0)), data.size(0) == 1, is_double(data),
+                   transpose);
     check_status();
     return out;
 }
@@ -233,8 +228,8 @@ struct CsrOuterFn : public torch::autograd::Function<CsrOuterFn> {
         OnDevice on(indices);
         Tensor out = new_tensor({indices.size(0)}, row_vector.scalar_type(), row_vector.device());
         bpl_csr_outer(on.stream, ptr(row_vector), ptr(col_vector), ptr(indices), ptr(indptr), ptr(out),
-                      static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(indices.size(0)),
-                      is_double(row_vector) ? 1 : 0);
+                      static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(col_vector.size(0)),
+                      static_cast<uint32_t>(indices.size(0)), is_double(row_vector) ? 1 : 0);
         check_status();
         return out;
     }
@@ -736,7 +731,8 @@ PyObject *py_csr_outer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     OnDevice on(indices);
     Tensor out = new_tensor({indices.size(0)}, row.scalar_type(), row.device());
     bpl_csr_outer(on.stream, ptr(row), ptr(col), ptr(indices), ptr(indptr), ptr(out),
-                  static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(indices.size(0)), is_double(row) ? 1 : 0);
+                  static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(col.size(0)), static_cast<uint32_t>(indices.size(0)),
+                  is_double(row) ? 1 : 0);
     check_status();
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS

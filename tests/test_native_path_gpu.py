@@ -7,6 +7,7 @@ import torch
 import cases
 import brainpylib_b200 as bpl
 from brainpylib_b200 import sparse_ops
+from oracle import cpu
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +54,26 @@ def test_second_order_gradients(cuda, transpose):
   x = torch.as_tensor(rng.standard_normal(30 if transpose else 40)).to(cuda).requires_grad_(True)
   op = lambda w, x: bpl.csr_matvec(w, indices, indptr, x, shape=(30, 40), transpose=transpose)
   assert torch.autograd.gradcheck(op, (w, x)) and torch.autograd.gradgradcheck(op, (w, x))
+
+
+@pytest.mark.parametrize('dtype', [np.float32, np.float64])
+@pytest.mark.parametrize('homo', [False, True])
+# the whole vector in shared memory: few columns, rows of every lane count, the longest vector that fits (4 and 8 bytes),
+# one element more (plain kernels); the entry count is no multiple of 4
+@pytest.mark.parametrize('n_row,n_col,mean', [(9000, 2000, 333), (300_000, 517, 7), (1201, 57_856, 2500), (1201, 28_928, 2500),
+                                              (1201, 57_857, 2500)])
+def test_products_with_the_vector_in_shared_memory(cuda, n_row, n_col, mean, homo, dtype):
+  rng = np.random.default_rng(17)
+  lens = rng.poisson(mean, n_row)
+  lens[[0, 5, n_row - 1]] = 0, 3 * mean, 1
+  lens[n_row // 2:n_row // 2 + 40] = 0
+  lens[1] += (1 - int(lens.sum())) % 4          # 4 k + 1 entries
+  data, indices, indptr, rng = cases.ragged_csr(lens, n_col, 19, dtype=dtype)
+  data = data[:1] if homo else data
+  d = [torch.as_tensor(a).to(cuda) for a in (data, indices, indptr)]
+  for transpose in (False, True):
+    x = rng.standard_normal(n_row if transpose else n_col).astype(dtype)
+    got = bpl.csr_matvec(*d, torch.as_tensor(x).to(cuda), shape=(n_row, n_col), transpose=transpose).cpu().numpy()
+    want = cpu.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
+    tol = 1e-5 if dtype == np.float32 else 1e-12
+    np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(max(mean, indices.size / n_col)))
