@@ -78,3 +78,15 @@ def test_probabilities_at_the_ends_of_the_range(cuda, prob):
   for kind in KINDS:
     _compare(cuda, ev, kind, prob, shape, True, True)
     _compare(cuda, ev.astype(np.float32), kind, prob, shape, True, False)
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+# X staged in shared memory (many columns: one tile, a ragged last tile, the ring going round), X read from L2 with 32, 64
+# and 128 rows per warp
+@pytest.mark.parametrize('m,k,n,prob', [(33, 383, 30_000, 0.05), (70, 2500, 25_001, 0.02), (7, 1537, 40_000, 0.1),
+                                        (31, 5000, 300, 0.01), (50, 5000, 300, 0.01), (150, 5000, 300, 0.01)])
+def test_matmat_from_lists_equals_the_inline_kernel(cuda, m, k, n, prob, dtype):
+  from brainpylib_b200 import jitconn_ops
+  X = torch.randn(m, k, dtype=dtype, generator=torch.Generator().manual_seed(5)).to(cuda)
+  kw = dict(kind='normal', w1=0., w2=0.01, conn_prob=prob, shape=(k, n), seed=11)
+  assert torch.equal(jitconn_ops.matmat_raw(X, **kw), jitconn_ops.matmat_raw(X, workspace=False, **kw))
