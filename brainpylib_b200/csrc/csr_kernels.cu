@@ -208,6 +208,18 @@ inline int persistent_blocks(int blocks_per_sm, uint64_t work_warps) {
     return static_cast<int>(need < 1 ? 1 : (need < cap ? need : cap));
 }
 
+// y = A events, the events gathered through L1
+template<typename T, typename E, bool HOMO>
+void event_gather(cudaStream_t stream, const uint32_t *indices, const uint32_t *indptr, const T *data, const E *events, T *y,
+                  const uint32_t n_row) {
+    const int grid = persistent_blocks(8, n_row);
+    if (aligned16(indices) && (HOMO || aligned16(data)))
+        row_gather_kernel<T, E, HOMO, true, true><<<grid, ROW_THREADS, 0, stream>>>(indices, indptr, data, events, n_row, y);
+    else
+        row_gather_kernel<T, E, HOMO, true, false><<<grid, ROW_THREADS, 0, stream>>>(indices, indptr, data, events, n_row, y);
+    launch_ok();
+}
+
 template<typename T, typename E, bool HOMO>
 void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len) {
     const TwoUintOneBoolDescriptor *d = unpack<TwoUintOneBoolDescriptor>(opaque, opaque_len);
@@ -279,14 +291,7 @@ void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaq
             launch_ok();
             return;
         }
-        const int grid = persistent_blocks(8, n_row);
-        if (vec)
-            row_gather_kernel<T, E, HOMO, true, true><<<grid, ROW_THREADS, 0, stream>>>(
-                indices, indptr, data, events, n_row, y);
-        else
-            row_gather_kernel<T, E, HOMO, true, false><<<grid, ROW_THREADS, 0, stream>>>(
-                indices, indptr, data, events, n_row, y);
-        launch_ok();
+        event_gather<T, E, HOMO>(stream, indices, indptr, data, events, y, n_row);
     }
 }
 
@@ -332,6 +337,25 @@ void csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, si
     csr_matvec_call<T, HOMO>(stream, static_cast<const T *>(buffers[0]), static_cast<const uint32_t *>(buffers[1]),
                              static_cast<const uint32_t *>(buffers[2]), static_cast<const T *>(buffers[vector_slot]),
                              static_cast<T *>(buffers[vector_slot + 1]), d->size_x, d->size_y, transpose);
+}
+
+template<typename T, typename E, bool HOMO>
+void event_csr_known(cudaStream_t stream, void **buffers, uint32_t n_row, uint32_t n_col, uint32_t nse, bool transpose) {
+    const CsrMatrix<T> m{static_cast<const uint32_t *>(buffers[1]), static_cast<const uint32_t *>(buffers[2]),
+                         static_cast<const T *>(buffers[0]), n_row, n_col, nse, HOMO};
+    if (!transpose) {
+        const E *events = static_cast<const E *>(buffers[3]);
+        T *y = static_cast<T *>(buffers[4]);
+        if (n_row != 0 && !gather_events(stream, m, events, static_cast<uint32_t *>(buffers[5]), y))
+            event_gather<T, E, HOMO>(stream, m.indices, m.indptr, m.data, events, y, n_row);
+        return;
+    }
+    TwoUintOneBoolDescriptor d;
+    __builtin_memset(&d, 0, sizeof(d));
+    d.uint_x = n_row;
+    d.uint_y = n_col;
+    d.bool_x = transpose;
+    event_csr_matvec_impl<T, E, HOMO>(stream, buffers, reinterpret_cast<const char *>(&d), sizeof(d));
 }
 
 // With the number of stored entries known: the kernels that hold the vector in shared memory where they are faster.
@@ -380,6 +404,17 @@ void bpl_csr_matvec(bpl_stream_t stream, const void *data, const void *indices, 
     const uint32_t *ix = static_cast<const uint32_t *>(indices), *ip = static_cast<const uint32_t *>(indptr);
     (is_double ? csr_matvec_known<double> : csr_matvec_known<float>)(stream, data, ix, ip, vector, out, n_row, n_col, nse,
                                                                     homo != 0, transpose != 0);
+}
+
+void bpl_event_csr_matvec(bpl_stream_t stream, void **buffers, uint32_t n_row, uint32_t n_col, uint32_t nse, int homo,
+                          int is_double, int bool_events, int transpose) {
+    using Call = void (*)(cudaStream_t, void **, uint32_t, uint32_t, uint32_t, bool);
+    static const Call calls[2][2][2] = {   // [double][bool events][homo]
+        {{event_csr_known<float, float, false>, event_csr_known<float, float, true>},
+         {event_csr_known<float, uint8_t, false>, event_csr_known<float, uint8_t, true>}},
+        {{event_csr_known<double, double, false>, event_csr_known<double, double, true>},
+         {event_csr_known<double, uint8_t, false>, event_csr_known<double, uint8_t, true>}}};
+    calls[is_double != 0][bool_events != 0][homo != 0](stream, buffers, n_row, n_col, nse, transpose != 0);
 }
 
 size_t bpl_event_csr_workspace_bytes(uint32_t n_row, int transpose) {

@@ -6,7 +6,7 @@
 // columns: 1.9e7 entries into 2185 sums took 853 us, here 46).  A lookup in shared memory takes a tenth of a clock, an
 // addition there 0.3.  So one block per SM holds the whole vector.
 //
-// Longer vectors stay with the plain kernels.  What shared memory takes from the 256 KB of an SM is missing for the
+// Longer vectors are gathered through L1 (bands_kernel) or scattered into L2 (csr_kernels.cu).  What shared memory takes from the 256 KB of an SM is missing for the
 // entries in flight, which pass through L1: 1e7 float entries, 80 MB, take 18.6 us with up to 132 KB of x, 19.9 with
 // 160 KB, 23 with 195 KB, 31 with 226 KB.  For that reason neither the first 160 KB of a longer vector here and the rest
 // by the plain ways (100,000 columns: gather 44 us against 39, scatter 78 against 65), nor slices of it in several blocks
@@ -182,6 +182,169 @@ gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     });
 }
 
+// y = A events: the events as one bit each in shared memory.  Homogeneous weights count hits and scale once (equal to the
+// reference CPU kernel's float64 accumulation, brainpylib/_src/event_ops/event_csr_matvec.py:334-357).
+template<typename T, bool HOMO>
+struct EventVisit {
+    const uint32_t *mask;
+    uint32_t lpr;
+    T homo_w, *y;
+    T acc;
+    uint32_t hits;
+    __device__ __forceinline__ int fetch(uint32_t) const { return 0; }
+    __device__ __forceinline__ void begin(int) {
+        acc = T(0);
+        hits = 0;
+    }
+    __device__ __forceinline__ uint32_t hit(const uint32_t c) const { return (mask[c >> 5] >> (c & 31u)) & 1u; }
+    template<bool FULL>
+    __device__ __forceinline__ void quad(uint32_t, const uint32_t (&c)[4], const T *w, const int lo, const int hi) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (!FULL && !(e >= lo && e < hi)) continue;
+            const uint32_t h = hit(c[e]);
+            if (HOMO) hits += h;
+            else if (h) acc += w[e];
+        }
+    }
+    __device__ __forceinline__ void entry(uint32_t, const uint32_t c, const T w) {
+        const uint32_t h = hit(c);
+        if (HOMO) hits += h;
+        else if (h) acc += w;
+    }
+    __device__ __forceinline__ void end(const uint32_t row, const bool lead) {
+        if (HOMO) {
+            hits = group_sum(hits, static_cast<int>(lpr));
+            // no hit leaves +0 like an empty sum (the product with a negative weight would give -0)
+            acc = hits ? static_cast<T>(static_cast<double>(hits) * static_cast<double>(homo_w)) : T(0);
+        } else {
+            acc = group_sum(acc, static_cast<int>(lpr));
+        }
+        if (lead) y[row] = acc;
+    }
+};
+
+template<typename T, typename E, bool HOMO, int U>
+__global__ void __launch_bounds__(SHARED_THREADS, 1)
+gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
+                     const E *__restrict__ events, const uint32_t *__restrict__ packed, T *__restrict__ y, const uint32_t n_row,
+                     const uint32_t nse, const uint32_t n_col) {
+    extern __shared__ __align__(16) unsigned char shared_vector[];
+    uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
+    const Deal deal(nse, n_row, 4 * U);
+    EventVisit<T, HOMO> visit{mask, deal.lpr, HOMO ? data[0] : T(0), y, T(0), 0u};
+    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
+        if (packed != nullptr) {
+            pdl_wait();
+            fill_shared(mask, packed, (n_col + 31u) / 32u);
+        } else {
+            pack_event_mask(events, n_col, mask);
+        }
+        __syncthreads();
+    });
+}
+
+// The bits of the events, once for all blocks.  (Every block packing them itself reads 148 times the events: a million
+// float events take 60 us, their 125 KB of bits 1.)
+template<typename E>
+__global__ void __launch_bounds__(256) pack_events_kernel(const E *__restrict__ events, uint32_t *__restrict__ packed, const uint32_t n) {
+    pdl_launch_dependents();
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t w = (static_cast<uint64_t>(blockIdx.x) * 256u + threadIdx.x) >> 5; w * 32u < n; w += static_cast<uint64_t>(gridDim.x) * 8u) {
+        const uint64_t i = w * 32u + lane;
+        const uint32_t bits = __ballot_sync(FULL_MASK, i < n && is_event(events[i]));
+        if (lane == 0) packed[w] = bits;
+    }
+}
+
+// The two gathering products for a longer vector x, read through L1.  What bounds them there is the traffic from L2, 34
+// bytes per clock and SM: every miss brings a sector of 32 bytes for one value, 2.7 times the matrix itself where most
+// gathers miss (1e7 float entries, 100,000 columns: 39 us).  Stored rows are nearly always sorted by column.  So few
+// lanes (one, where there are rows enough) walk a row together, 8 entries each at a time, and the rows of an SM, which
+// start together, sweep over x together: at any time they read in a band of x that fits L1, and each of its sectors comes
+// from L2 about once: 31 us, 80 % of the gathers hit.  More lanes per row, 1000 or 2000 per SM instead of 500: 37 and 45
+// us.  (Unsorted rows are summed as correctly, with the misses of the plain kernel.)
+//   OUTER = false: y[row] = sum of weight * x[column];  OUTER = true: g[entry] = row_vector[row] * x[column].
+constexpr int BAND_THREADS = 128;
+
+template<typename T, bool HOMO, bool OUTER>
+__global__ void __launch_bounds__(BAND_THREADS)
+bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
+             const T *__restrict__ x, T *__restrict__ out, const uint32_t n_row, const uint32_t nse, const uint32_t log_l) {
+    constexpr bool WEIGHTS = !HOMO && !OUTER;                  // (OUTER: data is the row vector)
+    struct Unit {
+        uint32_t c[8];
+        T w[WEIGHTS ? 8 : 1];
+    };
+    const uint32_t L = 1u << log_l, part = threadIdx.x & (L - 1u);
+    const uint32_t full = nse >> 3;                            // units that lie wholly inside the arrays
+    const uint64_t rows_per_grid = (static_cast<uint64_t>(gridDim.x) * BAND_THREADS) >> log_l;
+    for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * (BAND_THREADS >> log_l); base < n_row; base += rows_per_grid) {
+        const uint64_t row = base + (threadIdx.x >> log_l);
+        uint32_t start = 0, end = 0;
+        T w0 = T(0);
+        if (row < n_row) {
+            start = indptr[row];
+            end = indptr[row + 1];
+            if (!WEIGHTS) w0 = OUTER ? data[row] : data[0];
+        }
+        uint32_t u = (start >> 3) + part;
+        const uint32_t u_end = start < end ? (end + 7u) >> 3 : 0u;
+        auto load = [&](Unit &v, const uint32_t at) {
+            if (at < u_end && at < full) {
+                ldg_stream_8(indices + 8ull * at, v.c);
+                if (WEIGHTS) ldg_stream_8(data + 8ull * at, v.w);
+            }
+        };
+        T acc = T(0);
+        auto use = [&](const Unit &v, const uint32_t at) {
+            const uint32_t pos = 8u * at;
+            if (at >= full) {                                  // ragged end of the arrays
+                for (uint32_t e = max(pos, start); e < end; ++e) {
+                    const T p = (WEIGHTS ? data[e] : w0) * __ldg(x + indices[e]);
+                    if (OUTER) out[e] = p; else acc += p;
+                }
+                return;
+            }
+            T g[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                g[e] = T(0);
+                if (pos + e >= start && pos + e < end) g[e] = __ldg(x + v.c[e]);
+            }
+            if (OUTER) {
+                if (pos >= start && pos + 8u <= end) {
+                    store_quad(out + pos, w0 * g[0], w0 * g[1], w0 * g[2], w0 * g[3]);
+                    store_quad(out + pos + 4u, w0 * g[4], w0 * g[5], w0 * g[6], w0 * g[7]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (pos + e >= start && pos + e < end) out[pos + e] = w0 * g[e];
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (pos + e >= start && pos + e < end) acc += (WEIGHTS ? v.w[WEIGHTS ? e : 0] : w0) * g[e];
+            }
+        };
+        Unit a, b;
+        load(a, u);
+        while (u < u_end) {
+            load(b, u + L);
+            use(a, u);
+            if (u + L < u_end) {
+                load(a, u + 2u * L);
+                use(b, u + L);
+            }
+            u += 2u * L;
+        }
+        if (!OUTER) {
+            for (uint32_t o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL_MASK, acc, o);
+            if (part == 0 && row < n_row) out[row] = acc;
+        }
+    }
+}
+
 // y += A^T x: sums in shared memory, added to the zero-filled y at the end
 template<typename T, bool HOMO>
 struct ScatterVisit {
@@ -279,9 +442,31 @@ bool usable(const CsrMatrix<T> &m, const bool weights) {
            (!weights || aligned16(m.data));
 }
 
+// The bands pay where the sectors of x are used again in an SM (as many entries as sectors: 2e6 entries, 100,000 columns
+// 13.4 -> 11 us; two thirds, 400,000 columns: 26 -> 29), and where there are rows to sweep side by side (34 per SM: 26 ->
+// 29 us, 135: 37 -> 28).  500 lanes per SM, 16 entries or more for each.
+template<typename T, bool HOMO, bool OUTER>
+bool bands(cudaStream_t stream, const CsrMatrix<T> &m, const T *data, const T *x, T *out) {
+    const uint32_t sms = static_cast<uint32_t>(sm_count());
+    const auto aligned32 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; };
+    if (m.n_row < 100u * sms || static_cast<double>(m.nse) / sms < m.n_col * (sizeof(T) / 32.0) || !aligned32(m.indices) ||
+        (!HOMO && !OUTER && !aligned32(data)) || (OUTER && !aligned16(out)))
+        return false;
+    uint32_t log_l = 0;
+    while (log_l < 5 && (static_cast<uint64_t>(m.n_row) << log_l) < 512u * sms && (m.nse / m.n_row >> log_l) >= 16u) ++log_l;
+    const uint64_t blocks = ((static_cast<uint64_t>(m.n_row) << log_l) + BAND_THREADS - 1) / BAND_THREADS;
+    bands_kernel<T, HOMO, OUTER><<<static_cast<uint32_t>(std::min<uint64_t>(blocks, 64ull * sms)), BAND_THREADS, 0, stream>>>(
+        m.indices, m.indptr, data, x, out, m.n_row, m.nse, log_l);
+    launch_ok();
+    return true;
+}
+// columns from which the bands are faster than x in shared memory (200 KB of floats; of doubles, 164 KB)
+template<typename T> constexpr uint32_t BANDS_FROM = sizeof(T) == 4 ? 51200u : 21000u;
+
 template<typename T, bool HOMO>
 bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
     constexpr auto kernel = gather_shared_kernel<T, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    if (m.n_col > BANDS_FROM<T> && bands<T, HOMO, false>(stream, m, m.data, x, y)) return true;
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
@@ -289,6 +474,30 @@ bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
     kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, m.data, x, y,
                                                                                              m.n_row, m.nse, m.n_col);
     launch_ok();
+    return true;
+}
+
+template<typename T, typename E, bool HOMO>
+bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *workspace, T *y) {
+    constexpr auto kernel = gather_events_kernel<T, E, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    const uint32_t bytes = (m.n_col + 31u) / 32u * 4u;
+    if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
+        (!HOMO && !aligned16(m.data)))
+        return false;
+    // The bits are packed by a launch of their own where the events are more than a block reads in its time (34 bytes per
+    // clock).  The alternative gathers events through L1 and L2, 1.1 clocks each where they miss.
+    const double per = static_cast<double>(m.nse) / sm_count(), gather = m.n_col * sizeof(E) > 200000u ? 1.0 : 0.6;
+    const bool pack = m.n_col * sizeof(E) > 32768u;
+    if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
+    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
+    if (pack) {
+        const uint32_t blocks = std::min<uint32_t>((m.n_col + 255u) / 256u, 8u * static_cast<uint32_t>(sm_count()));
+        pack_events_kernel<E><<<blocks, 256, 0, stream>>>(events, workspace, m.n_col);
+        if (!launch_ok()) return true;
+    }
+    const cudaError_t e = launch_dependent(kernel, dim3(sm_count()), dim3(SHARED_THREADS), bytes, stream, m.indices, m.indptr, m.data,
+                                           events, pack ? workspace : nullptr, y, m.n_row, m.nse, m.n_col);
+    if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
     return true;
 }
 
@@ -311,6 +520,7 @@ bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) 
 template<typename T>
 bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g) {
     constexpr auto kernel = outer_shared_kernel<T, 2>;
+    if (m.n_col > BANDS_FROM<T> && bands<T, true, true>(stream, m, row_vector, col_vector, g)) return true;
     if (!usable(m, false) || !aligned16(g)) return false;
     const Plan<T> p(m, true);                // one index in, one value out
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
@@ -329,6 +539,15 @@ bool gather_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *
 bool gather_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *x, double *y) {
     return m.homo ? gather_impl<double, true>(stream, m, x, y) : gather_impl<double, false>(stream, m, x, y);
 }
+template<typename T, typename E>
+bool gather_events(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *workspace, T *y) {
+    return m.homo ? gather_events_impl<T, E, true>(stream, m, events, workspace, y)
+                  : gather_events_impl<T, E, false>(stream, m, events, workspace, y);
+}
+template bool gather_events(cudaStream_t, const CsrMatrix<float> &, const uint8_t *, uint32_t *, float *);
+template bool gather_events(cudaStream_t, const CsrMatrix<float> &, const float *, uint32_t *, float *);
+template bool gather_events(cudaStream_t, const CsrMatrix<double> &, const uint8_t *, uint32_t *, double *);
+template bool gather_events(cudaStream_t, const CsrMatrix<double> &, const double *, uint32_t *, double *);
 bool scatter_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *x, float *y) {
     return m.homo ? scatter_impl<float, true>(stream, m, x, y) : scatter_impl<float, false>(stream, m, x, y);
 }

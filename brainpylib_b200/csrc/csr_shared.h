@@ -19,6 +19,9 @@ struct CsrMatrix {
 // y = A x
 bool gather_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *x, float *y);
 bool gather_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *x, double *y);
+// y = A events (E: uint8_t, or T); workspace: n_col bits, in whole words
+template<typename T, typename E>
+bool gather_events(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *workspace, T *y);
 // y = A^T x; y need not be zero
 bool scatter_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *x, float *y);
 bool scatter_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *x, double *y);

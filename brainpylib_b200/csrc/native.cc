@@ -156,22 +156,13 @@ Tensor csr_product(const Tensor &data, const Tensor &indices, const Tensor &indp
 
 Tensor event_csr_product(const Tensor &data, const Tensor &indices, const Tensor &indptr, const Tensor &events,
                          int64_t n_row, int64_t n_col, bool transpose) {
-    static const Target targets[2][2][2] = {   // [double][homo][float events]
-        {{event_csr_matvec_heter_float_bool, event_csr_matvec_heter_float_float},
-         {event_csr_matvec_homo_float_bool, event_csr_matvec_homo_float_float}},
-        {{event_csr_matvec_heter_double_bool, event_csr_matvec_heter_double_double},
-         {event_csr_matvec_homo_double_bool, event_csr_matvec_homo_double_double}}};
     OnDevice on(data);
     Tensor out = new_tensor({transpose ? n_col : n_row}, data.scalar_type(), data.device());
-    bpl::TwoUintOneBoolDescriptor d;
-    std::memset(&d, 0, sizeof(d));
-    d.uint_x = static_cast<unsigned>(n_row);
-    d.uint_y = static_cast<unsigned>(n_col);
-    d.bool_x = transpose;
-    Scratch ws(bpl_event_csr_workspace_bytes(d.uint_x, transpose ? 1 : 0), on.stream);
+    Scratch ws(transpose ? bpl_event_csr_workspace_bytes(static_cast<uint32_t>(n_row), 1) : (n_col + 31) / 32 * 4, on.stream);
     void *buffers[6] = {ptr(data), ptr(indices), ptr(indptr), ptr(events), ptr(out), ws.ptr};
-    targets[is_double(data)][data.size(0) == 1][events.scalar_type() != at::kBool](
-        on.stream, buffers, reinterpret_cast<const char *>(&d), sizeof(d));
+    bpl_event_csr_matvec(on.stream, buffers, static_cast<uint32_t>(n_row), static_cast<uint32_t>(n_col),
+                         static_cast<uint32_t>(indices.size(0)), data.size(0) == 1, is_double(data),
+                         events.scalar_type() == at::kBool, transpose);
     check_status();
     return out;
 }

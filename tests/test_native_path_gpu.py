@@ -77,3 +77,49 @@ def test_products_with_the_vector_in_shared_memory(cuda, n_row, n_col, mean, hom
     want = cpu.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
     tol = 1e-5 if dtype == np.float32 else 1e-12
     np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(max(mean, indices.size / n_col)))
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('homo', [False, True])
+@pytest.mark.parametrize('n_row,n_col,mean', [(80_000, 60_000, 50), (16_000, 60_000, 400), (200_000, 47_000, 9)])
+def test_products_that_sweep_a_longer_vector(cuda, n_row, n_col, mean, homo, dtype):
+  """One lane, several lanes, less than a unit per row; unsorted rows, empty ones, a ragged end of the arrays."""
+  g = torch.Generator(device='cuda').manual_seed(23)
+  lens = torch.poisson(torch.full((n_row,), float(mean), device=cuda), generator=g).long()
+  lens[torch.tensor([0, 7, n_row - 2], device=cuda)] = torch.tensor([0, 3 * mean + 1, 0], device=cuda)
+  lens[1] += (3 - int(lens.sum())) % 8
+  indptr = torch.cat([lens.new_zeros(1), lens.cumsum(0)]).int()
+  indices = torch.randint(0, n_col, (int(lens.sum()),), dtype=torch.int32, device=cuda, generator=g)
+  data = torch.randn(1 if homo else indices.shape[0], dtype=dtype, device=cuda, generator=g).requires_grad_(not homo)
+  x = torch.randn(n_col, dtype=dtype, device=cuda, generator=g)
+  y = bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col))
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  want = torch.zeros(n_row, dtype=torch.float64, device=cuda).index_add_(0, row, (data.detach() * x[col]).double())
+  tol = dict(rtol=1e-5, atol=1e-4) if dtype == torch.float32 else dict(rtol=1e-12, atol=1e-11)
+  torch.testing.assert_close(y.detach().double(), want, **tol)
+  if not homo:
+    ct = torch.randn(n_row, dtype=dtype, device=cuda, generator=g)
+    torch.testing.assert_close(torch.autograd.grad(y, data, ct)[0], ct[row] * x[col])
+
+
+@pytest.mark.parametrize('dtype,bool_events', [(np.float32, True), (np.float32, False), (np.float64, True), (np.float64, False)])
+@pytest.mark.parametrize('homo', [False, True])
+@pytest.mark.parametrize('n_row,n_col,mean', [(9000, 2001, 333), (150_000, 33, 20), (2000, 1_000_003, 2500), (300, 517, 40),
+                                              (5000, 250_000, 40)])
+def test_event_gather_over_bits(cuda, n_row, n_col, mean, homo, dtype, bool_events):
+  rng = np.random.default_rng(29)
+  lens = rng.poisson(mean, n_row)
+  lens[[0, 3, n_row - 1]] = 0, 2 * mean, 0
+  lens[1] += (3 - int(lens.sum())) % 4
+  data, indices, indptr, rng = cases.ragged_csr(lens, n_col, 31, dtype=dtype)
+  data = -data[:1] if homo else data
+  events = rng.random(n_col) < 0.3
+  events = events if bool_events else (events * 2.5).astype(dtype)
+  d = [torch.as_tensor(a).to(cuda) for a in (data, indices, indptr, events)]
+  got = bpl.event_csr_matvec(*d, shape=(n_row, n_col)).cpu().numpy()
+  want = cpu.event_csr_matvec(data, indices, indptr, events, shape=(n_row, n_col))
+  if homo and dtype == np.float32:       # the reference counts in float64
+    assert got.tobytes() == want.tobytes()
+  else:
+    tol = 1e-5 if dtype == np.float32 else 1e-12
+    np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(mean))
