@@ -15,6 +15,8 @@
 #include <algorithm>
 #include <cmath>
 
+#include <math_constants.h>
+
 #include "abi.h"
 #include "common.cuh"
 #include "jit_stream.cuh"
@@ -145,23 +147,47 @@ __device__ __noinline__ void walk_column(const unsigned int seed, const GapParam
 //
 // What bounds it is the shared-memory pipe, and how many lanes of a warp have work in the tiles that are resident: the
 // number of connections per column and tile is Poisson.  With one tile of 768 positions at a time (mean 7.7 at 1 %) 55 % of
-// the lanes worked.  Now a warp moves on when all its lanes are through with the oldest tile, while a lane that is through
-// runs on into the next two, which have landed: 81 % (simulated; a ring of 4 tiles of 384, the fourth in flight).
-// C5 (256 x 65536 @ 65536^2, 1 %): 3.09 ms before.
+// the lanes worked, and the warps waited for the slowest one at every tile.  Now a warp moves on when all its lanes are
+// through with its oldest tile, while a lane that is through runs on into the next ones that have landed; and no warp waits
+// for another: each waits for the arrival of a tile only (an mbarrier per buffer), and the last warp to leave a tile
+// starts the copy (one bulk copy of 24 KB) that takes its place.
+// C5 (256 x 65536 @ 65536^2, 1 %): 3.09 ms with one tile at a time and block barriers, MATMAT_NOW ms now.
 //
 // Measured alternatives: lanes as rows (a warp owns 30 columns x 64 rows, entries broadcast from a staging buffer, every
 // lane works on every connection) 5.3 ms: 14 instructions per entry and 64 rows against 50 per 32 entries and 32 rows here;
 // the same without staging 7.7-10 ms.
-constexpr int RING = 4;                                     // buffers; RING - 1 tiles are open at a time
+constexpr unsigned int RING = 8;                            // buffers of 24 KB
 template<typename T> struct ApplyShape;
-template<> struct ApplyShape<float> { static constexpr int MAX_THREADS = 896, KT = 384, CHUNKS = 8; };
-template<> struct ApplyShape<double> { static constexpr int MAX_THREADS = 512, KT = 192, CHUNKS = 16; };   // 32 double sums
-constexpr unsigned int APPLY_SMEM = RING * 48u * 1024u;
+template<> struct ApplyShape<float> { static constexpr int MAX_THREADS = 896, KT = 192, CHUNKS = 8; };
+template<> struct ApplyShape<double> { static constexpr int MAX_THREADS = 512, KT = 96, CHUNKS = 16; };   // 32 double sums
+constexpr unsigned int TILE_BYTES = 24u * 1024u;
+constexpr unsigned int APPLY_SMEM = RING * TILE_BYTES;
 
-__device__ __forceinline__ void mm_cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-                 :: "r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(__cvta_generic_to_global(src))
-                 : "memory");
+__device__ __forceinline__ uint32_t shared_address(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void barrier_init(uint64_t *bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(shared_address(bar)) : "memory");
+}
+// the one arrival of a phase, and the bytes that complete it
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, const uint32_t bytes, uint64_t *bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(shared_address(bar)), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(shared_address(dst)), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(shared_address(bar)) : "memory");
+}
+__device__ __forceinline__ bool barrier_done(uint64_t *bar, const uint32_t parity) {
+    uint32_t done;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done) : "r"(shared_address(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
+// Waits for a phase; false when it has not come within a second or so.
+__device__ __forceinline__ bool barrier_wait(uint64_t *bar, const uint32_t parity) {
+    for (uint32_t i = 0; i < (1u << 20); ++i) {
+        uint32_t done;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(done) : "r"(shared_address(bar)), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
 }
 
 // grid = (row groups of 32, column blocks of blockDim.x columns): the blocks that walk the same columns' lists are
@@ -173,8 +199,10 @@ jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const un
                         const unsigned int *__restrict__ cnt, const MMEntry<T> *__restrict__ entries,
                         const unsigned int seed, const GapParams gp, const double w1, const double w2, T *__restrict__ Y) {
     constexpr int KT = ApplyShape<T>::KT, CHUNKS = ApplyShape<T>::CHUNKS, PER_CHUNK = 16 / sizeof(T);
-    constexpr unsigned int PIECES = KT * MM_ROWS * sizeof(T) / 16, ROW_PIECES = MM_ROWS * sizeof(T) / 16;
-    extern __shared__ __align__(16) unsigned char mm_smem[];
+    static_assert(KT * MM_ROWS * sizeof(T) == TILE_BYTES, "a tile");
+    extern __shared__ __align__(128) unsigned char mm_smem[];
+    __shared__ __align__(8) uint64_t landed_bar[RING];
+    __shared__ unsigned int left[RING];                                  // warps that are through with the tile of a buffer
     T *ring = reinterpret_cast<T *>(mm_smem);                            // [RING][KT][MM_ROWS]
 
     const unsigned int c = blockIdx.y * blockDim.x + threadIdx.x;       // column within the chunk
@@ -200,22 +228,37 @@ jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const un
 #pragma unroll
     for (int i = 0; i < static_cast<int>(MM_ROWS); ++i) sum[i] = T(0);
 
-    const unsigned int n_tiles = (k + KT - 1) / KT;
+    const unsigned int n_tiles = (k + KT - 1) / KT, n_warps = blockDim.x >> 5;
     auto issue = [&](const unsigned int t) {                             // tile t into buffer t mod RING
-        if (t < n_tiles) {
-            const unsigned int pieces = min(PIECES, (k - t * KT) * ROW_PIECES);
-            unsigned char *dst = mm_smem + (t % RING) * (PIECES * 16u);
-            const unsigned char *src = reinterpret_cast<const unsigned char *>(group + static_cast<size_t>(t) * KT * MM_ROWS);
-            for (unsigned int q = threadIdx.x; q < pieces; q += blockDim.x) mm_cp_async16(dst + q * 16u, src + q * 16u);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        const unsigned int rows = min(static_cast<unsigned int>(KT), k - t * KT);
+        bulk_copy(mm_smem + (t % RING) * TILE_BYTES, group + static_cast<size_t>(t) * KT * MM_ROWS,
+                  rows * static_cast<unsigned int>(MM_ROWS * sizeof(T)), &landed_bar[t % RING]);
     };
-    for (unsigned int t = 0; t < RING - 1; ++t) issue(t);
+    if (threadIdx.x == 0) {
+        for (unsigned int i = 0; i < RING; ++i) {
+            barrier_init(&landed_bar[i]);
+            left[i] = 0;
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        for (unsigned int t = 0; t < min(RING, n_tiles); ++t) issue(t);
+    }
+    __syncthreads();
+    unsigned int landed = 0;                                             // tiles that this warp knows to be there
+    bool lost = false;
     for (unsigned int t = 0; t < n_tiles; ++t) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");             // this thread's copies up to tile t + RING - 2
-        __syncthreads();                                                 // everyone's, and everyone is through with tile t - 1
-        issue(t + RING - 1);                                             // into the buffer of tile t - 1
-        const unsigned int first = t * KT, done = min(first + KT, k), open = min(first + (RING - 1) * KT, k);
+        if (landed == t) {
+            lost = !barrier_wait(&landed_bar[t % RING], (t / RING) & 1u);
+            if (__any_sync(FULL_MASK, lost)) {
+                lost = true;
+                break;
+            }
+            ++landed;
+        }
+        // further ones: below t + RING, whose buffer is the one of tile t
+        while (landed < min(t + RING, n_tiles) && __all_sync(FULL_MASK, barrier_done(&landed_bar[landed % RING], (landed / RING) & 1u)))
+            ++landed;
+        const unsigned int first = t * KT, done = min(first + KT, k), open = min(landed * KT, k);
         const unsigned int slot0 = (t % RING) * KT;
         while (__any_sync(FULL_MASK, pos < done)) {
             if (pos < open) {
@@ -242,6 +285,21 @@ jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const un
                 }
             }
         }
+        __syncwarp();
+        if (lane == 0 && t + RING < n_tiles) {
+            __threadfence_block();                                       // the reads of this warp are over
+            if (atomicAdd(&left[t % RING], 1u) == n_warps - 1u) {
+                __threadfence_block();                                   // and those of the others
+                left[t % RING] = 0;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                issue(t + RING);
+            }
+        }
+    }
+    if (lost) {                                                          // never seen: no result rather than a wrong one
+        for (unsigned int i = 0; i < RING; ++i) barrier_wait(&landed_bar[i], (landed / RING) & 1u);
+#pragma unroll
+        for (int i = 0; i < static_cast<int>(MM_ROWS); ++i) sum[i] = T(CUDART_NAN_F);
     }
     const unsigned int row0 = blockIdx.x * MM_ROWS;
     if (live && !overflow) {
