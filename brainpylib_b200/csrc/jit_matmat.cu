@@ -8,10 +8,10 @@
 //
 // Workspace of one chunk of C columns (the host walks the columns chunk by chunk):
 //   cnt u32[C] | Xt T[m_pad / 32][k][32] (X transposed in groups of 32 rows) | entries MMEntry<T>[C * stride]
-// Entry j of column c sits at c * stride + j (stride = cap + 1 rounded up to even), position and weight side by side (8
-// bytes for float, 16 for double); a list ends with an entry whose position is 0xffffffff.  cap = expected connections per
-// column + 10 standard deviations + 16.  A column with more (never seen; the bound is not a proof) reads as empty and is
-// walked again, stream and all, by the warp that owns it.
+// Entry j of column c sits at c * cap + j, position and weight side by side (8 bytes for float, 16 for double); a list
+// ends with an entry whose position is k or more.  cap = expected connections per column + 10 standard deviations + 16, a
+// multiple of 4.  A column with more (never seen; the bound is not a proof) reads as empty and is walked again, stream and
+// all, by the warp or thread that owns it.
 #include <algorithm>
 #include <cmath>
 
@@ -29,8 +29,17 @@ template<> struct __align__(8) MMEntry<float> { unsigned int pos; float w; };
 template<> struct __align__(16) MMEntry<double> { unsigned int pos, pad; double w; };
 template<typename T> struct __align__(16) MMEntryPair { MMEntry<T> a, b; };
 constexpr unsigned int LIST_END = 0xffffffffu;
-// slots per column: the entries, the terminating entry, rounded up to whole pairs
-__host__ __device__ inline unsigned int mm_list_stride(unsigned int cap) { return (cap + 2u) & ~1u; }
+// four entries, written as whole sectors
+template<typename T> struct __align__(32) MMEntryQuad { MMEntry<T> e[4]; };
+template<typename T>
+__device__ __forceinline__ void store_entries(MMEntry<T> *to, const MMEntryQuad<T> &q) {
+    const uint32_t *v = reinterpret_cast<const uint32_t *>(&q);
+#pragma unroll
+    for (unsigned int i = 0; i < sizeof(q) / 4; i += 8)
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                     :: "l"(reinterpret_cast<uint32_t *>(to) + i), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]),
+                        "r"(v[i + 4]), "r"(v[i + 5]), "r"(v[i + 6]), "r"(v[i + 7]) : "memory");
+}
 
 inline unsigned int blocks_for(unsigned long long n, unsigned int per_block) {
     return static_cast<unsigned int>((n + per_block - 1) / per_block);
@@ -48,36 +57,36 @@ constexpr int FILL_THREADS = 128;
 constexpr unsigned int MM_ROWS = 32;      // rows of X are padded to whole groups
 
 // One thread per column: bound by the latency of its chain (65,536 columns: 14 warps per SM), hence the batches of
-// jit_stream.cuh and small blocks, which spread over the SMs.
+// jit_stream.cuh and small blocks, which spread over the SMs; and by the writes, 32 lists per warp: a batch is four entries
+// and goes out as one sector (two for double), the last one with entries behind the end, which end the list.
 template<typename T, int KIND, bool QUICK>
 __device__ __forceinline__ void fill_list(const unsigned int seed, const GapParams &gp, const double w1, const double w2,
                                           const unsigned int k, const unsigned int cap, unsigned int *cnt, MMEntry<T> *mine) {
     Xorwow s;
     s.seed(seed);
-    Batch<KIND, QUICK> b;
+    Batch<KIND, QUICK, 4> b;
     unsigned int count = 0, at = 0;
     do {
         b.draw(s, at, k, gp);
-        T w[Batch<KIND, QUICK>::N];
+        T w[4];
         b.weights(w, w1, w2);
+        MMEntryQuad<T> q;
 #pragma unroll
-        for (int j = 0; j < b.N; ++j) {
-            if (b.pos[j] < k) {
-                if (count < cap) {
-                    MMEntry<T> e;
-                    e.pos = b.pos[j];
-                    e.w = w[j];
-                    mine[count] = e;
-                }
-                ++count;
-            }
+        for (int j = 0; j < 4; ++j) {
+            q.e[j].pos = b.pos[j];
+            q.e[j].w = w[j];
         }
+        if (count + 4u <= cap) store_entries(mine + count, q);
+        count += 4u;
     } while (at < k);
+    // of the last batch, the entries before the end
+#pragma unroll
+    for (int j = 0; j < 4; ++j) count -= b.pos[j] >= k;
+    if (((count + 4u) & ~3u) > cap) {     // the batch with the end did not fit: reads as empty
+        count = cap + 1u;
+        mine[0].pos = LIST_END;
+    }
     *cnt = count;
-    MMEntry<T> last;                      // a list that overflowed reads as empty
-    last.pos = LIST_END;
-    last.w = T(0);
-    mine[count <= cap ? count : 0u] = last;
 }
 
 // 32 x 32 tiles of X through shared memory into Xt; rows past m are zero
@@ -113,7 +122,7 @@ jit_matmat_prepare_kernel(const unsigned int seed, const GapParams gp, const dou
     if (blockIdx.x < fill_blocks) {
         const unsigned int c = blockIdx.x * FILL_THREADS + threadIdx.x;
         if (c < cols)
-            fill_list<T, KIND, QUICK>(seed + c, gp, w1, w2, k, cap, cnt + c, entries + static_cast<size_t>(c) * mm_list_stride(cap));
+            fill_list<T, KIND, QUICK>(seed + c, gp, w1, w2, k, cap, cnt + c, entries + static_cast<size_t>(c) * cap);
         return;
     }
     const unsigned int tiles_k = (k + 31u) / 32u, n_tiles = tiles_k * (m_pad / 32u);
@@ -213,14 +222,14 @@ jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const un
     // The list is read two entries at a time (every lane reads its own list, so a warp's load touches 32 different lines
     // and costs the load/store pipe as much as all shared loads of a connection together).  `cur` holds the pair being
     // consumed, `nxt` the pair after it, requested when `cur` is entered; `j` counts consumed entries.
-    const MMEntryPair<T> *pairs = reinterpret_cast<const MMEntryPair<T> *>(entries + static_cast<size_t>(c) * mm_list_stride(cap));
+    const MMEntryPair<T> *pairs = reinterpret_cast<const MMEntryPair<T> *>(entries + static_cast<size_t>(c) * cap);
     MMEntryPair<T> cur, nxt;
     cur.a.pos = cur.b.pos = nxt.a.pos = nxt.b.pos = LIST_END;
     cur.a.w = cur.b.w = nxt.a.w = nxt.b.w = T(0);
     unsigned int j = 0;
     if (live) {
         cur = pairs[0];
-        if (cur.a.pos != LIST_END && cur.b.pos != LIST_END) nxt = pairs[1];
+        if (max(cur.a.pos, cur.b.pos) < k) nxt = pairs[1];
     }
     unsigned int pos = cur.a.pos;
     T weight = cur.a.w;
@@ -274,7 +283,7 @@ jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const un
                     cur = nxt;                                           // list ends inside
                     pos = cur.a.pos;
                     weight = cur.a.w;
-                    if (cur.a.pos != LIST_END && cur.b.pos != LIST_END) nxt = pairs[(j >> 1) + 1];
+                    if (max(cur.a.pos, cur.b.pos) < k) nxt = pairs[(j >> 1) + 1];
                 }
 #pragma unroll
                 for (int cc = 0; cc < CHUNKS; ++cc) {
@@ -354,7 +363,7 @@ jit_matmat_gather_kernel(const T *__restrict__ Xt, const unsigned int m, const u
             for (int v = 0; v < V; ++v) sum[v] += (q.v[v] * w);
         };
         if (count <= cap) {
-            const MMEntry<T> *list = entries + static_cast<size_t>(c) * mm_list_stride(cap);
+            const MMEntry<T> *list = entries + static_cast<size_t>(c) * cap;
             MMEntry<T> e;
             e.pos = 0;
             e.w = T(0);
@@ -425,10 +434,11 @@ ListPlan list_plan(unsigned int m, unsigned int k, unsigned int n, double log_p,
     p.prob = -std::expm1(log_p);                              // log_p = log(1 - conn_prob)
     const double mean = static_cast<double>(k) * p.prob;
     const double cap_d = std::ceil(mean + 10.0 * std::sqrt(mean * (1.0 - p.prob) + 1.0)) + 16.0;
-    p.cap = static_cast<unsigned int>(std::min(cap_d, static_cast<double>(k) + 16.0));
+    p.cap = static_cast<unsigned int>(std::min(cap_d, static_cast<double>(k) + 16.0));   // (k, and a batch that ends it)
     if (g_list_cap_override != 0) p.cap = g_list_cap_override;
+    p.cap = (p.cap + 3u) & ~3u;
     const size_t entry = elem == 8 ? 16 : 8;        // sizeof(MMEntry<T>)
-    const size_t per_col = static_cast<size_t>(mm_list_stride(p.cap)) * entry + 4;
+    const size_t per_col = static_cast<size_t>(p.cap) * entry + 4;
     const size_t n_round = (static_cast<size_t>(n) + CHUNK_UNIT - 1) / CHUNK_UNIT * CHUNK_UNIT;
     const size_t budget = g_list_budget_override != 0 ? g_list_budget_override : LIST_BUDGET;
     const size_t chunk = std::min(std::max<size_t>(budget / per_col / CHUNK_UNIT * CHUNK_UNIT, CHUNK_UNIT), n_round);
@@ -437,7 +447,7 @@ ListPlan list_plan(unsigned int m, unsigned int k, unsigned int n, double log_p,
     p.m_pad = (m + MM_ROWS - 1) / MM_ROWS * MM_ROWS;
     p.xt_off = up(4 * chunk);
     p.entries_off = up(p.xt_off + elem * static_cast<size_t>(k) * p.m_pad);
-    p.bytes = up(p.entries_off + entry * chunk * static_cast<size_t>(mm_list_stride(p.cap)));
+    p.bytes = up(p.entries_off + entry * chunk * static_cast<size_t>(p.cap));
     return p;
 }
 

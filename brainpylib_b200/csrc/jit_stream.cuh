@@ -132,9 +132,10 @@ __device__ __forceinline__ T normal_weight(const uint32_t x, const uint32_t y, c
 // One batch of connections: positions and the raw draws of their weights.  QUICK = false: parameters outside gap_of's
 // range or streams too long for sums of gaps to stay below 2^32; the reference's expression for every draw, and a
 // position behind the end (`n`) stays there.
-template<int KIND, bool QUICK>
+// COUNT is even for normal weights, so that a batch starts with a new pair.
+template<int KIND, bool QUICK, int COUNT = KIND == W_NORMAL ? 4 : 5>
 struct Batch {
-    static constexpr int N = KIND == W_NORMAL ? 4 : 5;     // normal: even, so that a batch starts with a new pair
+    static constexpr int N = COUNT;
     uint32_t pos[N];
     uint32_t raw[KIND == W_HOMO ? 1 : N];
 
