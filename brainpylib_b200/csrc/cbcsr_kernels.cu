@@ -47,6 +47,7 @@ event_cb_scatter_kernel(const unsigned char *__restrict__ groups, const uint32_t
     extern __shared__ __align__(128) unsigned char cb_smem[];
     __shared__ uint32_t prefix[MAX_CHUNKS + 1];
     __shared__ uint32_t warp_total[CB_WARPS];
+    pdl_launch_dependents();     // (every dependent waits for this kernel's end, and this one for its predecessor's)
     cb_scatter_body<NBUF, FIXED, LOG_L>(groups, offsets, n_col, width, n_blocks, blockIdx.x / P, blockIdx.x % P, P, chunk,
                                         n_chunks, counts, ids, y, acc_bytes, cb_smem, prefix, warp_total, inv_scale, trace,
                                         blockIdx.x);

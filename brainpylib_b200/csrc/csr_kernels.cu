@@ -587,12 +587,13 @@ extern "C" void event_csr_matvec_list_heter_float(bpl_stream_t stream, void **bu
     float *y = static_cast<float *>(buffers[4]);
     const int grid = persistent_blocks(4, static_cast<uint64_t>(d->n_row) * 16);
     if (profile_before()) cudaEventRecord(profile_before(), stream);
-    if (aligned16(indices) && aligned16(data))
-        row_scatter_kernel<float, false, true, true, true><<<grid, ROW_THREADS, 0, stream>>>(
-            indices, indptr, data, nullptr, d->n_row, SCAN_TILE, d->n_chunks, list, list + MAX_CHUNKS, y);
-    else
-        row_scatter_kernel<float, false, true, false, true><<<grid, ROW_THREADS, 0, stream>>>(
-            indices, indptr, data, nullptr, d->n_row, SCAN_TILE, d->n_chunks, list, list + MAX_CHUNKS, y);
+    // behind lif_exp_step or another of these a dependent launch: its blocks are there when the list is (they wait for it)
+    const cudaError_t e = launch_dependent(
+        aligned16(indices) && aligned16(data) ? row_scatter_kernel<float, false, true, true, true>
+                                              : row_scatter_kernel<float, false, true, false, true>,
+        dim3(grid), dim3(ROW_THREADS), 0, stream, indices, indptr, data, static_cast<const float *>(nullptr), d->n_row,
+        static_cast<uint32_t>(SCAN_TILE), d->n_chunks, list, list + MAX_CHUNKS, y);
+    if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
     if (profile_after()) cudaEventRecord(profile_after(), stream);
     launch_ok();
 }

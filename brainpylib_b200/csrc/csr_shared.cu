@@ -490,13 +490,16 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     const bool pack = m.n_col * sizeof(E) > 32768u;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
     if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
-    if (pack) {
-        const uint32_t blocks = std::min<uint32_t>((m.n_col + 255u) / 256u, 8u * static_cast<uint32_t>(sm_count()));
-        pack_events_kernel<E><<<blocks, 256, 0, stream>>>(events, workspace, m.n_col);
-        if (!launch_ok()) return true;
+    const uint32_t sms = static_cast<uint32_t>(sm_count());
+    if (!pack) {
+        kernel<<<sms, SHARED_THREADS, bytes, stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col);
+        launch_ok();
+        return true;
     }
-    const cudaError_t e = launch_dependent(kernel, dim3(sm_count()), dim3(SHARED_THREADS), bytes, stream, m.indices, m.indptr, m.data,
-                                           events, pack ? workspace : nullptr, y, m.n_row, m.nse, m.n_col);
+    pack_events_kernel<E><<<std::min<uint32_t>((m.n_col + 255u) / 256u, 8u * sms), 256, 0, stream>>>(events, workspace, m.n_col);
+    if (!launch_ok()) return true;
+    const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(SHARED_THREADS), bytes, stream, m.indices, m.indptr, m.data,
+                                           events, workspace, y, m.n_row, m.nse, m.n_col);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
     return true;
 }

@@ -119,6 +119,7 @@ jit_matmat_prepare_kernel(const unsigned int seed, const GapParams gp, const dou
                           MMEntry<T> *__restrict__ entries, const unsigned int fill_blocks, const T *__restrict__ X,
                           const unsigned int m, const unsigned int m_pad, T *__restrict__ Xt) {
     __shared__ T tile[32][33];
+    pdl_launch_dependents();                   // the multiply's blocks come up while the last lists are written
     if (blockIdx.x < fill_blocks) {
         const unsigned int c = blockIdx.x * FILL_THREADS + threadIdx.x;
         if (c < cols)
@@ -160,7 +161,7 @@ __device__ __noinline__ void walk_column(const unsigned int seed, const GapParam
 // through with its oldest tile, while a lane that is through runs on into the next ones that have landed; and no warp waits
 // for another: each waits for the arrival of a tile only (an mbarrier per buffer), and the last warp to leave a tile
 // starts the copy (one bulk copy of 24 KB) that takes its place.
-// C5 (256 x 65536 @ 65536^2, 1 %): 3.09 ms with one tile at a time and block barriers, MATMAT_NOW ms now.
+// C5 (256 x 65536 @ 65536^2, 1 %): 3.09 ms with one tile at a time and block barriers, 2.39 ms now.
 //
 // Measured alternatives: lanes as rows (a warp owns 30 columns x 64 rows, entries broadcast from a staging buffer, every
 // lane works on every connection) 5.3 ms: 14 instructions per entry and 64 rows against 50 per 32 entries and 32 rows here;
@@ -213,6 +214,7 @@ jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const un
     __shared__ __align__(8) uint64_t landed_bar[RING];
     __shared__ unsigned int left[RING];                                  // warps that are through with the tile of a buffer
     T *ring = reinterpret_cast<T *>(mm_smem);                            // [RING][KT][MM_ROWS]
+    pdl_wait();
 
     const unsigned int c = blockIdx.y * blockDim.x + threadIdx.x;       // column within the chunk
     const bool live = c < cols;
@@ -348,6 +350,7 @@ jit_matmat_gather_kernel(const T *__restrict__ Xt, const unsigned int m, const u
                          const unsigned int seed, const GapParams gp, const double w1, const double w2, T *__restrict__ Y) {
     __shared__ T block[GATHER_COLS][32 * V + 1];
     const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    pdl_wait();
     const unsigned int c = blockIdx.x * GATHER_COLS + warp, row0 = blockIdx.y * 32u * V, row = row0 + lane * V;
     T sum[V];
 #pragma unroll
@@ -473,9 +476,11 @@ StagedChoice choose_staged(const ListPlan &p, unsigned int k, unsigned int cols)
 template<typename T, int KIND, int V>
 void launch_gather(cudaStream_t stream, const ListPlan &p, const MatMatJITProbDescriptor1 *d, unsigned int col0, unsigned int cols,
                    const unsigned int *cnt, const MMEntry<T> *entries, const GapParams &gp, const T *Xt, T *Y) {
-    jit_matmat_gather_kernel<T, KIND, V><<<dim3(blocks_for(cols, GATHER_COLS), blocks_for(p.m_pad, 32 * V)), GATHER_COLS * 32, 0,
-                                           stream>>>(Xt, d->m, p.m_pad, d->k, d->n, col0, cols, p.cap, cnt, entries, d->seed + col0,
-                                                     gp, d->w1, d->w2, Y);
+    const cudaError_t e = launch_dependent(
+        jit_matmat_gather_kernel<T, KIND, V>, dim3(blocks_for(cols, GATHER_COLS), blocks_for(p.m_pad, 32 * V)),
+        dim3(GATHER_COLS * 32), 0, stream, Xt, d->m, p.m_pad, d->k, d->n, col0, cols, p.cap, cnt, entries, d->seed + col0, gp,
+        d->w1, d->w2, Y);
+    if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
 }
 
 template<typename T, int KIND>
@@ -520,8 +525,10 @@ void jit_matmat_list_impl(cudaStream_t stream, void **buffers, const char *opaqu
         if (staged.clocks < visits * std::max(std::min(32.0 * v, 1.0 * p.m_pad) * sizeof(T) / 28, 4.0)) {
             constexpr auto kernel = jit_matmat_apply_kernel<T, KIND>;
             if (!allow_shared<kernel>(APPLY_SMEM)) break;
-            kernel<<<dim3(p.m_pad / MM_ROWS, blocks_for(cols, staged.threads)), staged.threads, APPLY_SMEM, stream>>>(
-                Xt, d->m, d->k, d->n, col0, cols, p.cap, cnt, entries, d->seed + col0, gp, d->w1, d->w2, Y);
+            const cudaError_t e = launch_dependent(
+                kernel, dim3(p.m_pad / MM_ROWS, blocks_for(cols, staged.threads)), dim3(staged.threads), APPLY_SMEM, stream, Xt,
+                d->m, d->k, d->n, col0, cols, p.cap, cnt, entries, d->seed + col0, gp, d->w1, d->w2, Y);
+            if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
         } else if (v == 1) {
             launch_gather<T, KIND, 1>(stream, p, d, col0, cols, cnt, entries, gp, Xt, Y);
         } else if (v == 2) {

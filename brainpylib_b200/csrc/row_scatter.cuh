@@ -183,6 +183,7 @@ row_scatter_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restr
                    const uint32_t *__restrict__ ids, T *__restrict__ y) {
     __shared__ uint32_t prefix[MAX_CHUNKS + 1];
     __shared__ uint32_t warp_total[ROW_WARPS];
+    if (LIST) pdl_launch_dependents();     // (every dependent waits for this kernel's end, and this one for its predecessor's)
     row_scatter_body<T, HOMO, LIST, VEC, false, LANE_PARALLEL>(indices, indptr, data, x, n_row, chunk, n_chunks, counts,
                                                                ids, y, prefix, warp_total, blockIdx.x, gridDim.x);
 }
