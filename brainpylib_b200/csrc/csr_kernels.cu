@@ -239,6 +239,22 @@ void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaq
             set_status(BPL_ERR_ARGUMENT, "event_csr_matvec(transpose=True) needs a workspace buffer");
             return;
         }
+        if (n_row <= DIRECT_ROWS) {
+            const uint32_t sms = static_cast<uint32_t>(sm_count());
+            const uint32_t zero_grid = static_cast<uint32_t>(
+                min((static_cast<uint64_t>(n_col) + 4 * ROW_THREADS - 1) / (4 * ROW_THREADS), static_cast<uint64_t>(8 * sms)));
+            zero_kernel<T><<<zero_grid, ROW_THREADS, 0, stream>>>(y, n_col);
+            if (!launch_ok() || n_row == 0) return;
+            const uint32_t warps = 4u * sms * ROW_WARPS;                           // resident, one group each
+            const uint32_t per_group = (n_row + warps - 1) / warps, n_groups = (n_row + per_group - 1) / per_group;
+            const dim3 grid((min(n_groups * 4u, warps) + ROW_WARPS - 1) / ROW_WARPS);   // (long rows are cut into pieces)
+            if (profile_before()) cudaEventRecord(profile_before(), stream);
+            const cudaError_t e = launch_dependent(vec ? event_scatter_kernel<T, E, HOMO, true> : event_scatter_kernel<T, E, HOMO, false>,
+                                                   grid, dim3(ROW_THREADS), 0, stream, indices, indptr, data, events, n_row, n_groups, y);
+            if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+            if (profile_after()) cudaEventRecord(profile_after(), stream);
+            return;
+        }
         uint32_t *counts = ws, *ids = ws + MAX_CHUNKS;
         const ScanPlan p = plan_scan(n_row);
         const uint64_t zero_blocks = (static_cast<uint64_t>(n_col) + SCAN_TILE - 1) / SCAN_TILE;

@@ -188,6 +188,48 @@ row_scatter_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restr
                                                                ids, y, prefix, warp_total, blockIdx.x, gridDim.x);
 }
 
+// Scatter product straight from the event vector, for matrices of few rows: y += sum of the rows whose event is set.
+//
+// A call on a small network is launch latency and a chain of dependent loads (event -> row pointers -> entries ->
+// reductions).  The spike list puts two more links and a kernel boundary into it (4000 rows: scan 3.4 us, then scatter 4.0);
+// here the only launch in front is the zero-fill of y, which this one overlaps.  A warp takes one piece (pieces_per_row) of
+// up to 32 rows, one event per lane.  The rows of a group lie n_groups apart, so that a run of neighbouring neurons that
+// fire together is spread over the warps.  From DIRECT_ROWS rows on the silent rows cost more than the list.
+constexpr uint32_t DIRECT_ROWS = 65536;
+
+template<typename T, typename E, bool HOMO, bool VEC>
+__global__ void __launch_bounds__(ROW_THREADS)
+event_scatter_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
+                     const E *__restrict__ events, const uint32_t n_row, const uint32_t n_groups, T *__restrict__ y) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t nse = indptr[n_row], S = pieces_per_row(nse, n_row);
+    const T homo_w = HOMO ? data[0] : T(0);
+    const uint32_t n_items = n_groups * S, n_warps = gridDim.x * ROW_WARPS;
+    for (uint32_t item = blockIdx.x * ROW_WARPS + (threadIdx.x >> 5); item < n_items; item += n_warps) {
+        const uint32_t group = item / S, h = item % S;
+        const uint64_t row = group + static_cast<uint64_t>(lane) * n_groups;
+        uint32_t a = 0, b = 0;
+        if (row < n_row && is_event(events[row])) {
+            const uint32_t start = indptr[row], end = indptr[row + 1];
+            a = piece_cut(start, end, h, S);
+            b = piece_cut(start, end, h + 1, S);
+        }
+        uint32_t active = __ballot_sync(FULL_MASK, a < b);
+        if (active) pdl_wait();                            // y is zero
+        for (; active; active &= active - 1u) {
+            const int l = __ffs(active) - 1;
+            scatter_span<T, HOMO, false, VEC, false>(indices, data, homo_w, T(1), __shfl_sync(FULL_MASK, a, l),
+                                                     __shfl_sync(FULL_MASK, b, l), nse, y, lane);
+        }
+    }
+}
+
+template<typename T>
+__global__ void __launch_bounds__(ROW_THREADS) zero_kernel(T *__restrict__ y, const uint32_t n) {
+    pdl_launch_dependents();
+    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * ROW_THREADS + threadIdx.x; i < n; i += gridDim.x * ROW_THREADS) y[i] = T(0);
+}
+
 }  // namespace
 }  // namespace bpl
 
