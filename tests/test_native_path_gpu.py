@@ -123,3 +123,25 @@ def test_event_gather_over_bits(cuda, n_row, n_col, mean, homo, dtype, bool_even
   else:
     tol = 1e-5 if dtype == np.float32 else 1e-12
     np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(mean))
+
+
+@pytest.mark.parametrize('dtype,bool_events', [(np.float32, True), (np.float32, False), (np.float64, True)])
+@pytest.mark.parametrize('homo', [False, True])
+# few columns (sums in shared memory); few rows (straight from the events): one, a group more than the warps, long pieces
+@pytest.mark.parametrize('n_row,n_col,mean', [(90_000, 2001, 250), (300_000, 701, 60), (1, 50, 20), (4737, 3000, 8), (65_536, 5000, 7),
+                                              (700, 40_000, 3000)])
+def test_event_scatter(cuda, n_row, n_col, mean, homo, dtype, bool_events):
+  rng = np.random.default_rng(37)
+  lens = rng.poisson(mean, n_row)
+  lens[n_row // 2:n_row // 2 + 3] = 0
+  data, indices, indptr, rng = cases.ragged_csr(lens, n_col, 41, dtype=dtype)
+  data = data[:1] if homo else data
+  events = rng.random(n_row) < 0.1
+  events[-1] = True
+  events = events if bool_events else (events * 2.5).astype(dtype)
+  d = [torch.as_tensor(a).to(cuda) for a in (data, indices, indptr, events)]
+  for ev, host in ((d[3], events), (torch.zeros_like(d[3]), np.zeros_like(events))):
+    got = bpl.event_csr_matvec(d[0], d[1], d[2], ev, shape=(n_row, n_col), transpose=True).cpu().numpy()
+    want = cpu.event_csr_matvec(data, indices, indptr, host, shape=(n_row, n_col), transpose=True)
+    tol = 1e-5 if dtype == np.float32 else 1e-12
+    np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(0.1 * indices.size / n_col + 1))
