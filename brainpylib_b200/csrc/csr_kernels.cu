@@ -239,13 +239,13 @@ void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaq
             set_status(BPL_ERR_ARGUMENT, "event_csr_matvec(transpose=True) needs a workspace buffer");
             return;
         }
-        if (n_row <= DIRECT_ROWS) {
-            const uint32_t sms = static_cast<uint32_t>(sm_count());
+        const uint32_t sms = static_cast<uint32_t>(sm_count());
+        const uint32_t warps = 8u * sms * ROW_WARPS;                               // resident, one group each
+        if (n_row <= DIRECT_ROWS && n_row <= 32u * warps) {
             const uint32_t zero_grid = static_cast<uint32_t>(
                 min((static_cast<uint64_t>(n_col) + 4 * ROW_THREADS - 1) / (4 * ROW_THREADS), static_cast<uint64_t>(8 * sms)));
             zero_kernel<T><<<zero_grid, ROW_THREADS, 0, stream>>>(y, n_col);
             if (!launch_ok() || n_row == 0) return;
-            const uint32_t warps = 4u * sms * ROW_WARPS;                           // resident, one group each
             const uint32_t per_group = (n_row + warps - 1) / warps, n_groups = (n_row + per_group - 1) / per_group;
             const dim3 grid((min(n_groups * 4u, warps) + ROW_WARPS - 1) / ROW_WARPS);   // (long rows are cut into pieces)
             if (profile_before()) cudaEventRecord(profile_before(), stream);

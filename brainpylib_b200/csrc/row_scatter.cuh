@@ -194,8 +194,10 @@ row_scatter_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restr
 // reductions).  The spike list puts two more links and a kernel boundary into it (4000 rows: scan 3.4 us, then scatter 4.0);
 // here the only launch in front is the zero-fill of y, which this one overlaps.  A warp takes one piece (pieces_per_row) of
 // up to 32 rows, one event per lane.  The rows of a group lie n_groups apart, so that a run of neighbouring neurons that
-// fire together is spread over the warps.  From DIRECT_ROWS rows on the silent rows cost more than the list.
-constexpr uint32_t DIRECT_ROWS = 65536;
+// fire together is spread over the warps.  Device time per call with the list and without: 4000 rows 6.4 / 3.2 us, 60,000
+// rows 7.2 / 5.6 (1 % active) and 15.5 / 13.4 (10 %), 200,000 rows 11.6 / 10.8.  DIRECT_ROWS: the warps of 148 SMs, 32 rows
+// each, hold a few more.
+constexpr uint32_t DIRECT_ROWS = 262144;
 
 template<typename T, typename E, bool HOMO, bool VEC>
 __global__ void __launch_bounds__(ROW_THREADS)
