@@ -220,6 +220,31 @@ void event_gather(cudaStream_t stream, const uint32_t *indices, const uint32_t *
     launch_ok();
 }
 
+inline uint32_t direct_warps() { return 8u * static_cast<uint32_t>(sm_count()) * ROW_WARPS; }    // resident, one group each
+inline bool direct_rows(const uint32_t n_row) { return n_row <= DIRECT_ROWS && n_row <= 32u * direct_warps(); }
+
+// y = A^T events without a list; false where there are too many rows
+template<typename T, typename E, bool HOMO>
+bool event_scatter_direct(cudaStream_t stream, const uint32_t *indices, const uint32_t *indptr, const T *data, const E *events, T *y,
+                          const uint32_t n_row, const uint32_t n_col) {
+    if (!direct_rows(n_row)) return false;
+    if (n_col == 0) return true;
+    const uint32_t sms = static_cast<uint32_t>(sm_count()), warps = direct_warps();
+    const uint32_t zero_grid = static_cast<uint32_t>(
+        min((static_cast<uint64_t>(n_col) + 4 * ROW_THREADS - 1) / (4 * ROW_THREADS), static_cast<uint64_t>(8 * sms)));
+    zero_kernel<T><<<zero_grid, ROW_THREADS, 0, stream>>>(y, n_col);
+    if (!launch_ok() || n_row == 0) return true;
+    const uint32_t per_group = (n_row + warps - 1) / warps, n_groups = (n_row + per_group - 1) / per_group;
+    const dim3 grid((min(n_groups * 4u, warps) + ROW_WARPS - 1) / ROW_WARPS);   // (long rows are cut into pieces)
+    if (profile_before()) cudaEventRecord(profile_before(), stream);
+    const bool vec = aligned16(indices) && (HOMO || aligned16(data));
+    const cudaError_t e = launch_dependent(vec ? event_scatter_kernel<T, E, HOMO, true> : event_scatter_kernel<T, E, HOMO, false>,
+                                           grid, dim3(ROW_THREADS), 0, stream, indices, indptr, data, events, n_row, n_groups, y);
+    if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+    if (profile_after()) cudaEventRecord(profile_after(), stream);
+    return true;
+}
+
 template<typename T, typename E, bool HOMO>
 void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaque, size_t opaque_len) {
     const TwoUintOneBoolDescriptor *d = unpack<TwoUintOneBoolDescriptor>(opaque, opaque_len);
@@ -239,22 +264,7 @@ void event_csr_matvec_impl(cudaStream_t stream, void **buffers, const char *opaq
             set_status(BPL_ERR_ARGUMENT, "event_csr_matvec(transpose=True) needs a workspace buffer");
             return;
         }
-        const uint32_t sms = static_cast<uint32_t>(sm_count());
-        const uint32_t warps = 8u * sms * ROW_WARPS;                               // resident, one group each
-        if (n_row <= DIRECT_ROWS && n_row <= 32u * warps) {
-            const uint32_t zero_grid = static_cast<uint32_t>(
-                min((static_cast<uint64_t>(n_col) + 4 * ROW_THREADS - 1) / (4 * ROW_THREADS), static_cast<uint64_t>(8 * sms)));
-            zero_kernel<T><<<zero_grid, ROW_THREADS, 0, stream>>>(y, n_col);
-            if (!launch_ok() || n_row == 0) return;
-            const uint32_t per_group = (n_row + warps - 1) / warps, n_groups = (n_row + per_group - 1) / per_group;
-            const dim3 grid((min(n_groups * 4u, warps) + ROW_WARPS - 1) / ROW_WARPS);   // (long rows are cut into pieces)
-            if (profile_before()) cudaEventRecord(profile_before(), stream);
-            const cudaError_t e = launch_dependent(vec ? event_scatter_kernel<T, E, HOMO, true> : event_scatter_kernel<T, E, HOMO, false>,
-                                                   grid, dim3(ROW_THREADS), 0, stream, indices, indptr, data, events, n_row, n_groups, y);
-            if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
-            if (profile_after()) cudaEventRecord(profile_after(), stream);
-            return;
-        }
+        if (event_scatter_direct<T, E, HOMO>(stream, indices, indptr, data, events, y, n_row, n_col)) return;
         uint32_t *counts = ws, *ids = ws + MAX_CHUNKS;
         const ScanPlan p = plan_scan(n_row);
         const uint64_t zero_blocks = (static_cast<uint64_t>(n_col) + SCAN_TILE - 1) / SCAN_TILE;
@@ -389,12 +399,15 @@ list_scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t 
 
 // How many rows are active is not known here; the rule supposes 1 %, a usual rate.  In clocks of one SM: a reduction takes
 // 1.85, and more the fewer columns share them; the sums take 0.4 each to clear and to add up, and 3000 in all.
+inline bool list_shared_pays(uint32_t n_row, uint32_t n_col, uint32_t nse, bool homo, size_t elem) {
+    const double active = 0.01 * nse / sm_count();
+    return !homo && n_row != 0 && n_col != 0 && n_col <= LIST_SHARED_SMEM / elem &&
+           active * (1.5 + 25000.0 / n_col) >= 3000 + 0.4 * (elem / 4) * n_col;
+}
+
 template<typename T, typename E>
 bool list_scatter_shared(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *ws, T *y) {
-    const double active = 0.01 * m.nse / sm_count();
-    if (m.homo || m.n_row == 0 || m.n_col == 0 || m.n_col > LIST_SHARED_SMEM / sizeof(T) ||
-        active * (1.5 + 25000.0 / m.n_col) < 3000 + 0.4 * (sizeof(T) / 4) * m.n_col)
-        return false;
+    if (!list_shared_pays(m.n_row, m.n_col, m.nse, m.homo, sizeof(T))) return false;
     const bool vec = aligned16(m.indices) && aligned16(m.data);
     constexpr auto wide = list_scatter_shared_kernel<T, true>, narrow = list_scatter_shared_kernel<T, false>;
     if (!(vec ? allow_shared<wide>(LIST_SHARED_SMEM) : allow_shared<narrow>(LIST_SHARED_SMEM))) return launch_ok(), true;
@@ -421,7 +434,9 @@ void event_csr_known(cudaStream_t stream, void **buffers, uint32_t n_row, uint32
         return;
     }
     if (list_scatter_shared<T, E>(stream, m, static_cast<const E *>(buffers[3]), static_cast<uint32_t *>(buffers[5]),
-                                        static_cast<T *>(buffers[4])))
+                                        static_cast<T *>(buffers[4])) ||
+        event_scatter_direct<T, E, HOMO>(stream, m.indices, m.indptr, m.data, static_cast<const E *>(buffers[3]),
+                                         static_cast<T *>(buffers[4]), n_row, n_col))
         return;
     TwoUintOneBoolDescriptor d;
     __builtin_memset(&d, 0, sizeof(d));
@@ -479,6 +494,11 @@ void bpl_csr_matvec(bpl_stream_t stream, const void *data, const void *indices, 
                                                                     homo != 0, transpose != 0);
 }
 
+size_t bpl_event_csr_matvec_workspace(uint32_t n_row, uint32_t n_col, uint32_t nse, int homo, int is_double, int transpose) {
+    if (!transpose) return (static_cast<size_t>(n_col) + 31) / 32 * 4;
+    const bool list = list_shared_pays(n_row, n_col, nse, homo != 0, is_double ? 8 : 4) || !direct_rows(n_row);
+    return list ? scatter_workspace_bytes(n_row) : 0;
+}
 void bpl_event_csr_matvec(bpl_stream_t stream, void **buffers, uint32_t n_row, uint32_t n_col, uint32_t nse, int homo,
                           int is_double, int bool_events, int transpose) {
     using Call = void (*)(cudaStream_t, void **, uint32_t, uint32_t, uint32_t, bool);

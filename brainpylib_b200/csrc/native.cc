@@ -158,7 +158,9 @@ Tensor event_csr_product(const Tensor &data, const Tensor &indices, const Tensor
                          int64_t n_row, int64_t n_col, bool transpose) {
     OnDevice on(data);
     Tensor out = new_tensor({transpose ? n_col : n_row}, data.scalar_type(), data.device());
-    Scratch ws(transpose ? bpl_event_csr_workspace_bytes(static_cast<uint32_t>(n_row), 1) : (n_col + 31) / 32 * 4, on.stream);
+    Scratch ws(bpl_event_csr_matvec_workspace(static_cast<uint32_t>(n_row), static_cast<uint32_t>(n_col),
+                                              static_cast<uint32_t>(indices.size(0)), data.size(0) == 1, is_double(data), transpose),
+               on.stream);
     void *buffers[6] = {ptr(data), ptr(indices), ptr(indptr), ptr(events), ptr(out), ws.ptr};
     bpl_event_csr_matvec(on.stream, buffers, static_cast<uint32_t>(n_row), static_cast<uint32_t>(n_col),
                          static_cast<uint32_t>(indices.size(0)), data.size(0) == 1, is_double(data),

@@ -278,8 +278,8 @@ BPL_FOR_EACH_TARGET(BPL_DECLARE_ONE)
  * (brainpylib/_src/sparse_ops/cusparse_matvec.py:292-304).
  * bpl_csr_matvec: csr_matvec_{homo,heter}_vector_* / csr_matvec_transpose_* without descriptor, for callers that know the
  * number of stored entries nse on the host (it selects the kernel).
- * bpl_event_csr_matvec: event_csr_matvec_* in the same way (buffers as there; the workspace holds n_col bits, in whole
- * words, when not transpose).
+ * bpl_event_csr_matvec: event_csr_matvec_* in the same way (buffers as there, with a workspace of
+ * bpl_event_csr_matvec_workspace bytes, which may be 0).
  * bpl_jit_matvec: gpu_matvec{,_atomic}_prob_*_v2 (events = 0) or gpu_event_matvec{,_atomic}_prob_*_v2 without descriptor
  * and with a factor: in_type 0 bool, 1 float32, 2 float64 (out: that type, float32 for bool); kind 0 homogeneous,
  * 1 uniform, 2 normal; rows: one stream per output.  scale multiplies, for homogeneous weights, the sums (rows) or the
@@ -288,6 +288,7 @@ size_t bpl_event_csr_workspace_bytes(uint32_t n_row, int transpose);
 void bpl_jit_matvec(bpl_stream_t stream, const void *in, void *out, int in_type, int events, int kind, int rows,
                     uint32_t n_row, uint32_t n_col, uint32_t seed, float log_p, float w1, float w2, double scale);
 size_t bpl_nonzero_workspace_bytes(uint32_t batch_size);
+size_t bpl_event_csr_matvec_workspace(uint32_t n_row, uint32_t n_col, uint32_t nse, int homo, int is_double, int transpose);
 void bpl_event_csr_matvec(bpl_stream_t stream, void **buffers, uint32_t n_row, uint32_t n_col, uint32_t nse, int homo,
                           int is_double, int bool_events, int transpose);
 void bpl_csr_outer(bpl_stream_t stream, const void *row_vector, const void *col_vector, const void *indices,
