@@ -127,8 +127,10 @@ def test_event_gather_over_bits(cuda, n_row, n_col, mean, homo, dtype, bool_even
 
 @pytest.mark.parametrize('dtype,bool_events', [(np.float32, True), (np.float32, False), (np.float64, True)])
 @pytest.mark.parametrize('homo', [False, True])
-# few columns (sums in shared memory); few rows (straight from the events): one, a group more than the warps, long pieces
-@pytest.mark.parametrize('n_row,n_col,mean', [(90_000, 2001, 250), (300_000, 701, 60), (1, 50, 20), (9473, 3000, 8), (262_144, 5000, 7),
+# small (one launch, columns owned by blocks): the most rows, long rows, many columns; few columns (sums in shared memory);
+# few rows (straight from the events): one, a group more than the warps, long pieces
+@pytest.mark.parametrize('n_row,n_col,mean', [(90_000, 2001, 250), (300_000, 701, 60), (1, 50, 20), (8192, 129, 9),
+                                              (40, 700, 2500), (300, 70_001, 31), (9473, 3000, 8), (262_144, 5000, 7),
                                               (262_145, 5000, 7),
                                               (700, 40_000, 3000)])
 def test_event_scatter(cuda, n_row, n_col, mean, homo, dtype, bool_events):
