@@ -212,19 +212,23 @@ struct CsrFn : public torch::autograd::Function<CsrFn> {
     static variable_list backward(AutogradContext *ctx, variable_list grads);
 };
 
+Tensor csr_outer(const Tensor &row_vector, const Tensor &col_vector, const Tensor &indices, const Tensor &indptr) {
+    OnDevice on(indices);
+    Tensor out = new_tensor({indices.size(0)}, row_vector.scalar_type(), row_vector.device());
+    bpl_csr_outer(on.stream, ptr(row_vector), ptr(col_vector), ptr(indices), ptr(indptr), ptr(out),
+                  static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(col_vector.size(0)),
+                  static_cast<uint32_t>(indices.size(0)), is_double(row_vector) ? 1 : 0);
+    check_status();
+    return out;
+}
+
 // g[e] = row_vector[row(e)] * col_vector[indices[e]] over the stored entries: the gradient of a product with respect to
 // the weights.  Bilinear, and its own derivatives are products with the matrix of cotangents.
 struct CsrOuterFn : public torch::autograd::Function<CsrOuterFn> {
     static Tensor forward(AutogradContext *ctx, const Tensor &row_vector, const Tensor &col_vector, const Tensor &indices,
                           const Tensor &indptr) {
         ctx->save_for_backward({row_vector, col_vector, indices, indptr});
-        OnDevice on(indices);
-        Tensor out = new_tensor({indices.size(0)}, row_vector.scalar_type(), row_vector.device());
-        bpl_csr_outer(on.stream, ptr(row_vector), ptr(col_vector), ptr(indices), ptr(indptr), ptr(out),
-                      static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(col_vector.size(0)),
-                      static_cast<uint32_t>(indices.size(0)), is_double(row_vector) ? 1 : 0);
-        check_status();
-        return out;
+        return csr_outer(row_vector, col_vector, indices, indptr);
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         const auto saved = ctx->get_saved_variables();
@@ -243,8 +247,15 @@ struct CsrOuterFn : public torch::autograd::Function<CsrOuterFn> {
     }
 };
 
+// In a backward pass without create_graph there is nothing to record: the kernels alone.
+Tensor csr_any(const Tensor &data, const Tensor &indices, const Tensor &indptr, const Tensor &x, int64_t n_row, int64_t n_col, bool t) {
+    return at::GradMode::is_enabled() ? CsrFn::apply(data, indices, indptr, x, n_row, n_col, t)
+                                      : csr_product(data, indices, indptr, x, n_row, n_col, t);
+}
+
 Tensor outer_of(const Tensor &indices, const Tensor &indptr, const Tensor &x, const Tensor &ct, bool transpose) {
-    return transpose ? CsrOuterFn::apply(x, ct, indices, indptr) : CsrOuterFn::apply(ct, x, indices, indptr);
+    const Tensor &row = transpose ? x : ct, &col = transpose ? ct : x;
+    return at::GradMode::is_enabled() ? CsrOuterFn::apply(row, col, indices, indptr) : csr_outer(row, col, indices, indptr);
 }
 
 variable_list CsrFn::backward(AutogradContext *ctx, variable_list grads) {
@@ -266,7 +277,7 @@ variable_list CsrFn::backward(AutogradContext *ctx, variable_list grads) {
                 g_data = outer_of(indices, indptr, x, ct, t);
             }
         }
-        if (ctx->needs_input_grad(3)) g_x = CsrFn::apply(data, indices, indptr, ct, n_row, n_col, !t);
+        if (ctx->needs_input_grad(3)) g_x = csr_any(data, indices, indptr, ct, n_row, n_col, !t);
     }
     return {g_data, Tensor(), Tensor(), g_x, Tensor(), Tensor(), Tensor()};
 }
@@ -299,7 +310,7 @@ struct EventCsrFn : public torch::autograd::Function<EventCsrFn> {
                     g_data = outer_of(indices, indptr, events.to(data.scalar_type()), ct, t);
                 }
             }
-            if (ctx->needs_input_grad(3)) g_events = CsrFn::apply(data, indices, indptr, ct, n_row, n_col, !t);
+            if (ctx->needs_input_grad(3)) g_events = csr_any(data, indices, indptr, ct, n_row, n_col, !t);
         }
         return {g_data, Tensor(), Tensor(), g_events, Tensor(), Tensor(), Tensor()};
     }
@@ -507,7 +518,7 @@ struct JitFn : public torch::autograd::Function<JitFn> {
         const JitArgs t = a.transposed();
         const Tensor ct = grads[0].contiguous();
         Tensor g;
-        if (plain_cotangent(ct)) g = JitFn::apply(ct, t, false);
+        if (plain_cotangent(ct)) g = at::GradMode::is_enabled() ? JitFn::apply(ct, t, false) : jit_product(ct, t, false);
         else g = python_jit_rule(ct, t);
         return {g, Tensor(), Tensor()};
     }
@@ -721,12 +732,7 @@ PyObject *py_csr_outer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     for (int i = 0; i < 4; ++i) NONE_UNLESS(THPVariable_Check(args[i]));
     const Tensor row = THPVariable_Unpack(args[0]).contiguous(), col = THPVariable_Unpack(args[1]).contiguous();
     const Tensor &indices = THPVariable_Unpack(args[2]), &indptr = THPVariable_Unpack(args[3]);
-    OnDevice on(indices);
-    Tensor out = new_tensor({indices.size(0)}, row.scalar_type(), row.device());
-    bpl_csr_outer(on.stream, ptr(row), ptr(col), ptr(indices), ptr(indptr), ptr(out),
-                  static_cast<uint32_t>(indptr.size(0) - 1), static_cast<uint32_t>(col.size(0)), static_cast<uint32_t>(indices.size(0)),
-                  is_double(row) ? 1 : 0);
-    check_status();
+    Tensor out = csr_outer(row, col, indices, indptr);
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
 }
