@@ -42,7 +42,7 @@ struct GapParams {
 // `lo` and `hi` enclose it with 1.1 times that bound.  Adding 2^23 with rounding up leaves 2^23 + ceil() in the mantissa;
 // where both ends agree that is the reference's gap.  Else (1 draw in 700 at a mean gap of 1000) the reference's own
 // logarithm decides, and where that lies too close to an integer, the reference's own expression.
-// `n`: length of a stream's range; a batch may run at most 5 gaps behind it.
+// `n`: length of a stream's range; a batch may run at most 8 gaps behind it (below 2^25 positions).
 inline GapParams gap_params(double log_p, uint32_t n) {
     GapParams g;
     g.one = 1u;
@@ -197,6 +197,54 @@ struct Batch {
                 w[j + 1] = (T) (v.y * w2 + w1);
             }
         }
+    }
+};
+
+// One stream walked by GROUP lanes together, GROUP connections per step, one each: where there are too few streams to fill
+// the SMs, the walk of one is a chain of some 1000 clocks per four connections (draws, logarithms, weights, all by one
+// lane).  Here every lane of the group runs the generator (the same instructions), and each converts its own connection;
+// the positions are a prefix sum over the group.  Four times the instructions per connection, a third of the time per
+// stream while issue slots are idle.  For `quick` parameters; all 32 lanes of the warp must call draw together.
+constexpr int GROUP = 8;
+
+template<int KIND>
+struct GroupStep {
+    uint32_t pos;              // of this lane's connection
+    uint32_t r0, r1;           // raw draws of its weight (normal: of its pair)
+
+    __device__ __forceinline__ void draw(Xorwow &s, uint32_t &at, const uint32_t n, const uint32_t sub, const GapParams &g) {
+        uint32_t x = 0;
+        r0 = r1 = 0;
+#pragma unroll
+        for (int j = 0; j < GROUP; ++j) {
+            const uint32_t d = s.next(g);
+            if (sub == j) x = d;
+            if (KIND == W_UNIFORM) {
+                const uint32_t r = s.next(g);
+                if (sub == j) r0 = r;
+            }
+            if (KIND == W_NORMAL && (j & 1) == 0) {
+                const uint32_t a = s.next(g), b = s.next(g);
+                if ((sub & ~1u) == j) {
+                    r0 = a;
+                    r1 = b;
+                }
+            }
+        }
+        uint32_t sum = static_cast<uint32_t>(gap_of(x, g));
+#pragma unroll
+        for (int o = 1; o < GROUP; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, sum, o, GROUP);
+            if (sub >= static_cast<uint32_t>(o)) sum += t;
+        }
+        pos = at + sum;
+        at = min(__shfl_sync(0xffffffffu, pos, GROUP - 1, GROUP), n);     // (a stream that is through stays at its end)
+    }
+    template<typename T>
+    __device__ __forceinline__ T weight(const uint32_t sub, const double w1, const double w2) const {
+        if (KIND == W_UNIFORM) return uniform_weight<T>(r0, w1, w2);
+        if (KIND == W_NORMAL) return normal_weight<T>(r0, r1, sub & 1u, w1, w2);
+        return T(1);
     }
 };
 

@@ -225,6 +225,57 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
     }
 }
 
+// Few rows (jit_stream.cuh, GroupStep): eight lanes per row, the input gathered from global memory while the next step is
+// drawn.  The sum takes the connections in stream order, as one lane would.  3000 rows of 200000 columns, p = 0.002, 3 %
+// of the events set: uniform 49 -> 35 us, normal 55 -> 41; dense, 1500 rows of 20000, p = 0.01: 19 -> 10.5, 21 -> 14.5,
+// 27 -> 18 (homogeneous, uniform, normal).
+constexpr int GROUP_THREADS = 128;
+
+template<typename T, typename E, int KIND, bool EVENT>
+__global__ void __launch_bounds__(GROUP_THREADS)
+jit_rows_group_kernel(const E *__restrict__ in, const unsigned int seed, const GapParams gp, const double w1, const double w2,
+                      const unsigned int num_row, const unsigned int num_col, const T scale, T *__restrict__ out) {
+    const unsigned int lane = threadIdx.x & 31u, sub = lane & (GROUP - 1u);
+    const unsigned int row = blockIdx.x * (GROUP_THREADS / GROUP) + threadIdx.x / GROUP;
+    const bool live = row < num_row;
+    if (!__any_sync(FULL_MASK, live)) return;
+    Xorwow s;
+    s.seed(seed + row);
+    GroupStep<KIND> now, next;
+    unsigned int at = live ? 0u : num_col;                 // (a group without a row is at the end from the start)
+    T sum = 0;
+    now.draw(s, at, num_col, sub, gp);
+    bool more = true;
+    while (more) {
+        E v = E(0);
+        const bool inside = live && now.pos < num_col;
+        if (inside) v = in[now.pos];
+        more = __any_sync(FULL_MASK, at < num_col);
+        if (more) next.draw(s, at, num_col, sub, gp);
+        // (rounded as by one lane: a product and its sum in one operation)
+        const bool has = inside && (!EVENT || is_event(v));
+        const T x = has && !EVENT ? static_cast<T>(v) : T(0);
+        const T w = has && KIND != W_HOMO ? now.template weight<T>(sub, w1, w2) : T(1);
+        unsigned int mine = (__ballot_sync(FULL_MASK, has) >> (lane & ~(GROUP - 1u))) & ((1u << GROUP) - 1u);
+        if (EVENT) {
+            while (__any_sync(FULL_MASK, mine != 0u)) {
+                const T t = __shfl_sync(FULL_MASK, w, mine ? __ffs(mine) - 1 : 0, GROUP);
+                if (mine) sum += t;
+                mine &= mine - 1u;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < GROUP; ++j) {
+                const T t = __shfl_sync(FULL_MASK, x, j, GROUP);
+                const T u = KIND == W_HOMO ? T(1) : __shfl_sync(FULL_MASK, w, j, GROUP);
+                if ((mine >> j) & 1u) sum += t * u;
+            }
+        }
+        now = next;
+    }
+    if (live && sub == 0) out[row] = KIND == W_HOMO ? sum * scale : sum;
+}
+
 // ------------------------------------------------------------------------------------------
 // Column-parallel (outdim_parallel = False): one thread walks the stream of one input column and scatters.
 // ------------------------------------------------------------------------------------------
@@ -280,6 +331,26 @@ jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const Gap
             }
         }
     }
+}
+
+// Few columns: eight lanes each.  30000 rows, 3000 columns, p = 0.01: uniform 32 -> 24 us, normal 46 -> 26.
+template<typename T, int KIND>
+__global__ void __launch_bounds__(GROUP_THREADS)
+jit_cols_group_kernel(const T *__restrict__ vector, const unsigned int seed, const GapParams gp, const double w1, const double w2,
+                      const unsigned int num_row, const unsigned int num_col, const T scale, T *__restrict__ out) {
+    const unsigned int sub = threadIdx.x & (GROUP - 1u);
+    const unsigned int col = blockIdx.x * (GROUP_THREADS / GROUP) + threadIdx.x / GROUP;
+    const bool live = col < num_col;
+    T v = live ? vector[col] : T(0);
+    if (KIND == W_HOMO) v = v * scale;
+    Xorwow s;
+    s.seed(seed + col);
+    GroupStep<KIND> step;
+    unsigned int at = live ? 0u : num_row;
+    do {
+        step.draw(s, at, num_row, sub, gp);
+        if (live && step.pos < num_row) red_add(out + step.pos, KIND == W_HOMO ? v : v * step.template weight<T>(sub, w1, w2));
+    } while (__any_sync(FULL_MASK, at < num_row));
 }
 
 // Event input: lib/gpu_jitconn_event_matvec_atomic.cu:30-58, :88-117, :150-178.  There every column walks its stream and
@@ -488,6 +559,14 @@ inline unsigned int tile_length(unsigned int n, size_t elem) {
     return blocks_for(blocks_for(n, tiles), 32) * 32u;
 }
 
+// Streams per SM up to which eight lanes walk one: beyond, the extra instructions no longer fit the idle issue slots.  One
+// lane per row takes dense homogeneous and uniform connections fast enough that the line lies lower (3000 rows, 100000
+// columns, p = 0.1, uniform: 441 us by one lane, 497 by eight; normal: 922 and 652), and an event bit of a homogeneous one
+// always (2300 rows, 20000 columns, p = 0.2: 133 and 172).
+constexpr int GROUP_COLS = 32;
+template<int KIND, bool EVENT>
+constexpr int GROUP_ROWS = KIND == W_NORMAL ? 40 : EVENT ? (KIND == W_UNIFORM ? 40 : 0) : 16;
+
 // Rules in clocks of one SM.  A gather through L1 takes one clock per connection.  Filling shared memory reads the whole
 // input per block, at about 56 bytes per clock, after a start of some 2000 clocks; a vector in several tiles is read
 // again for every wave of streams.
@@ -497,6 +576,14 @@ void jit_rows(const JitCall<T, E> &c) {
     const GapParams gp = gap_params(a.log_p, a.n_col);
     const double gathers = static_cast<double>(a.n_row) * a.n_col * -std::expm1(a.log_p) / sm_count();
     constexpr bool TRUTH_ONLY = EVENT && (KIND != W_HOMO || sizeof(E) == 1);
+    if constexpr (GROUP_ROWS<KIND, EVENT> > 0) {
+        if (gp.quick && a.n_row <= static_cast<unsigned int>(GROUP_ROWS<KIND, EVENT> * sm_count())) {
+            jit_rows_group_kernel<T, E, KIND, EVENT><<<blocks_for(a.n_row, GROUP_THREADS / GROUP), GROUP_THREADS, 0, c.stream>>>(
+                c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, c.scale, c.out);
+            launch_ok();
+            return;
+        }
+    }
     WalkGrid g(a.n_row, 512);
     // (n_col + 5 * 23 mean gaps stay below 2^24)
     if (gp.quick && TRUTH_ONLY && a.n_col <= MASK_MAX_BITS && -1.0 / a.log_p < 130000.0) {
@@ -563,6 +650,12 @@ void jit_cols(const JitCall<T, T> &c) {
     if (a.n_col == 0) return;
     const GapParams gp = gap_params(a.log_p, a.n_row);
     const double additions = static_cast<double>(a.n_row) * a.n_col * -std::expm1(a.log_p) / sm_count();
+    if (gp.quick && a.n_col <= static_cast<unsigned int>(GROUP_COLS * sm_count())) {
+        jit_cols_group_kernel<T, KIND><<<blocks_for(a.n_col, GROUP_THREADS / GROUP), GROUP_THREADS, 0, c.stream>>>(
+            c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, c.scale, c.out);
+        launch_ok();
+        return;
+    }
     const WalkGrid g(a.n_col, 512);
     if (gp.quick && 1.8 * additions > 0.3 * (sizeof(T) / 4) * additions + 0.8 * (sizeof(T) / 4) * a.n_row * g.waves + 5000) {
         const unsigned int len = tile_length(a.n_row, sizeof(T));

@@ -62,6 +62,27 @@ def test_dense_columns_against_the_oracle(cuda, kind):
 
 
 @pytest.mark.parametrize('kind', sorted(KINDS))
+# eight lanes per stream and one, on both sides of the lines between them; a single stream; a last block of one stream
+@pytest.mark.parametrize('streams,length,prob', [(1, 30_001, 0.01), (17, 3, 0.5), (2369, 901, 0.05), (4737, 500, 0.02),
+                                                 (5921, 500, 0.02)])
+def test_few_and_more_streams(cuda, streams, length, prob, kind):
+  rng = np.random.default_rng(6)
+  x = rng.standard_normal(length).astype(np.float32)
+  _compare(cuda, x, kind, prob, (streams, length), True, False)
+  _compare(cuda, x > 1., kind, prob, (streams, length), True, True)
+  x = rng.standard_normal(streams).astype(np.float32)
+  _compare(cuda, x, kind, prob, (length, streams), False, False)
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
+  test_dense_columns(cuda, (29_057, 6000), 0.01, dtype, kind)
+  x = np.random.default_rng(1).standard_normal(58_113).astype(str(dtype)[6:])
+  _compare(cuda, x, kind, 0.002, (6001, 58_113), True, False)
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [np.bool_, np.float32])
 # every input fires (full queues), ragged last word, more rows than threads, a mask of the largest size
 @pytest.mark.parametrize('shape,prob,rate', [((5000, 1000), 0.1, 1.0), ((2111, 4097), 0.2, 0.1), ((160000, 333), 0.1, 0.02),
