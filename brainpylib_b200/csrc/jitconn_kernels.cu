@@ -335,16 +335,12 @@ jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const Gap
 
 // Few columns: eight lanes each.  30000 rows, 3000 columns, p = 0.01: uniform 32 -> 24 us, normal 46 -> 26.
 template<typename T, int KIND>
-__global__ void __launch_bounds__(GROUP_THREADS)
-jit_cols_group_kernel(const T *__restrict__ vector, const unsigned int seed, const GapParams gp, const double w1, const double w2,
-                      const unsigned int num_row, const unsigned int num_col, const T scale, T *__restrict__ out) {
+__device__ __forceinline__ void scatter_group(const unsigned int stream_seed, const bool live, const T v,
+                                              const unsigned int num_row, const GapParams &gp, const double w1,
+                                              const double w2, T *__restrict__ out) {
     const unsigned int sub = threadIdx.x & (GROUP - 1u);
-    const unsigned int col = blockIdx.x * (GROUP_THREADS / GROUP) + threadIdx.x / GROUP;
-    const bool live = col < num_col;
-    T v = live ? vector[col] : T(0);
-    if (KIND == W_HOMO) v = v * scale;
     Xorwow s;
-    s.seed(seed + col);
+    s.seed(stream_seed);
     GroupStep<KIND> step;
     unsigned int at = live ? 0u : num_row;
     do {
@@ -353,18 +349,31 @@ jit_cols_group_kernel(const T *__restrict__ vector, const unsigned int seed, con
     } while (__any_sync(FULL_MASK, at < num_row));
 }
 
+template<typename T, int KIND>
+__global__ void __launch_bounds__(GROUP_THREADS)
+jit_cols_group_kernel(const T *__restrict__ vector, const unsigned int seed, const GapParams gp, const double w1, const double w2,
+                      const unsigned int num_row, const unsigned int num_col, const T scale, T *__restrict__ out) {
+    const unsigned int col = blockIdx.x * (GROUP_THREADS / GROUP) + threadIdx.x / GROUP;
+    const bool live = col < num_col;
+    T v = live ? vector[col] : T(0);
+    if (KIND == W_HOMO) v = v * scale;
+    scatter_group<T, KIND>(seed + col, live, v, num_row, gp, w1, w2, out);
+}
+
 // Event input: lib/gpu_jitconn_event_matvec_atomic.cu:30-58, :88-117, :150-178.  There every column walks its stream and
 // only the atomicAdd is conditional; a silent column contributes nothing and its stream is private, so it is skipped
-// here.  Each block compacts the firing columns of its chunk into shared memory and gives one thread to each of them.  The
+// here.  Each block compacts the firing columns of its chunk into shared memory and gives one thread to each of them, or eight
+// lanes where there are at most `few` (50000 x 50000, p = 0.004, 1 % firing, normal weights: 30 -> 20 us).  The
 // chunk (at most COL_CHUNK) is chosen for four blocks per SM: the walk of a stream is a chain, and a few thousand columns in
 // chunks of 2048 left most SMs without one (5796 columns, 10 % firing: 20 us).
 constexpr int COL_CHUNK = GATHER_THREADS * 8;
+
 
 template<typename T, typename E, int KIND, bool QUICK>
 __global__ void __launch_bounds__(GATHER_THREADS)
 jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, const GapParams gp, const double w1,
                       const double w2, const unsigned int num_row, const unsigned int num_col, const unsigned int chunk,
-                      T *__restrict__ out) {
+                      const unsigned int few, T *__restrict__ out) {
     __shared__ unsigned int active[COL_CHUNK];
     __shared__ unsigned int n_active;
     constexpr int N = Batch<KIND, QUICK>::N;
@@ -378,6 +387,12 @@ jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, con
     }
     __syncthreads();
     const unsigned int n = n_active;
+    if (QUICK && n <= few) {                               // (at most one per group)
+        const unsigned int i = threadIdx.x / GROUP;
+        if (threadIdx.x / 32 * (32 / GROUP) < n)
+            scatter_group<T, KIND>(seed + (i < n ? active[i] : 0u), i < n, T(1), num_row, gp, w1, w2, out);
+        return;
+    }
     for (unsigned int i = threadIdx.x; i < n; i += blockDim.x) {
         Xorwow s;
         s.seed(seed + active[i]);
@@ -564,6 +579,9 @@ inline unsigned int tile_length(unsigned int n, size_t elem) {
 // columns, p = 0.1, uniform: 441 us by one lane, 497 by eight; normal: 922 and 652), and an event bit of a homogeneous one
 // always (2300 rows, 20000 columns, p = 0.2: 133 and 172).
 constexpr int GROUP_COLS = 32;
+// (of firing columns; a block with one more than its share walks all of them by one lane each, beside blocks that do not)
+template<int KIND>
+constexpr unsigned int GROUP_EVENTS = KIND == W_NORMAL ? 24 : 12;
 template<int KIND, bool EVENT>
 constexpr int GROUP_ROWS = KIND == W_NORMAL ? 40 : EVENT ? (KIND == W_UNIFORM ? 40 : 0) : 16;
 
@@ -686,9 +704,11 @@ void jit_cols_event(const JitCall<T, E> &c) {
     if (a.n_col == 0) return;
     const GapParams gp = gap_params(a.log_p, a.n_row);
     const unsigned int chunk = std::min(static_cast<unsigned int>(COL_CHUNK), blocks_for(blocks_for(a.n_col, 4 * sm_count()), 32) * 32u);
+    const unsigned int blocks = blocks_for(a.n_col, chunk);
+    const unsigned int few = std::min(static_cast<unsigned int>(GATHER_THREADS / GROUP),
+                                      GROUP_EVENTS<KIND> * sm_count() / blocks);
     (gp.quick ? jit_cols_event_kernel<T, E, KIND, true> : jit_cols_event_kernel<T, E, KIND, false>)<<<
-        blocks_for(a.n_col, chunk), std::min(static_cast<unsigned int>(GATHER_THREADS), chunk), 0, c.stream>>>(
-        c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk, c.out);
+        blocks, GATHER_THREADS, 0, c.stream>>>(c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk, few, c.out);
     launch_ok();
 }
 

@@ -75,6 +75,14 @@ def test_few_and_more_streams(cuda, streams, length, prob, kind):
 
 
 @pytest.mark.parametrize('kind', sorted(KINDS))
+# firing columns of a block: none or one, about as many as are walked by eight lanes each, all
+@pytest.mark.parametrize('shape,prob,rate', [((900, 33), 0.1, 0.1), ((900, 33), 0.1, 1.0), ((500, 50_000), 0.02, 0.001),
+                                             ((500, 50_000), 0.02, 0.04), ((500, 50_000), 0.02, 0.07)])
+def test_event_columns(cuda, shape, prob, rate, kind):
+  _compare(cuda, np.random.default_rng(7).random(shape[1]) < rate, kind, prob, shape, False, True)
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
   test_dense_columns(cuda, (29_057, 6000), 0.01, dtype, kind)
