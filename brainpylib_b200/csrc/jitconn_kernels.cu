@@ -578,12 +578,15 @@ inline unsigned int tile_length(unsigned int n, size_t elem) {
 // lane per row takes dense homogeneous and uniform connections fast enough that the line lies lower (3000 rows, 100000
 // columns, p = 0.1, uniform: 441 us by one lane, 497 by eight; normal: 922 and 652), and an event bit of a homogeneous one
 // always (2300 rows, 20000 columns, p = 0.2: 133 and 172).
-constexpr int GROUP_COLS = 32;
+template<int KIND, bool EVENT>
+constexpr int GROUP_ROWS = EVENT ? (KIND == W_HOMO ? 0 : 60) : KIND == W_NORMAL ? 40 : 16;
+// Columns: reductions into a short output meet at the same addresses, where sums in shared memory are the better ones sooner
+// (9000 columns, p = 0.1, uniform: 3000 rows 65 us by one lane and 110 by eight, 30000 rows 468 and 357).
+constexpr unsigned int GROUP_LONG = 16384;
+constexpr int GROUP_COLS = 32, GROUP_COLS_LONG = 60;
 // (of firing columns; a block with one more than its share walks all of them by one lane each, beside blocks that do not)
 template<int KIND>
 constexpr unsigned int GROUP_EVENTS = KIND == W_NORMAL ? 24 : 12;
-template<int KIND, bool EVENT>
-constexpr int GROUP_ROWS = KIND == W_NORMAL ? 40 : EVENT ? (KIND == W_UNIFORM ? 40 : 0) : 16;
 
 // Rules in clocks of one SM.  A gather through L1 takes one clock per connection.  Filling shared memory reads the whole
 // input per block, at about 56 bytes per clock, after a start of some 2000 clocks; a vector in several tiles is read
@@ -668,7 +671,7 @@ void jit_cols(const JitCall<T, T> &c) {
     if (a.n_col == 0) return;
     const GapParams gp = gap_params(a.log_p, a.n_row);
     const double additions = static_cast<double>(a.n_row) * a.n_col * -std::expm1(a.log_p) / sm_count();
-    if (gp.quick && a.n_col <= static_cast<unsigned int>(GROUP_COLS * sm_count())) {
+    if (gp.quick && a.n_col <= static_cast<unsigned int>((a.n_row < GROUP_LONG ? GROUP_COLS : GROUP_COLS_LONG) * sm_count())) {
         jit_cols_group_kernel<T, KIND><<<blocks_for(a.n_col, GROUP_THREADS / GROUP), GROUP_THREADS, 0, c.stream>>>(
             c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, c.scale, c.out);
         launch_ok();

@@ -64,7 +64,7 @@ def test_dense_columns_against_the_oracle(cuda, kind):
 @pytest.mark.parametrize('kind', sorted(KINDS))
 # eight lanes per stream and one, on both sides of the lines between them; a single stream; a last block of one stream
 @pytest.mark.parametrize('streams,length,prob', [(1, 30_001, 0.01), (17, 3, 0.5), (2369, 901, 0.05), (4737, 500, 0.02),
-                                                 (5921, 500, 0.02)])
+                                                 (5921, 500, 0.02), (8881, 300, 0.05), (8880, 16_384, 0.001)])
 def test_few_and_more_streams(cuda, streams, length, prob, kind):
   rng = np.random.default_rng(6)
   x = rng.standard_normal(length).astype(np.float32)
@@ -85,7 +85,7 @@ def test_event_columns(cuda, shape, prob, rate, kind):
 @pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
-  test_dense_columns(cuda, (29_057, 6000), 0.01, dtype, kind)
+  test_dense_columns(cuda, (29_057, 8881), 0.01, dtype, kind)
   x = np.random.default_rng(1).standard_normal(58_113).astype(str(dtype)[6:])
   _compare(cuda, x, kind, 0.002, (6001, 58_113), True, False)
 
