@@ -182,9 +182,10 @@ gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     });
 }
 
-// y = A events: the events as one bit each in shared memory.  Homogeneous weights count hits and scale once (equal to the
+// y = A events: the events as one byte each in shared memory, or one bit where they are many.  The walk is bound by
+// instruction issue, and a byte needs no shifts (1e8 entries, rows of 121, 3000 columns: 140 -> 109 us).  Homogeneous weights count hits and scale once (equal to the
 // reference CPU kernel's float64 accumulation, brainpylib/_src/event_ops/event_csr_matvec.py:334-357).
-template<typename T, bool HOMO>
+template<typename T, bool HOMO, bool BYTES>
 struct EventVisit {
     const uint32_t *mask;
     uint32_t lpr;
@@ -196,7 +197,9 @@ struct EventVisit {
         acc = T(0);
         hits = 0;
     }
-    __device__ __forceinline__ uint32_t hit(const uint32_t c) const { return (mask[c >> 5] >> (c & 31u)) & 1u; }
+    __device__ __forceinline__ uint32_t hit(const uint32_t c) const {
+        return BYTES ? reinterpret_cast<const uint8_t *>(mask)[c] : (mask[c >> 5] >> (c & 31u)) & 1u;
+    }
     template<bool FULL>
     __device__ __forceinline__ void quad(uint32_t, const uint32_t (&c)[4], const T *w, const int lo, const int hi) {
 #pragma unroll
@@ -224,7 +227,21 @@ struct EventVisit {
     }
 };
 
-template<typename T, typename E, bool HOMO, int U>
+// One byte per event, 0 or 1, 16 bytes of events per load where they are aligned.
+template<typename E>
+__device__ __forceinline__ void fill_bytes(uint8_t *bytes, const E *__restrict__ events, const uint32_t n) {
+    constexpr uint32_t PER = 16 / sizeof(E);
+    const uint32_t whole = aligned16_device(events) ? n / PER : 0u;
+    for (uint32_t i = threadIdx.x; i < whole; i += blockDim.x) {
+        const uint4 raw = *reinterpret_cast<const uint4 *>(events + i * PER);
+        const E *e = reinterpret_cast<const E *>(&raw);
+#pragma unroll
+        for (uint32_t k = 0; k < PER; ++k) bytes[i * PER + k] = is_event(e[k]) ? 1 : 0;
+    }
+    for (uint32_t i = whole * PER + threadIdx.x; i < n; i += blockDim.x) bytes[i] = is_event(events[i]) ? 1 : 0;
+}
+
+template<typename T, typename E, bool HOMO, bool BYTES, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const E *__restrict__ events, const uint32_t *__restrict__ packed, T *__restrict__ y, const uint32_t n_row,
@@ -232,9 +249,11 @@ gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
-    EventVisit<T, HOMO> visit{mask, deal.lpr, HOMO ? data[0] : T(0), y, T(0), 0u};
+    EventVisit<T, HOMO, BYTES> visit{mask, deal.lpr, HOMO ? data[0] : T(0), y, T(0), 0u};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
-        if (packed != nullptr) {
+        if (BYTES) {
+            fill_bytes(shared_vector, events, n_col);
+        } else if (packed != nullptr) {
             pdl_wait();
             fill_shared(mask, packed, (n_col + 31u) / 32u);
         } else {
@@ -479,7 +498,8 @@ bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
 
 template<typename T, typename E, bool HOMO>
 bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *workspace, T *y) {
-    constexpr auto kernel = gather_events_kernel<T, E, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, sizeof(T) == 8 ? 1 : 2>;
+    constexpr auto kernel_bytes = gather_events_kernel<T, E, HOMO, true, sizeof(T) == 8 ? 1 : 2>;
     const uint32_t bytes = (m.n_col + 31u) / 32u * 4u;
     if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
         (!HOMO && !aligned16(m.data)))
@@ -488,9 +508,19 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     // clock).  The alternative gathers events through L1 and L2, 1.1 clocks each where they miss.
     const double per = static_cast<double>(m.nse) / sm_count(), gather = m.n_col * sizeof(E) > 200000u ? 1.0 : 0.6;
     const bool pack = m.n_col * sizeof(E) > 32768u;
+    // Few events, which L1 serves by broadcast: rows of one or two of the walk's steps, half of them empty, take it longer than
+    // the plain kernel (1e8 entries, rows of 121, 1037 columns: 106 us and 88; rows of 30: 35 and 41; of 700: 31 and 32).
+    const double mean_row = static_cast<double>(m.nse) / m.n_row;
+    if (HOMO && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
-    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
+    if (!allow_shared<kernel>(SHARED_SMEM) || !allow_shared<kernel_bytes>(SHARED_SMEM)) return launch_ok(), true;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
+    // Bytes take the vector's own length from L1, which streams the entries: 200 KB of them 157 us for 1e8 entries, bits 143.
+    if (m.n_col <= 131072u && m.n_col * sizeof(E) / 34.0 < (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0) + 0.08 * per) {
+        kernel_bytes<<<sms, SHARED_THREADS, m.n_col, stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col);
+        launch_ok();
+        return true;
+    }
     if (!pack) {
         kernel<<<sms, SHARED_THREADS, bytes, stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col);
         launch_ok();

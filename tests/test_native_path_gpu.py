@@ -125,6 +125,15 @@ def test_event_gather_over_bits(cuda, n_row, n_col, mean, homo, dtype, bool_even
     np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(mean))
 
 
+@pytest.mark.parametrize('homo', [True, False])
+@pytest.mark.parametrize('bool_events', [True, False])
+# events as bytes in shared memory: ragged ends, the most of them, one more (bits); few events with rows around the line
+@pytest.mark.parametrize('n_row,n_col,mean', [(40_000, 8203, 60), (30_000, 131_072, 90), (30_000, 131_073, 90),
+                                              (60_000, 2003, 64), (60_000, 2003, 63)])
+def test_event_gather_over_bytes(cuda, n_row, n_col, mean, homo, bool_events):
+  test_event_gather_over_bits(cuda, n_row, n_col, mean, homo, np.float32, bool_events)
+
+
 @pytest.mark.parametrize('dtype,bool_events', [(np.float32, True), (np.float32, False), (np.float64, True)])
 @pytest.mark.parametrize('homo', [False, True])
 # small (one launch, columns owned by blocks): the most rows, long rows, many columns; few columns (sums in shared memory);
