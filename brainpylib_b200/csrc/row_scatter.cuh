@@ -224,6 +224,9 @@ event_scatter_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
                                                      __shfl_sync(FULL_MASK, b, l), nse, y, lane);
         }
     }
+    // Where no row fires nothing above has waited.  This kernel's end must still come after the zero-fill's: what follows on
+    // the stream waits for this one only.
+    pdl_wait();
 }
 
 template<typename T>

@@ -157,3 +157,21 @@ def test_event_scatter(cuda, n_row, n_col, mean, homo, dtype, bool_events):
     want = cpu.event_csr_matvec(data, indices, indptr, host, shape=(n_row, n_col), transpose=True)
     tol = 1e-5 if dtype == np.float32 else 1e-12
     np.testing.assert_allclose(got, want, rtol=10 * tol, atol=20 * tol * np.sqrt(0.1 * indices.size / n_col + 1))
+
+
+def test_silent_event_scatter_orders_its_zeros(cuda):
+  """No row fires: the zeros must be there for a kernel behind the product that starts as early as it may."""
+  n_row, n = 20_000, 3_000_000
+  indptr = torch.arange(0, 4 * n_row + 1, 4, dtype=torch.int32, device=cuda)
+  indices = torch.randint(0, n, (4 * n_row,), dtype=torch.int32, device=cuda)
+  data, silent = torch.rand(4 * n_row, device=cuda), torch.zeros(n_row, dtype=torch.bool, device=cuda)
+  params = bpl.LifExpParams(dt=0.1, tau_syn=[5.0], E_rev=[0.0], ext_input=20.0, V_rest=-60.0, V_th=-50.0, V_reset=-60.0, R=1.0,
+                            tau=20.0, tau_ref=5.0)
+  V, t_last, g = torch.full((n,), -55., device=cuda), torch.full((n,), -1e7, device=cuda), torch.zeros(n, device=cuda)
+  spikes, spike_list = torch.empty(n, device=cuda), torch.empty(bpl.spike_list_bytes(n), dtype=torch.uint8, device=cuda)
+  for _ in range(20):
+    y = torch.full((n,), float('nan'), device=cuda)
+    del y                                # its memory is the next result's
+    y = bpl.event_csr_matvec(data, indices, indptr, silent, shape=(n_row, n), transpose=True)
+    bpl.lif_exp_step(y, g, V, t_last, params, 0.0, spikes=spikes, spike_list=spike_list)
+    assert torch.equal(g, torch.zeros_like(g))
