@@ -407,14 +407,6 @@ PyObject *py_event_csr_matvec(PyObject *, PyObject *const *args, Py_ssize_t narg
     END_HANDLE_TH_ERRORS
 }
 
-// Where the plain storage, the same matrix, multiplies faster than the prepared one: few entries (the prepared kernels clear
-// the result first and need every SM; 640,000 entries transposed 14 us, plain 7), and y = A x with a vector that fits shared
-// memory, which the prepared kernel adds into y from every block of columns (2e7 entries, 7502 columns: 108 us, plain 41; 1e7
-// entries, 100,000 columns: 26, plain 31).
-bool plain_is_faster(int64_t n_col, int64_t nse, bool transpose) {
-    return transpose ? nse < 1000000 : nse < 2000000 || n_col <= 51200;
-}
-
 // csr_matvec(data, indices, indptr, vector, shape, transpose, prepared)
 PyObject *py_csr_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
@@ -432,8 +424,6 @@ PyObject *py_csr_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         NONE_UNLESS(!is_double(*data) && data->size(0) != 1 && !wants_grad(*x) && m.read(args[6]) && !m.fixed &&
                     m.n_row == n_row && m.n_col == n_col && m.groups->device() == data->device() &&
                     m.offsets->device() == data->device());
-        if (plain_is_faster(n_col, indices->size(0), t != 0))
-            return THPVariable_Wrap(csr_product(*data, *indices, *indptr, *x, n_row, n_col, t != 0));
         OnDevice on(*data);
         Tensor out = new_tensor({t ? n_col : n_row}, at::kFloat, data->device());
         void *buffers[4] = {ptr(*m.groups), ptr(*m.offsets), ptr(*x), ptr(out)};

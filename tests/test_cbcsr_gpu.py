@@ -117,6 +117,21 @@ def test_cbcsr_empty_and_errors(cuda):
 
 
 @pytest.mark.parametrize('transpose', [True, False])
+@pytest.mark.parametrize('shape,density', [((3000, 2000), 0.02), ((1500, 51_300), 0.03)])     # 2.3e6 entries: longer vector
+def test_csr_product_is_the_prepared_matrix_s(cuda, shape, density, transpose):
+  """The weights are those that the matrix was prepared with, at every size and with or without a gradient."""
+  data, indices, indptr, rng = cases.csr_case(shape, density, 33)
+  d, ix, ptr = (torch.as_tensor(a).to(cuda) for a in (data, indices, indptr))
+  prepared = bpl.csr_to_column_blocked(d, ix, ptr, shape=shape)
+  x = torch.as_tensor(rng.uniform(-1, 1, shape[0] if transpose else shape[1]).astype(np.float32)).to(cuda)
+  want = bpl.csr_matvec(d, ix, ptr, x, shape=shape, transpose=transpose)
+  d.mul_(2)
+  for grad in (False, True):
+    y = bpl.csr_matvec(d, ix, ptr, x.clone().requires_grad_(grad), shape=shape, transpose=transpose, prepared=prepared)
+    torch.testing.assert_close(y.detach(), want, rtol=1e-5, atol=1e-5 * max(1.0, len(indices) / want.numel()))
+
+
+@pytest.mark.parametrize('transpose', [True, False])
 @pytest.mark.parametrize('shape,density,width', [((3000, 2000), 0.02, 512), ((20000, 50000), 0.002, None),
                                                  ((1, 40), 1.0, 32), ((700, 33000), 0.01, 32256)])
 def test_dense_vector_product_on_the_prepared_matrix(cuda, shape, density, width, transpose):
