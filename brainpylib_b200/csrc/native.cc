@@ -7,12 +7,13 @@
 //
 // Contract with the Python operators: a function returns None whenever the call is not the plain case it handles
 // (operands that are no CUDA tensors, anything that would raise, dtypes to convert, non-contiguous tensors, functorch
-// transforms, forward-mode duals, dispatch modes).  The Python code behind it then runs as it always did and raises,
+// transforms, forward-mode duals, dispatch modes, tracing).  The Python code behind it then runs as it always did and raises,
 // converts or differentiates; so no check and no error message lives here twice.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -47,10 +48,11 @@ bool plain_keys(const Tensor &t) {
     return (t.key_set().raw_repr() & ~allowed) == 0;
 }
 
-// no functorch transform and no dispatch mode is active on this thread
+// no functorch transform, no dispatch mode and no tracer (torch.jit.trace records the Python autograd functions) is active on
+// this thread
 bool plain_thread() {
     return !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
-           !c10::impl::TorchDispatchModeTLS::any_modes_set();
+           !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::tracer::impl::is_dispatch_enabled();
 }
 
 bool plain(const Tensor &t) {

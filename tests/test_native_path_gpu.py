@@ -175,3 +175,24 @@ def test_silent_event_scatter_orders_its_zeros(cuda):
     y = bpl.event_csr_matvec(data, indices, indptr, silent, shape=(n_row, n), transpose=True)
     bpl.lif_exp_step(y, g, V, t_last, params, 0.0, spikes=spikes, spike_list=spike_list)
     assert torch.equal(g, torch.zeros_like(g))
+
+
+@pytest.mark.filterwarnings('ignore')      # the tracer warns of the operators' checks
+@pytest.mark.parametrize('op', ['csr', 'event', 'info', 'jit', 'jit_event', 'matmat'])
+@pytest.mark.parametrize('grad', [False, True])
+def test_traced_operators_take_new_inputs(cuda, op, grad):
+  """A call recorded by torch.jit.trace runs again on the inputs it is given."""
+  if grad and op in ('info', 'matmat'):
+    pytest.skip('no gradient')
+  data, indices, indptr, rng = cases.csr_case((30, 40), 0.3, 11)
+  data, indices, indptr = (torch.as_tensor(a).to(cuda) for a in (data, indices, indptr))
+  conn = dict(conn_prob=0.2, seed=3)
+  call = {'csr': lambda x: bpl.csr_matvec(data, indices, indptr, x, shape=(30, 40)),
+          'event': lambda x: bpl.event_csr_matvec(data, indices, indptr, x, shape=(30, 40)),
+          'info': lambda x: bpl.event_info(x)[0],
+          'jit': lambda x: bpl.matvec_prob_conn_homo_weight(x, 0.5, shape=(50, 40), **conn),
+          'jit_event': lambda x: bpl.event_matvec_prob_conn_uniform_weight(x, w_low=0., w_high=1., shape=(50, 40), **conn),
+          'matmat': lambda x: bpl.matmat_prob_conn_normal_weight(x.reshape(2, 20), w_mu=0., w_sigma=1., shape=(20, 30), **conn)}[op]
+  x, other = (torch.as_tensor((rng.standard_normal(40) * (rng.random(40) < 0.5)).astype(np.float32)).to(cuda) for _ in range(2))
+  traced = torch.jit.trace(call, x.clone().requires_grad_(grad), check_trace=False)
+  torch.testing.assert_close(traced(other), call(other))
