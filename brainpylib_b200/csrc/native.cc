@@ -48,12 +48,13 @@ bool plain_keys(const Tensor &t) {
     return (t.key_set().raw_repr() & ~allowed) == 0;
 }
 
-// no functorch transform, no dispatch mode and no tracer (torch.jit.trace records the Python autograd functions) is active on
-// this thread
-bool plain_thread() {
+// no functorch transform and no dispatch mode is active on this thread
+bool untransformed() {
     return !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
-           !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::tracer::impl::is_dispatch_enabled();
+           !c10::impl::TorchDispatchModeTLS::any_modes_set();
 }
+// nor a tracer: torch.jit.trace records the Python autograd functions
+bool plain_thread() { return untransformed() && !at::tracer::impl::is_dispatch_enabled(); }
 
 bool plain(const Tensor &t) {
     return t.defined() && plain_keys(t) && t.is_contiguous() &&
@@ -442,7 +443,8 @@ PyObject *py_csr_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // event_info(events)
 PyObject *py_event_info(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
-    NONE_UNLESS(nargs == 1 && plain_thread());
+    // (Traced as well: neither way leaves a node in the trace, and here torch.jit.trace says so instead of keeping an empty result.)
+    NONE_UNLESS(nargs == 1 && untransformed());
     const Tensor *events = tensor_of(args[0]);
     NONE_UNLESS(events && (events->dim() == 1 || events->dim() == 2));
     Target target;

@@ -178,18 +178,17 @@ def test_silent_event_scatter_orders_its_zeros(cuda):
 
 
 @pytest.mark.filterwarnings('ignore')      # the tracer warns of the operators' checks
-@pytest.mark.parametrize('op', ['csr', 'event', 'info', 'jit', 'jit_event', 'matmat'])
+@pytest.mark.parametrize('op', ['csr', 'event', 'jit', 'jit_event', 'matmat'])
 @pytest.mark.parametrize('grad', [False, True])
 def test_traced_operators_take_new_inputs(cuda, op, grad):
   """A call recorded by torch.jit.trace runs again on the inputs it is given."""
-  if grad and op in ('info', 'matmat'):
+  if grad and op == 'matmat':
     pytest.skip('no gradient')
   data, indices, indptr, rng = cases.csr_case((30, 40), 0.3, 11)
   data, indices, indptr = (torch.as_tensor(a).to(cuda) for a in (data, indices, indptr))
   conn = dict(conn_prob=0.2, seed=3)
   call = {'csr': lambda x: bpl.csr_matvec(data, indices, indptr, x, shape=(30, 40)),
           'event': lambda x: bpl.event_csr_matvec(data, indices, indptr, x, shape=(30, 40)),
-          'info': lambda x: bpl.event_info(x)[0],
           'jit': lambda x: bpl.matvec_prob_conn_homo_weight(x, 0.5, shape=(50, 40), **conn),
           'jit_event': lambda x: bpl.event_matvec_prob_conn_uniform_weight(x, w_low=0., w_high=1., shape=(50, 40), **conn),
           'matmat': lambda x: bpl.matmat_prob_conn_normal_weight(x.reshape(2, 20), w_mu=0., w_sigma=1., shape=(20, 30), **conn)}[op]
