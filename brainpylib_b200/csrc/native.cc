@@ -103,6 +103,18 @@ bool wants_grad(const Tensor &t) { return t.requires_grad() && at::GradMode::is_
 // ---------------------------------------------------------------------------------------------------------
 // calling a target
 // ---------------------------------------------------------------------------------------------------------
+// A launch waits where the stream's queue is full, an allocation where memory has to be freed: other Python threads run
+// meanwhile.  (Backward passes come here without the lock.)
+struct NoGil {
+    PyThreadState *state = PyGILState_Check() ? PyEval_SaveThread() : nullptr;
+    NoGil() = default;
+    ~NoGil() {
+        if (state) PyEval_RestoreThread(state);
+    }
+    NoGil(const NoGil &) = delete;
+    NoGil &operator=(const NoGil &) = delete;
+};
+
 // Scratch of one call, from torch's stream-ordered allocator: taken and given back around the launches, so calls of
 // several threads and streams never share it, and the memory serves other tensors in between.
 struct Scratch {
@@ -148,6 +160,7 @@ void *ptr(const Tensor &t) { return const_cast<void *>(t.const_data_ptr()); }
 // ---------------------------------------------------------------------------------------------------------
 Tensor csr_product(const Tensor &data, const Tensor &indices, const Tensor &indptr, const Tensor &vector, int64_t n_row,
                    int64_t n_col, bool transpose) {
+    NoGil no_gil;
     OnDevice on(data);
     Tensor out = new_tensor({transpose ? n_col : n_row}, data.scalar_type(), data.device());
     bpl_csr_matvec(on.stream, ptr(data), ptr(indices), ptr(indptr), ptr(vector), ptr(out), static_cast<uint32_t>(n_row),
@@ -159,6 +172,7 @@ Tensor csr_product(const Tensor &data, const Tensor &indices, const Tensor &indp
 
 Tensor event_csr_product(const Tensor &data, const Tensor &indices, const Tensor &indptr, const Tensor &events,
                          int64_t n_row, int64_t n_col, bool transpose) {
+    NoGil no_gil;
     OnDevice on(data);
     Tensor out = new_tensor({transpose ? n_col : n_row}, data.scalar_type(), data.device());
     Scratch ws(bpl_event_csr_matvec_workspace(static_cast<uint32_t>(n_row), static_cast<uint32_t>(n_col),
@@ -216,6 +230,7 @@ struct CsrFn : public torch::autograd::Function<CsrFn> {
 };
 
 Tensor csr_outer(const Tensor &row_vector, const Tensor &col_vector, const Tensor &indices, const Tensor &indptr) {
+    NoGil no_gil;
     OnDevice on(indices);
     Tensor out = new_tensor({indices.size(0)}, row_vector.scalar_type(), row_vector.device());
     bpl_csr_outer(on.stream, ptr(row_vector), ptr(col_vector), ptr(indices), ptr(indptr), ptr(out),
@@ -333,7 +348,7 @@ bool csr_operands(const Tensor *data, const Tensor *indices, const Tensor *indpt
 PyObject *g_blocked_type = nullptr;
 
 struct Blocked {
-    const Tensor *groups = nullptr, *offsets = nullptr;
+    Tensor groups, offsets;               // (held: another thread may set the attributes while the lock is released)
     int64_t n_row = 0, n_col = 0, nse = -1;
     bool fixed = false;
     char opaque[32];
@@ -347,12 +362,13 @@ struct Blocked {
         Py_DECREF(a);
         return ok;
     }
-    static const Tensor *tensor(PyObject *o, const char *name) {
+    static Tensor tensor(PyObject *o, const char *name) {
         PyObject *a = PyObject_GetAttrString(o, name);
-        if (a == nullptr) return PyErr_Clear(), nullptr;
+        if (a == nullptr) return PyErr_Clear(), Tensor();
         const Tensor *t = tensor_of(a);
-        Py_DECREF(a);                       // the object keeps the attribute alive during the call
-        return t;
+        Tensor held = t ? *t : Tensor();
+        Py_DECREF(a);
+        return held;
     }
     bool read(PyObject *o) {
         if (g_blocked_type == nullptr || Py_TYPE(o) != reinterpret_cast<PyTypeObject *>(g_blocked_type)) return false;
@@ -363,7 +379,7 @@ struct Blocked {
         const bool shaped = shape_of(shape, n_row, n_col);
         Py_DECREF(shape);
         long width = 0, lanes = 0, scale = 0, entries = -1;
-        if (!groups || !offsets || !shaped || !integer(o, "block_width", width) || !integer(o, "team_lanes_log2", lanes))
+        if (!groups.defined() || !offsets.defined() || !shaped || !integer(o, "block_width", width) || !integer(o, "team_lanes_log2", lanes))
             return false;
         fixed = integer(o, "scale_log2", scale);       // None: float sums
         if (integer(o, "nse", entries)) nse = entries;
@@ -395,14 +411,18 @@ PyObject *py_event_csr_matvec(PyObject *, PyObject *const *args, Py_ssize_t narg
     if (args[6] != Py_None && t && !is_double(*data) && !grad) {
         Blocked m;
         NONE_UNLESS(m.read(args[6]) && m.n_row == n_row && m.n_col == n_col && m.nse == indices->size(0) &&
-                    m.groups->device() == data->device() && m.offsets->device() == data->device());
-        OnDevice on(*data);
-        Tensor out = new_tensor({n_col}, at::kFloat, data->device());
-        Scratch ws(bpl_event_csr_workspace_bytes(static_cast<uint32_t>(n_row), 1), on.stream);
-        void *buffers[5] = {ptr(*m.groups), ptr(*m.offsets), ptr(*events), ptr(out), ws.ptr};
-        (events->scalar_type() == at::kBool ? event_cbcsr_matvec_heter_float_bool : event_cbcsr_matvec_heter_float_float)(
-            on.stream, buffers, m.opaque, m.opaque_len);
-        check_status();
+                    m.groups.device() == data->device() && m.offsets.device() == data->device());
+        Tensor out;
+        {
+            NoGil no_gil;
+            OnDevice on(*data);
+            out = new_tensor({n_col}, at::kFloat, data->device());
+            Scratch ws(bpl_event_csr_workspace_bytes(static_cast<uint32_t>(n_row), 1), on.stream);
+            void *buffers[5] = {ptr(m.groups), ptr(m.offsets), ptr(*events), ptr(out), ws.ptr};
+            (events->scalar_type() == at::kBool ? event_cbcsr_matvec_heter_float_bool : event_cbcsr_matvec_heter_float_float)(
+                on.stream, buffers, m.opaque, m.opaque_len);
+            check_status();
+        }
         return THPVariable_Wrap(std::move(out));
     }
     return THPVariable_Wrap(grad ? EventCsrFn::apply(*data, *indices, *indptr, *events, n_row, n_col, t != 0)
@@ -425,13 +445,17 @@ PyObject *py_csr_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (args[6] != Py_None) {
         Blocked m;
         NONE_UNLESS(!is_double(*data) && data->size(0) != 1 && !wants_grad(*x) && m.read(args[6]) && !m.fixed &&
-                    m.n_row == n_row && m.n_col == n_col && m.groups->device() == data->device() &&
-                    m.offsets->device() == data->device());
-        OnDevice on(*data);
-        Tensor out = new_tensor({t ? n_col : n_row}, at::kFloat, data->device());
-        void *buffers[4] = {ptr(*m.groups), ptr(*m.offsets), ptr(*x), ptr(out)};
-        (t ? cbcsr_matvec_transpose_heter_float : cbcsr_matvec_heter_float)(on.stream, buffers, m.opaque, m.opaque_len);
-        check_status();
+                    m.n_row == n_row && m.n_col == n_col && m.groups.device() == data->device() &&
+                    m.offsets.device() == data->device());
+        Tensor out;
+        {
+            NoGil no_gil;
+            OnDevice on(*data);
+            out = new_tensor({t ? n_col : n_row}, at::kFloat, data->device());
+            void *buffers[4] = {ptr(m.groups), ptr(m.offsets), ptr(*x), ptr(out)};
+            (t ? cbcsr_matvec_transpose_heter_float : cbcsr_matvec_heter_float)(on.stream, buffers, m.opaque, m.opaque_len);
+            check_status();
+        }
         return THPVariable_Wrap(std::move(out));
     }
     return THPVariable_Wrap(wants_grad(*data) || wants_grad(*x)
@@ -458,14 +482,18 @@ PyObject *py_event_info(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     }
     const bool batched = events->dim() == 2;
     const int64_t batch = batched ? events->size(0) : 1, size = events->size(batched ? 1 : 0);
-    OnDevice on(*events);
-    Tensor ids = new_tensor(events->sizes(), at::kInt, events->device());
-    Tensor num = batched ? new_tensor({batch}, at::kInt, events->device()) : new_tensor({}, at::kInt, events->device());
-    const bpl::DoubleSizeDescriptor d{static_cast<unsigned>(size), static_cast<unsigned>(batch)};
-    Scratch ws(bpl_nonzero_workspace_bytes(static_cast<uint32_t>(batch)), on.stream);
-    void *buffers[4] = {ptr(*events), ptr(ids), ptr(num), ws.ptr};
-    target(on.stream, buffers, reinterpret_cast<const char *>(&d), sizeof(d));
-    check_status();
+    Tensor ids, num;
+    {
+        NoGil no_gil;
+        OnDevice on(*events);
+        ids = new_tensor(events->sizes(), at::kInt, events->device());
+        num = batched ? new_tensor({batch}, at::kInt, events->device()) : new_tensor({}, at::kInt, events->device());
+        const bpl::DoubleSizeDescriptor d{static_cast<unsigned>(size), static_cast<unsigned>(batch)};
+        Scratch ws(bpl_nonzero_workspace_bytes(static_cast<uint32_t>(batch)), on.stream);
+        void *buffers[4] = {ptr(*events), ptr(ids), ptr(num), ws.ptr};
+        target(on.stream, buffers, reinterpret_cast<const char *>(&d), sizeof(d));
+        check_status();
+    }
     PyObject *r = PyTuple_New(2);
     if (r == nullptr) return nullptr;
     PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(ids)));
@@ -495,6 +523,7 @@ struct JitArgs {
 
 // The descriptor's real fields are float32-rounded, here as in bpl_build_jitconn_prob_*_descriptor.
 Tensor jit_product(const Tensor &x, const JitArgs &a, const bool events) {
+    NoGil no_gil;
     OnDevice on(x);
     const bool b = x.scalar_type() == at::kBool;
     Tensor out = new_tensor({a.n_out}, b ? at::kFloat : x.scalar_type(), x.device());
@@ -575,18 +604,22 @@ PyObject *py_jit_matmat(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     NONE_UNLESS(x && x->dim() == 2 && float_like(*x) && !wants_grad(*x) && number_of(args[1], kind) &&
                 number_of(args[2], w1) && number_of(args[3], w2) && number_of(args[4], log_p) && shape_of(args[5], k, n) &&
                 x->size(1) == k && x->size(0) <= 0xffffffffll && PyLong_CheckExact(args[6]));
-    OnDevice on(*x);
-    Tensor out = new_tensor({x->size(0), n}, x->scalar_type(), x->device());
-    char opaque[64];
-    const size_t len = bpl_build_matmat_jit_prob_descriptor1(
-        static_cast<uint32_t>(x->size(0)), static_cast<uint32_t>(k), static_cast<uint32_t>(n),
-        static_cast<uint32_t>(PyLong_AsUnsignedLongMask(args[6])), static_cast<float>(log_p), static_cast<float>(w1),
-        static_cast<float>(w2), opaque, sizeof(opaque));
-    Scratch ws(bpl_workspace_bytes(is_double(*x) ? "gpu_matmat_prob_prob_normal_double_v1_ws"
-                                                 : "gpu_matmat_prob_prob_normal_float_v1_ws", opaque, len), on.stream);
-    void *buffers[3] = {ptr(*x), ptr(out), ws.ptr};
-    targets[kind > 1.5][is_double(*x)](on.stream, buffers, opaque, len);
-    check_status();
+    const uint32_t seed = static_cast<uint32_t>(PyLong_AsUnsignedLongMask(args[6]));
+    Tensor out;
+    {
+        NoGil no_gil;
+        OnDevice on(*x);
+        out = new_tensor({x->size(0), n}, x->scalar_type(), x->device());
+        char opaque[64];
+        const size_t len = bpl_build_matmat_jit_prob_descriptor1(
+            static_cast<uint32_t>(x->size(0)), static_cast<uint32_t>(k), static_cast<uint32_t>(n), seed, static_cast<float>(log_p),
+            static_cast<float>(w1), static_cast<float>(w2), opaque, sizeof(opaque));
+        Scratch ws(bpl_workspace_bytes(is_double(*x) ? "gpu_matmat_prob_prob_normal_double_v1_ws"
+                                                     : "gpu_matmat_prob_prob_normal_float_v1_ws", opaque, len), on.stream);
+        void *buffers[3] = {ptr(*x), ptr(out), ws.ptr};
+        targets[kind > 1.5][is_double(*x)](on.stream, buffers, opaque, len);
+        check_status();
+    }
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
 }
@@ -685,9 +718,12 @@ PyObject *py_lif_exp_step(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
                                                     decay, e_rev, ext, v_rest, v_th, v_reset, r, lif, tau_ref, opaque,
                                                     sizeof(opaque));
     NONE_UNLESS(len != 0);
-    void *buffers[6] = {ptr(*y), ptr(*g), ptr(*V), ptr(*t_last), ptr(spikes), ptr(list)};
-    lif_exp_step_float(on.stream, buffers, opaque, len);
-    check_status();
+    {
+        NoGil no_gil;
+        void *buffers[6] = {ptr(*y), ptr(*g), ptr(*V), ptr(*t_last), ptr(spikes), ptr(list)};
+        lif_exp_step_float(on.stream, buffers, opaque, len);
+        check_status();
+    }
     PyObject *res = PyTuple_New(2);
     if (res == nullptr) return nullptr;
     PyTuple_SET_ITEM(res, 0, THPVariable_Wrap(std::move(spikes)));
@@ -707,10 +743,12 @@ PyObject *py_list_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
                 list->device() == y->device());
     if (args[6] != Py_None) {
         Blocked m;
-        NONE_UNLESS(m.read(args[6]) && m.n_row == n_row && m.n_col == n_col && m.groups->device() == y->device());
+        NONE_UNLESS(m.read(args[6]) && m.n_row == n_row && m.n_col == n_col && m.groups.device() == y->device());
+        NoGil no_gil;
         OnDevice on(*y);
-        void *buffers[4] = {ptr(*m.groups), ptr(*m.offsets), ptr(*list), ptr(*y)};
+        void *buffers[4] = {ptr(m.groups), ptr(m.offsets), ptr(*list), ptr(*y)};
         event_cbcsr_matvec_list_heter_float(on.stream, buffers, m.opaque, m.opaque_len);
+        check_status();
     } else {
         const Tensor *data = tensor_of(args[0]), *indices = tensor_of(args[1]), *indptr = tensor_of(args[2]);
         NONE_UNLESS(data && indices && indptr && data->scalar_type() == at::kFloat && int32_like(*indices) &&
@@ -720,11 +758,12 @@ PyObject *py_list_matvec(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         char opaque[16];
         const size_t len = bpl_build_triple_size_descriptor(static_cast<uint32_t>(n_row), static_cast<uint32_t>(n_col),
                                                             static_cast<uint32_t>((n_row + 4095) / 4096), opaque, sizeof(opaque));
+        NoGil no_gil;
         OnDevice on(*y);
         void *buffers[5] = {ptr(*data), ptr(*indices), ptr(*indptr), ptr(*list), ptr(*y)};
         event_csr_matvec_list_heter_float(on.stream, buffers, opaque, len);
+        check_status();
     }
-    check_status();
     Py_RETURN_TRUE;
     END_HANDLE_TH_ERRORS
 }

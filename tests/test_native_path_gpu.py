@@ -1,5 +1,8 @@
 """The native host path: its gradients (C++ nodes, weight gradient in one kernel) against index arithmetic in float64, on
 row lengths around the kernel's units of 4 entries and 4..32 lanes, and its second-order gradients."""
+import threading
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -195,3 +198,45 @@ def test_traced_operators_take_new_inputs(cuda, op, grad):
   x, other = (torch.as_tensor((rng.standard_normal(40) * (rng.random(40) < 0.5)).astype(np.float32)).to(cuda) for _ in range(2))
   traced = torch.jit.trace(call, x.clone().requires_grad_(grad), check_trace=False)
   torch.testing.assert_close(traced(other), call(other))
+
+
+@pytest.mark.parametrize('op', ['csr', 'event', 'jit', 'step'])
+def test_other_threads_run_while_the_launch_queue_is_full(cuda, op):
+  """More launches than the queue of a stream holds, behind half a second of other work: the calls wait for room, and
+  meanwhile a thread that needs the interpreter goes on."""
+  data, indices, indptr, rng = cases.csr_case((30, 40), 0.3, 11)
+  data, indices, indptr = (torch.as_tensor(a).to(cuda) for a in (data, indices, indptr))
+  x = torch.rand(40, device=cuda)
+  params = bpl.LifExpParams(dt=0.1, tau_syn=[5.0], E_rev=[0.0], ext_input=20.0, V_rest=-60.0, V_th=-50.0, V_reset=-60.0, R=1.0,
+                            tau=20.0, tau_ref=5.0)
+  y, g, V, t_last, spikes = (torch.zeros(40, device=cuda) for _ in range(5))
+  spike_list = torch.empty(bpl.spike_list_bytes(40), dtype=torch.uint8, device=cuda)
+  call = {'csr': lambda: bpl.csr_matvec(data, indices, indptr, x, shape=(30, 40)),
+          'event': lambda: bpl.event_csr_matvec(data, indices, indptr, x, shape=(30, 40)),
+          'jit': lambda: bpl.matvec_prob_conn_homo_weight(x, 0.5, conn_prob=0.2, shape=(50, 40), seed=3),
+          'step': lambda: bpl.lif_exp_step(y, g, V, t_last, params, 0.0, spikes=spikes, spike_list=spike_list)}[op]
+  call()
+  torch.cuda.synchronize()
+  gaps, stop = [], threading.Event()
+
+  def beat():
+    last = time.perf_counter()
+    while not stop.is_set():
+      time.sleep(0.001)
+      now = time.perf_counter()
+      gaps.append(now - last)
+      last = now
+
+  thread = threading.Thread(target=beat)
+  thread.start()
+  begin = time.perf_counter()
+  torch.cuda._sleep(1_000_000_000)
+  for _ in range(6000):
+    call()
+  took = time.perf_counter() - begin
+  stop.set()
+  thread.join()
+  torch.cuda.synchronize()
+  if took < 0.3:
+    pytest.skip('the queue took every launch')
+  assert max(gaps) < 0.15
