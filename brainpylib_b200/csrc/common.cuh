@@ -125,6 +125,16 @@ __device__ __forceinline__ void add_sums(const T *sums, T *__restrict__ out, con
     }
 }
 
+// Per-entry results of entries that no row owns (arrays longer than the matrix): zero, by the whole grid.
+template<typename T>
+__device__ __forceinline__ void zero_outside_rows(T *__restrict__ g, const uint32_t *__restrict__ indptr, const uint32_t n_row,
+                                                  const uint32_t nse) {
+    const uint64_t first = indptr[0], from = indptr[n_row], step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    const uint64_t me = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (uint64_t i = me; i < first; i += step) g[i] = T(0);
+    for (uint64_t i = from + me; i < nse; i += step) g[i] = T(0);
+}
+
 // *p = v in shared memory where `yes` is not zero, without a branch
 __device__ __forceinline__ void store_shared_if(const uint32_t yes, uint32_t *p, const uint32_t v) {
     asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.shared.u32 [%1], %2; }"

@@ -197,6 +197,7 @@ csr_outer_kernel(const T *__restrict__ row_vector, const T *__restrict__ col_vec
             for (uint32_t pos = start + sl; pos < end; pos += lpr) g[pos] = r * col_vector[indices[pos]];
         }
     }
+    zero_outside_rows(g, indptr, n_row, nse);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -615,7 +616,11 @@ void csr_matvec_known(cudaStream_t stream, const void *data, const uint32_t *ind
 template<typename T>
 void csr_outer_impl(cudaStream_t stream, const void *row_vector, const void *col_vector, const uint32_t *indices,
                     const uint32_t *indptr, void *out, uint32_t n_row, uint32_t n_col, uint32_t nse) {
-    if (n_row == 0 || nse == 0) return;
+    if (nse == 0) return;
+    if (n_row == 0) {
+        if (cudaMemsetAsync(out, 0, sizeof(T) * static_cast<size_t>(nse), stream) != cudaSuccess) launch_ok();
+        return;
+    }
     const int grid = persistent_blocks(8, n_row);
     const T *r = static_cast<const T *>(row_vector), *c = static_cast<const T *>(col_vector);
     T *g = static_cast<T *>(out);

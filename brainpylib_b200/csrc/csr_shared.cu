@@ -362,6 +362,7 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
             if (part == 0 && row < n_row) out[row] = acc;
         }
     }
+    if (OUTER) zero_outside_rows(out, indptr, n_row, nse);
 }
 
 // y += A^T x: sums in shared memory, added to the zero-filled y at the end
@@ -436,6 +437,7 @@ outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__rest
     OuterVisit<T> visit{xs, row_vector, g, n_row, T(0)};
     walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, deal, visit, [&]() {
         fill_shared(xs, col_vector, n_col);
+        zero_outside_rows(g, indptr, n_row, nse);
         __syncthreads();
     });
 }

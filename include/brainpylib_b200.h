@@ -275,7 +275,7 @@ BPL_FOR_EACH_TARGET(BPL_DECLARE_ONE)
  * size of a spike list of n_row neurons) and nonzero_*.
  * bpl_csr_outer: g[e] = row_vector[row of entry e] * col_vector[indices[e]] for the nse stored entries of a CSR matrix
  * (float32, or float64 with is_double): the gradient of a CSR product with respect to its weights
- * (brainpylib/_src/sparse_ops/cusparse_matvec.py:292-304).
+ * (brainpylib/_src/sparse_ops/cusparse_matvec.py:292-304).  Zero for entries that no row owns.
  * bpl_csr_matvec: csr_matvec_{homo,heter}_vector_* / csr_matvec_transpose_* without descriptor, for callers that know the
  * number of stored entries nse on the host (it selects the kernel).
  * bpl_event_csr_matvec: event_csr_matvec_* in the same way (buffers as there, with a workspace of

@@ -49,6 +49,33 @@ def test_gradients_of_weights_and_vector(cuda, rows, dtype, transpose, event, of
     torch.testing.assert_close(g.double(), want, **tol)
 
 
+@pytest.mark.parametrize('event', [False, True])
+@pytest.mark.parametrize('transpose', [False, True])
+# the three kernels: vector in shared memory, longer vector swept in bands, neither; no rows at all
+@pytest.mark.parametrize('n_row,n_col,mean', [(20_000, 3000, 60), (20_000, 60_000, 120), (300, 60_000, 9), (0, 40, 0)])
+def test_gradient_of_entries_that_no_row_owns(cuda, n_row, n_col, mean, transpose, event):
+  """Arrays with room in front of and behind the matrix: the product does not use it, so its gradient is zero."""
+  front, back = 5, 3011
+  indptr = torch.arange(front, front + n_row * mean + 1, max(mean, 1), dtype=torch.int32, device=cuda)[:n_row + 1]
+  g = torch.Generator(device=cuda).manual_seed(1)
+  nse = front + n_row * mean + back
+  indices = torch.randint(0, n_col, (nse,), dtype=torch.int32, device=cuda, generator=g)
+  data = torch.rand(nse, device=cuda, generator=g).requires_grad_(True)
+  x = torch.rand(n_row if transpose else n_col, device=cuda, generator=g)
+  op = bpl.event_csr_matvec if event else bpl.csr_matvec
+  y = op(data, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
+  ct = torch.rand_like(y)
+  junk = torch.full_like(data, float('nan'))
+  del junk                               # its memory is the gradient's
+  got = torch.autograd.grad(y, data, ct)[0]
+  want = torch.zeros_like(got)
+  if n_row:
+    row = torch.arange(n_row, device=cuda).repeat_interleave(mean)
+    col = indices[front:nse - back].long()
+    want[front:nse - back] = x[row] * ct[col] if transpose else x[col] * ct[row]
+  torch.testing.assert_close(got, want)
+
+
 @pytest.mark.parametrize('transpose', [False, True])
 def test_second_order_gradients(cuda, transpose):
   data, indices, indptr, rng = cases.csr_case((30, 40), 0.3, 11, dtype=np.float64)
