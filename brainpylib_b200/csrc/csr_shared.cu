@@ -46,6 +46,13 @@ struct Deal {
     }
 };
 
+// The entries [first, last) of a quad at `base` that belong to a row which reaches into it.  Positions have 32 bits, and a
+// row may have more than 2^31 entries.
+__host__ __device__ constexpr int quad_first(const uint32_t row_start, const uint32_t base) { return row_start > base ? static_cast<int>(row_start - base) : 0; }
+__host__ __device__ constexpr int quad_last(const uint32_t row_end, const uint32_t base) { return row_end - base < 4u ? static_cast<int>(row_end - base) : 4; }
+static_assert(quad_first(0x80000001u, 0x80000000u) == 1 && quad_first(0x80000002u, 0x7ffffffcu) == 6 && quad_first(3u, 0xf0000000u) == 0, "");
+static_assert(quad_last(0x80000003u, 0x80000000u) == 3 && quad_last(0xfffffff0u, 8u) == 4 && quad_last(0x80000010u, 0x7ffffff0u) == 4, "");
+
 // `visit` has
 //   fetch(row)                            what is needed of a row besides its entries (requested one row ahead)
 //   quad<FULL>(base, c[4], w[4], lo, hi)  entries base .. base + 3, of which lo <= e < hi belong to the row (FULL: all)
@@ -103,8 +110,8 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
             if (!__any_sync(FULL_MASK, here)) continue;
             const uint32_t c[4] = {now.ix[u].x, now.ix[u].y, now.ix[u].z, now.ix[u].w};
             const T *v = now.w[WEIGHTS ? u : 0].v;
-            const int lo = static_cast<int>(row.start) - static_cast<int>(base), hi = static_cast<int>(row.end) - static_cast<int>(base);
-            if (__all_sync(FULL_MASK, here && lo <= 0 && hi >= 4)) visit.template quad<true>(base, c, v, lo, hi);
+            const int lo = quad_first(row.start, base), hi = quad_last(row.end, base);
+            if (__all_sync(FULL_MASK, here && lo == 0 && hi == 4)) visit.template quad<true>(base, c, v, lo, hi);
             else visit.template quad<false>(base, c, v, lo, here ? hi : 0);
         }
         if (more) return;
