@@ -110,9 +110,8 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
             if (!__any_sync(FULL_MASK, here)) continue;
             const uint32_t c[4] = {now.ix[u].x, now.ix[u].y, now.ix[u].z, now.ix[u].w};
             const T *v = now.w[WEIGHTS ? u : 0].v;
-            const int lo = quad_first(row.start, base), hi = quad_last(row.end, base);
-            if (__all_sync(FULL_MASK, here && lo == 0 && hi == 4)) visit.template quad<true>(base, c, v, lo, hi);
-            else visit.template quad<false>(base, c, v, lo, here ? hi : 0);
+            if (__all_sync(FULL_MASK, here && row.start <= base && row.end - base >= 4u)) visit.template quad<true>(base, c, v, 0, 4);
+            else visit.template quad<false>(base, c, v, quad_first(row.start, base), here ? quad_last(row.end, base) : 0);
         }
         if (more) return;
         if (sl == 0)
