@@ -46,12 +46,11 @@ struct Deal {
     }
 };
 
-// The entries [first, last) of a quad at `base` that belong to a row which reaches into it.  Positions have 32 bits, and a
-// row may have more than 2^31 entries.
-__host__ __device__ constexpr int quad_first(const uint32_t row_start, const uint32_t base) { return row_start > base ? static_cast<int>(row_start - base) : 0; }
-__host__ __device__ constexpr int quad_last(const uint32_t row_end, const uint32_t base) { return row_end - base < 4u ? static_cast<int>(row_end - base) : 4; }
-static_assert(quad_first(0x80000001u, 0x80000000u) == 1 && quad_first(0x80000002u, 0x7ffffffcu) == 6 && quad_first(3u, 0xf0000000u) == 0, "");
-static_assert(quad_last(0x80000003u, 0x80000000u) == 3 && quad_last(0xfffffff0u, 8u) == 4 && quad_last(0x80000010u, 0x7ffffff0u) == 4, "");
+// Where a position lies from the first entry of a quad.  Positions have 32 bits; the host sends no matrix of 2^31 entries or
+// more here, so that a row's ends lie less than that from any of its quads.
+__host__ __device__ constexpr int from_quad(const uint32_t position, const uint32_t base) { return static_cast<int>(position - base); }
+static_assert(from_quad(0x80000001u, 0x7ffffffcu) == 5 && from_quad(0x7ffffffdu, 0x80000000u) == -3, "");
+constexpr uint32_t MOST_ENTRIES = 0x7fffffffu;
 
 // `visit` has
 //   fetch(row)                            what is needed of a row besides its entries (requested one row ahead)
@@ -110,8 +109,9 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
             if (!__any_sync(FULL_MASK, here)) continue;
             const uint32_t c[4] = {now.ix[u].x, now.ix[u].y, now.ix[u].z, now.ix[u].w};
             const T *v = now.w[WEIGHTS ? u : 0].v;
-            if (__all_sync(FULL_MASK, here && row.start <= base && row.end - base >= 4u)) visit.template quad<true>(base, c, v, 0, 4);
-            else visit.template quad<false>(base, c, v, quad_first(row.start, base), here ? quad_last(row.end, base) : 0);
+            const int lo = from_quad(row.start, base), hi = from_quad(row.end, base);
+            if (__all_sync(FULL_MASK, here && lo <= 0 && hi >= 4)) visit.template quad<true>(base, c, v, lo, hi);
+            else visit.template quad<false>(base, c, v, lo, here ? hi : 0);
         }
         if (more) return;
         if (sl == 0)
@@ -465,7 +465,7 @@ struct Plan {
 
 template<typename T>
 bool usable(const CsrMatrix<T> &m, const bool weights) {
-    return m.n_row != 0 && m.n_col != 0 && m.nse != 0 && m.n_col <= SHARED_SMEM / sizeof(T) && aligned16(m.indices) &&
+    return m.n_row != 0 && m.n_col != 0 && m.nse != 0 && m.nse <= MOST_ENTRIES && m.n_col <= SHARED_SMEM / sizeof(T) && aligned16(m.indices) &&
            (!weights || aligned16(m.data));
 }
 
@@ -509,7 +509,7 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, sizeof(T) == 8 ? 1 : 2>;
     constexpr auto kernel_bytes = gather_events_kernel<T, E, HOMO, true, sizeof(T) == 8 ? 1 : 2>;
     const uint32_t bytes = (m.n_col + 31u) / 32u * 4u;
-    if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
+    if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.nse > MOST_ENTRIES || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
         (!HOMO && !aligned16(m.data)))
         return false;
     // The bits are packed by a launch of their own where the events are more than a block reads in its time (34 bytes per
