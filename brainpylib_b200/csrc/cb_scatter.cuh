@@ -173,7 +173,7 @@ __device__ __forceinline__ void cb_accumulate(float *acc, const unsigned char *b
 __device__ __forceinline__ uint32_t cb_chunk_prefix(const uint32_t *__restrict__ counts, const uint32_t n_chunks,
                                                     uint32_t *prefix, uint32_t *warp_total) {
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t c = t < n_chunks ? counts[t] : 0u;
+    const uint32_t c = t < n_chunks ? __ldca(counts + t) : 0u;
     uint32_t incl = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

@@ -52,6 +52,9 @@ __device__ __forceinline__ uint2 ldg_stream_u2(const void *p) {
 // scatter does everything that needs no input from the scan (clearing its shared memory) and then waits here until
 // the scan has completed and its writes are visible.  In a kernel that was launched the ordinary way the wait returns
 // at once.
+// What the launch in front writes must not be read through the read-only path (`ld.global.nc`, which the compiler also takes
+// for a `const __restrict__` kernel argument): it is specified for data that stays constant while the kernel runs, and the
+// reading kernel runs already.  Such reads are written as __ldcg or __ldca, or their pointers carry no __restrict__.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -452,7 +452,7 @@ event_columns_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             const uint32_t i = base + k * OWN_THREADS + threadIdx.x;
-            act[k] = i < n_row && is_event(events[i]);
+            act[k] = i < n_row && is_event(__ldcg(events + i));
         }
 #pragma unroll
         for (int k = 0; k < PER; ++k) {

@@ -152,6 +152,15 @@ __device__ __forceinline__ void fill_shared(T *shared, const T *__restrict__ p, 
     for (uint32_t i = n_vec * PER + threadIdx.x; i < count; i += SHARED_THREADS) shared[i] = __ldg(p + i);
 }
 
+// The same for words that the launch in front has written.
+__device__ __forceinline__ void fill_words(uint32_t *shared, const uint32_t *p, const uint32_t count) {
+    const uint32_t n_vec = aligned16_device(p) ? count / 4u : 0u;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < n_vec; i += SHARED_THREADS)
+        reinterpret_cast<uint4 *>(shared)[i] = __ldcg(reinterpret_cast<const uint4 *>(p) + i);
+    for (uint32_t i = n_vec * 4u + threadIdx.x; i < count; i += SHARED_THREADS) shared[i] = __ldcg(p + i);
+}
+
 // y = A x
 template<typename T, bool HOMO>
 struct GatherVisit {
@@ -250,7 +259,7 @@ __device__ __forceinline__ void fill_bytes(uint8_t *bytes, const E *__restrict__
 template<typename T, typename E, bool HOMO, bool BYTES, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
-                     const E *__restrict__ events, const uint32_t *__restrict__ packed, T *__restrict__ y, const uint32_t n_row,
+                     const E *__restrict__ events, const uint32_t *packed, T *__restrict__ y, const uint32_t n_row,
                      const uint32_t nse, const uint32_t n_col) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
@@ -261,7 +270,7 @@ gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
             fill_bytes(shared_vector, events, n_col);
         } else if (packed != nullptr) {
             pdl_wait();
-            fill_shared(mask, packed, (n_col + 31u) / 32u);
+            fill_words(mask, packed, (n_col + 31u) / 32u);
         } else {
             pack_event_mask(events, n_col, mask);
         }

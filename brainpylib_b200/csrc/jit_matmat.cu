@@ -204,9 +204,9 @@ __device__ __forceinline__ bool barrier_wait(uint64_t *bar, const uint32_t parit
 // launched side by side, so the lists come from DRAM once and from L2 for the other row groups.
 template<typename T, int KIND>
 __global__ void __launch_bounds__(ApplyShape<T>::MAX_THREADS, 1)
-jit_matmat_apply_kernel(const T *__restrict__ Xt, const unsigned int m, const unsigned int k, const unsigned int n,
+jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k, const unsigned int n,
                         const unsigned int col0, const unsigned int cols, const unsigned int cap,
-                        const unsigned int *__restrict__ cnt, const MMEntry<T> *__restrict__ entries,
+                        const unsigned int *cnt, const MMEntry<T> *entries,
                         const unsigned int seed, const GapParams gp, const double w1, const double w2, T *__restrict__ Y) {
     constexpr int KT = ApplyShape<T>::KT, CHUNKS = ApplyShape<T>::CHUNKS, PER_CHUNK = 16 / sizeof(T);
     static_assert(KT * MM_ROWS * sizeof(T) == TILE_BYTES, "a tile");
@@ -344,9 +344,9 @@ constexpr int GATHER_COLS = 8;
 
 template<typename T, int KIND, int V>
 __global__ void __launch_bounds__(GATHER_COLS * 32)
-jit_matmat_gather_kernel(const T *__restrict__ Xt, const unsigned int m, const unsigned int m_pad, const unsigned int k,
+jit_matmat_gather_kernel(const T *Xt, const unsigned int m, const unsigned int m_pad, const unsigned int k,
                          const unsigned int n, const unsigned int col0, const unsigned int cols, const unsigned int cap,
-                         const unsigned int *__restrict__ cnt, const MMEntry<T> *__restrict__ entries,
+                         const unsigned int *cnt, const MMEntry<T> *entries,
                          const unsigned int seed, const GapParams gp, const double w1, const double w2, T *__restrict__ Y) {
     __shared__ T block[GATHER_COLS][32 * V + 1];
     const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;

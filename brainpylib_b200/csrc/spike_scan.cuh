@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t chunk_prefix(const uint32_t *__restrict__ co
     uint32_t s = 0;
     for (uint32_t j = 0; j < per; ++j) {
         const uint32_t k = threadIdx.x * per + j;
-        c[j] = k < n_chunks ? counts[k] : 0u;
+        c[j] = k < n_chunks ? __ldca(counts + k) : 0u;
         s += c[j];
     }
     uint32_t incl = s;
@@ -147,7 +147,7 @@ __device__ __forceinline__ uint32_t list_row(const uint32_t *prefix, const uint3
         const uint32_t mid = (lo + hi) >> 1;
         if (prefix[mid] <= li) lo = mid; else hi = mid;
     }
-    return ids[static_cast<uint64_t>(lo) * chunk + (li - prefix[lo])];
+    return __ldca(ids + static_cast<uint64_t>(lo) * chunk + (li - prefix[lo]));
 }
 
 }  // namespace
