@@ -417,9 +417,11 @@ bool list_scatter_shared(cudaStream_t stream, const CsrMatrix<T> &m, const E *ev
     scan_events_kernel<T, E><<<max(p.n_chunks, (m.n_col + SCAN_TILE - 1) / SCAN_TILE), SCAN_THREADS, 0, stream>>>(
         events, m.n_row, p.chunk, p.n_chunks, y, m.n_col, counts, ids);
     if (!launch_ok()) return true;
+    if (profile_before()) cudaEventRecord(profile_before(), stream);
     const cudaError_t e = launch_dependent(vec ? wide : narrow, dim3(sm_count()), dim3(LIST_SHARED_THREADS), m.n_col * sizeof(T), stream,
                                            m.indices, m.indptr, m.data, m.n_row, m.n_col, p.chunk, p.n_chunks, counts, ids, y);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+    if (profile_after()) cudaEventRecord(profile_after(), stream);
     return true;
 }
 
@@ -569,10 +571,12 @@ bool event_scatter_columns(cudaStream_t stream, const CsrMatrix<T> &m, const E *
     constexpr auto wide = event_columns_kernel<T, E, HOMO, true>, narrow = event_columns_kernel<T, E, HOMO, false>;
     constexpr unsigned most = 100u * 1024u;
     if (!(vec ? allow_shared<wide>(most) : allow_shared<narrow>(most))) return launch_ok(), true;
+    if (profile_before()) cudaEventRecord(profile_before(), stream);
     const cudaError_t e = launch_dependent(vec ? wide : narrow, dim3(blocks), dim3(OWN_THREADS),
                                            width * sizeof(T) + sizeof(uint2) * static_cast<size_t>(m.n_row), stream, m.indices, m.indptr, m.data,
                                            events, m.n_row, m.n_col, m.nse, width, log_lpr, y);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+    if (profile_after()) cudaEventRecord(profile_after(), stream);
     return true;
 }
 

@@ -267,3 +267,25 @@ def test_other_threads_run_while_the_launch_queue_is_full(cuda, op):
   if took < 0.3:
     pytest.skip('the queue took every launch')
   assert max(gaps) < 0.15
+
+
+@pytest.mark.parametrize('n_row,n_col,mean', [(300, 517, 40), (90_000, 2001, 250), (20_000, 9000, 20), (270_000, 5000, 3)])
+def test_every_event_scatter_records_the_profile_events(cuda, n_row, n_col, mean):
+  """One launch, sums in shared memory, straight from the events, from a list."""
+  import ctypes
+  from brainpylib_b200 import _lib
+  indptr = torch.arange(0, n_row * mean + 1, mean, dtype=torch.int32, device=cuda)
+  indices = torch.randint(0, n_col, (n_row * mean,), dtype=torch.int32, device=cuda)
+  data, events = torch.rand(n_row * mean, device=cuda), torch.rand(n_row, device=cuda) < 0.1
+  before, after = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+  before.record(), after.record()        # the events exist from their first record on
+  torch.cuda.synchronize()
+  idle = before.elapsed_time(after)
+  lib = _lib.lib()
+  lib.bpl_profile_scatter_events(ctypes.c_void_p(before.cuda_event), ctypes.c_void_p(after.cuda_event))
+  try:
+    bpl.event_csr_matvec(data, indices, indptr, events, shape=(n_row, n_col), transpose=True)
+  finally:
+    lib.bpl_profile_scatter_events(None, None)
+  torch.cuda.synchronize()
+  assert before.elapsed_time(after) != idle
