@@ -179,6 +179,7 @@ void bpl_profile_scatter_events(void *before, void *after);
  *   The same product, bit for bit, with every column's stream generated once instead of once per 32 rows of X:
  *   one pass writes the connections (position, weight) of a chunk of columns into the workspace, a second multiplies
  *   from the lists.  buffers [X T(m,k), Y T(m,n), workspace (bpl_workspace_bytes(), 256-byte aligned)]; same opaque.
+ *   The multiply's waits for its copies are bounded; a block whose copy does not arrive writes NaN for its outputs.
  * gpu_matmat_prob_prob_normal_{float,double}_{v2,v3}
  *   replace lib/gpu_jitconn_matmat.cu:138-231 (v2: 32 streams per column, one per range of ceil(k / 32) rows) and
  *   :19-135 (v3: one stream per row of X, pairs shared by a block of rows); registered lib/gpu_ops.cc:166-169.
