@@ -28,6 +28,7 @@ FLAGS = ['-O3', '-std=c++17', '-gencode', 'arch=compute_100a,code=sm_100a', '-li
 
 NATIVE_SOURCE = os.path.join(CSRC, 'native.cc')
 NATIVE = os.path.join(HERE, '_native' + sysconfig.get_config_var('EXT_SUFFIX'))
+NATIVE_STAMP = os.path.join(BUILD_DIR, 'native_torch.txt')     # the torch that NATIVE was compiled against
 CXX = os.environ.get('CXX', 'g++')
 
 
@@ -68,14 +69,27 @@ def _native_command():
            '-Wl,-rpath,$ORIGIN'])
 
 
+def _torch_stamp():
+  import torch
+  return f'{torch.__version__} abi={int(torch._C._GLIBCXX_USE_CXX11_ABI)}\n'
+
+
+def _native_stale(deps):
+  if _stale(NATIVE, deps) or not os.path.exists(NATIVE_STAMP):
+    return True
+  with open(NATIVE_STAMP) as f:
+    return f.read() != _torch_stamp()
+
+
 def _build_native(force, verbose):
-  """The extension module.  Its text depends on the C ABI only, so it is linked again when the headers change and not
-  when a kernel does.  The object goes to a temporary name first: a reader never sees half a file."""
+  """The extension module.  Its text depends on the C ABI and on torch's headers and libraries, so it is linked again when
+  those change and not when a kernel does.  The object goes to a name of this process first: a reader never sees half a
+  file, nor do two builds write one."""
   deps = [NATIVE_SOURCE, os.path.join(CSRC, 'abi.h'), os.path.join(CSRC, HEADERS[-1]), os.path.abspath(__file__)]
-  if not force and not _stale(NATIVE, deps):
+  if not force and not _native_stale(deps):
     return
   cmd = _native_command()
-  out = NATIVE + '.tmp'
+  out = f'{NATIVE}.{os.getpid()}.tmp'
   cmd[cmd.index(NATIVE)] = out
   if verbose:
     print(' '.join(cmd), flush=True)
@@ -83,6 +97,9 @@ def _build_native(force, verbose):
   if p.returncode != 0:
     raise RuntimeError(f'{CXX} failed on native.cc:\n{p.stdout}')
   os.replace(out, NATIVE)
+  os.makedirs(BUILD_DIR, exist_ok=True)
+  with open(NATIVE_STAMP, 'w') as f:
+    f.write(_torch_stamp())
 
 
 def build(force=False, verbose=False):
