@@ -428,7 +428,9 @@ bool list_scatter_shared(cudaStream_t stream, const CsrMatrix<T> &m, const E *ev
 // y = A^T events in ONE launch, for small matrices.  A launch costs the host 2.7 us, half of such a call.  Every block owns
 // a range of the columns, finds the active rows itself, reads ALL their entries (from L2, where the blocks read them side by
 // side) and adds those of its range in shared memory; y is written once and needs no zero-fill, and a column's sum is formed
-// in one place (equal weights add up to the reference's bits).  Teams of lpr lanes take a row each.
+// in one place (equal weights add up to the reference's bits).  Teams of lpr lanes take a row each, a row of more than `piece`
+// entries (four steps of a team) in pieces: how long single rows are is not known when the team is chosen, and every block
+// would wait for the longest (4096 rows, 150,000 entries, half of them in one row: 808 us by one team, 18 in pieces).
 constexpr uint32_t OWN_THREADS = 1024;
 constexpr uint32_t OWN_ROWS = 8192;
 
@@ -436,11 +438,11 @@ template<typename T, typename E, bool HOMO, bool VEC>
 __global__ void __launch_bounds__(OWN_THREADS)
 event_columns_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const E *__restrict__ events, const uint32_t n_row, const uint32_t n_col, const uint32_t nse,
-                     const uint32_t width, const uint32_t log_lpr, T *__restrict__ y) {
+                     const uint32_t width, const uint32_t log_lpr, const uint32_t piece, T *__restrict__ y) {
     extern __shared__ __align__(16) unsigned char own_smem[];
     __shared__ uint32_t n_active;
     T *sums = reinterpret_cast<T *>(own_smem);
-    uint2 *list = reinterpret_cast<uint2 *>(own_smem + static_cast<size_t>(width) * sizeof(T));    // where active rows lie
+    uint2 *list = reinterpret_cast<uint2 *>(own_smem + static_cast<size_t>(width) * sizeof(T));    // where pieces of active rows lie
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t first = blockIdx.x * width, count = min(width, n_col - first);
     if (threadIdx.x == 0) n_active = 0;
@@ -465,7 +467,13 @@ event_columns_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
             at = __shfl_sync(FULL_MASK, at, 0) + __popc(bits & ((1u << lane) - 1u));
             if (act[k]) {
                 const uint32_t row = base + k * OWN_THREADS + threadIdx.x;
-                list[at] = make_uint2(indptr[row], indptr[row + 1]);
+                const uint32_t start = indptr[row], end = indptr[row + 1];
+                list[at] = make_uint2(start, min(end, start + piece));
+                if (end - start > piece) {
+                    const uint32_t more = (end - start - 1u) / piece, from = atomicAdd(&n_active, more);
+                    for (uint32_t j = 0; j < more; ++j)
+                        list[from + j] = make_uint2(start + (j + 1u) * piece, min(end, start + (j + 2u) * piece));
+                }
             }
         }
     }
@@ -569,12 +577,15 @@ bool event_scatter_columns(cudaStream_t stream, const CsrMatrix<T> &m, const E *
     const uint32_t log_lpr = mean <= 4u * per ? 2u : mean <= 8u * per ? 3u : mean <= 16u * per ? 4u : 5u;
     const bool vec = aligned16(m.indices) && (HOMO || aligned16(m.data));
     constexpr auto wide = event_columns_kernel<T, E, HOMO, true>, narrow = event_columns_kernel<T, E, HOMO, false>;
-    constexpr unsigned most = 100u * 1024u;
+    const uint32_t piece = (4u * per) << log_lpr;
+    const size_t items = static_cast<size_t>(m.n_row) + m.nse / piece;         // of the list, at most
+    constexpr unsigned most = 110u * 1024u;                                    // (8192 rows, 108,333 doubles, 500,000 columns: 104 KB)
+    const size_t smem = width * sizeof(T) + sizeof(uint2) * items;
+    if (smem > most) return false;
     if (!(vec ? allow_shared<wide>(most) : allow_shared<narrow>(most))) return launch_ok(), true;
     if (profile_before()) cudaEventRecord(profile_before(), stream);
     const cudaError_t e = launch_dependent(vec ? wide : narrow, dim3(blocks), dim3(OWN_THREADS),
-                                           width * sizeof(T) + sizeof(uint2) * static_cast<size_t>(m.n_row), stream, m.indices, m.indptr, m.data,
-                                           events, m.n_row, m.n_col, m.nse, width, log_lpr, y);
+                                           smem, stream, m.indices, m.indptr, m.data, events, m.n_row, m.n_col, m.nse, width, log_lpr, piece, y);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
     if (profile_after()) cudaEventRecord(profile_after(), stream);
     return true;

@@ -289,3 +289,48 @@ def test_every_event_scatter_records_the_profile_events(cuda, n_row, n_col, mean
     lib.bpl_profile_scatter_events(None, None)
   torch.cuda.synchronize()
   assert before.elapsed_time(after) != idle
+
+
+# ---- rows of very different lengths: how long single rows are is not known to the rules, which see the mean only ----
+def _skewed(n_row, n_col, lens, dtype, device, seed=43):
+  g = torch.Generator(device=device).manual_seed(seed)
+  lens = torch.as_tensor(lens, device=device).long()
+  indptr = torch.cat([lens.new_zeros(1), lens.cumsum(0)]).int()
+  indices = torch.randint(0, n_col, (int(lens.sum()),), dtype=torch.int32, device=device, generator=g)
+  return torch.randn(indices.shape[0], dtype=dtype, device=device, generator=g), indices, indptr
+
+
+def _one_long_row(n_row, nse):
+  lens = np.full(n_row, nse // 2 // n_row)
+  lens[n_row // 3] += nse // 2
+  return lens
+
+
+def _device_us(call, n=10):
+  call()
+  best = float('inf')
+  for _ in range(5):
+    begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    begin.record()
+    for _ in range(n):
+      call()
+    end.record()
+    end.synchronize()
+    best = min(best, begin.elapsed_time(end) * 1e3 / n)
+  return best
+
+
+@pytest.mark.parametrize('homo', [False, True])
+@pytest.mark.parametrize('n_row,n_col', [(4096, 1000), (64, 1000), (1, 30_000)])
+def test_small_event_scatter_of_one_long_row(cuda, n_row, n_col, homo):
+  """Half of the entries in one row; a wrong list would lose or repeat pieces.  One team alone walked it in 230 us or more."""
+  data, indices, indptr = _skewed(n_row, n_col, _one_long_row(n_row, 150_000), torch.float32, cuda)
+  weights = torch.full((1,), 0.5, device=cuda) if homo else data
+  events = torch.rand(n_row, device=cuda, generator=torch.Generator(device=cuda).manual_seed(2)) < 0.2
+  events[n_row // 3] = True
+  call = lambda: bpl.event_csr_matvec(weights, indices, indptr, events, shape=(n_row, n_col), transpose=True)
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  want = torch.zeros(n_col, dtype=torch.float64, device=cuda).index_add_(
+    0, col, torch.where(events[row], weights.double().expand(indices.shape[0]), 0.))
+  torch.testing.assert_close(call().double(), want, rtol=1e-5, atol=1e-4)
+  assert _device_us(call) < 100.
