@@ -33,10 +33,11 @@ constexpr int ROW_WARPS = ROW_THREADS / 32;
 
 // How many pieces a row is cut into so that work items stay near 256 entries: keeps the
 // last wave of a persistent grid short.  Uniform over the grid (a function of the mean row length).
-__device__ __forceinline__ uint32_t pieces_per_row(uint32_t nse, uint32_t n_row) {
+constexpr uint32_t MOST_PIECES = 16;
+__host__ __device__ __forceinline__ uint32_t pieces_per_row(uint32_t nse, uint32_t n_row) {
     const uint32_t mean = n_row ? nse / n_row : 0;
     const uint32_t s = mean / 320u;
-    return s < 1u ? 1u : (s > 16u ? 16u : s);
+    return s < 1u ? 1u : (s > MOST_PIECES ? MOST_PIECES : s);
 }
 
 // Boundary h (0..S) of row [start, end) cut into S pieces; interior cuts fall on multiples of 4

@@ -334,3 +334,15 @@ def test_small_event_scatter_of_one_long_row(cuda, n_row, n_col, homo):
     0, col, torch.where(events[row], weights.double().expand(indices.shape[0]), 0.))
   torch.testing.assert_close(call().double(), want, rtol=1e-5, atol=1e-4)
   assert _device_us(call) < 100.
+
+
+def test_event_scatter_of_few_long_rows(cuda):
+  """Enough warps for the pieces of the rows (a warp for four of them took twice as long as the list-driven product)."""
+  n_row, n_col = 256, 300_000
+  data, indices, indptr = _skewed(n_row, n_col, np.full(n_row, 78_125), torch.float32, cuda)
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  events = torch.rand(n_row, device=cuda, generator=torch.Generator(device=cuda).manual_seed(2)) < 0.2
+  call = lambda: bpl.event_csr_matvec(data, indices, indptr, events, shape=(n_row, n_col), transpose=True)
+  want = torch.zeros(n_col, dtype=torch.float64, device=cuda).index_add_(0, col, torch.where(events[row], data.double(), 0.))
+  torch.testing.assert_close(call().double(), want, rtol=1e-5, atol=1e-4)
+  assert _device_us(call) < 85.
