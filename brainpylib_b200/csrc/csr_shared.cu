@@ -13,6 +13,7 @@
 // that read the same rows side by side (58 us) paid; and reading a neighbour's slice out of its shared memory moves 0.33
 // random words per clock and SM.
 #include <algorithm>
+#include <type_traits>
 
 #include "abi.h"
 #include "common.cuh"
@@ -34,12 +35,20 @@ constexpr uint32_t SHARED_SMEM = 226u * 1024u;       // the longest vector
 // entry (30 instructions each; the entries of a quad go through predicates now, and whether any lane's quad crosses the
 // ends of its row is asked once per quad and warp), and a warp that waited for a step's entries before it asked for the
 // next.  The entries of the next step, of this row or the next, are therefore requested before a step is worked on.
+//
+// The lanes of a row are chosen for the mean length.  A row that would keep them for more than 8 steps, and for more than
+// twice a warp's share of all steps, is put off: behind the walk the block takes the rows that it put off, up to BLOCK_ROW
+// entries with a warp each, longer ones with all its warps.  (Lengths with a heavy tail: 100,000 rows of 20 on average, the
+// longest 30,000, y = A^T x: 858 us by the lanes of each row.)  LONG_ROWS at most; the lanes take the rest after all.
+constexpr uint32_t LONG_ROWS = 128, BLOCK_ROW = 4096;
+
 struct Deal {
-    uint32_t lpr, rows_per_warp;
+    uint32_t lpr, rows_per_warp, long_from;
     __device__ __forceinline__ Deal(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
         const uint32_t want = (nse / n_row + per_step - 1u) / per_step;
         lpr = want <= 4u ? 4u : want <= 8u ? 8u : want <= 16u ? 16u : 32u;
         rows_per_warp = 32u / lpr;
+        long_from = max(8u * per_step, nse / (gridDim.x * SHARED_WARPS) / 16u) * lpr;
     }
     __device__ __forceinline__ uint32_t row(const uint32_t local_group, const uint32_t sub) const {
         return (local_group * gridDim.x + blockIdx.x) * rows_per_warp + sub;
@@ -56,7 +65,9 @@ constexpr uint32_t MOST_ENTRIES = 0x7fffffffu;
 //   fetch(row)                            what is needed of a row besides its entries (requested one row ahead)
 //   quad<FULL>(base, c[4], w[4], lo, hi)  entries base .. base + 3, of which lo <= e < hi belong to the row (FULL: all)
 //   entry(pos, c, w)                      one entry (the ragged end of the arrays)
-//   begin(fetched), end(row, lead)        around a row; lead: this lane speaks for it
+//   begin(fetched)                        before a row
+//   SUMS, Sum, total(lanes), put(row, s)  behind a row, where it has a result: the sum over aligned groups of lanes, and where
+//                                         one lane leaves it
 // `ready` runs before the first entry is visited, behind the first loads: it fills shared memory and ends with a barrier.
 template<typename T, bool WEIGHTS, int U, typename Visit, typename Ready>
 __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
@@ -66,6 +77,8 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
     const uint32_t sub = lane / lpr, sl = lane % lpr;
     const uint32_t g_full = nse >> 2;
     using Fetched = decltype(visit.fetch(0u));
+    __shared__ uint32_t n_long, long_row[LONG_ROWS];
+    __shared__ typename Visit::Sum part[2][SHARED_WARPS];
     struct Step {
         uint4 ix[U];
         Quad<T> w[WEIGHTS ? U : 1];
@@ -92,12 +105,28 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
             }
         }
     };
+    // a long row becomes an empty one
+    auto put_off = [&](Row &r, const uint32_t row) {
+        const bool is_long = r.end - r.start > deal.long_from;
+        if (!__any_sync(FULL_MASK, is_long)) return;
+        uint32_t at = LONG_ROWS;
+        if (is_long && sl == 0) at = atomicAdd(&n_long, 1u);
+        at = __shfl_sync(FULL_MASK, at, lane - sl);
+        if (is_long && at < LONG_ROWS) {
+            if (sl == 0) long_row[at] = row;
+            r.start = r.end = 0;
+        }
+    };
     uint32_t group = threadIdx.x >> 5;
     Row row = pointers(group), next = pointers(group + SHARED_WARPS);
+    if (threadIdx.x == 0) n_long = 0;
+    __syncthreads();
+    put_off(row, deal.row(group, sub));
     // one step: request what comes after it (`after`), then work on it
     auto step = [&](Step &now, Step &after) {
         const uint32_t g_stop = min((row.end + 3u) >> 2, g_full);
         const bool more = __any_sync(FULL_MASK, now.g0 + U * lpr < g_stop);
+        if (!more) put_off(next, deal.row(group + SHARED_WARPS, sub));
         after.g0 = more ? now.g0 + U * lpr : (next.start >> 2) + sl;
         load(after, more ? row : next);
         Row later{0u, 0u, Fetched()};
@@ -117,7 +146,10 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         if (sl == 0)
             for (uint32_t pos = max(4u * g_full, row.start); pos < row.end; ++pos)
                 visit.entry(pos, indices[pos], WEIGHTS ? data[pos] : T(0));
-        visit.end(deal.row(group, sub), sl == 0 && deal.row(group, sub) < n_row);
+        if (Visit::SUMS) {
+            const typename Visit::Sum s = visit.total(static_cast<int>(lpr));
+            if (sl == 0 && deal.row(group, sub) < n_row) visit.put(deal.row(group, sub), s);
+        }
         group += SHARED_WARPS;
         row = next;
         next = later;
@@ -138,6 +170,57 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         step(a, b);
         if (deal.row(group, 0) >= n_row) break;
         step(b, a);
+    }
+    // the rows that were put off
+    __syncthreads();
+    const uint32_t n = min(n_long, LONG_ROWS), warp = threadIdx.x >> 5;
+    auto span = [&](const uint32_t r, const uint32_t start, const uint32_t end, const uint32_t first, const uint32_t lanes) {
+        constexpr int AHEAD = sizeof(T) == 8 ? 2 : 4;
+        visit.begin(visit.fetch(r));
+        const uint32_t g_stop = min((end + 3u) >> 2, g_full);
+        for (uint32_t g0 = (start >> 2) + first; g0 < g_stop; g0 += AHEAD * lanes) {
+            uint4 ix[AHEAD];
+            Quad<T> w[WEIGHTS ? AHEAD : 1];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const uint32_t g = g0 + u * lanes;
+                if (g >= g_stop) continue;
+                ix[u] = ldg_stream_u4(indices + 4ull * g);
+                if (WEIGHTS) load_quad(data + 4ull * g, w[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const uint32_t g = g0 + u * lanes, c[4] = {ix[u].x, ix[u].y, ix[u].z, ix[u].w};
+                if (g < g_stop) visit.template quad<false>(4u * g, c, w[WEIGHTS ? u : 0].v, from_quad(start, 4u * g), from_quad(end, 4u * g));
+            }
+        }
+        if (first == 0)
+            for (uint32_t pos = max(4u * g_full, start); pos < end; ++pos) visit.entry(pos, indices[pos], WEIGHTS ? data[pos] : T(0));
+    };
+    for (uint32_t i = warp; i < n; i += SHARED_WARPS) {
+        const uint32_t r = long_row[i], start = indptr[r], end = indptr[r + 1];
+        if (end - start > BLOCK_ROW) continue;
+        span(r, start, end, lane, 32u);
+        if (Visit::SUMS) {
+            const typename Visit::Sum s = visit.total(32);
+            if (lane == 0) visit.put(r, s);
+        }
+    }
+    uint32_t turn = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t r = long_row[i], start = indptr[r], end = indptr[r + 1];
+        if (end - start <= BLOCK_ROW) continue;
+        span(r, start, end, threadIdx.x, SHARED_THREADS);
+        if (!Visit::SUMS) continue;
+        // one barrier per row: the sums of the next go to the other half, and who reads these is through at the barrier after
+        const typename Visit::Sum s = visit.total(32);
+        if (lane == 0) part[turn & 1u][warp] = s;
+        __syncthreads();
+        if (warp == turn % SHARED_WARPS) {
+            const typename Visit::Sum t = group_sum(lane < SHARED_WARPS ? part[turn & 1u][lane] : typename Visit::Sum(0), 32);
+            if (lane == 0) visit.put(r, t);
+        }
+        ++turn;
     }
 }
 
@@ -165,7 +248,6 @@ __device__ __forceinline__ void fill_words(uint32_t *shared, const uint32_t *p, 
 template<typename T, bool HOMO>
 struct GatherVisit {
     const T *xs;
-    uint32_t lpr;
     T homo_w, *y;
     T acc;
     __device__ __forceinline__ int fetch(uint32_t) const { return 0; }
@@ -177,10 +259,10 @@ struct GatherVisit {
             if (FULL || (e >= lo && e < hi)) acc += (HOMO ? homo_w : w[e]) * xs[c[e]];
     }
     __device__ __forceinline__ void entry(uint32_t, const uint32_t c, const T w) { acc += (HOMO ? homo_w : w) * xs[c]; }
-    __device__ __forceinline__ void end(const uint32_t row, const bool lead) {
-        acc = group_sum(acc, static_cast<int>(lpr));
-        if (lead) y[row] = acc;
-    }
+    static constexpr bool SUMS = true;
+    using Sum = T;
+    __device__ __forceinline__ Sum total(const int lanes) const { return group_sum(acc, lanes); }
+    __device__ __forceinline__ void put(const uint32_t row, const Sum s) const { y[row] = s; }
 };
 
 template<typename T, bool HOMO, int U>
@@ -190,7 +272,7 @@ gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
-    GatherVisit<T, HOMO> visit{xs, deal.lpr, HOMO ? data[0] : T(0), y, T(0)};
+    GatherVisit<T, HOMO> visit{xs, HOMO ? data[0] : T(0), y, T(0)};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
         fill_shared(xs, x, n_col);
         __syncthreads();
@@ -203,7 +285,6 @@ gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
 template<typename T, bool HOMO, bool BYTES>
 struct EventVisit {
     const uint32_t *mask;
-    uint32_t lpr;
     T homo_w, *y;
     T acc;
     uint32_t hits;
@@ -230,15 +311,16 @@ struct EventVisit {
         if (HOMO) hits += h;
         else if (h) acc += w;
     }
-    __device__ __forceinline__ void end(const uint32_t row, const bool lead) {
-        if (HOMO) {
-            hits = group_sum(hits, static_cast<int>(lpr));
-            // no hit leaves +0 like an empty sum (the product with a negative weight would give -0)
-            acc = hits ? static_cast<T>(static_cast<double>(hits) * static_cast<double>(homo_w)) : T(0);
-        } else {
-            acc = group_sum(acc, static_cast<int>(lpr));
-        }
-        if (lead) y[row] = acc;
+    static constexpr bool SUMS = true;
+    using Sum = std::conditional_t<HOMO, uint32_t, T>;
+    __device__ __forceinline__ Sum total(const int lanes) const {
+        if constexpr (HOMO) return group_sum(hits, lanes);
+        else return group_sum(acc, lanes);
+    }
+    __device__ __forceinline__ void put(const uint32_t row, const Sum s) const {
+        // no hit leaves +0 like an empty sum (the product with a negative weight would give -0)
+        if constexpr (HOMO) y[row] = s ? static_cast<T>(static_cast<double>(s) * static_cast<double>(homo_w)) : T(0);
+        else y[row] = s;
     }
 };
 
@@ -264,7 +346,7 @@ gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
-    EventVisit<T, HOMO, BYTES> visit{mask, deal.lpr, HOMO ? data[0] : T(0), y, T(0), 0u};
+    EventVisit<T, HOMO, BYTES> visit{mask, HOMO ? data[0] : T(0), y, T(0), 0u};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
         if (BYTES) {
             fill_bytes(shared_vector, events, n_col);
@@ -396,7 +478,10 @@ struct ScatterVisit {
             if (FULL || (e >= lo && e < hi)) atomicAdd(sums + c[e], (HOMO ? homo_w : w[e]) * scale);
     }
     __device__ __forceinline__ void entry(uint32_t, const uint32_t c, const T w) { atomicAdd(sums + c, (HOMO ? homo_w : w) * scale); }
-    __device__ __forceinline__ void end(uint32_t, bool) {}
+    static constexpr bool SUMS = false;
+    using Sum = T;
+    __device__ __forceinline__ Sum total(int) const { return T(0); }
+    __device__ __forceinline__ void put(uint32_t, Sum) const {}
 };
 
 template<typename T, bool HOMO, int U>
@@ -438,7 +523,10 @@ struct OuterVisit {
         }
     }
     __device__ __forceinline__ void entry(const uint32_t pos, const uint32_t c, T) { g[pos] = r * xs[c]; }
-    __device__ __forceinline__ void end(uint32_t, bool) {}
+    static constexpr bool SUMS = false;
+    using Sum = T;
+    __device__ __forceinline__ Sum total(int) const { return T(0); }
+    __device__ __forceinline__ void put(uint32_t, Sum) const {}
 };
 
 template<typename T, int U>
