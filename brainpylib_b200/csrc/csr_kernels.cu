@@ -455,6 +455,7 @@ event_columns_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     constexpr int PER = 4;
     for (uint32_t base = 0; base < n_row; base += PER * OWN_THREADS) {
         bool act[PER];
+        uint32_t at[PER], start[PER], end[PER];            // (all loads of the four before a branch on any: 0.6 us)
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             const uint32_t i = base + k * OWN_THREADS + threadIdx.x;
@@ -462,20 +463,31 @@ event_columns_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
         }
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
+            start[k] = end[k] = 0;
             const uint32_t bits = __ballot_sync(FULL_MASK, act[k]);
             if (bits == 0) continue;
-            uint32_t at = 0;
-            if (lane == 0) at = atomicAdd(&n_active, static_cast<uint32_t>(__popc(bits)));
-            at = __shfl_sync(FULL_MASK, at, 0) + __popc(bits & ((1u << lane) - 1u));
+            uint32_t first = 0;
+            if (lane == 0) first = atomicAdd(&n_active, static_cast<uint32_t>(__popc(bits)));
+            at[k] = __shfl_sync(FULL_MASK, first, 0) + __popc(bits & ((1u << lane) - 1u));
             if (act[k]) {
                 const uint32_t row = base + k * OWN_THREADS + threadIdx.x;
-                const uint32_t start = indptr[row], end = indptr[row + 1];
-                list[at] = make_uint2(start, min(end, start + piece));
-                if (end - start > piece) {
-                    const uint32_t more = (end - start - 1u) / piece, from = atomicAdd(&n_active, more);
-                    for (uint32_t j = 0; j < more; ++j)
-                        list[from + j] = make_uint2(start + (j + 1u) * piece, min(end, start + (j + 2u) * piece));
-                }
+                start[k] = indptr[row];
+                end[k] = indptr[row + 1];
+            }
+        }
+        bool pieces = false;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            if (act[k]) list[at[k]] = make_uint2(start[k], min(end[k], start[k] + piece));
+            pieces |= end[k] - start[k] > piece;
+        }
+        if (pieces) {
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                if (end[k] - start[k] <= piece) continue;
+                const uint32_t more = (end[k] - start[k] - 1u) / piece, from = atomicAdd(&n_active, more);
+                for (uint32_t j = 0; j < more; ++j)
+                    list[from + j] = make_uint2(start[k] + (j + 1u) * piece, min(end[k], start[k] + (j + 2u) * piece));
             }
         }
     }

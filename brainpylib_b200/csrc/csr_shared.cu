@@ -37,21 +37,32 @@ constexpr uint32_t SHARED_SMEM = 226u * 1024u;       // the longest vector
 // next.  The entries of the next step, of this row or the next, are therefore requested before a step is worked on.
 //
 // The lanes of a row are chosen for the mean length.  A row that would keep them for more than 8 steps, and for more than
-// twice a warp's share of all steps, is put off: behind the walk the block takes the rows that it put off, up to BLOCK_ROW
-// entries with a warp each, longer ones with all its warps.  (Lengths with a heavy tail: 100,000 rows of 20 on average, the
-// longest 30,000, y = A^T x: 858 us by the lanes of each row.)  LONG_ROWS at most; the lanes take the rest after all.
+// twice a warp's share of all steps, is cut there (`long_from`).  Behind its walk a warp takes its cut rows with all its
+// lanes; those of more than BLOCK_ROW entries (LONG_ROWS of them at most) are left to all warps of the block.  (Lengths with a
+// heavy tail: 100,000 rows of 20 on average, the longest 30,000, y = A^T x: 858 us by the lanes of each row.  A test of every
+// row's length inside the walk, with a branch to a list, cost the event gather 1 to 5 us of 21.)
 constexpr uint32_t LONG_ROWS = 128, BLOCK_ROW = 4096;
 
+inline __host__ __device__ uint32_t lanes_per_row(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
+    const uint32_t want = (nse / n_row + per_step - 1u) / per_step;
+    return want <= 4u ? 4u : want <= 8u ? 8u : want <= 16u ? 16u : 32u;
+}
+inline uint32_t long_rows_from(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
+    const uint32_t share = nse / (static_cast<uint32_t>(sm_count()) * SHARED_WARPS);
+    return std::max(8u * per_step, share / 16u) * lanes_per_row(nse, n_row, per_step);
+}
 struct Deal {
-    uint32_t lpr, rows_per_warp, long_from;
+    uint32_t lpr, rows_per_warp;
     __device__ __forceinline__ Deal(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
-        const uint32_t want = (nse / n_row + per_step - 1u) / per_step;
-        lpr = want <= 4u ? 4u : want <= 8u ? 8u : want <= 16u ? 16u : 32u;
+        lpr = lanes_per_row(nse, n_row, per_step);
         rows_per_warp = 32u / lpr;
-        long_from = max(8u * per_step, nse / (gridDim.x * SHARED_WARPS) / 16u) * lpr;
     }
     __device__ __forceinline__ uint32_t row(const uint32_t local_group, const uint32_t sub) const {
         return (local_group * gridDim.x + blockIdx.x) * rows_per_warp + sub;
+    }
+    // the i-th row that a warp walks (in an order of its groups)
+    __device__ __forceinline__ uint32_t row_of_warp(const uint32_t warp, const uint32_t i) const {
+        return row(warp + (i >> (__ffs(rows_per_warp) - 1)) * SHARED_WARPS, i & (rows_per_warp - 1u));
     }
 };
 
@@ -68,17 +79,109 @@ constexpr uint32_t MOST_ENTRIES = 0x7fffffffu;
 //   begin(fetched)                        before a row
 //   SUMS, Sum, total(lanes), put(row, s)  behind a row, where it has a result: the sum over aligned groups of lanes, and where
 //                                         one lane leaves it
+// (Behind the vector in dynamic shared memory: with static shared memory in the kernel the vector no longer lies at the address
+// 0, and every look-up adds its base: 2 us of the event gather's 20.)
+template<typename Sum>
+struct CutRows {
+    uint32_t n, row[LONG_ROWS];
+    bool block[SHARED_WARPS];          // a warp has rows of more than BLOCK_ROW
+    Sum part[2][SHARED_WARPS];
+};
+
+inline __host__ __device__ uint32_t behind_vector(const size_t bytes) { return static_cast<uint32_t>((bytes + 15u) & ~static_cast<size_t>(15u)); }
+template<typename Sum>
+__device__ __forceinline__ CutRows<Sum> &cut_rows_at(unsigned char *shared, const size_t bytes) {
+    return *reinterpret_cast<CutRows<Sum> *>(shared + behind_vector(bytes));
+}
+template<typename Sum>
+uint32_t shared_bytes(const size_t vector_bytes) { return behind_vector(vector_bytes) + sizeof(CutRows<Sum>); }
+constexpr uint32_t ALL_SMEM = 227u * 1024u;
+static_assert(SHARED_SMEM + sizeof(CutRows<double>) <= ALL_SMEM, "the longest vector and the list");
+
+// The rows that the walk has cut; `mine`: this warp has some, `block`: some warps of the block have rows for all of it.
+template<typename T, bool WEIGHTS, typename Visit>
+__device__ __noinline__ void walk_cut_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
+                                           const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
+                                           const uint32_t long_from, const Deal deal, Visit visit, const bool mine, const bool block,
+                                           CutRows<typename Visit::Sum> &cut_rows) {
+    const uint32_t lane = threadIdx.x & 31, g_full = nse >> 2;
+    auto span = [&](const uint32_t r, const uint32_t start, const uint32_t end, const uint32_t first, const uint32_t lanes) {
+        constexpr int AHEAD = sizeof(T) == 8 ? 2 : 4;
+        visit.begin(visit.fetch(r));
+        const uint32_t g_stop = min((end + 3u) >> 2, g_full);
+        for (uint32_t g0 = (start >> 2) + first; g0 < g_stop; g0 += AHEAD * lanes) {
+            uint4 ix[AHEAD];
+            Quad<T> w[WEIGHTS ? AHEAD : 1];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const uint32_t g = g0 + u * lanes;
+                if (g >= g_stop) continue;
+                ix[u] = ldg_stream_u4(indices + 4ull * g);
+                if (WEIGHTS) load_quad(data + 4ull * g, w[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const uint32_t g = g0 + u * lanes, c[4] = {ix[u].x, ix[u].y, ix[u].z, ix[u].w};
+                if (g < g_stop) visit.template quad<false>(4u * g, c, w[WEIGHTS ? u : 0].v, from_quad(start, 4u * g), from_quad(end, 4u * g));
+            }
+        }
+        if (first == 0)
+            for (uint32_t pos = max(4u * g_full, start); pos < end; ++pos) visit.entry(pos, indices[pos], WEIGHTS ? data[pos] : T(0));
+    };
+    const uint32_t warp = threadIdx.x >> 5, skip = Visit::SUMS ? 0u : long_from;     // (a sum is taken again as a whole)
+    __syncwarp();                                          // (its results are replaced by other lanes)
+    for (uint32_t i = 0; mine && deal.row_of_warp(warp, i) < n_row; i += 32u) {     // the warp's rows again, one per lane
+        const uint32_t r = deal.row_of_warp(warp, i + lane);
+        const uint32_t start = r < n_row ? indptr[r] : 0u, end = r < n_row ? indptr[r + 1] : 0u;
+        for (uint32_t some = __ballot_sync(FULL_MASK, end - start > long_from); some; some &= some - 1u) {
+            const int l = __ffs(some) - 1;
+            const uint32_t r0 = __shfl_sync(FULL_MASK, r, l), s0 = __shfl_sync(FULL_MASK, start, l), e0 = __shfl_sync(FULL_MASK, end, l);
+            uint32_t at = LONG_ROWS;
+            if (e0 - s0 > BLOCK_ROW) {
+                if (lane == 0) at = atomicAdd(&cut_rows.n, 1u);
+                at = __shfl_sync(FULL_MASK, at, 0);
+            }
+            if (at < LONG_ROWS) {
+                if (lane == 0) cut_rows.row[at] = r0;
+                continue;
+            }
+            span(r0, s0 + skip, e0, lane, 32u);
+            if (Visit::SUMS) {
+                const typename Visit::Sum s = visit.total(32);
+                if (lane == 0) visit.put(r0, s);
+            }
+        }
+    }
+    if (!block) return;
+    __syncthreads();
+    const uint32_t n = min(cut_rows.n, LONG_ROWS);
+    uint32_t turn = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t r = cut_rows.row[i];
+        span(r, indptr[r] + skip, indptr[r + 1], threadIdx.x, SHARED_THREADS);
+        if (!Visit::SUMS) continue;
+        // one barrier per row: the sums of the next go to the other half, and who reads these is through at the barrier after
+        const typename Visit::Sum s = visit.total(32);
+        if (lane == 0) cut_rows.part[turn & 1u][warp] = s;
+        __syncthreads();
+        if (warp == turn % SHARED_WARPS) {
+            const typename Visit::Sum t = group_sum(lane < SHARED_WARPS ? cut_rows.part[turn & 1u][lane] : typename Visit::Sum(0), 32);
+            if (lane == 0) visit.put(r, t);
+        }
+        ++turn;
+    }
+}
+
 // `ready` runs before the first entry is visited, behind the first loads: it fills shared memory and ends with a barrier.
 template<typename T, bool WEIGHTS, int U, typename Visit, typename Ready>
 __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                                           const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
-                                          const Deal deal, Visit &visit, Ready ready) {
+                                          const uint32_t long_from, const Deal deal, Visit &visit,
+                                          CutRows<typename Visit::Sum> &cut_rows, Ready ready) {
     const uint32_t lane = threadIdx.x & 31, lpr = deal.lpr;
     const uint32_t sub = lane / lpr, sl = lane % lpr;
     const uint32_t g_full = nse >> 2;
     using Fetched = decltype(visit.fetch(0u));
-    __shared__ uint32_t n_long, long_row[LONG_ROWS];
-    __shared__ typename Visit::Sum part[2][SHARED_WARPS];
     struct Step {
         uint4 ix[U];
         Quad<T> w[WEIGHTS ? U : 1];
@@ -105,28 +208,16 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
             }
         }
     };
-    // a long row becomes an empty one
-    auto put_off = [&](Row &r, const uint32_t row) {
-        const bool is_long = r.end - r.start > deal.long_from;
-        if (!__any_sync(FULL_MASK, is_long)) return;
-        uint32_t at = LONG_ROWS;
-        if (is_long && sl == 0) at = atomicAdd(&n_long, 1u);
-        at = __shfl_sync(FULL_MASK, at, lane - sl);
-        if (is_long && at < LONG_ROWS) {
-            if (sl == 0) long_row[at] = row;
-            r.start = r.end = 0;
-        }
-    };
+    auto cut = [&](Row &r) { r.end = min(r.end, r.start + long_from); };     // (where the pointers are needed, not where they are asked for)
     uint32_t group = threadIdx.x >> 5;
     Row row = pointers(group), next = pointers(group + SHARED_WARPS);
-    if (threadIdx.x == 0) n_long = 0;
-    __syncthreads();
-    put_off(row, deal.row(group, sub));
+    cut(row);
+    cut(next);
+    if (threadIdx.x == 0) cut_rows.n = 0;
     // one step: request what comes after it (`after`), then work on it
     auto step = [&](Step &now, Step &after) {
         const uint32_t g_stop = min((row.end + 3u) >> 2, g_full);
         const bool more = __any_sync(FULL_MASK, now.g0 + U * lpr < g_stop);
-        if (!more) put_off(next, deal.row(group + SHARED_WARPS, sub));
         after.g0 = more ? now.g0 + U * lpr : (next.start >> 2) + sl;
         load(after, more ? row : next);
         Row later{0u, 0u, Fetched()};
@@ -153,6 +244,7 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         group += SHARED_WARPS;
         row = next;
         next = later;
+        cut(next);
         visit.begin(row.fetched);
     };
     Step a, b;
@@ -164,6 +256,26 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         for (int e = 0; e < 4; ++e) a.w[u].v[e] = b.w[u].v[e] = T(0);
     a.g0 = (row.start >> 2) + sl;
     load(a, row);
+    // Has the warp rows that it will cut?  Asked here, where the answer comes with what the warp waits for anyway: behind the
+    // walk it took 2 us of the event gather's 21.
+    const uint32_t warp = threadIdx.x >> 5;
+    bool some_cut = false, for_block = false;
+    for (uint32_t i = 0; deal.row_of_warp(warp, i) < n_row; i += 128u) {
+        uint32_t length[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t r = deal.row_of_warp(warp, i + 32u * k + lane);
+            length[k] = r < n_row ? indptr[r + 1] - indptr[r] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            some_cut |= length[k] > long_from;
+            for_block |= length[k] > max(long_from, BLOCK_ROW);
+        }
+    }
+    some_cut = __any_sync(FULL_MASK, some_cut);
+    for_block = __any_sync(FULL_MASK, for_block);
+    if (lane == 0) cut_rows.block[warp] = for_block;
     ready();
     visit.begin(row.fetched);
     while (deal.row(group, 0) < n_row) {
@@ -171,57 +283,9 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         if (deal.row(group, 0) >= n_row) break;
         step(b, a);
     }
-    // the rows that were put off
-    __syncthreads();
-    const uint32_t n = min(n_long, LONG_ROWS), warp = threadIdx.x >> 5;
-    auto span = [&](const uint32_t r, const uint32_t start, const uint32_t end, const uint32_t first, const uint32_t lanes) {
-        constexpr int AHEAD = sizeof(T) == 8 ? 2 : 4;
-        visit.begin(visit.fetch(r));
-        const uint32_t g_stop = min((end + 3u) >> 2, g_full);
-        for (uint32_t g0 = (start >> 2) + first; g0 < g_stop; g0 += AHEAD * lanes) {
-            uint4 ix[AHEAD];
-            Quad<T> w[WEIGHTS ? AHEAD : 1];
-#pragma unroll
-            for (int u = 0; u < AHEAD; ++u) {
-                const uint32_t g = g0 + u * lanes;
-                if (g >= g_stop) continue;
-                ix[u] = ldg_stream_u4(indices + 4ull * g);
-                if (WEIGHTS) load_quad(data + 4ull * g, w[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < AHEAD; ++u) {
-                const uint32_t g = g0 + u * lanes, c[4] = {ix[u].x, ix[u].y, ix[u].z, ix[u].w};
-                if (g < g_stop) visit.template quad<false>(4u * g, c, w[WEIGHTS ? u : 0].v, from_quad(start, 4u * g), from_quad(end, 4u * g));
-            }
-        }
-        if (first == 0)
-            for (uint32_t pos = max(4u * g_full, start); pos < end; ++pos) visit.entry(pos, indices[pos], WEIGHTS ? data[pos] : T(0));
-    };
-    for (uint32_t i = warp; i < n; i += SHARED_WARPS) {
-        const uint32_t r = long_row[i], start = indptr[r], end = indptr[r + 1];
-        if (end - start > BLOCK_ROW) continue;
-        span(r, start, end, lane, 32u);
-        if (Visit::SUMS) {
-            const typename Visit::Sum s = visit.total(32);
-            if (lane == 0) visit.put(r, s);
-        }
-    }
-    uint32_t turn = 0;
-    for (uint32_t i = 0; i < n; ++i) {
-        const uint32_t r = long_row[i], start = indptr[r], end = indptr[r + 1];
-        if (end - start <= BLOCK_ROW) continue;
-        span(r, start, end, threadIdx.x, SHARED_THREADS);
-        if (!Visit::SUMS) continue;
-        // one barrier per row: the sums of the next go to the other half, and who reads these is through at the barrier after
-        const typename Visit::Sum s = visit.total(32);
-        if (lane == 0) part[turn & 1u][warp] = s;
-        __syncthreads();
-        if (warp == turn % SHARED_WARPS) {
-            const typename Visit::Sum t = group_sum(lane < SHARED_WARPS ? part[turn & 1u][lane] : typename Visit::Sum(0), 32);
-            if (lane == 0) visit.put(r, t);
-        }
-        ++turn;
-    }
+    for_block = __any_sync(FULL_MASK, lane < SHARED_WARPS && cut_rows.block[lane]);
+    if (some_cut || for_block)
+        walk_cut_rows<T, WEIGHTS>(indices, indptr, data, n_row, nse, long_from, deal, visit, some_cut, for_block, cut_rows);
 }
 
 // The first `count` elements of x into shared memory, by the whole block.
@@ -268,12 +332,14 @@ struct GatherVisit {
 template<typename T, bool HOMO, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
-                     const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col) {
+                     const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col,
+                     const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
     GatherVisit<T, HOMO> visit{xs, HOMO ? data[0] : T(0), y, T(0)};
-    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
+    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         fill_shared(xs, x, n_col);
         __syncthreads();
     });
@@ -324,16 +390,22 @@ struct EventVisit {
     }
 };
 
-// One byte per event, 0 or 1, 16 bytes of events per load where they are aligned.
+// One byte per event, 0 or 1, 16 bytes of events per load where they are aligned, and their bytes in one store (single bytes
+// meet in the banks).
 template<typename E>
 __device__ __forceinline__ void fill_bytes(uint8_t *bytes, const E *__restrict__ events, const uint32_t n) {
     constexpr uint32_t PER = 16 / sizeof(E);
     const uint32_t whole = aligned16_device(events) ? n / PER : 0u;
+#pragma unroll 4
     for (uint32_t i = threadIdx.x; i < whole; i += blockDim.x) {
         const uint4 raw = *reinterpret_cast<const uint4 *>(events + i * PER);
         const E *e = reinterpret_cast<const E *>(&raw);
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-        for (uint32_t k = 0; k < PER; ++k) bytes[i * PER + k] = is_event(e[k]) ? 1 : 0;
+        for (uint32_t k = 0; k < PER; ++k) w[k / 4] |= (is_event(e[k]) ? 1u : 0u) << (8u * (k % 4));
+        if (PER == 16) reinterpret_cast<uint4 *>(bytes)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        else if (PER == 4) reinterpret_cast<uint32_t *>(bytes)[i] = w[0];
+        else reinterpret_cast<uint16_t *>(bytes)[i] = static_cast<uint16_t>(w[0]);
     }
     for (uint32_t i = whole * PER + threadIdx.x; i < n; i += blockDim.x) bytes[i] = is_event(events[i]) ? 1 : 0;
 }
@@ -342,12 +414,14 @@ template<typename T, typename E, bool HOMO, bool BYTES, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const E *__restrict__ events, const uint32_t *packed, T *__restrict__ y, const uint32_t n_row,
-                     const uint32_t nse, const uint32_t n_col) {
+                     const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
+    using Sum = typename EventVisit<T, HOMO, BYTES>::Sum;
+    auto &cut_rows = cut_rows_at<Sum>(shared_vector, BYTES ? n_col : (n_col + 31u) / 32u * 4u);
     EventVisit<T, HOMO, BYTES> visit{mask, HOMO ? data[0] : T(0), y, T(0), 0u};
-    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
+    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         if (BYTES) {
             fill_bytes(shared_vector, events, n_col);
         } else if (packed != nullptr) {
@@ -488,12 +562,13 @@ template<typename T, bool HOMO, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                       const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse,
-                      const uint32_t n_col) {
+                      const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *sums = reinterpret_cast<T *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
     ScatterVisit<T, HOMO> visit{sums, n_row, x, HOMO ? data[0] : T(0), T(0)};
-    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, deal, visit, [&]() {
+    walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         for (uint32_t i = threadIdx.x; i < n_col; i += SHARED_THREADS) sums[i] = T(0);
         __syncthreads();
     });
@@ -533,12 +608,13 @@ template<typename T, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                     const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g,
-                    const uint32_t n_row, const uint32_t nse, const uint32_t n_col) {
+                    const uint32_t n_row, const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
     OuterVisit<T> visit{xs, row_vector, g, n_row, T(0)};
-    walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, deal, visit, [&]() {
+    walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         fill_shared(xs, col_vector, n_col);
         zero_outside_rows(g, indptr, n_row, nse);
         __syncthreads();
@@ -589,22 +665,25 @@ template<typename T> constexpr uint32_t BANDS_FROM = sizeof(T) == 4 ? 51200u : 2
 
 template<typename T, bool HOMO>
 bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
-    constexpr auto kernel = gather_shared_kernel<T, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    constexpr int U = sizeof(T) == 8 ? 1 : 2;
+    constexpr auto kernel = gather_shared_kernel<T, HOMO, U>;
     if (m.n_col > BANDS_FROM<T> && bands<T, HOMO, false>(stream, m, m.data, x, y)) return true;
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, m.data, x, y,
-                                                                                             m.n_row, m.nse, m.n_col);
+    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
+        m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
     launch_ok();
     return true;
 }
 
 template<typename T, typename E, bool HOMO>
 bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *workspace, T *y) {
-    constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, sizeof(T) == 8 ? 1 : 2>;
-    constexpr auto kernel_bytes = gather_events_kernel<T, E, HOMO, true, sizeof(T) == 8 ? 1 : 2>;
+    constexpr int U = sizeof(T) == 8 ? 1 : 2;
+    constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, U>;
+    constexpr auto kernel_bytes = gather_events_kernel<T, E, HOMO, true, U>;
+    using Sum = std::conditional_t<HOMO, uint32_t, T>;
     const uint32_t bytes = (m.n_col + 31u) / 32u * 4u;
     if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.nse > MOST_ENTRIES || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
         (!HOMO && !aligned16(m.data)))
@@ -618,53 +697,57 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     const double mean_row = static_cast<double>(m.nse) / m.n_row;
     if (HOMO && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
-    if (!allow_shared<kernel>(SHARED_SMEM) || !allow_shared<kernel_bytes>(SHARED_SMEM)) return launch_ok(), true;
-    const uint32_t sms = static_cast<uint32_t>(sm_count());
+    if (!allow_shared<kernel>(ALL_SMEM) || !allow_shared<kernel_bytes>(ALL_SMEM)) return launch_ok(), true;
+    const uint32_t sms = static_cast<uint32_t>(sm_count()), long_from = long_rows_from(m.nse, m.n_row, 4 * U);
     // Bytes take the vector's own length from L1, which streams the entries: 200 KB of them 157 us for 1e8 entries, bits 143.
     if (m.n_col <= 131072u && m.n_col * sizeof(E) / 34.0 < (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0) + 0.08 * per) {
-        kernel_bytes<<<sms, SHARED_THREADS, m.n_col, stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col);
+        kernel_bytes<<<sms, SHARED_THREADS, shared_bytes<Sum>(m.n_col), stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col,
+                                                              long_from);
         launch_ok();
         return true;
     }
     if (!pack) {
-        kernel<<<sms, SHARED_THREADS, bytes, stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col);
+        kernel<<<sms, SHARED_THREADS, shared_bytes<Sum>(bytes), stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col,
+                                                              long_from);
         launch_ok();
         return true;
     }
     pack_events_kernel<E><<<std::min<uint32_t>((m.n_col + 255u) / 256u, 8u * sms), 256, 0, stream>>>(events, workspace, m.n_col);
     if (!launch_ok()) return true;
-    const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(SHARED_THREADS), bytes, stream, m.indices, m.indptr, m.data,
-                                           events, workspace, y, m.n_row, m.nse, m.n_col);
+    const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(SHARED_THREADS), shared_bytes<Sum>(bytes), stream, m.indices, m.indptr, m.data,
+                                           events, workspace, y, m.n_row, m.nse, m.n_col, long_from);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
     return true;
 }
 
 template<typename T, bool HOMO>
 bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
-    constexpr auto kernel = scatter_shared_kernel<T, HOMO, sizeof(T) == 8 ? 1 : 2>;
+    constexpr int U = sizeof(T) == 8 ? 1 : 2;
+    constexpr auto kernel = scatter_shared_kernel<T, HOMO, U>;
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     // a reduction into L2: slower the fewer columns share them (20,000 columns 3.1 clocks, 2000 columns 13), and in double
     const double words = sizeof(T) / 4, reduction = (1.85 + 25000.0 / m.n_col) * (sizeof(T) == 8 ? 1.25 : 1.0);
     if (p.fill + 0.3 * words * m.n_col + p.per * (p.entry + 0.3 * words) > 0.95 * (reduction * p.per + 1500)) return false;
     if (cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(m.n_col), stream) != cudaSuccess) return launch_ok(), true;
-    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, m.data, x, y,
-                                                                                             m.n_row, m.nse, m.n_col);
+    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
+        m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
     launch_ok();
     return true;
 }
 
 template<typename T>
 bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g) {
-    constexpr auto kernel = outer_shared_kernel<T, 2>;
+    constexpr int U = 2;
+    constexpr auto kernel = outer_shared_kernel<T, U>;
     if (m.n_col > BANDS_FROM<T> && bands<T, true, true>(stream, m, row_vector, col_vector, g)) return true;
     if (!usable(m, false) || !aligned16(g)) return false;
     const Plan<T> p(m, true);                // one index in, one value out
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    if (!allow_shared<kernel>(SHARED_SMEM)) return launch_ok(), true;
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, m.n_col * sizeof(T), stream>>>(m.indices, m.indptr, row_vector,
-                                                                                             col_vector, g, m.n_row, m.nse, m.n_col);
+    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
+        m.indices, m.indptr, row_vector, col_vector, g, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
     launch_ok();
     return true;
 }

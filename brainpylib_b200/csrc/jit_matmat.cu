@@ -309,7 +309,7 @@ jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k,
     }
     if (lost) {                                                          // never seen: no result rather than a wrong one
         // the copies that may be in flight, each by the phase of its own tile (one that was never started runs the wait out)
-        for (unsigned int t = landed; t < min(landed + RING, n_tiles); ++t) barrier_wait(&landed_bar[t % RING], (t / RING) & 1u);
+        for (unsigned int i = 0; i < RING; ++i) barrier_wait(&landed_bar[i], ((landed + (i - landed) % RING) / RING) & 1u);
 #pragma unroll
         for (int i = 0; i < static_cast<int>(MM_ROWS); ++i) sum[i] = T(CUDART_NAN_F);
     }

@@ -208,7 +208,8 @@ event_scatter_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
     const uint32_t nse = indptr[n_row], S = pieces_per_row(nse, n_row);
     const T homo_w = HOMO ? data[0] : T(0);
     const uint32_t n_items = n_groups * S, n_warps = gridDim.x * ROW_WARPS;
-    for (uint32_t item = blockIdx.x * ROW_WARPS + (threadIdx.x >> 5); item < n_items; item += n_warps) {
+    // neighbouring items, a row's pieces, in different blocks
+    for (uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; item < n_items; item += n_warps) {
         const uint32_t group = item / S, h = item % S;
         const uint64_t row = group + static_cast<uint64_t>(lane) * n_groups;
         uint32_t a = 0, b = 0;

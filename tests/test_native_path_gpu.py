@@ -346,3 +346,60 @@ def test_event_scatter_of_few_long_rows(cuda):
   want = torch.zeros(n_col, dtype=torch.float64, device=cuda).index_add_(0, col, torch.where(events[row], data.double(), 0.))
   torch.testing.assert_close(call().double(), want, rtol=1e-5, atol=1e-4)
   assert _device_us(call) < 85.
+
+
+def _uneven(kind):
+  if kind == 'shared':           # a block full of cut rows, one of several warps' worth, two for the block
+    n_row, n_col, lens = 150_000, 3000, np.full(150_000, 20)
+    block = (np.arange(n_row) // 8) % 148 == 5
+    lens[np.flatnonzero(block)[::6][:160]] = 401
+    lens[[7, 77_777]] = 30_011, 4099
+  elif kind == 'shared_many':    # more rows for a block than it has room for
+    n_row, n_col, lens = 150_000, 3000, np.full(150_000, 20)
+    lens[np.flatnonzero((np.arange(n_row) // 8) % 148 == 5)[::6][:140]] = 4501
+  else:                          # fewer rows than warps, each long
+    n_row, n_col, lens = 60, 9001, np.full(60, 8003)
+    lens[5] = 0
+  return n_row, n_col, lens
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('homo', [False, True])
+@pytest.mark.parametrize('kind', ['shared', 'shared_many', 'shared_few'])
+def test_products_of_rows_of_very_different_lengths(cuda, kind, homo, dtype):
+  n_row, n_col, lens = _uneven(kind)
+  data, indices, indptr = _skewed(n_row, n_col, lens, dtype, cuda)
+  data = data[:1].clone() if homo else data
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  g = torch.Generator(device=cuda).manual_seed(47)
+  w = data.double().expand(indices.shape[0])
+  tol = dict(rtol=1e-5, atol=1e-3) if dtype == torch.float32 else dict(rtol=1e-12, atol=1e-10)
+  for transpose in (False, True):
+    n_in, n_out, src, dst = (n_row, n_col, row, col) if transpose else (n_col, n_row, col, row)
+    x = torch.randn(n_in, dtype=dtype, device=cuda, generator=g)
+    d = data.clone().requires_grad_(not homo)
+    y = bpl.csr_matvec(d, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
+    want = torch.zeros(n_out, dtype=torch.float64, device=cuda).index_add_(0, dst, w * x[src].double())
+    torch.testing.assert_close(y.detach().double(), want, **tol)
+    if not homo:
+      ct = torch.randn(n_out, dtype=dtype, device=cuda, generator=g)
+      torch.testing.assert_close(torch.autograd.grad(y, d, ct)[0], ct[dst] * x[src])
+    events = x > 0.5
+    y = bpl.event_csr_matvec(data, indices, indptr, events, shape=(n_row, n_col), transpose=transpose)
+    want = torch.zeros(n_out, dtype=torch.float64, device=cuda).index_add_(0, dst, torch.where(events[src], w, 0.))
+    torch.testing.assert_close(y.double(), want, **tol)
+
+
+# Bounds several times above what the calls take, far below what the lanes of single rows would (0.9 to 7 ms).
+@pytest.mark.parametrize('n_row,n_col,op,bound', [(100_000, 30_000, 'transposed', 350.)])
+def test_time_of_a_product_with_a_long_row(cuda, n_row, n_col, op, bound):
+  lens = np.full(n_row, 2_000_000 // n_row)
+  lens[n_row // 3] = min(n_col, 250_000)
+  data, indices, indptr = _skewed(n_row, n_col, lens, torch.float32, cuda)
+  x, xt = torch.rand(n_col, device=cuda), torch.rand(n_row, device=cuda)
+  data.requires_grad_(op == 'gradient')
+  y = bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col))
+  call = {'transposed': lambda: bpl.csr_matvec(data, indices, indptr, xt, shape=(n_row, n_col), transpose=True),
+          'product': lambda: bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col)),
+          'gradient': lambda: torch.autograd.grad(y, data, xt, retain_graph=True)}[op]
+  assert _device_us(call) < bound
