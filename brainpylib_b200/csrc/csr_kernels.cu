@@ -156,25 +156,27 @@ csr_outer_kernel(const T *__restrict__ row_vector, const T *__restrict__ col_vec
     const uint32_t sub = lane / lpr, sl = lane % lpr;
     const uint64_t n_warps = static_cast<uint64_t>(gridDim.x) * ROW_WARPS;
     const uint64_t n_groups = (static_cast<uint64_t>(n_row) + rows_per_warp - 1) / rows_per_warp;
+    // A row that would keep its lanes for more than 8 steps, and for more than twice a warp's share of all, is put off and
+    // taken by the whole block (20,000 rows, 2e6 entries, 300,000 of them in one row: 4.8 ms by the lanes of each row).
+    constexpr uint32_t LONG_ROWS = 256;
+    __shared__ uint32_t n_long, long_row[LONG_ROWS];
+    const uint32_t long_from = max(128u, nse / (gridDim.x * ROW_WARPS) / 16u) * lpr;
     const uint32_t g_full = nse >> 2;
     constexpr int UNROLL = 4;
-    for (uint64_t wg = static_cast<uint64_t>(blockIdx.x) * ROW_WARPS + (threadIdx.x >> 5); wg < n_groups; wg += n_warps) {
-        const uint64_t row = wg * rows_per_warp + sub;
-        if (row >= n_row) continue;
-        const uint32_t start = indptr[row], end = indptr[row + 1];
-        const T r = row_vector[row];
+    // entries [start, end) by every `lanes`-th of some threads, the `first` this one
+    auto span = [&](const uint32_t start, const uint32_t end, const T r, const uint32_t first, const uint32_t lanes) {
         if (VEC) {
             const uint32_t g_end = (end + 3u) >> 2;
-            for (uint32_t g0 = (start >> 2) + sl; g0 < g_end; g0 += lpr * UNROLL) {
+            for (uint32_t g0 = (start >> 2) + first; g0 < g_end; g0 += lanes * UNROLL) {
                 uint4 ix[UNROLL];
 #pragma unroll
                 for (int u = 0; u < UNROLL; ++u) {
-                    const uint32_t q = g0 + u * lpr;
+                    const uint32_t q = g0 + u * lanes;
                     if (q < g_end && q < g_full) ix[u] = ldg_stream_u4(indices + 4ull * q);
                 }
 #pragma unroll
                 for (int u = 0; u < UNROLL; ++u) {
-                    const uint32_t q = g0 + u * lpr;
+                    const uint32_t q = g0 + u * lanes;
                     if (q >= g_end) continue;
                     if (q < g_full) {
                         const uint32_t c[4] = {ix[u].x, ix[u].y, ix[u].z, ix[u].w};
@@ -194,9 +196,29 @@ csr_outer_kernel(const T *__restrict__ row_vector, const T *__restrict__ col_vec
                 }
             }
         } else {
-            for (uint32_t pos = start + sl; pos < end; pos += lpr) g[pos] = r * col_vector[indices[pos]];
+            for (uint32_t pos = start + first; pos < end; pos += lanes) g[pos] = r * col_vector[indices[pos]];
         }
+    };
+    if (threadIdx.x == 0) n_long = 0;
+    __syncthreads();
+    for (uint64_t wg = static_cast<uint64_t>(blockIdx.x) * ROW_WARPS + (threadIdx.x >> 5); wg < n_groups; wg += n_warps) {
+        const uint64_t row = wg * rows_per_warp + sub;
+        if (row >= n_row) continue;
+        const uint32_t start = indptr[row], end = indptr[row + 1];
+        if (end - start > long_from) {
+            uint32_t at = 0;
+            if (sl == 0) at = atomicAdd(&n_long, 1u);
+            at = __shfl_sync((FULL_MASK >> (32u - lpr)) << (sub * lpr), at, sub * lpr);      // (all lanes of the row are here)
+            if (at < LONG_ROWS) {
+                if (sl == 0) long_row[at] = static_cast<uint32_t>(row);
+                continue;
+            }
+        }
+        span(start, end, row_vector[row], sl, lpr);
     }
+    __syncthreads();
+    const uint32_t n = min(n_long, LONG_ROWS);
+    for (uint32_t i = 0; i < n; ++i) span(indptr[long_row[i]], indptr[long_row[i] + 1], row_vector[long_row[i]], threadIdx.x, ROW_THREADS);
     zero_outside_rows(g, indptr, n_row, nse);
 }
 

@@ -454,84 +454,135 @@ __global__ void __launch_bounds__(256) pack_events_kernel(const E *__restrict__ 
 // start together, sweep over x together: at any time they read in a band of x that fits L1, and each of its sectors comes
 // from L2 about once: 31 us, 80 % of the gathers hit.  More lanes per row, 1000 or 2000 per SM instead of 500: 37 and 45
 // us.  (Unsorted rows are summed as correctly, with the misses of the plain kernel.)
+// Rows that would keep their lanes far longer than an average one are put off and taken by whole warps, those of more than
+// BAND_WARP_ROW entries by the block (100,000 rows, 2e7 entries, heavy tail up to 300,000: 15.6 ms by the lanes of each row).
 //   OUTER = false: y[row] = sum of weight * x[column];  OUTER = true: g[entry] = row_vector[row] * x[column].
 constexpr int BAND_THREADS = 128;
+constexpr uint32_t BAND_WARP_ROW = 2048;
 
 template<typename T, bool HOMO, bool OUTER>
 __global__ void __launch_bounds__(BAND_THREADS)
 bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
              const T *__restrict__ x, T *__restrict__ out, const uint32_t n_row, const uint32_t nse, const uint32_t log_l) {
     constexpr bool WEIGHTS = !HOMO && !OUTER;                  // (OUTER: data is the row vector)
+    __shared__ uint32_t n_long, long_row[BAND_THREADS];
+    __shared__ T warp_part[2][BAND_THREADS / 32];
     struct Unit {
         uint32_t c[8];
         T w[WEIGHTS ? 8 : 1];
     };
-    const uint32_t L = 1u << log_l, part = threadIdx.x & (L - 1u);
+    const uint32_t L = 1u << log_l, part = threadIdx.x & (L - 1u), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t full = nse >> 3;                            // units that lie wholly inside the arrays
     const uint64_t rows_per_grid = (static_cast<uint64_t>(gridDim.x) * BAND_THREADS) >> log_l;
-    for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * (BAND_THREADS >> log_l); base < n_row; base += rows_per_grid) {
-        const uint64_t row = base + (threadIdx.x >> log_l);
-        uint32_t start = 0, end = 0;
-        T w0 = T(0);
-        if (row < n_row) {
-            start = indptr[row];
-            end = indptr[row + 1];
-            if (!WEIGHTS) w0 = OUTER ? data[row] : data[0];
+    const uint32_t long_from = max(128u, nse >> 15) << log_l;
+    uint32_t start = 0, end = 0, u_end = 0;                    // the row that is walked
+    T w0 = T(0), acc = T(0);
+    auto enter = [&](const uint32_t row) {
+        start = indptr[row];
+        end = indptr[row + 1];
+        if (!WEIGHTS) w0 = OUTER ? data[row] : data[0];
+    };
+    auto load = [&](Unit &v, const uint32_t at) {
+        if (at < u_end && at < full) {
+            ldg_stream_8(indices + 8ull * at, v.c);
+            if (WEIGHTS) ldg_stream_8(data + 8ull * at, v.w);
         }
-        uint32_t u = (start >> 3) + part;
-        const uint32_t u_end = start < end ? (end + 7u) >> 3 : 0u;
-        auto load = [&](Unit &v, const uint32_t at) {
-            if (at < u_end && at < full) {
-                ldg_stream_8(indices + 8ull * at, v.c);
-                if (WEIGHTS) ldg_stream_8(data + 8ull * at, v.w);
+    };
+    auto use = [&](const Unit &v, const uint32_t at) {
+        const uint32_t pos = 8u * at;
+        if (at >= full) {                                      // ragged end of the arrays
+            for (uint32_t e = max(pos, start); e < end; ++e) {
+                const T p = (WEIGHTS ? data[e] : w0) * __ldg(x + indices[e]);
+                if (OUTER) out[e] = p; else acc += p;
             }
-        };
-        T acc = T(0);
-        auto use = [&](const Unit &v, const uint32_t at) {
-            const uint32_t pos = 8u * at;
-            if (at >= full) {                                  // ragged end of the arrays
-                for (uint32_t e = max(pos, start); e < end; ++e) {
-                    const T p = (WEIGHTS ? data[e] : w0) * __ldg(x + indices[e]);
-                    if (OUTER) out[e] = p; else acc += p;
-                }
-                return;
-            }
-            T g[8];
+            return;
+        }
+        T g[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                g[e] = T(0);
-                if (pos + e >= start && pos + e < end) g[e] = __ldg(x + v.c[e]);
-            }
-            if (OUTER) {
-                if (pos >= start && pos + 8u <= end) {
-                    store_quad(out + pos, w0 * g[0], w0 * g[1], w0 * g[2], w0 * g[3]);
-                    store_quad(out + pos + 4u, w0 * g[4], w0 * g[5], w0 * g[6], w0 * g[7]);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (pos + e >= start && pos + e < end) out[pos + e] = w0 * g[e];
-                }
+        for (int e = 0; e < 8; ++e) {
+            g[e] = T(0);
+            if (pos + e >= start && pos + e < end) g[e] = __ldg(x + v.c[e]);
+        }
+        if (OUTER) {
+            if (pos >= start && pos + 8u <= end) {
+                store_quad(out + pos, w0 * g[0], w0 * g[1], w0 * g[2], w0 * g[3]);
+                store_quad(out + pos + 4u, w0 * g[4], w0 * g[5], w0 * g[6], w0 * g[7]);
             } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                    if (pos + e >= start && pos + e < end) acc += (WEIGHTS ? v.w[WEIGHTS ? e : 0] : w0) * g[e];
+                    if (pos + e >= start && pos + e < end) out[pos + e] = w0 * g[e];
             }
-        };
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (pos + e >= start && pos + e < end) acc += (WEIGHTS ? v.w[WEIGHTS ? e : 0] : w0) * g[e];
+        }
+    };
+    // the units of the row from its `first` on, every `lanes`-th
+    auto walk = [&](const uint32_t first, const uint32_t lanes) {
+        uint32_t u = (start >> 3) + first;
+        u_end = start < end ? (end + 7u) >> 3 : 0u;
+        acc = T(0);
         Unit a, b;
         load(a, u);
         while (u < u_end) {
-            load(b, u + L);
+            load(b, u + lanes);
             use(a, u);
-            if (u + L < u_end) {
-                load(a, u + 2u * L);
-                use(b, u + L);
+            if (u + lanes < u_end) {
+                load(a, u + 2u * lanes);
+                use(b, u + lanes);
             }
-            u += 2u * L;
+            u += 2u * lanes;
         }
+    };
+    if (threadIdx.x == 0) n_long = 0;
+    __syncthreads();
+    for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * (BAND_THREADS >> log_l); base < n_row; base += rows_per_grid) {
+        const uint64_t row = base + (threadIdx.x >> log_l);
+        start = end = 0;
+        if (row < n_row) enter(static_cast<uint32_t>(row));
+        bool later = end - start > long_from;
+        if (__any_sync(FULL_MASK, later)) {                    // put off, as many as there is room for
+            uint32_t at = BAND_THREADS;
+            if (later && part == 0) at = atomicAdd(&n_long, 1u);
+            later = __shfl_sync(FULL_MASK, at, lane - part) < BAND_THREADS;
+            if (later) {
+                if (part == 0) long_row[at] = static_cast<uint32_t>(row);
+                start = end = 0;
+            }
+        }
+        walk(part, L);
         if (!OUTER) {
             for (uint32_t o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL_MASK, acc, o);
-            if (part == 0 && row < n_row) out[row] = acc;
+            if (part == 0 && row < n_row && !later) out[row] = acc;
         }
+    }
+    __syncthreads();
+    const uint32_t n = min(n_long, static_cast<uint32_t>(BAND_THREADS));
+    for (uint32_t i = warp; i < n; i += BAND_THREADS / 32) {
+        enter(long_row[i]);
+        if (end - start > BAND_WARP_ROW) continue;
+        walk(lane, 32u);
+        if (!OUTER) {
+            acc = warp_sum(acc);
+            if (lane == 0) out[long_row[i]] = acc;
+        }
+    }
+    uint32_t turn = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        enter(long_row[i]);
+        if (end - start <= BAND_WARP_ROW) continue;
+        walk(threadIdx.x, BAND_THREADS);
+        if (OUTER) continue;
+        acc = warp_sum(acc);                                   // (a barrier per row: as in walk_cut_rows)
+        if (lane == 0) warp_part[turn & 1u][warp] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            T sum = T(0);
+            for (uint32_t k = 0; k < BAND_THREADS / 32; ++k) sum += warp_part[turn & 1u][k];
+            out[long_row[i]] = sum;
+        }
+        ++turn;
     }
     if (OUTER) zero_outside_rows(out, indptr, n_row, nse);
 }

@@ -357,15 +357,24 @@ def _uneven(kind):
   elif kind == 'shared_many':    # more rows for a block than it has room for
     n_row, n_col, lens = 150_000, 3000, np.full(150_000, 20)
     lens[np.flatnonzero((np.arange(n_row) // 8) % 148 == 5)[::6][:140]] = 4501
-  else:                          # fewer rows than warps, each long
+  elif kind == 'shared_few':     # fewer rows than warps, each long
     n_row, n_col, lens = 60, 9001, np.full(60, 8003)
     lens[5] = 0
+  elif kind == 'bands':          # a whole block of long rows; one lane per row
+    n_row, n_col, lens = 100_000, 60_000, np.full(100_000, 31)
+    lens[256:384], lens[70_001] = 499, 59_999
+  elif kind == 'bands_teams':    # several lanes per row
+    n_row, n_col, lens = 16_000, 60_000, np.full(16_000, 401)
+    lens[[3, 9000, 9001]] = 0, 50_003, 5400
+  else:                          # plain: vector too long for shared memory, too few rows for the bands
+    n_row, n_col, lens = 3000, 300_000, np.full(3000, 33)
+    lens[[1, 2999]], lens[100:700] = 250_001, 1500
   return n_row, n_col, lens
 
 
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 @pytest.mark.parametrize('homo', [False, True])
-@pytest.mark.parametrize('kind', ['shared', 'shared_many', 'shared_few'])
+@pytest.mark.parametrize('kind', ['shared', 'shared_many', 'shared_few', 'bands', 'bands_teams', 'plain'])
 def test_products_of_rows_of_very_different_lengths(cuda, kind, homo, dtype):
   n_row, n_col, lens = _uneven(kind)
   data, indices, indptr = _skewed(n_row, n_col, lens, dtype, cuda)
@@ -391,7 +400,8 @@ def test_products_of_rows_of_very_different_lengths(cuda, kind, homo, dtype):
 
 
 # Bounds several times above what the calls take, far below what the lanes of single rows would (0.9 to 7 ms).
-@pytest.mark.parametrize('n_row,n_col,op,bound', [(100_000, 30_000, 'transposed', 350.)])
+@pytest.mark.parametrize('n_row,n_col,op,bound', [(100_000, 30_000, 'transposed', 350.), (100_000, 60_000, 'product', 350.),
+                                                  (100_000, 60_000, 'gradient', 400.), (20_000, 300_000, 'gradient', 400.)])
 def test_time_of_a_product_with_a_long_row(cuda, n_row, n_col, op, bound):
   lens = np.full(n_row, 2_000_000 // n_row)
   lens[n_row // 3] = min(n_col, 250_000)
