@@ -45,8 +45,8 @@ def test_dense_rows(cuda, shape, prob, dtype, kind):
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 @pytest.mark.parametrize('shape,prob', [((901, 3000), 0.3), ((58113, 4000), 0.01), ((29057, 2500), 0.02)])
 def test_dense_columns(cuda, shape, prob, dtype, kind):
-  """Sums in tiles of the output against the same streams (seed + column) a few columns at a time, which are too few for
-  tiles.  (One connection that the oracle moves would shift all that follow in its stream.)"""
+  """Against the same streams (seed + column) a few columns at a time.  (One connection that the oracle moves would shift all
+  that follow in its stream.)"""
   x = torch.randn(shape[1], dtype=dtype, generator=torch.Generator().manual_seed(2)).to(cuda)
   got = _call(x, kind, prob, shape, False, False).double()
   want = torch.zeros(shape[0], dtype=torch.float64, device=cuda)
@@ -85,9 +85,47 @@ def test_event_columns(cuda, shape, prob, rate, kind):
 @pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
+  """More streams than eight lanes each are given to, with too few connections for tiles: reductions and gathers."""
   test_dense_columns(cuda, (29_057, 8881), 0.01, dtype, kind)
   x = np.random.default_rng(1).standard_normal(58_113).astype(str(dtype)[6:])
   _compare(cuda, x, kind, 0.002, (6001, 58_113), True, False)
+
+
+def _tiles(n, other, prob, size, columns):
+  """The lines between the walks (jitconn_kernels.cu) for 148 SMs: whether one lane per stream works in tiles of the output
+  (`columns`: n outputs, `other` streams) or of the vector (n inputs)."""
+  per_sm, waves = n * other * prob / 148, -(-(-(-other // 148)) // 1024)
+  if columns:
+    return other > 60 * 148 and 1.8 * per_sm > 0.3 * (size // 4) * per_sm + 0.8 * (size // 4) * n * waves + 5000
+  return other > 40 * 148 and 0.75 * per_sm > n * size / 56 * (1 if n * size <= 227 * 1024 else waves) + 2000
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+# one tile, one element more, exactly two and one more, of either type
+@pytest.mark.parametrize('n', [29_056, 29_057, 58_112, 58_113, 116_225])
+def test_sums_in_tiles_of_the_output(cuda, n, dtype, kind):
+  columns, prob, few = 12_001, 0.03, 4000           # `few` columns are too few: eight lanes each, reductions
+  assert _tiles(n, columns, prob, dtype.itemsize, True) and few <= 32 * 148
+  x = torch.randn(columns, dtype=dtype, generator=torch.Generator().manual_seed(2)).to(cuda)
+  got = _call(x, kind, prob, (n, columns), False, False).double()
+  want = torch.zeros(n, dtype=torch.float64, device=cuda)
+  for lo in range(0, columns, few):
+    part = x[lo:lo + few].contiguous()
+    want += _call(part, kind, prob, (n, part.shape[0]), False, False, seed=77 + lo).double()
+  torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('n', [29_057, 58_112, 58_113])
+def test_vector_in_tiles(cuda, n, dtype, kind):
+  rows, prob, few = 6001, 0.02, 2000                # `few` rows: eight lanes each, or gathers from global memory
+  assert _tiles(n, rows, prob, dtype.itemsize, False) and not _tiles(n, few, prob, dtype.itemsize, False)
+  x = torch.randn(n, dtype=dtype, generator=torch.Generator().manual_seed(3)).to(cuda)
+  got = _call(x, kind, prob, (rows, n), True, False)
+  want = torch.cat([_call(x, kind, prob, (min(few, rows - lo), n), True, False, seed=77 + lo) for lo in range(0, rows, few)])
+  torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * float(want.abs().max()))
 
 
 @pytest.mark.parametrize('kind', sorted(KINDS))
