@@ -220,6 +220,11 @@ def cpu_reference_kernel():
   return 'port'
 
 
+# what the reference arm ran, by the kind that cpu_reference_kernel() found
+REFERENCE_CODE = {
+  'reference': 'lib/cpu_event_sum.cc cpu_csr_event_sum_heter_f32_i32 (serial C++) on the host',
+  'port': "oracle/synaptic_oracle.c, this repository's serial C restatement of lib/cpu_event_sum.cc, on the host: not the "
+          "reference's own code, and no base for a speed-up over it"}
 CPU_SAMPLE = 'the whole 1e6 x 1e6 matrix (1e9 synapses) on the host, the same spike vectors: ~1e7 synaptic ops per step'
 
 
@@ -266,8 +271,7 @@ def run_reference(args):
     'impl': 'reference', 'metric': METRIC, 'value': value, 'unit': UNIT, 'n_gpus': args.gpus, 'steps': done,
     'warmup': args.warmup, 'ms_per_step': seconds / done * 1e3, 'higher_is_better': True, 'scaling': 'strong',
     'vs_baseline': None, 'dtype': 'f32', 'data': 'synthetic',
-    'config': {'workload': WORKLOAD, 'reference_code': 'lib/cpu_event_sum.cc cpu_csr_event_sum_heter_f32_i32 '
-               '(serial C++) on the host'},
+    'config': {'workload': WORKLOAD, 'reference_code': REFERENCE_CODE[kind]},
     'cpu_baseline': {'value': value, 'unit': UNIT, 'cores': 1, 'kind': kind,
                      'sample': f'{done} steps on {CPU_SAMPLE}', 'host_cores_available': os.cpu_count()},
     'e2e': {'value': value, 'unit': UNIT, 'h2d_bytes_per_step': 0, 'd2h_bytes_per_step': 0},

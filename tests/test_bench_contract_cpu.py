@@ -29,6 +29,7 @@ def test_reference_arm_prints_one_json_line_with_the_agreed_keys():
   assert d['vs_baseline'] is None and d['data'] == 'synthetic' and d['dtype'] == 'f32'
   assert 'workload' in d['config'] and 'model' not in d['config']
   cb = d['cpu_baseline']
+  assert ('oracle/' in d['config']['reference_code']) == (cb['kind'] == 'port')     # names the code that ran
   assert cb['kind'] in ('reference', 'port') and cb['cores'] == 1 and cb['value'] == d['value'] and cb['sample']
   e2e = d['e2e']
   assert e2e['value'] == d['value'] and e2e['unit'] == d['unit']
