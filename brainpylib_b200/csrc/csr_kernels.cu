@@ -422,7 +422,7 @@ list_scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t 
     if (n_list != 0) add_sums(sums, y, n_col, blockIdx.x, gridDim.x);
 }
 
-// How many rows are active is not known here; the rule supposes 1 %, a usual rate.  In clocks of one SM: a reduction takes
+// How many rows are active is not known here; the rule supposes 1 % (a convention, not a measurement).  In clocks of one SM: a reduction takes
 // 1.85, and more the fewer columns share them; the sums take 0.4 each to clear and to add up, and 3000 in all.
 inline bool list_shared_pays(uint32_t n_row, uint32_t n_col, uint32_t nse, bool homo, size_t elem) {
     const double active = 0.01 * nse / sm_count();
@@ -595,7 +595,7 @@ event_columns_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
 
 // Every block reads what the others read: the events, and the entries of the active rows, at 34 bytes per clock.  With the
 // 10 % of a lively network active, OWN_BYTES of matrix take the 2 us that the second launch would (4000 x 4000, 320,000
-// synapses, 5 %: 5.3 us per call, 6.9 with two launches).
+// synapses, 5 %: 5.3 us per call, 6.9 with two launches; with 10 % 7.4 and 7.0: at that size and activity the line is late).
 constexpr double OWN_BYTES = 1.3e6;
 
 inline bool columns_pay(uint32_t n_row, uint32_t n_col, uint32_t nse, size_t per_entry, size_t event) {

@@ -6,8 +6,8 @@
 // columns: 1.9e7 entries into 2185 sums took 853 us, here 46).  A lookup in shared memory takes a tenth of a clock, an
 // addition there 0.3.  So one block per SM holds the whole vector.
 //
-// Longer vectors are gathered through L1 (bands_kernel) or scattered into L2 (csr_kernels.cu).  What shared memory takes from the 256 KB of an SM is missing for the
-// entries in flight, which pass through L1: 1e7 float entries, 80 MB, take 18.6 us with up to 132 KB of x, 19.9 with
+// Longer vectors are gathered through L1 (bands_kernel) or scattered into L2 (csr_kernels.cu).  What shared memory takes from
+// the 256 KB of an SM is missing for the entries in flight, which pass through L1: 1e7 float entries, 80 MB, take 18.6 us with up to 132 KB of x, 19.9 with
 // 160 KB, 23 with 195 KB, 31 with 226 KB.  For that reason neither the first 160 KB of a longer vector here and the rest
 // by the plain ways (100,000 columns: gather 44 us against 39, scatter 78 against 65), nor slices of it in several blocks
 // that read the same rows side by side (58 us) paid; and reading a neighbour's slice out of its shared memory moves 0.33
@@ -346,8 +346,8 @@ gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
 }
 
 // y = A events: the events as one byte each in shared memory, or one bit where they are many.  The walk is bound by
-// instruction issue, and a byte needs no shifts (1e8 entries, rows of 121, 3000 columns: 140 -> 109 us).  Homogeneous weights count hits and scale once (equal to the
-// reference CPU kernel's float64 accumulation, brainpylib/_src/event_ops/event_csr_matvec.py:334-357).
+// instruction issue, and a byte needs no shifts (1e8 entries, rows of 121, 3000 columns: 140 -> 109 us).  Homogeneous weights
+// count hits and scale once (equal to the reference CPU kernel's float64 accumulation, brainpylib/_src/event_ops/event_csr_matvec.py:334-357).
 template<typename T, bool HOMO, bool BYTES>
 struct EventVisit {
     const uint32_t *mask;
@@ -745,6 +745,7 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     const bool pack = m.n_col * sizeof(E) > 32768u;
     // Few events, which L1 serves by broadcast: rows of one or two of the walk's steps, half of them empty, take it longer than
     // the plain kernel (1e8 entries, rows of 121, 1037 columns: 106 us and 88; rows of 30: 35 and 41; of 700: 31 and 32).
+    // The lines lie between these three; where exactly both take the same was not measured.
     const double mean_row = static_cast<double>(m.nse) / m.n_row;
     if (HOMO && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
