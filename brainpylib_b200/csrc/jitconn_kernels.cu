@@ -62,15 +62,42 @@ jit_rows_dense_v1_kernel(const T *__restrict__ vector, const unsigned int seed, 
 //   FROM_MASK    events as one bit each in shared memory (1e6 inputs = 125 KB): truthiness is all that is needed.  A hit
 //                leaves its raw draws in a queue of its thread (shared memory); the weights are computed when a queue is
 //                full, by all threads of the warp together, instead of by one thread at a time where it hits
+//   FROM_BYTES   the same with one byte per event where they fit beside the queues: three instructions fewer per connection
 //   FROM_TILES   the vector in shared memory, in as few tiles as fit (58,000 floats each).  Positions ascend along a
 //                stream, so all streams of a block cross one tile together; a batch that straddles the end of a tile is
 //                simply looked at again in the next one, where the other positions fall into range.
-enum { FROM_GLOBAL = 0, FROM_MASK = 1, FROM_TILES = 2 };
+// A hit (the top bit of `hit`) leaves its draws at `next`, which moves on.  One comparison for both, no branch.
+__device__ __forceinline__ void push_if(const uint32_t hit, uint32_t &next, const uint32_t x, const uint32_t step) {
+    asm volatile("{ .reg .pred q; setp.lt.s32 q, %1, 0; @q st.shared.u32 [%0], %2; @q add.u32 %0, %0, %3; }"
+                 : "+r"(next) : "r"(hit), "r"(x), "r"(step) : "memory");
+}
+// (`seconds`: one bit per hit, the last one lowest)
+__device__ __forceinline__ void push_pair_if(const bool second, const uint32_t hit, uint32_t &next, const uint32_t x, const uint32_t y,
+                                             const uint32_t step, uint32_t &seconds) {
+    if (second)
+        asm volatile("{ .reg .pred q; setp.lt.s32 q, %2, 0; @q st.shared.v2.u32 [%0], {%3, %4}; @q add.u32 %0, %0, %5; @q mad.lo.u32 %1, %1, 2, 1; }"
+                     : "+r"(next), "+r"(seconds) : "r"(hit), "r"(x), "r"(y), "r"(step) : "memory");
+    else
+        asm volatile("{ .reg .pred q; setp.lt.s32 q, %2, 0; @q st.shared.v2.u32 [%0], {%3, %4}; @q add.u32 %0, %0, %5; @q add.u32 %1, %1, %1; }"
+                     : "+r"(next), "+r"(seconds) : "r"(hit), "r"(x), "r"(y), "r"(step) : "memory");
+}
+
+enum { FROM_GLOBAL = 0, FROM_MASK = 1, FROM_TILES = 2, FROM_BYTES = 3 };
 
 constexpr int WALK_THREADS = 1024;                          // per block with shared memory, one block per SM
 constexpr int GATHER_THREADS = 256;                         // at most, per block without
 constexpr unsigned int WALK_SMEM = 227u * 1024u;            // all that a block can have
 constexpr unsigned int MASK_MAX_BITS = 200u * 1024u * 8u;   // the rest of it: the queues of hits
+
+// Connections that a walk over truths takes at a time.  (Uniform weights, 1e9 connections: 1517 us with 5, 1392 with 8, 1420
+// with 10, where the registers of 1024 threads run out; normal 1669 with 4, 1530 with 8.)
+constexpr int TRUTH_BATCH = 8;
+// and a walk over tiles (homogeneous weights, 100,000 streams of 400: 155 us with 5, 149 with 8; uniform and normal: 2 % and 1 %
+// faster with 6 than with 5 and 4)
+template<int KIND> constexpr int TILE_BATCH = KIND == W_HOMO ? 8 : 6;
+__host__ __device__ constexpr unsigned int queue_slot_bytes(int kind) { return kind == W_NORMAL ? 8u : 4u; }
+// shared memory of the events, as bits or bytes
+__host__ __device__ constexpr unsigned int truth_bytes(unsigned int n, bool bytes) { return ((bytes ? n : (n + 7u) >> 3) + 7u) & ~7u; }
 
 // The rows (columns) of a block: equal shares, so that no SM is left with a last wave of its own.
 struct Share {
@@ -93,6 +120,25 @@ __device__ __forceinline__ void load_tile(T *tile, const T *__restrict__ src, co
     for (unsigned int i = n_vec * PER + threadIdx.x; i < count; i += blockDim.x) tile[i] = p[i];
 }
 
+// One byte per event, 0 or -1, by the whole block.
+template<typename E>
+__device__ __forceinline__ void event_bytes(const E *__restrict__ in, const unsigned int n, unsigned char *bytes) {
+    constexpr unsigned int PER = 16 / sizeof(E);
+    const unsigned int whole = aligned16_device(in) ? n / PER : 0u;
+#pragma unroll 4
+    for (unsigned int i = threadIdx.x; i < whole; i += blockDim.x) {
+        const uint4 raw = *reinterpret_cast<const uint4 *>(in + i * PER);
+        const E *e = reinterpret_cast<const E *>(&raw);
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (unsigned int k = 0; k < PER; ++k) w[k / 4] |= (is_event(e[k]) ? 0xffu : 0u) << (8u * (k % 4));
+        if (PER == 16) reinterpret_cast<uint4 *>(bytes)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        else if (PER == 4) reinterpret_cast<uint32_t *>(bytes)[i] = w[0];
+        else reinterpret_cast<uint16_t *>(bytes)[i] = static_cast<uint16_t>(w[0]);
+    }
+    for (unsigned int i = whole * PER + threadIdx.x; i < n; i += blockDim.x) bytes[i] = is_event(in[i]) ? 0xff : 0;
+}
+
 template<typename T, typename E, int KIND, bool EVENT, int FROM, bool QUICK>
 __global__ void __launch_bounds__(FROM == FROM_GLOBAL ? GATHER_THREADS : WALK_THREADS)
 jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapParams gp, const double w1, const double w2,
@@ -100,9 +146,14 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
                 const T scale, T *__restrict__ out) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(walk_smem);
-    uint32_t *queue = mask + ((num_col + 31u) >> 5) + threadIdx.x;     // slot i of this thread: queue[i * blockDim.x]
+    constexpr bool BYTES = FROM == FROM_BYTES, TRUTH = FROM == FROM_MASK || BYTES;
+    // the queue of hits of this thread behind the events: slots of 4 (normal: 8) bytes, `queue_step` apart
+    constexpr uint32_t SLOT = queue_slot_bytes(KIND);
+    const uint32_t queue_step = SLOT * blockDim.x;
+    const uint32_t queue = static_cast<uint32_t>(__cvta_generic_to_shared(walk_smem)) + truth_bytes(num_col, BYTES) + SLOT * threadIdx.x;
     E *tile = reinterpret_cast<E *>(walk_smem);
-    constexpr int N = Batch<KIND, QUICK>::N;
+    constexpr bool SUMS = TRUTH || FROM == FROM_TILES;
+    constexpr int N = TRUTH ? TRUTH_BATCH : FROM == FROM_TILES ? TILE_BATCH<KIND> : Batch<KIND, QUICK>::N;
     const Share share(num_row);
     const bool one_tile = tile_len >= num_col;
 
@@ -112,6 +163,9 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
         // the first event of a word in its top bit: one shift by the position brings an event into the sign bit
         for (unsigned int i = threadIdx.x; i < ((num_col + 31u) >> 5); i += blockDim.x) mask[i] = __brev(mask[i]);
         __syncthreads();
+    } else if (BYTES) {
+        event_bytes(in, num_col, walk_smem);
+        __syncthreads();
     } else if (FROM == FROM_TILES && one_tile) {
         load_tile(tile, in, 0, num_col);
         __syncthreads();
@@ -120,10 +174,10 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
         const unsigned int row = row0 + threadIdx.x;
         const bool live = row < share.end;
         if (FROM == FROM_GLOBAL && !live) break;
-        if (FROM == FROM_MASK && !__any_sync(FULL_MASK, live)) break;
+        if (TRUTH && !__any_sync(FULL_MASK, live)) break;
         Xorwow s;
         s.seed(seed + row);
-        Batch<KIND, QUICK> b;
+        Batch<KIND, QUICK, N, SUMS> b;
         unsigned int at = 0;
         T sum = 0;
         if (FROM == FROM_TILES) {
@@ -150,53 +204,61 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
                     b.draw(s, at, num_col, gp);
                 }
             }
-        } else if (FROM == FROM_MASK) {
+        } else if (TRUTH) {
             // all lanes of the warp stay in the loop until the last is done: what a lane draws behind its end is no hit
             unsigned int hits = 0;                         // homogeneous: the float sum of 0/1 events is the exact count
-            unsigned int queued = 0, seconds = 0;
+            uint32_t next = queue, seconds = 0;            // where the next hit goes; which hits are the second of their pair
+            const uint32_t full = queue + (slots - min(slots, static_cast<unsigned int>(N) - 1u)) * queue_step;
             if (!live) at = num_col;                       // draws behind the end from the start
             auto drain = [&]() {
-                const unsigned int most = __reduce_max_sync(FULL_MASK, queued);
-                for (unsigned int i = 0; i < most; ++i) {
-                    if (i < queued) {
-                        if (KIND == W_UNIFORM) sum += uniform_weight<T>(queue[i * blockDim.x], w1, w2);
-                        if (KIND == W_NORMAL)
-                            sum += normal_weight<T>(queue[2 * i * blockDim.x], queue[(2 * i + 1) * blockDim.x],
-                                                    (seconds >> i) & 1u, w1, w2);
+                uint32_t last = KIND == W_NORMAL ? (next - queue) / queue_step : 0u;
+                for (uint32_t from = queue; __any_sync(FULL_MASK, from < next); from += queue_step) {
+                    if (from >= next) continue;
+                    if (KIND == W_UNIFORM) {
+                        uint32_t x;
+                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(from) : "memory");
+                        sum += uniform_weight<T>(x, w1, w2);
+                    }
+                    if (KIND == W_NORMAL) {
+                        uint32_t x, y;
+                        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(from) : "memory");
+                        sum += normal_weight<T>(x, y, (seconds >> --last) & 1u, w1, w2);
                     }
                 }
-                queued = seconds = 0;
+                next = queue;
             };
             // checked: positions may lie behind the end
             auto look = [&](auto checked) {
 #pragma unroll
                 for (int j = 0; j < N; ++j) {
-                    uint32_t word = 0;                     // 24 bits of the position hold it: the mask has at most 2^21
-                    if (!checked.value || (b.pos[j] & 0xffffffu) < num_col)
-                        word = *reinterpret_cast<const uint32_t *>(walk_smem + ((b.pos[j] >> 3) & 0x1ffffcu));
-                    const uint32_t hit = __funnelshift_l(0u, word, b.pos[j]) >> 31;
-                    if (KIND == W_HOMO) {
-                        hits += hit;
+                    uint32_t hit = 0;                      // its top bit
+                    if (BYTES) {
+                        if (!checked.value || b.pos[j] < num_col) hit = static_cast<int>(reinterpret_cast<const signed char *>(walk_smem)[b.pos[j]]);
+                        if (KIND == W_HOMO) hits -= hit;
                     } else {
-                        if (KIND == W_UNIFORM) store_shared_if(hit, queue + queued * blockDim.x, b.raw[j]);
-                        if (KIND == W_NORMAL) {
-                            store_shared_if(hit, queue + 2 * queued * blockDim.x, b.raw[j & ~1]);
-                            store_shared_if(hit, queue + (2 * queued + 1) * blockDim.x, b.raw[j | 1]);
-                            if (j & 1) seconds |= hit << queued;
-                        }
-                        queued += hit;
+                        uint32_t word = 0;                 // 24 bits of the position hold it: the mask has at most 2^21
+                        if (!checked.value || (b.pos[j] & 0xffffffu) < num_col)
+                            word = *reinterpret_cast<const uint32_t *>(walk_smem + ((b.pos[j] >> 3) & 0x1ffffcu));
+                        hit = __funnelshift_l(0u, word, b.pos[j]);
+                        if (KIND == W_HOMO) hits += hit >> 31;
                     }
+                    if (KIND == W_UNIFORM) push_if(hit, next, b.raw[j], queue_step);
+                    if (KIND == W_NORMAL) push_pair_if(j & 1, hit, next, b.raw[j & ~1], b.raw[j | 1], queue_step, seconds);
                 }
-                if (KIND != W_HOMO && __any_sync(FULL_MASK, queued + N > slots)) drain();
+                if (KIND != W_HOMO && __any_sync(FULL_MASK, next >= full)) drain();
             };
-            b.template draw<true>(s, at, num_col, gp);
+            auto draw = [&]() {
+                b.template draw<FROM == FROM_MASK>(s, at, num_col, gp);
+                if (BYTES) at = min(at, num_col);
+            };
+            draw();
             while (__all_sync(FULL_MASK, at < num_col)) {
                 look(std::false_type());
-                b.template draw<true>(s, at, num_col, gp);
+                draw();
             }
             look(std::true_type());
             while (__any_sync(FULL_MASK, at < num_col)) {
-                b.template draw<true>(s, at, num_col, gp);
+                draw();
                 look(std::true_type());
             }
             if (KIND == W_HOMO) sum = static_cast<T>(hits);
@@ -290,7 +352,7 @@ jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const Gap
                 T *__restrict__ out) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     T *tile = reinterpret_cast<T *>(walk_smem);
-    constexpr int N = Batch<KIND, QUICK>::N;
+    constexpr int N = TILES ? TILE_BATCH<KIND> : Batch<KIND, QUICK>::N;
     const Share share(num_col);
     for (unsigned int col0 = share.begin; col0 < share.end; col0 += blockDim.x) {
         const unsigned int col = col0 + threadIdx.x;
@@ -298,7 +360,7 @@ jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const Gap
         if (!TILES && !live) break;
         Xorwow s;
         s.seed(seed + col);
-        Batch<KIND, QUICK> b;
+        Batch<KIND, QUICK, N, TILES> b;
         unsigned int at = 0;
         T v = live ? vector[col] : T(0);
         if (KIND == W_HOMO) v = v * scale;
@@ -606,32 +668,35 @@ void jit_rows(const JitCall<T, E> &c) {
         }
     }
     WalkGrid g(a.n_row, 512);
-    // (n_col + 5 * 23 mean gaps stay below 2^24)
-    if (gp.quick && TRUTH_ONLY && a.n_col <= MASK_MAX_BITS && -1.0 / a.log_p < 130000.0) {
-        if (gathers > static_cast<double>(a.n_col) * sizeof(E) / 56 + 2000) {
-            constexpr auto kernel = jit_rows_kernel<T, E, KIND, EVENT, TRUTH_ONLY ? FROM_MASK : FROM_GLOBAL, true>;
-            if (!allow_shared<kernel>(WALK_SMEM)) {
+    if constexpr (TRUTH_ONLY) {
+        // Bytes where they leave room for queues of 12 (normal: 10) hits of 1024 threads; then bits, whose walk keeps positions
+        // in 24 bits (a batch runs TRUTH_BATCH gaps, each below 23 mean ones, behind the end).
+        const unsigned int room = KIND == W_HOMO ? 0u : (KIND == W_UNIFORM ? 48u : 80u) * 1024u;
+        const bool bytes = truth_bytes(a.n_col, true) <= WALK_SMEM - room && a.n_col <= WALK_SMEM;
+        const bool bits = a.n_col <= MASK_MAX_BITS && a.n_col - TRUTH_BATCH * 23.0 / a.log_p < 16777216.0;
+        if (gp.quick && (bytes || bits) && gathers > static_cast<double>(a.n_col) * sizeof(E) / 56 + 2000) {
+            constexpr auto byte_kernel = jit_rows_kernel<T, E, KIND, EVENT, FROM_BYTES, true>;
+            constexpr auto bit_kernel = jit_rows_kernel<T, E, KIND, EVENT, FROM_MASK, true>;
+            if (!(bytes ? allow_shared<byte_kernel>(WALK_SMEM) : allow_shared<bit_kernel>(WALK_SMEM))) {
                 launch_ok();
                 return;
             }
-            // what the mask leaves holds the queues of hits, up to 16 slots per thread (`seconds` has 32 bits); beside a
-            // mask of the largest size only those of 512 threads fit
-            const unsigned int mask_bytes = blocks_for(a.n_col, 32) * 4u, slot_bytes = KIND == W_HOMO ? 0u : KIND == W_UNIFORM ? 4u : 8u;
+            // what the events leave holds the queues of hits, up to 16 slots per thread (`seconds` has 32 bits), and one more
+            // than a batch at least: beside a mask of the largest size only those of some threads fit
+            const unsigned int taken = truth_bytes(a.n_col, bytes), slot_bytes = queue_slot_bytes(KIND);
             unsigned int slots = 0;
-            if (slot_bytes != 0) {
-                slots = (WALK_SMEM - mask_bytes) / (slot_bytes * g.threads);
-                if (slots < 6u) {
-                    g.threads = 512;
-                    slots = (WALK_SMEM - mask_bytes) / (slot_bytes * g.threads);
-                }
-                slots = std::min(slots, 16u);
+            if (KIND != W_HOMO) {
+                const unsigned int fit = (WALK_SMEM - taken) / (slot_bytes * (TRUTH_BATCH + 1));
+                g.threads = std::min(g.threads, fit & ~31u);
+                slots = std::min(16u, (WALK_SMEM - taken) / (slot_bytes * g.threads));
             }
-            kernel<<<g.blocks, g.threads, static_cast<size_t>(mask_bytes) + slots * slot_bytes * g.threads, c.stream>>>(
+            (bytes ? byte_kernel : bit_kernel)<<<g.blocks, g.threads, static_cast<size_t>(taken) + slots * slot_bytes * g.threads, c.stream>>>(
                 c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, 0, slots, c.scale, c.out);
             launch_ok();
             return;
         }
-    } else if (gp.quick && !TRUTH_ONLY && (KIND == W_HOMO || !EVENT)) {
+    }
+    if (gp.quick && !TRUTH_ONLY && (KIND == W_HOMO || !EVENT)) {
         const unsigned int len = tile_length(a.n_col, sizeof(E));
         const double loads = static_cast<double>(a.n_col) * sizeof(E) / 56 * (len >= a.n_col ? 1 : g.waves);
         if (0.75 * gathers > loads + 2000) {

@@ -138,6 +138,23 @@ def test_event_rows(cuda, shape, prob, rate, dtype, kind):
   _compare(cuda, x, kind, prob, shape, True, True)
 
 
+@pytest.mark.parametrize('kind,most', [('homo', 227 * 1024), ('uniform', 179 * 1024), ('normal', 147 * 1024)])
+@pytest.mark.parametrize('more', [0, 1])
+def test_events_as_bytes_and_as_bits(cuda, kind, most, more):
+  """The longest event vector that a walk keeps as bytes beside its queues, and the first that it keeps as bits; every input
+  fires in half of the vector, so that queues fill."""
+  x = np.random.default_rng(8).random(most + more) < 0.05
+  x[:most // 2] = True
+  _compare(cuda, x, kind, 0.001, (9001, most + more), True, True)
+
+
+@pytest.mark.parametrize('prob', [1.22e-5, 1.2e-5])      # the last mean gap whose positions bits keep in 24 bits; one beyond
+def test_events_as_bits_far_apart(cuda, prob):
+  n = 1_638_400
+  assert (n + 8 * 23 / prob < 1 << 24) == (prob == 1.22e-5)
+  _compare(cuda, np.random.default_rng(9).random(n) < 0.5, 'homo', prob, (250_000, n), True, True)
+
+
 @pytest.mark.parametrize('prob', [6e-6, 2e-5, 1.0])      # outside the quick test's range, sparse, every position
 def test_probabilities_at_the_ends_of_the_range(cuda, prob):
   shape = (600, 200) if prob == 1.0 else (600, 300_000)
