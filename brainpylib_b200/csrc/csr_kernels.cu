@@ -683,12 +683,33 @@ void csr_outer_impl(cudaStream_t stream, const void *row_vector, const void *col
     launch_ok();
 }
 
+// Both gradients of a product of per-entry weights.
+template<typename T>
+void csr_gradients_impl(cudaStream_t stream, const void *data, const uint32_t *indices, const uint32_t *indptr, const void *x,
+                        const void *ct, void *g_data, void *g_x, uint32_t n_row, uint32_t n_col, uint32_t nse, bool transpose) {
+    const CsrMatrix<T> m{indices, indptr, static_cast<const T *>(data), n_row, n_col, nse, false};
+    const T *row_vector = static_cast<const T *>(transpose ? x : ct), *col_vector = static_cast<const T *>(transpose ? ct : x);
+    T *g = static_cast<T *>(g_data), *y = static_cast<T *>(g_x);
+    if (transpose ? gather_outer_shared(stream, m, row_vector, col_vector, g, y) : outer_scatter_shared(stream, m, row_vector, col_vector, g, y))
+        return;
+    csr_outer_impl<T>(stream, row_vector, col_vector, indices, indptr, g_data, n_row, n_col, nse);
+    csr_matvec_known<T>(stream, data, indices, indptr, ct, g_x, n_row, n_col, nse, false, !transpose);
+}
+
 }  // namespace
 }  // namespace bpl
 
 using namespace bpl;
 
 extern "C" {
+
+void bpl_csr_gradients(bpl_stream_t stream, const void *data, const void *indices, const void *indptr, const void *vector,
+                       const void *cotangent, void *data_gradient, void *vector_gradient, uint32_t n_row, uint32_t n_col,
+                       uint32_t nse, int is_double, int transpose) {
+    const uint32_t *ix = static_cast<const uint32_t *>(indices), *ip = static_cast<const uint32_t *>(indptr);
+    (is_double ? csr_gradients_impl<double> : csr_gradients_impl<float>)(stream, data, ix, ip, vector, cotangent, data_gradient,
+                                                                        vector_gradient, n_row, n_col, nse, transpose != 0);
+}
 
 void bpl_csr_outer(bpl_stream_t stream, const void *row_vector, const void *col_vector, const void *indices,
                    const void *indptr, void *out, uint32_t n_row, uint32_t n_col, uint32_t nse, int is_double) {

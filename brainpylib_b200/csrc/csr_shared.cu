@@ -456,15 +456,17 @@ __global__ void __launch_bounds__(256) pack_events_kernel(const E *__restrict__ 
 // us.  (Unsorted rows are summed as correctly, with the misses of the plain kernel.)
 // Rows that would keep their lanes far longer than an average one are put off and taken by whole warps, those of more than
 // BAND_WARP_ROW entries by the block (100,000 rows, 2e7 entries, heavy tail up to 300,000: 15.6 ms by the lanes of each row).
-//   OUTER = false: y[row] = sum of weight * x[column];  OUTER = true: g[entry] = row_vector[row] * x[column].
+//   SUM: y[row] = sum of weight * x[column];  OUTER: g[entry] = row_vector[row] * x[column];  SUM + OUTER: both, for one gather.
+enum { BAND_SUM = 1, BAND_OUTER = 2 };
 constexpr int BAND_THREADS = 128;
 constexpr uint32_t BAND_WARP_ROW = 2048;
 
-template<typename T, bool HOMO, bool OUTER>
+template<typename T, bool HOMO, int MODE>
 __global__ void __launch_bounds__(BAND_THREADS)
 bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
-             const T *__restrict__ x, T *__restrict__ out, const uint32_t n_row, const uint32_t nse, const uint32_t log_l) {
-    constexpr bool WEIGHTS = !HOMO && !OUTER;                  // (OUTER: data is the row vector)
+             const T *__restrict__ row_vector, const T *__restrict__ x, T *__restrict__ y, T *__restrict__ out, const uint32_t n_row,
+             const uint32_t nse, const uint32_t log_l) {
+    constexpr bool SUM = (MODE & BAND_SUM) != 0, OUTER = (MODE & BAND_OUTER) != 0, WEIGHTS = SUM && !HOMO;
     __shared__ uint32_t n_long, long_row[BAND_THREADS];
     __shared__ T warp_part[2][BAND_THREADS / 32];
     struct Unit {
@@ -476,11 +478,12 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
     const uint64_t rows_per_grid = (static_cast<uint64_t>(gridDim.x) * BAND_THREADS) >> log_l;
     const uint32_t long_from = max(128u, nse >> 15) << log_l;
     uint32_t start = 0, end = 0, u_end = 0;                    // the row that is walked
-    T w0 = T(0), acc = T(0);
+    T r = T(0), acc = T(0);
+    const T homo_w = SUM && HOMO ? data[0] : T(0);
     auto enter = [&](const uint32_t row) {
         start = indptr[row];
         end = indptr[row + 1];
-        if (!WEIGHTS) w0 = OUTER ? data[row] : data[0];
+        if (OUTER) r = row_vector[row];
     };
     auto load = [&](Unit &v, const uint32_t at) {
         if (at < u_end && at < full) {
@@ -492,8 +495,9 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
         const uint32_t pos = 8u * at;
         if (at >= full) {                                      // ragged end of the arrays
             for (uint32_t e = max(pos, start); e < end; ++e) {
-                const T p = (WEIGHTS ? data[e] : w0) * __ldg(x + indices[e]);
-                if (OUTER) out[e] = p; else acc += p;
+                const T v = __ldg(x + indices[e]);
+                if (OUTER) out[e] = r * v;
+                if (SUM) acc += (WEIGHTS ? data[e] : homo_w) * v;
             }
             return;
         }
@@ -505,17 +509,18 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
         }
         if (OUTER) {
             if (pos >= start && pos + 8u <= end) {
-                store_quad(out + pos, w0 * g[0], w0 * g[1], w0 * g[2], w0 * g[3]);
-                store_quad(out + pos + 4u, w0 * g[4], w0 * g[5], w0 * g[6], w0 * g[7]);
+                store_quad(out + pos, r * g[0], r * g[1], r * g[2], r * g[3]);
+                store_quad(out + pos + 4u, r * g[4], r * g[5], r * g[6], r * g[7]);
             } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                    if (pos + e >= start && pos + e < end) out[pos + e] = w0 * g[e];
+                    if (pos + e >= start && pos + e < end) out[pos + e] = r * g[e];
             }
-        } else {
+        }
+        if (SUM) {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                if (pos + e >= start && pos + e < end) acc += (WEIGHTS ? v.w[WEIGHTS ? e : 0] : w0) * g[e];
+                if (pos + e >= start && pos + e < end) acc += (WEIGHTS ? v.w[WEIGHTS ? e : 0] : homo_w) * g[e];
         }
     };
     // the units of the row from its `first` on, every `lanes`-th
@@ -552,9 +557,9 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
             }
         }
         walk(part, L);
-        if (!OUTER) {
+        if (SUM) {
             for (uint32_t o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL_MASK, acc, o);
-            if (part == 0 && row < n_row && !later) out[row] = acc;
+            if (part == 0 && row < n_row && !later) y[row] = acc;
         }
     }
     __syncthreads();
@@ -563,9 +568,9 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
         enter(long_row[i]);
         if (end - start > BAND_WARP_ROW) continue;
         walk(lane, 32u);
-        if (!OUTER) {
+        if (SUM) {
             acc = warp_sum(acc);
-            if (lane == 0) out[long_row[i]] = acc;
+            if (lane == 0) y[long_row[i]] = acc;
         }
     }
     uint32_t turn = 0;
@@ -573,14 +578,14 @@ bands_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ 
         enter(long_row[i]);
         if (end - start <= BAND_WARP_ROW) continue;
         walk(threadIdx.x, BAND_THREADS);
-        if (OUTER) continue;
+        if (!SUM) continue;
         acc = warp_sum(acc);                                   // (a barrier per row: as in walk_cut_rows)
         if (lane == 0) warp_part[turn & 1u][warp] = acc;
         __syncthreads();
         if (threadIdx.x == 0) {
             T sum = T(0);
             for (uint32_t k = 0; k < BAND_THREADS / 32; ++k) sum += warp_part[turn & 1u][k];
-            out[long_row[i]] = sum;
+            y[long_row[i]] = sum;
         }
         ++turn;
     }
@@ -624,6 +629,7 @@ scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__re
         __syncthreads();
     });
     __syncthreads();
+    pdl_wait();                                            // y is zero
     add_sums(sums, y, n_col, blockIdx.x, gridDim.x);
 }
 
@@ -655,17 +661,75 @@ struct OuterVisit {
     __device__ __forceinline__ void put(uint32_t, Sum) const {}
 };
 
+// (`zero`: n_zero elements to clear for the launch behind this one)
 template<typename T, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
-                    const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g,
-                    const uint32_t n_row, const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
+                    const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g, T *__restrict__ zero,
+                    const uint32_t n_zero, const uint32_t n_row, const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
+    pdl_launch_dependents();
+    for (uint32_t i = blockIdx.x * SHARED_THREADS + threadIdx.x; i < n_zero; i += gridDim.x * SHARED_THREADS) zero[i] = T(0);
     T *xs = reinterpret_cast<T *>(shared_vector);
     const Deal deal(nse, n_row, 4 * U);
     auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
     OuterVisit<T> visit{xs, row_vector, g, n_row, T(0)};
     walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
+        fill_shared(xs, col_vector, n_col);
+        zero_outside_rows(g, indptr, n_row, nse);
+        __syncthreads();
+    });
+}
+
+// Both of one gather: y[row] = sum of weight * col_vector[column] and g[e] = row_vector[row] * col_vector[column], the two
+// gradients of y = A^T x.  The indices are read once, and so is the vector (a row that is cut writes its g twice, the same).
+template<typename T>
+struct GatherOuterVisit {
+    const T *xs, *row_vector;
+    T *g, *y;
+    uint32_t n_row;
+    T r, acc;
+    __device__ __forceinline__ T fetch(const uint32_t row) const { return row < n_row ? row_vector[row] : T(0); }
+    __device__ __forceinline__ void begin(const T v) {
+        r = v;
+        acc = T(0);
+    }
+    template<bool FULL>
+    __device__ __forceinline__ void quad(const uint32_t base, const uint32_t (&c)[4], const T *w, const int lo, const int hi) {
+        if (FULL || (lo <= 0 && hi >= 4)) {
+            const T v[4] = {xs[c[0]], xs[c[1]], xs[c[2]], xs[c[3]]};
+            store_quad(g + base, r * v[0], r * v[1], r * v[2], r * v[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc += w[e] * v[e];
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (e >= lo && e < hi) entry(base + e, c[e], w[e]);
+        }
+    }
+    __device__ __forceinline__ void entry(const uint32_t pos, const uint32_t c, const T w) {
+        const T v = xs[c];
+        g[pos] = r * v;
+        acc += w * v;
+    }
+    static constexpr bool SUMS = true;
+    using Sum = T;
+    __device__ __forceinline__ Sum total(const int lanes) const { return group_sum(acc, lanes); }
+    __device__ __forceinline__ void put(const uint32_t row, const Sum s) const { y[row] = s; }
+};
+
+template<typename T, int U>
+__global__ void __launch_bounds__(SHARED_THREADS, 1)
+gather_outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
+                           const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g,
+                           T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col,
+                           const uint32_t long_from) {
+    extern __shared__ __align__(16) unsigned char shared_vector[];
+    T *xs = reinterpret_cast<T *>(shared_vector);
+    const Deal deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
+    GatherOuterVisit<T> visit{xs, row_vector, g, y, n_row, T(0), T(0)};
+    walk_rows<T, true, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         fill_shared(xs, col_vector, n_col);
         zero_outside_rows(g, indptr, n_row, nse);
         __syncthreads();
@@ -696,18 +760,18 @@ bool usable(const CsrMatrix<T> &m, const bool weights) {
 // The bands pay where the sectors of x are used again in an SM (as many entries as sectors: 2e6 entries, 100,000 columns
 // 13.4 -> 11 us; two thirds, 400,000 columns: 26 -> 29), and where there are rows to sweep side by side (34 per SM: 26 ->
 // 29 us, 135: 37 -> 28).  500 lanes per SM, 16 entries or more for each.
-template<typename T, bool HOMO, bool OUTER>
-bool bands(cudaStream_t stream, const CsrMatrix<T> &m, const T *data, const T *x, T *out) {
+template<typename T, bool HOMO, int MODE>
+bool bands(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *x, T *y, T *out) {
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     const auto aligned32 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; };
     if (m.n_row < 100u * sms || static_cast<double>(m.nse) / sms < m.n_col * (sizeof(T) / 32.0) || !aligned32(m.indices) ||
-        (!HOMO && !OUTER && !aligned32(data)) || (OUTER && !aligned16(out)))
+        ((MODE & BAND_SUM) && !HOMO && !aligned32(m.data)) || ((MODE & BAND_OUTER) && !aligned16(out)))
         return false;
     uint32_t log_l = 0;
     while (log_l < 5 && (static_cast<uint64_t>(m.n_row) << log_l) < 512u * sms && (m.nse / m.n_row >> log_l) >= 16u) ++log_l;
     const uint64_t blocks = ((static_cast<uint64_t>(m.n_row) << log_l) + BAND_THREADS - 1) / BAND_THREADS;
-    bands_kernel<T, HOMO, OUTER><<<static_cast<uint32_t>(std::min<uint64_t>(blocks, 64ull * sms)), BAND_THREADS, 0, stream>>>(
-        m.indices, m.indptr, data, x, out, m.n_row, m.nse, log_l);
+    bands_kernel<T, HOMO, MODE><<<static_cast<uint32_t>(std::min<uint64_t>(blocks, 64ull * sms)), BAND_THREADS, 0, stream>>>(
+        m.indices, m.indptr, m.data, row_vector, x, y, out, m.n_row, m.nse, log_l);
     launch_ok();
     return true;
 }
@@ -718,7 +782,7 @@ template<typename T, bool HOMO>
 bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
     constexpr auto kernel = gather_shared_kernel<T, HOMO, U>;
-    if (m.n_col > BANDS_FROM<T> && bands<T, HOMO, false>(stream, m, m.data, x, y)) return true;
+    if (m.n_col > BANDS_FROM<T> && bands<T, HOMO, BAND_SUM>(stream, m, nullptr, x, y, nullptr)) return true;
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
@@ -773,35 +837,73 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
 }
 
 template<typename T, bool HOMO>
-bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
-    constexpr int U = sizeof(T) == 8 ? 1 : 2;
-    constexpr auto kernel = scatter_shared_kernel<T, HOMO, U>;
+bool scatter_pays(const CsrMatrix<T> &m) {
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     // a reduction into L2: slower the fewer columns share them (20,000 columns 3.1 clocks, 2000 columns 13), and in double
     const double words = sizeof(T) / 4, reduction = (1.85 + 25000.0 / m.n_col) * (sizeof(T) == 8 ? 1.25 : 1.0);
-    if (p.fill + 0.3 * words * m.n_col + p.per * (p.entry + 0.3 * words) > 0.95 * (reduction * p.per + 1500)) return false;
-    if (cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(m.n_col), stream) != cudaSuccess) return launch_ok(), true;
+    return p.fill + 0.3 * words * m.n_col + p.per * (p.entry + 0.3 * words) <= 0.95 * (reduction * p.per + 1500);
+}
+
+// `behind_zero`: the launch in front clears y
+template<typename T, bool HOMO>
+bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y, const bool behind_zero = false) {
+    constexpr int U = sizeof(T) == 8 ? 1 : 2;
+    constexpr auto kernel = scatter_shared_kernel<T, HOMO, U>;
+    if (!scatter_pays<T, HOMO>(m)) return false;
+    if (!behind_zero && cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(m.n_col), stream) != cudaSuccess) return launch_ok(), true;
     if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
+    if (behind_zero) {
+        const cudaError_t e = launch_dependent(kernel, dim3(sm_count()), dim3(SHARED_THREADS), shared_bytes<T>(m.n_col * sizeof(T)), stream,
+                                               m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col,
+                                               long_rows_from(m.nse, m.n_row, 4 * U));
+        if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+        return true;
+    }
     kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
         m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
     launch_ok();
     return true;
 }
 
+// `zero`: elements to clear; false, and nothing cleared, where another kernel has to do the product
 template<typename T>
-bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g) {
+bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g, T *zero = nullptr,
+                const uint32_t n_zero = 0) {
     constexpr int U = 2;
     constexpr auto kernel = outer_shared_kernel<T, U>;
-    if (m.n_col > BANDS_FROM<T> && bands<T, true, true>(stream, m, row_vector, col_vector, g)) return true;
+    if (zero == nullptr && m.n_col > BANDS_FROM<T> && bands<T, true, BAND_OUTER>(stream, m, row_vector, col_vector, nullptr, g)) return true;
     if (!usable(m, false) || !aligned16(g)) return false;
     const Plan<T> p(m, true);                // one index in, one value out
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
     if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
     kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
-        m.indices, m.indptr, row_vector, col_vector, g, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
+        m.indices, m.indptr, row_vector, col_vector, g, zero, n_zero, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
     launch_ok();
     return true;
+}
+
+// The gradients of a product, one launch (transposed product) or two without a memset between them.  A training step of a few
+// million entries is bound by the host, and each launch costs it 2 to 3 us.
+template<typename T>
+bool gather_outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g, T *y) {
+    constexpr int U = sizeof(T) == 8 ? 1 : 2;
+    constexpr auto kernel = gather_outer_shared_kernel<T, U>;
+    if (m.n_col > BANDS_FROM<T> && bands<T, false, BAND_SUM | BAND_OUTER>(stream, m, row_vector, col_vector, y, g)) return true;
+    if (!usable(m, true) || !aligned16(g)) return false;
+    const Plan<T> p(m, true);
+    if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
+    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
+    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
+        m.indices, m.indptr, m.data, row_vector, col_vector, g, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
+    launch_ok();
+    return true;
+}
+
+template<typename T>
+bool outer_scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g, T *y) {
+    return m.n_col <= BANDS_FROM<T> && scatter_pays<T, false>(m) && outer_impl<T>(stream, m, row_vector, col_vector, g, y, m.n_col) &&
+           scatter_impl<T, false>(stream, m, row_vector, y, true);
 }
 
 }  // namespace
@@ -832,6 +934,19 @@ bool outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *r
 }
 bool outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *r, const double *c, double *g) {
     return outer_impl<double>(stream, m, r, c, g);
+}
+
+bool gather_outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *r, const float *c, float *g, float *y) {
+    return gather_outer_impl<float>(stream, m, r, c, g, y);
+}
+bool gather_outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *r, const double *c, double *g, double *y) {
+    return gather_outer_impl<double>(stream, m, r, c, g, y);
+}
+bool outer_scatter_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *r, const float *c, float *g, float *y) {
+    return outer_scatter_impl<float>(stream, m, r, c, g, y);
+}
+bool outer_scatter_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *r, const double *c, double *g, double *y) {
+    return outer_scatter_impl<double>(stream, m, r, c, g, y);
 }
 
 }  // namespace bpl

@@ -28,6 +28,12 @@ bool scatter_shared(cudaStream_t stream, const CsrMatrix<double> &m, const doubl
 // g[e] = row_vector[row of e] * col_vector[indices[e]]; m.data is not read
 bool outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *row_vector, const float *col_vector, float *g);
 bool outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *row_vector, const double *col_vector, double *g);
+// g as above and y[row] = sum of data * col_vector[column] (the gradients of a transposed product), or y[column] = sum of
+// data * row_vector[row] (of the other one); y need not be zero
+bool gather_outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *row_vector, const float *col_vector, float *g, float *y);
+bool gather_outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *row_vector, const double *col_vector, double *g, double *y);
+bool outer_scatter_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *row_vector, const float *col_vector, float *g, float *y);
+bool outer_scatter_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *row_vector, const double *col_vector, double *g, double *y);
 
 }  // namespace bpl
 

@@ -276,6 +276,20 @@ Tensor outer_of(const Tensor &indices, const Tensor &indptr, const Tensor &x, co
     return at::GradMode::is_enabled() ? CsrOuterFn::apply(row, col, indices, indptr) : csr_outer(row, col, indices, indptr);
 }
 
+// Both gradients of a product of per-entry weights, without a graph of their own: (of the weights, of the vector)
+std::pair<Tensor, Tensor> csr_gradients(const Tensor &data, const Tensor &indices, const Tensor &indptr, const Tensor &x,
+                                        const Tensor &ct, int64_t n_row, int64_t n_col, bool transpose) {
+    NoGil no_gil;
+    OnDevice on(data);
+    Tensor g_data = new_tensor({indices.size(0)}, data.scalar_type(), data.device());
+    Tensor g_x = new_tensor({x.size(0)}, data.scalar_type(), data.device());
+    bpl_csr_gradients(on.stream, ptr(data), ptr(indices), ptr(indptr), ptr(x), ptr(ct), ptr(g_data), ptr(g_x),
+                      static_cast<uint32_t>(n_row), static_cast<uint32_t>(n_col), static_cast<uint32_t>(indices.size(0)),
+                      is_double(data) ? 1 : 0, transpose ? 1 : 0);
+    check_status();
+    return {g_data, g_x};
+}
+
 variable_list CsrFn::backward(AutogradContext *ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &data = saved[0], &indices = saved[1], &indptr = saved[2], &x = saved[3];
@@ -286,6 +300,9 @@ variable_list CsrFn::backward(AutogradContext *ctx, variable_list grads) {
     if (!plain_cotangent(ct)) {
         std::tie(g_data, g_x) = python_rule(g_csr_backward, {data, indices, indptr, x, ct}, n_row, n_col, t,
                                             ctx->needs_input_grad(0), ctx->needs_input_grad(3));
+    } else if (ctx->needs_input_grad(0) && ctx->needs_input_grad(3) && data.size(0) == indices.size(0) && data.size(0) != 1 &&
+               !at::GradMode::is_enabled()) {
+        std::tie(g_data, g_x) = csr_gradients(data, indices, indptr, x, ct, n_row, n_col, t);
     } else {
         if (ctx->needs_input_grad(0)) {
             if (data.size(0) == 1) {

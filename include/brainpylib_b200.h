@@ -277,6 +277,8 @@ BPL_FOR_EACH_TARGET(BPL_DECLARE_ONE)
  * bpl_csr_outer: g[e] = row_vector[row of entry e] * col_vector[indices[e]] for the nse stored entries of a CSR matrix
  * (float32, or float64 with is_double): the gradient of a CSR product with respect to its weights
  * (brainpylib/_src/sparse_ops/cusparse_matvec.py:292-304).  Zero for entries that no row owns.
+ * bpl_csr_gradients: the gradients of a CSR product y = A x (or A^T x with transpose) of nse weights with respect to both
+ * operands: data_gradient (nse, as bpl_csr_outer) and vector_gradient (as long as the vector; need not be zero).
  * bpl_csr_matvec: csr_matvec_{homo,heter}_vector_* / csr_matvec_transpose_* without descriptor, for callers that know the
  * number of stored entries nse on the host (it selects the kernel).
  * bpl_event_csr_matvec: event_csr_matvec_* in the same way (buffers as there, with a workspace of
@@ -294,6 +296,9 @@ void bpl_event_csr_matvec(bpl_stream_t stream, void **buffers, uint32_t n_row, u
                           int is_double, int bool_events, int transpose);
 void bpl_csr_outer(bpl_stream_t stream, const void *row_vector, const void *col_vector, const void *indices,
                    const void *indptr, void *out, uint32_t n_row, uint32_t n_col, uint32_t nse, int is_double);
+void bpl_csr_gradients(bpl_stream_t stream, const void *data, const void *indices, const void *indptr, const void *vector,
+                       const void *cotangent, void *data_gradient, void *vector_gradient, uint32_t n_row, uint32_t n_col,
+                       uint32_t nse, int is_double, int transpose);
 void bpl_csr_matvec(bpl_stream_t stream, const void *data, const void *indices, const void *indptr, const void *vector,
                     void *out, uint32_t n_row, uint32_t n_col, uint32_t nse, int homo, int is_double, int transpose);
 

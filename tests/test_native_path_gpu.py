@@ -413,3 +413,29 @@ def test_time_of_a_product_with_a_long_row(cuda, n_row, n_col, op, bound):
           'product': lambda: bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col)),
           'gradient': lambda: torch.autograd.grad(y, data, xt, retain_graph=True)}[op]
   assert _device_us(call) < bound
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('transpose', [False, True])
+# vector in shared memory with rows cut for warps and blocks, swept in bands by one lane and by several, neither; aligned or not
+@pytest.mark.parametrize('kind', ['shared', 'shared_many', 'bands', 'bands_teams', 'plain'])
+@pytest.mark.parametrize('front', [0, 5])
+def test_both_gradients_at_once(cuda, kind, front, transpose, dtype):
+  """One or two launches for both gradients; entries in front of and behind the matrix have the gradient zero."""
+  n_row, n_col, lens = _uneven(kind)
+  data, indices, indptr = _skewed(n_row, n_col, lens, dtype, cuda)
+  pad = lambda a: torch.cat([a.new_zeros(front), a, a.new_zeros(front)])
+  data, indices, indptr = pad(data).requires_grad_(True), pad(indices), indptr + front
+  g = torch.Generator(device=cuda).manual_seed(51)
+  x = torch.randn(n_row if transpose else n_col, dtype=dtype, device=cuda, generator=g).requires_grad_(True)
+  y = bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
+  ct = torch.randn(y.shape[0], dtype=dtype, device=cuda, generator=g)
+  junk = [torch.full_like(data, float('nan')), torch.full_like(x, float('nan'))]
+  del junk                               # their memory is the gradients'
+  g_data, g_x = torch.autograd.grad(y, (data, x), ct)
+  inner = slice(front, indices.shape[0] - front)
+  want_data, want_x = _expected(data[inner], indices[inner], indptr - front, x, ct, (n_row, n_col), transpose)
+  torch.testing.assert_close(g_data[inner], want_data.to(dtype))
+  assert not g_data[:front].any() and not g_data[indices.shape[0] - front:].any()
+  tol = dict(rtol=1e-5, atol=1e-3) if dtype == torch.float32 else dict(rtol=1e-12, atol=1e-10)
+  torch.testing.assert_close(g_x.double(), want_x, **tol)
