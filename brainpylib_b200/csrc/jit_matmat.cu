@@ -152,25 +152,30 @@ __device__ __noinline__ void walk_column(const unsigned int seed, const GapParam
 // A thread owns one column and 32 rows of X and walks its own list; Xt is staged tile by tile into a ring of buffers, one
 // block of up to 896 threads per SM.  A connection is 32 products against 8 reads of 16 bytes per lane: the lanes of a warp
 // read different tile rows (their positions are unrelated), which would put them on the same banks, so lane l reads the
-// 16-byte chunks of its row in the rotated order (c + l) mod CHUNKS: the eight lanes served together touch eight different
-// chunks.  The register (c, i) of lane l belongs to row ((c + l) mod CHUNKS) * PER_CHUNK + i.
+// 16-byte chunks of its row in the order c ^ (l mod CHUNKS): the eight lanes served together touch eight different chunks.
+// The register (c, i) of lane l belongs to row (c ^ (l mod CHUNKS)) * PER_CHUNK + i.
 //
-// What bounds it is the shared-memory pipe, and how many lanes of a warp have work in the tiles that are resident: the
-// number of connections per column and tile is Poisson.  With one tile of 768 positions at a time (mean 7.7 at 1 %) 55 % of
-// the lanes worked, and the warps waited for the slowest one at every tile.  Now a warp moves on when all its lanes are
-// through with its oldest tile, while a lane that is through runs on into the next ones that have landed; and no warp waits
-// for another: each waits for the arrival of a tile only (an mbarrier per buffer), and the last warp to leave a tile
-// starts the copy (one bulk copy of 24 KB) that takes its place.
-// C5 (256 x 65536 @ 65536^2, 1 %): 3.09 ms with one tile at a time and block barriers, 2.39 ms now.
+// What bounds it is the shared-memory pipe, how many lanes of a warp have work in the tiles that are resident (the number of
+// connections per column and tile is Poisson), and what a warp does once per tile.  It moves on when all its lanes are through
+// with its oldest tile, while a lane that is through runs on into the next ones that have landed; and no warp waits for
+// another: each waits for the arrival of a tile only (an mbarrier per buffer), and the last warp to leave a tile starts the
+// copy (one bulk copy) that takes its place.  With eight tiles of 192 positions a warp spent 140 instructions per tile on that,
+// twice what a connection takes: four tiles of 384 hold the same positions (192 KB: with more, L1 no longer holds the other
+// half of the sectors that the lists come in), and it waits for the tile after its own before it goes on, so that lanes have
+// somewhere to run on to.
+// 256 x 65536 @ 65536^2, 1 %: 3.09 ms with one tile at a time and block barriers, 2.39 ms with the ring (without the lists),
+// 2.25 now; 100 x 30000 @ 30000 x 40000, 0.5 %: whole call 321 -> 271 us.
 //
 // Measured alternatives: lanes as rows (a warp owns 30 columns x 64 rows, entries broadcast from a staging buffer, every
 // lane works on every connection) 5.3 ms: 14 instructions per entry and 64 rows against 50 per 32 entries and 32 rows here;
-// the same without staging 7.7-10 ms.
-constexpr unsigned int RING = 8;                            // buffers of 24 KB
+// the same without staging 7.7-10 ms.  Lists read four entries at a time: 3 to 25 % slower.  Steps while some number of lanes
+// have work, tiles given back behind the last lane of all: 5 to 60 % slower.  Packed multiply-adds: no change.
+constexpr unsigned int RING = 4;                            // buffers of 48 KB
+constexpr unsigned int AHEAD = 2;                           // tiles that have landed before a warp works on the first of them
 template<typename T> struct ApplyShape;
-template<> struct ApplyShape<float> { static constexpr int MAX_THREADS = 896, KT = 192, CHUNKS = 8; };
-template<> struct ApplyShape<double> { static constexpr int MAX_THREADS = 512, KT = 96, CHUNKS = 16; };   // 32 double sums
-constexpr unsigned int TILE_BYTES = 24u * 1024u;
+template<> struct ApplyShape<float> { static constexpr int MAX_THREADS = 896, KT = 384, CHUNKS = 8; };
+template<> struct ApplyShape<double> { static constexpr int MAX_THREADS = 512, KT = 192, CHUNKS = 16; };   // 32 double sums
+constexpr unsigned int TILE_BYTES = 48u * 1024u;
 constexpr unsigned int APPLY_SMEM = RING * TILE_BYTES;
 
 __device__ __forceinline__ uint32_t shared_address(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -200,6 +205,20 @@ __device__ __forceinline__ bool barrier_wait(uint64_t *bar, const uint32_t parit
     return false;
 }
 
+// sum[0 ..] += w * the 16 bytes at `at`
+__device__ __forceinline__ void add_chunk(float *sum, const uint32_t at, const float w) {
+    float x[4];
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(at) : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] += (x[i] * w);
+}
+__device__ __forceinline__ void add_chunk(double *sum, const uint32_t at, const double w) {
+    double x[2];
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "r"(at) : "memory");
+#pragma unroll
+    for (int i = 0; i < 2; ++i) sum[i] += (x[i] * w);
+}
+
 // grid = (row groups of 32, column blocks of blockDim.x columns): the blocks that walk the same columns' lists are
 // launched side by side, so the lists come from DRAM once and from L2 for the other row groups.
 template<typename T, int KIND>
@@ -210,10 +229,9 @@ jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k,
                         const unsigned int seed, const GapParams gp, const double w1, const double w2, T *__restrict__ Y) {
     constexpr int KT = ApplyShape<T>::KT, CHUNKS = ApplyShape<T>::CHUNKS, PER_CHUNK = 16 / sizeof(T);
     static_assert(KT * MM_ROWS * sizeof(T) == TILE_BYTES, "a tile");
-    extern __shared__ __align__(128) unsigned char mm_smem[];
+    extern __shared__ __align__(256) unsigned char mm_smem[];           // T [RING][KT][MM_ROWS]; a row of it (128 or 256 bytes) aligned to itself
     __shared__ __align__(8) uint64_t landed_bar[RING];
     __shared__ unsigned int left[RING];                                  // warps that are through with the tile of a buffer
-    T *ring = reinterpret_cast<T *>(mm_smem);                            // [RING][KT][MM_ROWS]
     pdl_wait();
 
     const unsigned int c = blockIdx.y * blockDim.x + threadIdx.x;       // column within the chunk
@@ -221,20 +239,24 @@ jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k,
     const unsigned int lane = threadIdx.x & 31u;
     const T *group = Xt + static_cast<size_t>(blockIdx.x) * k * MM_ROWS;
     const bool overflow = live && cnt[c] > cap;                         // its list reads as empty
-    // The list is read two entries at a time (every lane reads its own list, so a warp's load touches 32 different lines
-    // and costs the load/store pipe as much as all shared loads of a connection together).  `cur` holds the pair being
-    // consumed, `nxt` the pair after it, requested when `cur` is entered; `j` counts consumed entries.
+    // The list is read two entries at a time (every lane reads its own list, so a warp's load touches 32 different lines).
+    // `pos` and `weight` are the entry to come, `second` is the other one of its pair (while `odd`), and `next` the pair behind
+    // it, requested when its predecessor is entered.  Positions ascend: a pair whose second is inside has a successor.
     const MMEntryPair<T> *pairs = reinterpret_cast<const MMEntryPair<T> *>(entries + static_cast<size_t>(c) * cap);
-    MMEntryPair<T> cur, nxt;
-    cur.a.pos = cur.b.pos = nxt.a.pos = nxt.b.pos = LIST_END;
-    cur.a.w = cur.b.w = nxt.a.w = nxt.b.w = T(0);
-    unsigned int j = 0;
+    MMEntry<T> second;
+    MMEntryPair<T> next;
+    unsigned int pos = LIST_END;
+    T weight = T(0);
+    bool odd = true;
+    second.pos = next.a.pos = next.b.pos = LIST_END;
+    second.w = next.a.w = next.b.w = T(0);
     if (live) {
-        cur = pairs[0];
-        if (max(cur.a.pos, cur.b.pos) < k) nxt = pairs[1];
+        next = *pairs++;
+        pos = next.a.pos;
+        weight = next.a.w;
+        second = next.b;
+        if (max(pos, second.pos) < k) next = *pairs;
     }
-    unsigned int pos = cur.a.pos;
-    T weight = cur.a.w;
     T sum[MM_ROWS];
 #pragma unroll
     for (int i = 0; i < static_cast<int>(MM_ROWS); ++i) sum[i] = T(0);
@@ -256,16 +278,15 @@ jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k,
     }
     __syncthreads();
     unsigned int landed = 0;                                             // tiles that this warp knows to be there
+    const uint32_t home = shared_address(mm_smem) + (lane & (CHUNKS - 1)) * 16u;
     bool lost = false;
     for (unsigned int t = 0; t < n_tiles; ++t) {
-        if (landed == t) {
-            lost = !barrier_wait(&landed_bar[t % RING], (t / RING) & 1u);
-            if (__any_sync(FULL_MASK, lost)) {
-                lost = true;
-                break;
-            }
+        while (landed < min(t + AHEAD, n_tiles)) {                       // (below t + RING: started, at the latest when the last warp leaves tile t - 1)
+            lost = __any_sync(FULL_MASK, !barrier_wait(&landed_bar[landed % RING], (landed / RING) & 1u));
+            if (lost) break;
             ++landed;
         }
+        if (lost) break;
         // further ones: below t + RING, whose buffer is the one of tile t
         while (landed < min(t + RING, n_tiles) && __all_sync(FULL_MASK, barrier_done(&landed_bar[landed % RING], (landed / RING) & 1u)))
             ++landed;
@@ -275,25 +296,21 @@ jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k,
             if (pos < open) {
                 unsigned int slot = slot0 + (pos - first);
                 if (slot >= RING * KT) slot -= RING * KT;
-                const T *row = ring + slot * MM_ROWS;
+                const uint32_t row = home + slot * static_cast<uint32_t>(MM_ROWS * sizeof(T));
                 const T w = weight;
-                ++j;
-                if (j & 1u) {                                            // second entry of the pair
-                    pos = cur.b.pos;
-                    weight = cur.b.w;
-                } else {                                                 // next pair; request the one after it unless the
-                    cur = nxt;                                           // list ends inside
-                    pos = cur.a.pos;
-                    weight = cur.a.w;
-                    if (max(cur.a.pos, cur.b.pos) < k) nxt = pairs[(j >> 1) + 1];
+                if (odd) {
+                    pos = second.pos;
+                    weight = second.w;
+                } else {
+                    pos = next.a.pos;
+                    weight = next.a.w;
+                    second = next.b;
+                    ++pairs;
+                    if (second.pos < k) next = *pairs;
                 }
+                odd = !odd;
 #pragma unroll
-                for (int cc = 0; cc < CHUNKS; ++cc) {
-                    const unsigned int chunk = (cc + lane) & (CHUNKS - 1);
-                    const Values<T, PER_CHUNK> x = *reinterpret_cast<const Values<T, PER_CHUNK> *>(row + chunk * PER_CHUNK);
-#pragma unroll
-                    for (int i = 0; i < PER_CHUNK; ++i) sum[cc * PER_CHUNK + i] += (x.v[i] * w);
-                }
+                for (int cc = 0; cc < CHUNKS; ++cc) add_chunk(&sum[cc * PER_CHUNK], row ^ (cc * 16u), w);
             }
         }
         __syncwarp();
@@ -317,7 +334,7 @@ jit_matmat_apply_kernel(const T *Xt, const unsigned int m, const unsigned int k,
     if (live && !overflow) {
 #pragma unroll
         for (int cc = 0; cc < CHUNKS; ++cc) {
-            const unsigned int chunk = (cc + lane) & (CHUNKS - 1);
+            const unsigned int chunk = cc ^ (lane & (CHUNKS - 1));
 #pragma unroll
             for (int i = 0; i < PER_CHUNK; ++i) {
                 const unsigned int row = row0 + chunk * PER_CHUNK + i;
@@ -467,7 +484,8 @@ StagedChoice choose_staged(const ListPlan &p, unsigned int k, unsigned int cols)
     for (unsigned int th = 128; th <= static_cast<unsigned int>(ApplyShape<T>::MAX_THREADS); th += 32) {
         const double waves = std::ceil(blocks_for(cols, th) * groups / sms);
         // per position: its copy into shared memory (16 bytes per clock: a tile is in flight while one is worked on), or the
-        // connections that use it (measured: 2.5 clocks for 32 float rows)
+        // connections that use it (2.5 clocks for 32 float rows; 2.0 to 3.7 measured, the more the fewer share a tile: where
+        // the choice against the other kernel is close, both take the same to 6 %)
         const double clocks = waves * k * std::max(row_bytes / 16, th * p.prob * 2.5 * row_bytes / 128);
         if (clocks <= best.clocks) best = {th, clocks};
     }

@@ -174,3 +174,13 @@ def test_matmat_from_lists_equals_the_inline_kernel(cuda, m, k, n, prob, dtype):
   X = torch.randn(m, k, dtype=dtype, generator=torch.Generator().manual_seed(5)).to(cuda)
   kw = dict(kind='normal', w1=0., w2=0.01, conn_prob=prob, shape=(k, n), seed=11)
   assert torch.equal(jitconn_ops.matmat_raw(X, **kw), jitconn_ops.matmat_raw(X, workspace=False, **kw))
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+# tiles of 384 (float64: 192) positions, a ring of four: one, one and a position, the whole ring, the first tile behind it
+@pytest.mark.parametrize('k', [192, 193, 384, 385, 768, 769, 1536, 1537, 3073])
+def test_matmat_at_the_edges_of_tiles(cuda, k, dtype):
+  from brainpylib_b200 import jitconn_ops
+  X = torch.randn(34, k, dtype=dtype, generator=torch.Generator().manual_seed(6)).to(cuda)
+  kw = dict(kind='uniform', w1=-0.1, w2=0.2, conn_prob=0.03, shape=(k, 20_001), seed=12)
+  assert torch.equal(jitconn_ops.matmat_raw(X, **kw), jitconn_ops.matmat_raw(X, workspace=False, **kw))
