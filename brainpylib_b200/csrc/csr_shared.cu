@@ -410,6 +410,11 @@ __device__ __forceinline__ void fill_bytes(uint8_t *bytes, const E *__restrict__
     for (uint32_t i = whole * PER + threadIdx.x; i < n; i += blockDim.x) bytes[i] = is_event(events[i]) ? 1 : 0;
 }
 
+// Entries of a lane for which its row gets one lane more.  Doubles take one quad per step, two words each; with a lane per quad
+// the sums over the lanes cost more than the steps they save (5e6 entries, rows of 64: 32.8 us by 16 lanes, 26.7 by 4; of 24:
+// 34.8 by 8, 28.7 by 4; of 250: 26.7 by 32, 26.6 by 16).
+template<typename T> constexpr uint32_t EVENT_STEP = sizeof(T) == 8 ? 16u : 8u;
+
 template<typename T, typename E, bool HOMO, bool BYTES, int U>
 __global__ void __launch_bounds__(SHARED_THREADS, 1)
 gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
@@ -417,7 +422,7 @@ gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__res
                      const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
-    const Deal deal(nse, n_row, 4 * U);
+    const Deal deal(nse, n_row, EVENT_STEP<T>);
     using Sum = typename EventVisit<T, HOMO, BYTES>::Sum;
     auto &cut_rows = cut_rows_at<Sum>(shared_vector, BYTES ? n_col : (n_col + 31u) / 32u * 4u);
     EventVisit<T, HOMO, BYTES> visit{mask, HOMO ? data[0] : T(0), y, T(0), 0u};
@@ -814,7 +819,7 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     if (HOMO && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
     if (!allow_shared<kernel>(ALL_SMEM) || !allow_shared<kernel_bytes>(ALL_SMEM)) return launch_ok(), true;
-    const uint32_t sms = static_cast<uint32_t>(sm_count()), long_from = long_rows_from(m.nse, m.n_row, 4 * U);
+    const uint32_t sms = static_cast<uint32_t>(sm_count()), long_from = long_rows_from(m.nse, m.n_row, EVENT_STEP<T>);
     // Bytes take the vector's own length from L1, which streams the entries: 200 KB of them 157 us for 1e8 entries, bits 143.
     if (m.n_col <= 131072u && m.n_col * sizeof(E) / 34.0 < (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0) + 0.08 * per) {
         kernel_bytes<<<sms, SHARED_THREADS, shared_bytes<Sum>(m.n_col), stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col,

@@ -439,3 +439,9 @@ def test_both_gradients_at_once(cuda, kind, front, transpose, dtype):
   assert not g_data[:front].any() and not g_data[indices.shape[0] - front:].any()
   tol = dict(rtol=1e-5, atol=1e-3) if dtype == torch.float32 else dict(rtol=1e-12, atol=1e-10)
   torch.testing.assert_close(g_x.double(), want_x, **tol)
+
+
+@pytest.mark.parametrize('homo', [True, False])
+@pytest.mark.parametrize('mean', [60, 100, 200, 300])         # 4, 8, 16 and 32 lanes per row
+def test_event_gather_of_doubles(cuda, mean, homo):
+  test_event_gather_over_bits(cuda, 30_000, 3001, mean, homo, np.float64, True)
