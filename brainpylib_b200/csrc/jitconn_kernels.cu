@@ -425,37 +425,55 @@ jit_cols_group_kernel(const T *__restrict__ vector, const unsigned int seed, con
 // Event input: lib/gpu_jitconn_event_matvec_atomic.cu:30-58, :88-117, :150-178.  There every column walks its stream and
 // only the atomicAdd is conditional; a silent column contributes nothing and its stream is private, so it is skipped
 // here.  Each block compacts the firing columns of its chunk into shared memory and gives one thread to each of them, or eight
-// lanes where there are at most `few` (50000 x 50000, p = 0.004, 1 % firing, normal weights: 30 -> 20 us).  The
-// chunk (at most COL_CHUNK) is chosen for four blocks per SM: the walk of a stream is a chain, and a few thousand columns in
-// chunks of 2048 left most SMs without one (5796 columns, 10 % firing: 20 us).
-constexpr int COL_CHUNK = GATHER_THREADS * 8;
+// lanes where there are at most `few`.  One block per SM: where four of them shared one, some ten firing columns each, give or
+// take three, single blocks went the other way than their neighbours and held them up (1e6 x 1e6, p = 0.001, normal weights,
+// 0.5 % firing: 125 us, now 90; 300,000 columns, 100,000 rows, p = 0.005, 0.5 %: 64, now 38).
+constexpr unsigned int COL_CHUNK = 8192;
 
+template<typename T>
+__global__ void __launch_bounds__(256) jit_clear_kernel(T *__restrict__ out, const unsigned int n) {
+    pdl_launch_dependents();
+    for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) out[i] = T(0);
+}
 
 template<typename T, typename E, int KIND, bool QUICK>
-__global__ void __launch_bounds__(GATHER_THREADS)
+__global__ void __launch_bounds__(WALK_THREADS)
 jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, const GapParams gp, const double w1,
                       const double w2, const unsigned int num_row, const unsigned int num_col, const unsigned int chunk,
                       const unsigned int few, T *__restrict__ out) {
     __shared__ unsigned int active[COL_CHUNK];
     __shared__ unsigned int n_active;
     constexpr int N = Batch<KIND, QUICK>::N;
+    constexpr unsigned int PER = 16 / sizeof(E);           // events per load; chunk is a multiple of 16
     if (threadIdx.x == 0) n_active = 0;
     __syncthreads();
-    const unsigned long long base = static_cast<unsigned long long>(blockIdx.x) * chunk;
-    const unsigned long long end = min(base + chunk, static_cast<unsigned long long>(num_col));
-#pragma unroll 8
-    for (unsigned long long c = base + threadIdx.x; c < end; c += blockDim.x) {
-        if (is_event(events[c])) active[atomicAdd(&n_active, 1u)] = static_cast<unsigned int>(c);
+    const unsigned int base = blockIdx.x * chunk, end = num_col - base < chunk ? num_col : base + chunk;
+    const unsigned int whole = aligned16_device(events) ? base + (end - base) / PER * PER : base;
+    for (unsigned int c = base + threadIdx.x * PER; c < whole; c += blockDim.x * PER) {
+        const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(events + c));
+        const E *e = reinterpret_cast<const E *>(&raw);
+        if ((raw.x | raw.y | raw.z | raw.w) == 0u) continue;
+#pragma unroll
+        for (unsigned int k = 0; k < PER; ++k)
+            if (is_event(e[k])) active[atomicAdd(&n_active, 1u)] = c + k;
     }
+    for (unsigned int c = whole + threadIdx.x; c < end; c += blockDim.x)
+        if (is_event(events[c])) active[atomicAdd(&n_active, 1u)] = c;
     __syncthreads();
-    const unsigned int n = n_active;
-    if (QUICK && n <= few) {                               // (at most one per group)
-        const unsigned int i = threadIdx.x / GROUP;
-        if (threadIdx.x / 32 * (32 / GROUP) < n)
+    pdl_wait();                                            // the output is zero
+    const unsigned int n = n_active, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    if (QUICK && n <= few) {
+        constexpr unsigned int PER_WARP = 32 / GROUP;
+        for (unsigned int i0 = warp * PER_WARP; i0 < n; i0 += warps * PER_WARP) {
+            const unsigned int i = i0 + (threadIdx.x & 31u) / GROUP;
             scatter_group<T, KIND>(seed + (i < n ? active[i] : 0u), i < n, T(1), num_row, gp, w1, w2, out);
+        }
         return;
     }
-    for (unsigned int i = threadIdx.x; i < n; i += blockDim.x) {
+    // As few warps as hold the columns, as many for each scheduler: a walk issues for all lanes of its warp.
+    const unsigned int per_warp = (n + 4u * ((n + 127u) / 128u) - 1u) / max(4u * ((n + 127u) / 128u), 1u), lane = threadIdx.x & 31u;
+    if (lane >= per_warp) return;
+    for (unsigned int i = warp * per_warp + lane; i < n; i += warps * per_warp) {
         Xorwow s;
         s.seed(seed + active[i]);
         Batch<KIND, QUICK> b;
@@ -646,9 +664,11 @@ constexpr int GROUP_ROWS = EVENT ? (KIND == W_HOMO ? 0 : 60) : KIND == W_NORMAL 
 // (9000 columns, p = 0.1, uniform: 3000 rows 65 us by one lane and 110 by eight, 30000 rows 468 and 357).
 constexpr unsigned int GROUP_LONG = 16384;
 constexpr int GROUP_COLS = 32, GROUP_COLS_LONG = 60;
-// (of firing columns; a block with one more than its share walks all of them by one lane each, beside blocks that do not)
+// Firing columns: at 30, 47 and 68 per SM of 1000 connections each, by eight lanes 77, 100 and 123 us, by one 113, 114 and 115 (normal);
+// 61, 84 and 95 against 66, 68 and 80 (uniform); 47, 60 and 80 against 55, 58 and 78 (homogeneous).  A little above where both
+// take the same: single blocks have more than others, and the slower of two kinds counts.
 template<int KIND>
-constexpr unsigned int GROUP_EVENTS = KIND == W_NORMAL ? 24 : 12;
+constexpr unsigned int GROUP_EVENTS = KIND == W_NORMAL ? 72 : KIND == W_UNIFORM ? 42 : 60;
 
 // Rules in clocks of one SM.  A gather through L1 takes one clock per connection.  Filling shared memory reads the whole
 // input per block, at about 56 bytes per clock, after a start of some 2000 clocks; a vector in several tiles is read
@@ -765,19 +785,19 @@ void jit_cols(const JitCall<T, T> &c) {
 template<typename T, typename E, int KIND>
 void jit_cols_event(const JitCall<T, E> &c) {
     const JitArgs &a = c.a;
-    if (cudaMemsetAsync(c.out, 0, sizeof(T) * static_cast<size_t>(a.n_row), c.stream) != cudaSuccess) {
-        launch_ok();
-        return;
-    }
-    if (a.n_col == 0) return;
+    const unsigned int sms = static_cast<unsigned int>(sm_count());
+    jit_clear_kernel<T><<<std::min(blocks_for(a.n_row, 1024), 8 * sms), 256, 0, c.stream>>>(c.out, a.n_row);
+    if (!launch_ok() || a.n_col == 0) return;
     const GapParams gp = gap_params(a.log_p, a.n_row);
-    const unsigned int chunk = std::min(static_cast<unsigned int>(COL_CHUNK), blocks_for(blocks_for(a.n_col, 4 * sm_count()), 32) * 32u);
-    const unsigned int blocks = blocks_for(a.n_col, chunk);
-    const unsigned int few = std::min(static_cast<unsigned int>(GATHER_THREADS / GROUP),
-                                      GROUP_EVENTS<KIND> * sm_count() / blocks);
-    (gp.quick ? jit_cols_event_kernel<T, E, KIND, true> : jit_cols_event_kernel<T, E, KIND, false>)<<<
-        blocks, GATHER_THREADS, 0, c.stream>>>(c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk, few, c.out);
-    launch_ok();
+    const unsigned int chunk = std::min(COL_CHUNK, blocks_for(blocks_for(a.n_col, sms), 16) * 16u), blocks = blocks_for(a.n_col, chunk);
+    const unsigned int threads = std::max(128u, std::min(static_cast<unsigned int>(WALK_THREADS), blocks_for(chunk, 4) * 32u));
+    // (In a short output the lanes of a warp that each walk a stream of their own meet at the same addresses: 101 firing columns
+    // per SM, 900 rows, 146 us by eight lanes, 183 by one; 3000 rows 28.7 and 30.7; 8000 rows 43.4 and 37.7.)
+    const unsigned int few = a.n_row < 4096u ? COL_CHUNK : blocks <= sms ? GROUP_EVENTS<KIND> : GROUP_EVENTS<KIND> * sms / blocks;
+    const cudaError_t e = launch_dependent(gp.quick ? jit_cols_event_kernel<T, E, KIND, true> : jit_cols_event_kernel<T, E, KIND, false>,
+                                           dim3(blocks), dim3(threads), 0, c.stream, c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk,
+                                           few, c.out);
+    if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
 }
 
 template<typename T, int KIND, bool ROWS>

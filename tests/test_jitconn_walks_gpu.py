@@ -83,6 +83,22 @@ def test_event_columns(cuda, shape, prob, rate, kind):
 
 
 @pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('dtype', [torch.bool, torch.float32, torch.float64])
+# events read 16 bytes at a time: fewer than that, ragged ends; several rounds of eight lanes; more columns than the SMs' lists hold
+@pytest.mark.parametrize('shape,prob,rate', [((900, 1), 0.2, 1.0), ((900, 15), 0.1, 1.0), ((700, 2371), 0.05, 0.0), ((700, 2371), 0.05, 0.5),
+                                             ((900, 40_009), 0.02, 1.0), ((5000, 40_009), 0.004, 0.9), ((300, 1_250_003), 0.02, 0.01)])
+@pytest.mark.parametrize('offset', [0, 1])                # 1: events not 16-byte aligned
+def test_event_columns_by_chunks(cuda, shape, prob, rate, offset, dtype, kind):
+  """Against the dense product of the events as zeros and ones, which walks every column."""
+  n_row, n_col = shape
+  fires = torch.rand(n_col + offset, generator=torch.Generator().manual_seed(8)) < rate
+  x = fires.to(dtype).to(cuda)[offset:]
+  got = _call(x, kind, prob, shape, False, True).double()
+  want = _call(x.double(), kind, prob, shape, False, False)
+  torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * max(float(want.abs().max()), 1e-3))
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
   """More streams than eight lanes each are given to, with too few connections for tiles: reductions and gathers."""
