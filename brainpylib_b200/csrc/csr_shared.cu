@@ -23,8 +23,11 @@
 namespace bpl {
 namespace {
 
-constexpr int SHARED_THREADS = 768;                  // one block per SM
-constexpr uint32_t SHARED_WARPS = SHARED_THREADS / 32;
+// Warps of a block, one block per SM: as many as there may be beside a vector of up to 131 KB; with more of shared memory taken,
+// the entries that so many have in flight no longer fit what is left of L1.  (24 and 32 warps: 1.57e7 double entries and
+// events, 1 KB, 55.8 and 49.3 us; 1.2e7 floats, 80 KB of x, 23.7 and 22.1, transposed 36.4 and 34.9; 4.8e6 floats, 180 KB, 15.0
+// and 16.4.)
+constexpr uint32_t FEW_WARPS = 24, MANY_WARPS = 32, MANY_SMEM = 131u * 1024u;
 constexpr uint32_t SHARED_SMEM = 226u * 1024u;       // the longest vector
 
 // The rows of one block, in one walk that all three products share.
@@ -47,10 +50,11 @@ inline __host__ __device__ uint32_t lanes_per_row(const uint32_t nse, const uint
     const uint32_t want = (nse / n_row + per_step - 1u) / per_step;
     return want <= 4u ? 4u : want <= 8u ? 8u : want <= 16u ? 16u : 32u;
 }
-inline uint32_t long_rows_from(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
-    const uint32_t share = nse / (static_cast<uint32_t>(sm_count()) * SHARED_WARPS);
+inline uint32_t long_rows_from(const uint32_t nse, const uint32_t n_row, const uint32_t per_step, const uint32_t warps) {
+    const uint32_t share = nse / (static_cast<uint32_t>(sm_count()) * warps);
     return std::max(8u * per_step, share / 16u) * lanes_per_row(nse, n_row, per_step);
 }
+template<uint32_t W>
 struct Deal {
     uint32_t lpr, rows_per_warp;
     __device__ __forceinline__ Deal(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
@@ -62,7 +66,7 @@ struct Deal {
     }
     // the i-th row that a warp walks (in an order of its groups)
     __device__ __forceinline__ uint32_t row_of_warp(const uint32_t warp, const uint32_t i) const {
-        return row(warp + (i >> (__ffs(rows_per_warp) - 1)) * SHARED_WARPS, i & (rows_per_warp - 1u));
+        return row(warp + (i >> (__ffs(rows_per_warp) - 1)) * W, i & (rows_per_warp - 1u));
     }
 };
 
@@ -81,29 +85,29 @@ constexpr uint32_t MOST_ENTRIES = 0x7fffffffu;
 //                                         one lane leaves it
 // (Behind the vector in dynamic shared memory: with static shared memory in the kernel the vector no longer lies at the address
 // 0, and every look-up adds its base: 2 us of the event gather's 20.)
-template<typename Sum>
+template<typename Sum, uint32_t W>
 struct CutRows {
     uint32_t n, row[LONG_ROWS];
-    bool block[SHARED_WARPS];          // a warp has rows of more than BLOCK_ROW
-    Sum part[2][SHARED_WARPS];
+    bool block[W];          // a warp has rows of more than BLOCK_ROW
+    Sum part[2][W];
 };
 
 inline __host__ __device__ uint32_t behind_vector(const size_t bytes) { return static_cast<uint32_t>((bytes + 15u) & ~static_cast<size_t>(15u)); }
-template<typename Sum>
-__device__ __forceinline__ CutRows<Sum> &cut_rows_at(unsigned char *shared, const size_t bytes) {
-    return *reinterpret_cast<CutRows<Sum> *>(shared + behind_vector(bytes));
+template<typename Sum, uint32_t W>
+__device__ __forceinline__ CutRows<Sum, W> &cut_rows_at(unsigned char *shared, const size_t bytes) {
+    return *reinterpret_cast<CutRows<Sum, W> *>(shared + behind_vector(bytes));
 }
-template<typename Sum>
-uint32_t shared_bytes(const size_t vector_bytes) { return behind_vector(vector_bytes) + sizeof(CutRows<Sum>); }
+template<typename Sum, uint32_t W>
+uint32_t shared_bytes(const size_t vector_bytes) { return behind_vector(vector_bytes) + sizeof(CutRows<Sum, W>); }
 constexpr uint32_t ALL_SMEM = 227u * 1024u;
-static_assert(SHARED_SMEM + sizeof(CutRows<double>) <= ALL_SMEM, "the longest vector and the list");
+static_assert(SHARED_SMEM + sizeof(CutRows<double, FEW_WARPS>) <= ALL_SMEM, "the longest vector and the list");
 
 // The rows that the walk has cut; `mine`: this warp has some, `block`: some warps of the block have rows for all of it.
-template<typename T, bool WEIGHTS, typename Visit>
+template<typename T, bool WEIGHTS, uint32_t W, typename Visit>
 __device__ __noinline__ void walk_cut_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                                            const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
-                                           const uint32_t long_from, const Deal deal, Visit visit, const bool mine, const bool block,
-                                           CutRows<typename Visit::Sum> &cut_rows) {
+                                           const uint32_t long_from, const Deal<W> deal, Visit visit, const bool mine, const bool block,
+                                           CutRows<typename Visit::Sum, W> &cut_rows) {
     const uint32_t lane = threadIdx.x & 31, g_full = nse >> 2;
     auto span = [&](const uint32_t r, const uint32_t start, const uint32_t end, const uint32_t first, const uint32_t lanes) {
         constexpr int AHEAD = sizeof(T) == 8 ? 2 : 4;
@@ -158,14 +162,14 @@ __device__ __noinline__ void walk_cut_rows(const uint32_t *__restrict__ indices,
     uint32_t turn = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const uint32_t r = cut_rows.row[i];
-        span(r, indptr[r] + skip, indptr[r + 1], threadIdx.x, SHARED_THREADS);
+        span(r, indptr[r] + skip, indptr[r + 1], threadIdx.x, W * 32u);
         if (!Visit::SUMS) continue;
         // one barrier per row: the sums of the next go to the other half, and who reads these is through at the barrier after
         const typename Visit::Sum s = visit.total(32);
         if (lane == 0) cut_rows.part[turn & 1u][warp] = s;
         __syncthreads();
-        if (warp == turn % SHARED_WARPS) {
-            const typename Visit::Sum t = group_sum(lane < SHARED_WARPS ? cut_rows.part[turn & 1u][lane] : typename Visit::Sum(0), 32);
+        if (warp == turn % W) {
+            const typename Visit::Sum t = group_sum(lane < W ? cut_rows.part[turn & 1u][lane] : typename Visit::Sum(0), 32);
             if (lane == 0) visit.put(r, t);
         }
         ++turn;
@@ -173,11 +177,11 @@ __device__ __noinline__ void walk_cut_rows(const uint32_t *__restrict__ indices,
 }
 
 // `ready` runs before the first entry is visited, behind the first loads: it fills shared memory and ends with a barrier.
-template<typename T, bool WEIGHTS, int U, typename Visit, typename Ready>
+template<typename T, bool WEIGHTS, int U, uint32_t W, typename Visit, typename Ready>
 __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                                           const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
-                                          const uint32_t long_from, const Deal deal, Visit &visit,
-                                          CutRows<typename Visit::Sum> &cut_rows, Ready ready) {
+                                          const uint32_t long_from, const Deal<W> deal, Visit &visit,
+                                          CutRows<typename Visit::Sum, W> &cut_rows, Ready ready) {
     const uint32_t lane = threadIdx.x & 31, lpr = deal.lpr;
     const uint32_t sub = lane / lpr, sl = lane % lpr;
     const uint32_t g_full = nse >> 2;
@@ -210,7 +214,7 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
     };
     auto cut = [&](Row &r) { r.end = min(r.end, r.start + long_from); };     // (where the pointers are needed, not where they are asked for)
     uint32_t group = threadIdx.x >> 5;
-    Row row = pointers(group), next = pointers(group + SHARED_WARPS);
+    Row row = pointers(group), next = pointers(group + W);
     cut(row);
     cut(next);
     if (threadIdx.x == 0) cut_rows.n = 0;
@@ -221,7 +225,7 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         after.g0 = more ? now.g0 + U * lpr : (next.start >> 2) + sl;
         load(after, more ? row : next);
         Row later{0u, 0u, Fetched()};
-        if (!more) later = pointers(group + 2 * SHARED_WARPS);
+        if (!more) later = pointers(group + 2 * W);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t base = 4u * (now.g0 + u * lpr);
@@ -241,7 +245,7 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
             const typename Visit::Sum s = visit.total(static_cast<int>(lpr));
             if (sl == 0 && deal.row(group, sub) < n_row) visit.put(deal.row(group, sub), s);
         }
-        group += SHARED_WARPS;
+        group += W;
         row = next;
         next = later;
         cut(next);
@@ -283,7 +287,7 @@ __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, 
         if (deal.row(group, 0) >= n_row) break;
         step(b, a);
     }
-    for_block = __any_sync(FULL_MASK, lane < SHARED_WARPS && cut_rows.block[lane]);
+    for_block = __any_sync(FULL_MASK, lane < W && cut_rows.block[lane]);
     if (some_cut || for_block)
         walk_cut_rows<T, WEIGHTS>(indices, indptr, data, n_row, nse, long_from, deal, visit, some_cut, for_block, cut_rows);
 }
@@ -294,18 +298,18 @@ __device__ __forceinline__ void fill_shared(T *shared, const T *__restrict__ p, 
     constexpr uint32_t PER = 16 / sizeof(T);
     const uint32_t n_vec = aligned16_device(p) ? count / PER : 0u;
 #pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < n_vec; i += SHARED_THREADS)
+    for (uint32_t i = threadIdx.x; i < n_vec; i += blockDim.x)
         reinterpret_cast<uint4 *>(shared)[i] = __ldg(reinterpret_cast<const uint4 *>(p) + i);
-    for (uint32_t i = n_vec * PER + threadIdx.x; i < count; i += SHARED_THREADS) shared[i] = __ldg(p + i);
+    for (uint32_t i = n_vec * PER + threadIdx.x; i < count; i += blockDim.x) shared[i] = __ldg(p + i);
 }
 
 // The same for words that the launch in front has written.
 __device__ __forceinline__ void fill_words(uint32_t *shared, const uint32_t *p, const uint32_t count) {
     const uint32_t n_vec = aligned16_device(p) ? count / 4u : 0u;
 #pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < n_vec; i += SHARED_THREADS)
+    for (uint32_t i = threadIdx.x; i < n_vec; i += blockDim.x)
         reinterpret_cast<uint4 *>(shared)[i] = __ldcg(reinterpret_cast<const uint4 *>(p) + i);
-    for (uint32_t i = n_vec * 4u + threadIdx.x; i < count; i += SHARED_THREADS) shared[i] = __ldcg(p + i);
+    for (uint32_t i = n_vec * 4u + threadIdx.x; i < count; i += blockDim.x) shared[i] = __ldcg(p + i);
 }
 
 // y = A x
@@ -329,15 +333,15 @@ struct GatherVisit {
     __device__ __forceinline__ void put(const uint32_t row, const Sum s) const { y[row] = s; }
 };
 
-template<typename T, bool HOMO, int U>
-__global__ void __launch_bounds__(SHARED_THREADS, 1)
+template<typename T, bool HOMO, int U, uint32_t W>
+__global__ void __launch_bounds__(W * 32, 1)
 gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col,
                      const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
-    const Deal deal(nse, n_row, 4 * U);
-    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
+    const Deal<W> deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     GatherVisit<T, HOMO> visit{xs, HOMO ? data[0] : T(0), y, T(0)};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         fill_shared(xs, x, n_col);
@@ -415,16 +419,16 @@ __device__ __forceinline__ void fill_bytes(uint8_t *bytes, const E *__restrict__
 // 34.8 by 8, 28.7 by 4; of 250: 26.7 by 32, 26.6 by 16).
 template<typename T> constexpr uint32_t EVENT_STEP = sizeof(T) == 8 ? 16u : 8u;
 
-template<typename T, typename E, bool HOMO, bool BYTES, int U>
-__global__ void __launch_bounds__(SHARED_THREADS, 1)
+template<typename T, typename E, bool HOMO, bool BYTES, int U, uint32_t W>
+__global__ void __launch_bounds__(W * 32, 1)
 gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const E *__restrict__ events, const uint32_t *packed, T *__restrict__ y, const uint32_t n_row,
                      const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
-    const Deal deal(nse, n_row, EVENT_STEP<T>);
+    const Deal<W> deal(nse, n_row, EVENT_STEP<T>);
     using Sum = typename EventVisit<T, HOMO, BYTES>::Sum;
-    auto &cut_rows = cut_rows_at<Sum>(shared_vector, BYTES ? n_col : (n_col + 31u) / 32u * 4u);
+    auto &cut_rows = cut_rows_at<Sum, W>(shared_vector, BYTES ? n_col : (n_col + 31u) / 32u * 4u);
     EventVisit<T, HOMO, BYTES> visit{mask, HOMO ? data[0] : T(0), y, T(0), 0u};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         if (BYTES) {
@@ -619,18 +623,18 @@ struct ScatterVisit {
     __device__ __forceinline__ void put(uint32_t, Sum) const {}
 };
 
-template<typename T, bool HOMO, int U>
-__global__ void __launch_bounds__(SHARED_THREADS, 1)
+template<typename T, bool HOMO, int U, uint32_t W>
+__global__ void __launch_bounds__(W * 32, 1)
 scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                       const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse,
                       const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *sums = reinterpret_cast<T *>(shared_vector);
-    const Deal deal(nse, n_row, 4 * U);
-    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
+    const Deal<W> deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     ScatterVisit<T, HOMO> visit{sums, n_row, x, HOMO ? data[0] : T(0), T(0)};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
-        for (uint32_t i = threadIdx.x; i < n_col; i += SHARED_THREADS) sums[i] = T(0);
+        for (uint32_t i = threadIdx.x; i < n_col; i += W * 32u) sums[i] = T(0);
         __syncthreads();
     });
     __syncthreads();
@@ -667,17 +671,17 @@ struct OuterVisit {
 };
 
 // (`zero`: n_zero elements to clear for the launch behind this one)
-template<typename T, int U>
-__global__ void __launch_bounds__(SHARED_THREADS, 1)
+template<typename T, int U, uint32_t W>
+__global__ void __launch_bounds__(W * 32, 1)
 outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                     const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g, T *__restrict__ zero,
                     const uint32_t n_zero, const uint32_t n_row, const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     pdl_launch_dependents();
-    for (uint32_t i = blockIdx.x * SHARED_THREADS + threadIdx.x; i < n_zero; i += gridDim.x * SHARED_THREADS) zero[i] = T(0);
+    for (uint32_t i = blockIdx.x * (W * 32u) + threadIdx.x; i < n_zero; i += gridDim.x * (W * 32u)) zero[i] = T(0);
     T *xs = reinterpret_cast<T *>(shared_vector);
-    const Deal deal(nse, n_row, 4 * U);
-    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
+    const Deal<W> deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     OuterVisit<T> visit{xs, row_vector, g, n_row, T(0)};
     walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         fill_shared(xs, col_vector, n_col);
@@ -723,16 +727,16 @@ struct GatherOuterVisit {
     __device__ __forceinline__ void put(const uint32_t row, const Sum s) const { y[row] = s; }
 };
 
-template<typename T, int U>
-__global__ void __launch_bounds__(SHARED_THREADS, 1)
+template<typename T, int U, uint32_t W>
+__global__ void __launch_bounds__(W * 32, 1)
 gather_outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                            const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g,
                            T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col,
                            const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
-    const Deal deal(nse, n_row, 4 * U);
-    auto &cut_rows = cut_rows_at<T>(shared_vector, n_col * sizeof(T));
+    const Deal<W> deal(nse, n_row, 4 * U);
+    auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     GatherOuterVisit<T> visit{xs, row_vector, g, y, n_row, T(0), T(0)};
     walk_rows<T, true, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
         fill_shared(xs, col_vector, n_col);
@@ -783,26 +787,34 @@ bool bands(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, cons
 // columns from which the bands are faster than x in shared memory (200 KB of floats; of doubles, 164 KB)
 template<typename T> constexpr uint32_t BANDS_FROM = sizeof(T) == 4 ? 51200u : 21000u;
 
+// go(warps of a block, a constant), for so much shared memory
+template<typename Go>
+void with_warps(const size_t vector_bytes, Go go) {
+    if (vector_bytes <= MANY_SMEM) go(std::integral_constant<uint32_t, MANY_WARPS>());
+    else go(std::integral_constant<uint32_t, FEW_WARPS>());
+}
+
 template<typename T, bool HOMO>
 bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
-    constexpr auto kernel = gather_shared_kernel<T, HOMO, U>;
     if (m.n_col > BANDS_FROM<T> && bands<T, HOMO, BAND_SUM>(stream, m, nullptr, x, y, nullptr)) return true;
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
-        m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
-    launch_ok();
+    with_warps(m.n_col * sizeof(T), [&](auto warps) {
+        constexpr uint32_t W = decltype(warps)::value;
+        constexpr auto kernel = gather_shared_kernel<T, HOMO, U, W>;
+        if (allow_shared<kernel>(ALL_SMEM))
+            kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
+                m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U, W));
+        launch_ok();
+    });
     return true;
 }
 
 template<typename T, typename E, bool HOMO>
 bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, uint32_t *workspace, T *y) {
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
-    constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, U>;
-    constexpr auto kernel_bytes = gather_events_kernel<T, E, HOMO, true, U>;
     using Sum = std::conditional_t<HOMO, uint32_t, T>;
     const uint32_t bytes = (m.n_col + 31u) / 32u * 4u;
     if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.nse > MOST_ENTRIES || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
@@ -818,26 +830,34 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     const double mean_row = static_cast<double>(m.nse) / m.n_row;
     if (HOMO && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
-    if (!allow_shared<kernel>(ALL_SMEM) || !allow_shared<kernel_bytes>(ALL_SMEM)) return launch_ok(), true;
-    const uint32_t sms = static_cast<uint32_t>(sm_count()), long_from = long_rows_from(m.nse, m.n_row, EVENT_STEP<T>);
+    const uint32_t sms = static_cast<uint32_t>(sm_count());
     // Bytes take the vector's own length from L1, which streams the entries: 200 KB of them 157 us for 1e8 entries, bits 143.
-    if (m.n_col <= 131072u && m.n_col * sizeof(E) / 34.0 < (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0) + 0.08 * per) {
-        kernel_bytes<<<sms, SHARED_THREADS, shared_bytes<Sum>(m.n_col), stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col,
-                                                              long_from);
-        launch_ok();
-        return true;
-    }
-    if (!pack) {
-        kernel<<<sms, SHARED_THREADS, shared_bytes<Sum>(bytes), stream>>>(m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col,
-                                                              long_from);
-        launch_ok();
+    const bool as_bytes = m.n_col <= 131072u && m.n_col * sizeof(E) / 34.0 < (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0) + 0.08 * per;
+    if (as_bytes || !pack) {
+        with_warps(as_bytes ? m.n_col : bytes, [&](auto warps) {
+            constexpr uint32_t W = decltype(warps)::value;
+            constexpr auto of_bytes = gather_events_kernel<T, E, HOMO, true, U, W>, of_bits = gather_events_kernel<T, E, HOMO, false, U, W>;
+            if (as_bytes ? allow_shared<of_bytes>(ALL_SMEM) : allow_shared<of_bits>(ALL_SMEM))
+                (as_bytes ? of_bytes : of_bits)<<<sms, W * 32, shared_bytes<Sum, W>(as_bytes ? m.n_col : bytes), stream>>>(
+                    m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, EVENT_STEP<T>, W));
+            launch_ok();
+        });
         return true;
     }
     pack_events_kernel<E><<<std::min<uint32_t>((m.n_col + 255u) / 256u, 8u * sms), 256, 0, stream>>>(events, workspace, m.n_col);
     if (!launch_ok()) return true;
-    const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(SHARED_THREADS), shared_bytes<Sum>(bytes), stream, m.indices, m.indptr, m.data,
-                                           events, workspace, y, m.n_row, m.nse, m.n_col, long_from);
-    if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+    with_warps(bytes, [&](auto warps) {
+        constexpr uint32_t W = decltype(warps)::value;
+        constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, U, W>;
+        if (!allow_shared<kernel>(ALL_SMEM)) {
+            launch_ok();
+            return;
+        }
+        const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(W * 32), shared_bytes<Sum, W>(bytes), stream, m.indices, m.indptr, m.data,
+                                               events, workspace, y, m.n_row, m.nse, m.n_col,
+                                               long_rows_from(m.nse, m.n_row, EVENT_STEP<T>, W));
+        if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+    });
     return true;
 }
 
@@ -854,20 +874,24 @@ bool scatter_pays(const CsrMatrix<T> &m) {
 template<typename T, bool HOMO>
 bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y, const bool behind_zero = false) {
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
-    constexpr auto kernel = scatter_shared_kernel<T, HOMO, U>;
     if (!scatter_pays<T, HOMO>(m)) return false;
     if (!behind_zero && cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(m.n_col), stream) != cudaSuccess) return launch_ok(), true;
-    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
-    if (behind_zero) {
-        const cudaError_t e = launch_dependent(kernel, dim3(sm_count()), dim3(SHARED_THREADS), shared_bytes<T>(m.n_col * sizeof(T)), stream,
-                                               m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col,
-                                               long_rows_from(m.nse, m.n_row, 4 * U));
-        if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
-        return true;
-    }
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
-        m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
-    launch_ok();
+    with_warps(m.n_col * sizeof(T), [&](auto warps) {
+        constexpr uint32_t W = decltype(warps)::value;
+        constexpr auto kernel = scatter_shared_kernel<T, HOMO, U, W>;
+        const uint32_t smem = shared_bytes<T, W>(m.n_col * sizeof(T)), sms = static_cast<uint32_t>(sm_count());
+        const uint32_t long_from = long_rows_from(m.nse, m.n_row, 4 * U, W);
+        if (!allow_shared<kernel>(ALL_SMEM)) {
+            launch_ok();
+        } else if (behind_zero) {
+            const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(W * 32), smem, stream, m.indices, m.indptr, m.data, x, y, m.n_row,
+                                                   m.nse, m.n_col, long_from);
+            if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
+        } else {
+            kernel<<<sms, W * 32, smem, stream>>>(m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_from);
+            launch_ok();
+        }
+    });
     return true;
 }
 
@@ -876,15 +900,18 @@ template<typename T>
 bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g, T *zero = nullptr,
                 const uint32_t n_zero = 0) {
     constexpr int U = 2;
-    constexpr auto kernel = outer_shared_kernel<T, U>;
     if (zero == nullptr && m.n_col > BANDS_FROM<T> && bands<T, true, BAND_OUTER>(stream, m, row_vector, col_vector, nullptr, g)) return true;
     if (!usable(m, false) || !aligned16(g)) return false;
     const Plan<T> p(m, true);                // one index in, one value out
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
-        m.indices, m.indptr, row_vector, col_vector, g, zero, n_zero, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
-    launch_ok();
+    with_warps(m.n_col * sizeof(T), [&](auto warps) {
+        constexpr uint32_t W = decltype(warps)::value;
+        constexpr auto kernel = outer_shared_kernel<T, U, W>;
+        if (allow_shared<kernel>(ALL_SMEM))
+            kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
+                m.indices, m.indptr, row_vector, col_vector, g, zero, n_zero, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U, W));
+        launch_ok();
+    });
     return true;
 }
 
@@ -893,14 +920,15 @@ bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector,
 template<typename T>
 bool gather_outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, const T *col_vector, T *g, T *y) {
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
-    constexpr auto kernel = gather_outer_shared_kernel<T, U>;
     if (m.n_col > BANDS_FROM<T> && bands<T, false, BAND_SUM | BAND_OUTER>(stream, m, row_vector, col_vector, y, g)) return true;
     if (!usable(m, true) || !aligned16(g)) return false;
     const Plan<T> p(m, true);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    if (!allow_shared<kernel>(ALL_SMEM)) return launch_ok(), true;
-    kernel<<<static_cast<uint32_t>(sm_count()), SHARED_THREADS, shared_bytes<T>(m.n_col * sizeof(T)), stream>>>(
-        m.indices, m.indptr, m.data, row_vector, col_vector, g, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U));
+    constexpr uint32_t W = FEW_WARPS;        // (80 registers)
+    constexpr auto kernel = gather_outer_shared_kernel<T, U, W>;
+    if (allow_shared<kernel>(ALL_SMEM))
+        kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
+            m.indices, m.indptr, m.data, row_vector, col_vector, g, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U, W));
     launch_ok();
     return true;
 }

@@ -445,3 +445,23 @@ def test_both_gradients_at_once(cuda, kind, front, transpose, dtype):
 @pytest.mark.parametrize('mean', [60, 100, 200, 300])         # 4, 8, 16 and 32 lanes per row
 def test_event_gather_of_doubles(cuda, mean, homo):
   test_event_gather_over_bits(cuda, 30_000, 3001, mean, homo, np.float64, True)
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('more', [0, 1])           # the longest vector beside which a block has 32 warps; one element more: 24
+def test_products_by_more_and_fewer_warps(cuda, more, dtype):
+  n_row, n_col = 40_000, 131 * 1024 // dtype.itemsize + more
+  data, indices, indptr = _skewed(n_row, n_col, np.random.default_rng(3).poisson(130, n_row), dtype, cuda)
+  data.requires_grad_(True)
+  g = torch.Generator(device=cuda).manual_seed(9)
+  tol = dict(rtol=1e-5, atol=1e-3) if dtype == torch.float32 else dict(rtol=1e-12, atol=1e-10)
+  for transpose in (False, True):
+    x = torch.randn(n_row if transpose else n_col, dtype=dtype, device=cuda, generator=g).requires_grad_(True)
+    y = bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
+    ct = torch.randn(y.shape[0], dtype=dtype, device=cuda, generator=g)
+    row, col = sparse_ops.csr_to_coo(indices, indptr)
+    src, dst = (row, col) if transpose else (col, row)
+    want = torch.zeros_like(y, dtype=torch.float64).index_add_(0, dst, data.detach().double() * x.detach().double()[src])
+    torch.testing.assert_close(y.detach().double(), want, **tol)
+    for got, want in zip(torch.autograd.grad(y, (data, x), ct), _expected(data, indices, indptr, x, ct, (n_row, n_col), transpose)):
+      torch.testing.assert_close(got.double(), want, **tol)
