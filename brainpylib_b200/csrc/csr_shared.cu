@@ -33,40 +33,55 @@ constexpr uint32_t SHARED_SMEM = 226u * 1024u;       // the longest vector
 // The rows of one block, in one walk that all three products share.
 //
 // A warp takes 32 / lpr rows at a time, lpr lanes each: a lane takes 4 consecutive entries per 128-bit load and U such
-// loads per step, so that an average row takes one step.  Row groups are dealt out to the blocks in turn: neither a run of
-// empty rows nor a run of long ones falls to one SM.  Two things held the first form at half the memory rate: a branch per
-// entry (30 instructions each; the entries of a quad go through predicates now, and whether any lane's quad crosses the
-// ends of its row is asked once per quad and warp), and a warp that waited for a step's entries before it asked for the
-// next.  The entries of the next step, of this row or the next, are therefore requested before a step is worked on.
+// loads per step.  Row groups are dealt out to the blocks in turn: neither a run of empty rows nor a run of long ones falls
+// to one SM.  Two things held the first form at half the memory rate: a branch per entry (30 instructions each; the entries
+// of a quad go through predicates now, and whether any lane's quad crosses the ends of its row is asked once per quad and
+// warp), and a warp that waited for a step's entries before it asked for the next.  The entries of the next step, of this
+// row or the next, are therefore requested before a step is worked on.
 //
-// The lanes of a row are chosen for the mean length.  A row that would keep them for more than 8 steps, and for more than
-// twice a warp's share of all steps, is cut there (`long_from`).  Behind its walk a warp takes its cut rows with all its
+// The lanes of a row are chosen for the mean length.  A row that would keep them for 64 entries each, and for more than
+// twice a warp's share of all entries, is cut there (`long_from`).  Behind its walk a warp takes its cut rows with all its
 // lanes; those of more than BLOCK_ROW entries (LONG_ROWS of them at most) are left to all warps of the block.  (Lengths with a
 // heavy tail: 100,000 rows of 20 on average, the longest 30,000, y = A^T x: 858 us by the lanes of each row.  A test of every
 // row's length inside the walk, with a branch to a list, cost the event gather 1 to 5 us of 21.)
 constexpr uint32_t LONG_ROWS = 128, BLOCK_ROW = 4096;
 
-inline __host__ __device__ uint32_t lanes_per_row(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
-    const uint32_t want = (nse / n_row + per_step - 1u) / per_step;
-    return want <= 4u ? 4u : want <= 8u ? 8u : want <= 16u ? 16u : 32u;
+// Mean rows up to which 4, 8 and 16 lanes take a row.  More lanes mean fewer steps for a row, but each warp has fewer rows for
+// what a row costs besides its entries: its pointers, the sum over the lanes, lanes that have nothing left.  8e6 ragged entries, float,
+// by 4, 8, 16 and 32 lanes, us: events, rows of 40 (one weight) 18.5, 22.5, 28.8, 50.6; of 64 20.1, 18.5, 21.3, 26.1; of 150 18.6, 16.4,
+// 17.6, 18.3; of 300 17.9, 17.3, 15.9, 17.7; products, rows of 64 20.0, 17.2, 20.5, 25.1; of 100 20.0, 17.4, 16.5, 19.0; of 300 17.0, 16.3,
+// 15.9, 15.9; of 900 32.4, 26.5, 15.6, 14.0.  4e6 double: products, rows of 100 20.9, 17.9, 16.0, 16.5; transposed, rows of 64 31.7, 32.0,
+// 30.8, 32.3, of 100 36.0, 31.7, 30.2, 28.7.  (The lanes that finish a mean row in one step, which is what all of them had: events, rows
+// of 150 by 32 lanes 20.6.)  The lanes are constants of the kernels: as numbers they cost 3 to 10 % (rows of 300, 16 lanes, 16.9 us
+// and 15.9).  Products with outer values store what they read, and keep the lanes of one step.
+// Where few rows leave most warps with one group, or with none, the longest chain counts: a warp's groups, times the steps of `step`
+// entries per lane and one for the row.  (Products, 12,000 rows of 300, 12,000 columns: by 16 lanes 11.5 us, by 8, one group each,
+// 10.2; 6000 rows of 433 transposed, 1700 columns: by 32 lanes 16.4, by 16 14.4.  With up to two groups per warp, rows of 900, the
+// uneven lengths count for more: by 16 lanes 15.6, by 32 14.0.)
+struct LaneRule { uint32_t four, eight, sixteen, step; };
+template<typename T> constexpr LaneRule PRODUCT_LANES = sizeof(T) == 8 ? LaneRule{32, 80, 200, 4} : LaneRule{48, 80, 400, 8};
+template<typename T> constexpr LaneRule SCATTER_LANES = sizeof(T) == 8 ? LaneRule{16, 40, 80, 4} : LaneRule{48, 80, 400, 8};
+template<typename T> constexpr LaneRule EVENT_LANES = sizeof(T) == 8 ? LaneRule{80, 120, 400, 16} : LaneRule{48, 192, 400, 8};
+template<int U> constexpr LaneRule STEP_LANES{16u * U, 32u * U, 64u * U, 4u * U};
+inline uint32_t lanes_per_row(const uint32_t nse, const uint32_t n_row, const uint32_t warps, const LaneRule &rule) {
+    const uint32_t mean = nse / n_row;
+    const uint32_t lanes = mean <= rule.four ? 4u : mean <= rule.eight ? 8u : mean <= rule.sixteen ? 16u : 32u;
+    if (static_cast<uint64_t>(n_row) * lanes >= 48u * warps) return lanes;
+    auto chain = [&](const uint64_t l) { return (n_row * l + 32u * warps - 1u) / (32u * warps) * ((mean + l * rule.step - 1u) / (l * rule.step) + 1u); };
+    uint32_t best = 32u;
+    for (uint32_t l = 16u; l >= 4u; l /= 2u)
+        if (chain(l) < chain(best)) best = l;
+    return best;
 }
-inline uint32_t long_rows_from(const uint32_t nse, const uint32_t n_row, const uint32_t per_step, const uint32_t warps) {
-    const uint32_t share = nse / (static_cast<uint32_t>(sm_count()) * warps);
-    return std::max(8u * per_step, share / 16u) * lanes_per_row(nse, n_row, per_step);
-}
-template<uint32_t W>
+template<uint32_t W, uint32_t LANES>
 struct Deal {
-    uint32_t lpr, rows_per_warp;
-    __device__ __forceinline__ Deal(const uint32_t nse, const uint32_t n_row, const uint32_t per_step) {
-        lpr = lanes_per_row(nse, n_row, per_step);
-        rows_per_warp = 32u / lpr;
-    }
+    static constexpr uint32_t lpr = LANES, rows_per_warp = 32u / LANES;
     __device__ __forceinline__ uint32_t row(const uint32_t local_group, const uint32_t sub) const {
         return (local_group * gridDim.x + blockIdx.x) * rows_per_warp + sub;
     }
     // the i-th row that a warp walks (in an order of its groups)
     __device__ __forceinline__ uint32_t row_of_warp(const uint32_t warp, const uint32_t i) const {
-        return row(warp + (i >> (__ffs(rows_per_warp) - 1)) * W, i & (rows_per_warp - 1u));
+        return row(warp + i / rows_per_warp * W, i % rows_per_warp);
     }
 };
 
@@ -103,10 +118,10 @@ constexpr uint32_t ALL_SMEM = 227u * 1024u;
 static_assert(SHARED_SMEM + sizeof(CutRows<double, FEW_WARPS>) <= ALL_SMEM, "the longest vector and the list");
 
 // The rows that the walk has cut; `mine`: this warp has some, `block`: some warps of the block have rows for all of it.
-template<typename T, bool WEIGHTS, uint32_t W, typename Visit>
+template<typename T, bool WEIGHTS, uint32_t W, uint32_t LANES, typename Visit>
 __device__ __noinline__ void walk_cut_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                                            const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
-                                           const uint32_t long_from, const Deal<W> deal, Visit visit, const bool mine, const bool block,
+                                           const uint32_t long_from, const Deal<W, LANES> deal, Visit visit, const bool mine, const bool block,
                                            CutRows<typename Visit::Sum, W> &cut_rows) {
     const uint32_t lane = threadIdx.x & 31, g_full = nse >> 2;
     auto span = [&](const uint32_t r, const uint32_t start, const uint32_t end, const uint32_t first, const uint32_t lanes) {
@@ -177,12 +192,13 @@ __device__ __noinline__ void walk_cut_rows(const uint32_t *__restrict__ indices,
 }
 
 // `ready` runs before the first entry is visited, behind the first loads: it fills shared memory and ends with a barrier.
-template<typename T, bool WEIGHTS, int U, uint32_t W, typename Visit, typename Ready>
+template<typename T, bool WEIGHTS, int U, uint32_t W, uint32_t LANES, typename Visit, typename Ready>
 __device__ __forceinline__ void walk_rows(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                                           const T *__restrict__ data, const uint32_t n_row, const uint32_t nse,
-                                          const uint32_t long_from, const Deal<W> deal, Visit &visit,
+                                          const uint32_t long_from, const Deal<W, LANES> deal, Visit &visit,
                                           CutRows<typename Visit::Sum, W> &cut_rows, Ready ready) {
-    const uint32_t lane = threadIdx.x & 31, lpr = deal.lpr;
+    const uint32_t lane = threadIdx.x & 31;
+    constexpr uint32_t lpr = LANES;
     const uint32_t sub = lane / lpr, sl = lane % lpr;
     const uint32_t g_full = nse >> 2;
     using Fetched = decltype(visit.fetch(0u));
@@ -333,14 +349,14 @@ struct GatherVisit {
     __device__ __forceinline__ void put(const uint32_t row, const Sum s) const { y[row] = s; }
 };
 
-template<typename T, bool HOMO, int U, uint32_t W>
+template<typename T, bool HOMO, int U, uint32_t W, uint32_t LANES>
 __global__ void __launch_bounds__(W * 32, 1)
 gather_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse, const uint32_t n_col,
                      const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
-    const Deal<W> deal(nse, n_row, 4 * U);
+    constexpr Deal<W, LANES> deal;
     auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     GatherVisit<T, HOMO> visit{xs, HOMO ? data[0] : T(0), y, T(0)};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
@@ -414,19 +430,14 @@ __device__ __forceinline__ void fill_bytes(uint8_t *bytes, const E *__restrict__
     for (uint32_t i = whole * PER + threadIdx.x; i < n; i += blockDim.x) bytes[i] = is_event(events[i]) ? 1 : 0;
 }
 
-// Entries of a lane for which its row gets one lane more.  Doubles take one quad per step, two words each; with a lane per quad
-// the sums over the lanes cost more than the steps they save (5e6 entries, rows of 64: 32.8 us by 16 lanes, 26.7 by 4; of 24:
-// 34.8 by 8, 28.7 by 4; of 250: 26.7 by 32, 26.6 by 16).
-template<typename T> constexpr uint32_t EVENT_STEP = sizeof(T) == 8 ? 16u : 8u;
-
-template<typename T, typename E, bool HOMO, bool BYTES, int U, uint32_t W>
+template<typename T, typename E, bool HOMO, bool BYTES, int U, uint32_t W, uint32_t LANES>
 __global__ void __launch_bounds__(W * 32, 1)
 gather_events_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                      const E *__restrict__ events, const uint32_t *packed, T *__restrict__ y, const uint32_t n_row,
                      const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(shared_vector);
-    const Deal<W> deal(nse, n_row, EVENT_STEP<T>);
+    constexpr Deal<W, LANES> deal;
     using Sum = typename EventVisit<T, HOMO, BYTES>::Sum;
     auto &cut_rows = cut_rows_at<Sum, W>(shared_vector, BYTES ? n_col : (n_col + 31u) / 32u * 4u);
     EventVisit<T, HOMO, BYTES> visit{mask, HOMO ? data[0] : T(0), y, T(0), 0u};
@@ -623,14 +634,14 @@ struct ScatterVisit {
     __device__ __forceinline__ void put(uint32_t, Sum) const {}
 };
 
-template<typename T, bool HOMO, int U, uint32_t W>
+template<typename T, bool HOMO, int U, uint32_t W, uint32_t LANES>
 __global__ void __launch_bounds__(W * 32, 1)
 scatter_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                       const T *__restrict__ x, T *__restrict__ y, const uint32_t n_row, const uint32_t nse,
                       const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *sums = reinterpret_cast<T *>(shared_vector);
-    const Deal<W> deal(nse, n_row, 4 * U);
+    constexpr Deal<W, LANES> deal;
     auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     ScatterVisit<T, HOMO> visit{sums, n_row, x, HOMO ? data[0] : T(0), T(0)};
     walk_rows<T, !HOMO, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
@@ -671,7 +682,7 @@ struct OuterVisit {
 };
 
 // (`zero`: n_zero elements to clear for the launch behind this one)
-template<typename T, int U, uint32_t W>
+template<typename T, int U, uint32_t W, uint32_t LANES>
 __global__ void __launch_bounds__(W * 32, 1)
 outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                     const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g, T *__restrict__ zero,
@@ -680,7 +691,7 @@ outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__rest
     pdl_launch_dependents();
     for (uint32_t i = blockIdx.x * (W * 32u) + threadIdx.x; i < n_zero; i += gridDim.x * (W * 32u)) zero[i] = T(0);
     T *xs = reinterpret_cast<T *>(shared_vector);
-    const Deal<W> deal(nse, n_row, 4 * U);
+    constexpr Deal<W, LANES> deal;
     auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     OuterVisit<T> visit{xs, row_vector, g, n_row, T(0)};
     walk_rows<T, false, U>(indices, indptr, nullptr, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
@@ -727,7 +738,7 @@ struct GatherOuterVisit {
     __device__ __forceinline__ void put(const uint32_t row, const Sum s) const { y[row] = s; }
 };
 
-template<typename T, int U, uint32_t W>
+template<typename T, int U, uint32_t W, uint32_t LANES>
 __global__ void __launch_bounds__(W * 32, 1)
 gather_outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr, const T *__restrict__ data,
                            const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g,
@@ -735,7 +746,7 @@ gather_outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t 
                            const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
     T *xs = reinterpret_cast<T *>(shared_vector);
-    const Deal<W> deal(nse, n_row, 4 * U);
+    constexpr Deal<W, LANES> deal;
     auto &cut_rows = cut_rows_at<T, W>(shared_vector, n_col * sizeof(T));
     GatherOuterVisit<T> visit{xs, row_vector, g, y, n_row, T(0), T(0)};
     walk_rows<T, true, U>(indices, indptr, data, n_row, nse, long_from, deal, visit, cut_rows, [&]() {
@@ -787,11 +798,21 @@ bool bands(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector, cons
 // columns from which the bands are faster than x in shared memory (200 KB of floats; of doubles, 164 KB)
 template<typename T> constexpr uint32_t BANDS_FROM = sizeof(T) == 4 ? 51200u : 21000u;
 
-// go(warps of a block, a constant), for so much shared memory
-template<typename Go>
-void with_warps(const size_t vector_bytes, Go go) {
-    if (vector_bytes <= MANY_SMEM) go(std::integral_constant<uint32_t, MANY_WARPS>());
-    else go(std::integral_constant<uint32_t, FEW_WARPS>());
+// go(warps of a block, lanes of a row, where rows are cut): the first two are constants
+template<uint32_t W, typename Go>
+void with_lanes(const uint32_t nse, const uint32_t n_row, const LaneRule &rule, Go go) {
+    const uint32_t warps = static_cast<uint32_t>(sm_count()) * W, lanes = lanes_per_row(nse, n_row, warps, rule);
+    const uint32_t long_from = std::max(64u, nse / warps / 16u) * lanes;
+    constexpr std::integral_constant<uint32_t, W> w;
+    if (lanes == 4u) go(w, std::integral_constant<uint32_t, 4>(), long_from);
+    else if (lanes == 8u) go(w, std::integral_constant<uint32_t, 8>(), long_from);
+    else if (lanes == 16u) go(w, std::integral_constant<uint32_t, 16>(), long_from);
+    else go(w, std::integral_constant<uint32_t, 32>(), long_from);
+}
+template<typename T, typename Go>
+void with_block(const CsrMatrix<T> &m, const size_t vector_bytes, const LaneRule &rule, Go go) {
+    if (vector_bytes <= MANY_SMEM) with_lanes<MANY_WARPS>(m.nse, m.n_row, rule, go);
+    else with_lanes<FEW_WARPS>(m.nse, m.n_row, rule, go);
 }
 
 template<typename T, bool HOMO>
@@ -801,12 +822,12 @@ bool gather_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y) {
     if (!usable(m, !HOMO)) return false;
     const Plan<T> p(m, !HOMO);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    with_warps(m.n_col * sizeof(T), [&](auto warps) {
-        constexpr uint32_t W = decltype(warps)::value;
-        constexpr auto kernel = gather_shared_kernel<T, HOMO, U, W>;
+    with_block(m, m.n_col * sizeof(T), PRODUCT_LANES<T>, [&](auto warps, auto lanes, const uint32_t long_from) {
+        constexpr uint32_t W = decltype(warps)::value, L = decltype(lanes)::value;
+        constexpr auto kernel = gather_shared_kernel<T, HOMO, U, W, L>;
         if (allow_shared<kernel>(ALL_SMEM))
             kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
-                m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U, W));
+                m.indices, m.indptr, m.data, x, y, m.n_row, m.nse, m.n_col, long_from);
         launch_ok();
     });
     return true;
@@ -834,28 +855,28 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     // Bytes take the vector's own length from L1, which streams the entries: 200 KB of them 157 us for 1e8 entries, bits 143.
     const bool as_bytes = m.n_col <= 131072u && m.n_col * sizeof(E) / 34.0 < (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0) + 0.08 * per;
     if (as_bytes || !pack) {
-        with_warps(as_bytes ? m.n_col : bytes, [&](auto warps) {
-            constexpr uint32_t W = decltype(warps)::value;
-            constexpr auto of_bytes = gather_events_kernel<T, E, HOMO, true, U, W>, of_bits = gather_events_kernel<T, E, HOMO, false, U, W>;
+        with_block(m, as_bytes ? m.n_col : bytes, EVENT_LANES<T>, [&](auto warps, auto lanes, const uint32_t long_from) {
+            constexpr uint32_t W = decltype(warps)::value, L = decltype(lanes)::value;
+            constexpr auto of_bytes = gather_events_kernel<T, E, HOMO, true, U, W, L>, of_bits = gather_events_kernel<T, E, HOMO, false, U, W, L>;
             if (as_bytes ? allow_shared<of_bytes>(ALL_SMEM) : allow_shared<of_bits>(ALL_SMEM))
                 (as_bytes ? of_bytes : of_bits)<<<sms, W * 32, shared_bytes<Sum, W>(as_bytes ? m.n_col : bytes), stream>>>(
-                    m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, EVENT_STEP<T>, W));
+                    m.indices, m.indptr, m.data, events, nullptr, y, m.n_row, m.nse, m.n_col, long_from);
             launch_ok();
         });
         return true;
     }
     pack_events_kernel<E><<<std::min<uint32_t>((m.n_col + 255u) / 256u, 8u * sms), 256, 0, stream>>>(events, workspace, m.n_col);
     if (!launch_ok()) return true;
-    with_warps(bytes, [&](auto warps) {
-        constexpr uint32_t W = decltype(warps)::value;
-        constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, U, W>;
+    with_block(m, bytes, EVENT_LANES<T>, [&](auto warps, auto lanes, const uint32_t long_from) {
+        constexpr uint32_t W = decltype(warps)::value, L = decltype(lanes)::value;
+        constexpr auto kernel = gather_events_kernel<T, E, HOMO, false, U, W, L>;
         if (!allow_shared<kernel>(ALL_SMEM)) {
             launch_ok();
             return;
         }
         const cudaError_t e = launch_dependent(kernel, dim3(sms), dim3(W * 32), shared_bytes<Sum, W>(bytes), stream, m.indices, m.indptr, m.data,
                                                events, workspace, y, m.n_row, m.nse, m.n_col,
-                                               long_rows_from(m.nse, m.n_row, EVENT_STEP<T>, W));
+                                               long_from);
         if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
     });
     return true;
@@ -876,11 +897,10 @@ bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y, 
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
     if (!scatter_pays<T, HOMO>(m)) return false;
     if (!behind_zero && cudaMemsetAsync(y, 0, sizeof(T) * static_cast<size_t>(m.n_col), stream) != cudaSuccess) return launch_ok(), true;
-    with_warps(m.n_col * sizeof(T), [&](auto warps) {
-        constexpr uint32_t W = decltype(warps)::value;
-        constexpr auto kernel = scatter_shared_kernel<T, HOMO, U, W>;
+    with_block(m, m.n_col * sizeof(T), SCATTER_LANES<T>, [&](auto warps, auto lanes, const uint32_t long_from) {
+        constexpr uint32_t W = decltype(warps)::value, L = decltype(lanes)::value;
+        constexpr auto kernel = scatter_shared_kernel<T, HOMO, U, W, L>;
         const uint32_t smem = shared_bytes<T, W>(m.n_col * sizeof(T)), sms = static_cast<uint32_t>(sm_count());
-        const uint32_t long_from = long_rows_from(m.nse, m.n_row, 4 * U, W);
         if (!allow_shared<kernel>(ALL_SMEM)) {
             launch_ok();
         } else if (behind_zero) {
@@ -904,12 +924,12 @@ bool outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_vector,
     if (!usable(m, false) || !aligned16(g)) return false;
     const Plan<T> p(m, true);                // one index in, one value out
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
-    with_warps(m.n_col * sizeof(T), [&](auto warps) {
-        constexpr uint32_t W = decltype(warps)::value;
-        constexpr auto kernel = outer_shared_kernel<T, U, W>;
+    with_block(m, m.n_col * sizeof(T), STEP_LANES<U>, [&](auto warps, auto lanes, const uint32_t long_from) {
+        constexpr uint32_t W = decltype(warps)::value, L = decltype(lanes)::value;
+        constexpr auto kernel = outer_shared_kernel<T, U, W, L>;
         if (allow_shared<kernel>(ALL_SMEM))
             kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
-                m.indices, m.indptr, row_vector, col_vector, g, zero, n_zero, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U, W));
+                m.indices, m.indptr, row_vector, col_vector, g, zero, n_zero, m.n_row, m.nse, m.n_col, long_from);
         launch_ok();
     });
     return true;
@@ -925,11 +945,13 @@ bool gather_outer_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *row_
     const Plan<T> p(m, true);
     if (p.fill + p.per * p.entry > 0.95 * (p.per * std::max(1.0, p.entry) + 1500)) return false;
     constexpr uint32_t W = FEW_WARPS;        // (80 registers)
-    constexpr auto kernel = gather_outer_shared_kernel<T, U, W>;
-    if (allow_shared<kernel>(ALL_SMEM))
-        kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
-            m.indices, m.indptr, m.data, row_vector, col_vector, g, y, m.n_row, m.nse, m.n_col, long_rows_from(m.nse, m.n_row, 4 * U, W));
-    launch_ok();
+    with_lanes<W>(m.nse, m.n_row, STEP_LANES<U>, [&](auto, auto lanes, const uint32_t long_from) {
+        constexpr auto kernel = gather_outer_shared_kernel<T, U, W, decltype(lanes)::value>;
+        if (allow_shared<kernel>(ALL_SMEM))
+            kernel<<<static_cast<uint32_t>(sm_count()), W * 32, shared_bytes<T, W>(m.n_col * sizeof(T)), stream>>>(
+                m.indices, m.indptr, m.data, row_vector, col_vector, g, y, m.n_row, m.nse, m.n_col, long_from);
+        launch_ok();
+    });
     return true;
 }
 
