@@ -149,7 +149,7 @@ struct Batch {
     uint32_t raw[KIND == W_HOMO ? 1 : N];
 
     // LOW24: positions below 2^24, whose upper 8 bits are left undefined in pos[]; a stream that is through stays at n, so
-    // that a batch reaches n + 5 gaps at most
+    // that a batch reaches n + COUNT gaps at most
     template<bool LOW24 = false>
     __device__ __forceinline__ void draw(Xorwow &s, uint32_t &at, const uint32_t n, const GapParams &g) {
         uint32_t x[N];
