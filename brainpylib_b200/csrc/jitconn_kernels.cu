@@ -447,18 +447,20 @@ jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, con
     constexpr unsigned int PER = 16 / sizeof(E);           // events per load; chunk is a multiple of 16
     if (threadIdx.x == 0) n_active = 0;
     __syncthreads();
-    const unsigned int base = blockIdx.x * chunk, end = num_col - base < chunk ? num_col : base + chunk;
-    const unsigned int whole = aligned16_device(events) ? base + (end - base) / PER * PER : base;
-    for (unsigned int c = base + threadIdx.x * PER; c < whole; c += blockDim.x * PER) {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(events + c));
+    // (counted from the first column of the chunk: numbers of columns go up to 2^32 - 1)
+    const unsigned int base = blockIdx.x * chunk, count = min(chunk, num_col - base);
+    const E *mine = events + base;
+    const unsigned int whole = aligned16_device(events) ? count / PER * PER : 0u;
+    for (unsigned int i = threadIdx.x * PER; i < whole; i += blockDim.x * PER) {
+        const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(mine + i));
         const E *e = reinterpret_cast<const E *>(&raw);
         if ((raw.x | raw.y | raw.z | raw.w) == 0u) continue;
 #pragma unroll
         for (unsigned int k = 0; k < PER; ++k)
-            if (is_event(e[k])) active[atomicAdd(&n_active, 1u)] = c + k;
+            if (is_event(e[k])) active[atomicAdd(&n_active, 1u)] = base + i + k;
     }
-    for (unsigned int c = whole + threadIdx.x; c < end; c += blockDim.x)
-        if (is_event(events[c])) active[atomicAdd(&n_active, 1u)] = c;
+    for (unsigned int i = whole + threadIdx.x; i < count; i += blockDim.x)
+        if (is_event(mine[i])) active[atomicAdd(&n_active, 1u)] = base + i;
     __syncthreads();
     pdl_wait();                                            // the output is zero
     const unsigned int n = n_active, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;

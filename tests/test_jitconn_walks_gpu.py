@@ -100,6 +100,20 @@ def test_event_columns_by_chunks(cuda, shape, prob, rate, offset, dtype, kind):
   torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * max(float(want.abs().max()), 1e-3))
 
 
+# the largest number of columns; the first whose last chunk ends less than a round of loads before 2^32
+@pytest.mark.parametrize('n_col', [(1 << 32) - 1, (1 << 32) - 16_383])
+def test_event_columns_up_to_32_bits(cuda, n_col):
+  """Firing columns at both ends and in between, against calls with each of them alone."""
+  firing = [0, 8191, 1_000_003, (1 << 31) + 5, n_col - 8195, n_col - 2, n_col - 1]
+  x = torch.zeros(n_col, dtype=torch.bool, device=cuda)
+  x[firing] = True
+  one = torch.ones(1, dtype=torch.bool, device=cuda)
+  for kind in sorted(KINDS):
+    got = _call(x, kind, 0.2, (501, n_col), False, True).double()
+    want = sum(_call(one, kind, 0.2, (501, 1), False, True, seed=(77 + c) % (1 << 32)).double() for c in firing)
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-6)
+
+
 @pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
