@@ -427,8 +427,10 @@ jit_cols_group_kernel(const T *__restrict__ vector, const unsigned int seed, con
 // here.  Each block compacts the firing columns of its chunk into shared memory and gives one thread to each of them, or eight
 // lanes where there are at most `few`.  One block per SM: where four of them shared one, some ten firing columns each, give or
 // take three, single blocks went the other way than their neighbours and held them up (1e6 x 1e6, p = 0.001, normal weights,
-// 0.5 % firing: 125 us, now 90; 300,000 columns, 100,000 rows, p = 0.005, 0.5 %: 64, now 38).
-constexpr unsigned int COL_CHUNK = 8192;
+// 0.5 % firing: 125 us, now 77; 300,000 columns, 100,000 rows, p = 0.005, 0.5 %: 64, now 37).  The list has room for every
+// column of the chunk, up to all of shared memory; more columns take several equal waves.  (With lists of 8192 and a second wave
+// behind them, 1,250,000 columns, 2 % firing: 250 us, now 169.)
+constexpr unsigned int COL_CHUNK = WALK_SMEM / sizeof(unsigned int) / 1024u * 1024u;
 
 template<typename T>
 __global__ void __launch_bounds__(256) jit_clear_kernel(T *__restrict__ out, const unsigned int n) {
@@ -441,7 +443,7 @@ __global__ void __launch_bounds__(WALK_THREADS)
 jit_cols_event_kernel(const E *__restrict__ events, const unsigned int seed, const GapParams gp, const double w1,
                       const double w2, const unsigned int num_row, const unsigned int num_col, const unsigned int chunk,
                       const unsigned int few, T *__restrict__ out) {
-    __shared__ unsigned int active[COL_CHUNK];
+    extern __shared__ unsigned int active[];               // [chunk]
     __shared__ unsigned int n_active;
     constexpr int N = Batch<KIND, QUICK>::N;
     constexpr unsigned int PER = 16 / sizeof(E);           // events per load; chunk is a multiple of 16
@@ -802,14 +804,19 @@ void jit_cols_event(const JitCall<T, E> &c) {
     jit_clear_kernel<T><<<std::min(blocks_for(a.n_row, 1024), 8 * sms), 256, 0, c.stream>>>(c.out, a.n_row);
     if (!launch_ok() || a.n_col == 0) return;
     const GapParams gp = gap_params(a.log_p, a.n_row);
-    const unsigned int chunk = std::min(COL_CHUNK, blocks_for(blocks_for(a.n_col, sms), 16) * 16u), blocks = blocks_for(a.n_col, chunk);
+    const unsigned int waves = blocks_for(a.n_col, sms * COL_CHUNK);
+    const unsigned int chunk = blocks_for(blocks_for(a.n_col, sms * waves), 16) * 16u, blocks = blocks_for(a.n_col, chunk);
     const unsigned int threads = std::max(128u, std::min(static_cast<unsigned int>(WALK_THREADS), blocks_for(chunk, 4) * 32u));
     // (In a short output the lanes of a warp that each walk a stream of their own meet at the same addresses: 101 firing columns
     // per SM, 900 rows, 146 us by eight lanes, 183 by one; 3000 rows 28.7 and 30.7; 8000 rows 43.4 and 37.7.)
-    const unsigned int few = a.n_row < 4096u ? COL_CHUNK : blocks <= sms ? GROUP_EVENTS<KIND> : GROUP_EVENTS<KIND> * sms / blocks;
-    const cudaError_t e = launch_dependent(gp.quick ? jit_cols_event_kernel<T, E, KIND, true> : jit_cols_event_kernel<T, E, KIND, false>,
-                                           dim3(blocks), dim3(threads), 0, c.stream, c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk,
-                                           few, c.out);
+    const unsigned int few = a.n_row < 4096u ? chunk : GROUP_EVENTS<KIND>;
+    constexpr auto quick = jit_cols_event_kernel<T, E, KIND, true>, any = jit_cols_event_kernel<T, E, KIND, false>;
+    if (!(gp.quick ? allow_shared<quick>(COL_CHUNK * sizeof(unsigned int)) : allow_shared<any>(COL_CHUNK * sizeof(unsigned int)))) {
+        launch_ok();
+        return;
+    }
+    const cudaError_t e = launch_dependent(gp.quick ? quick : any, dim3(blocks), dim3(threads), chunk * sizeof(unsigned int), c.stream, c.in,
+                                           a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk, few, c.out);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));
 }
 

@@ -9,6 +9,7 @@ import torch
 
 import brainpylib_b200 as bpl
 from oracle import cpu
+from test_native_path_gpu import _device_us
 
 pytestmark = pytest.mark.gpu
 
@@ -98,6 +99,14 @@ def test_event_columns_by_chunks(cuda, shape, prob, rate, offset, dtype, kind):
   got = _call(x, kind, prob, shape, False, True).double()
   want = _call(x.double(), kind, prob, shape, False, False)
   torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * max(float(want.abs().max()), 1e-3))
+
+
+def test_time_of_event_columns_above_one_list(cuda):
+  """A few more columns than lists of 8192 on 148 SMs: no second wave of blocks (1.05 times the time; with it, 1.55)."""
+  def us(n_col):
+    x = torch.rand(n_col, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4)) < 0.02
+    return _device_us(lambda: _call(x, 'normal', 0.001, (1_000_000, n_col), False, True))
+  assert us(1_250_000) < 1.25 * us(1_200_000)
 
 
 # the largest number of columns; the first whose last chunk ends less than a round of loads before 2^32
