@@ -807,9 +807,13 @@ void jit_cols_event(const JitCall<T, E> &c) {
     const unsigned int waves = blocks_for(a.n_col, sms * COL_CHUNK);
     const unsigned int chunk = blocks_for(blocks_for(a.n_col, sms * waves), 16) * 16u, blocks = blocks_for(a.n_col, chunk);
     const unsigned int threads = std::max(128u, std::min(static_cast<unsigned int>(WALK_THREADS), blocks_for(chunk, 4) * 32u));
-    // (In a short output the lanes of a warp that each walk a stream of their own meet at the same addresses: 101 firing columns
-    // per SM, 900 rows, 146 us by eight lanes, 183 by one; 3000 rows 28.7 and 30.7; 8000 rows 43.4 and 37.7.)
-    const unsigned int few = a.n_row < 4096u ? chunk : GROUP_EVENTS<KIND>;
+    // In a short output the lanes of a warp that each walk a stream of their own meet at the same addresses; eight lanes of one
+    // stream do not, but seed it and draw for it eight times, which streams of a few connections do not pay back.  3000 rows, 1e6
+    // columns, 10 % firing, by eight lanes and by one, us (normal): 0.15 connections per stream 12.5, 8.2; 5 20.9, 24.6; 10 35.8, 51.3; 40 137,
+    // 265; half of them firing, 3 connections 53.6, 50.4.  300,000 columns, 5 %: 5 connections 8.2, 8.2; 80 53.3, 59.5.  8000 rows, 101
+    // firing columns per SM: 43.4, 37.7.
+    const bool meet = a.n_row < 4096u && a.n_row * -std::expm1(a.log_p) >= 4.0;
+    const unsigned int few = meet ? chunk : GROUP_EVENTS<KIND>;
     constexpr auto quick = jit_cols_event_kernel<T, E, KIND, true>, any = jit_cols_event_kernel<T, E, KIND, false>;
     if (!(gp.quick ? allow_shared<quick>(COL_CHUNK * sizeof(unsigned int)) : allow_shared<any>(COL_CHUNK * sizeof(unsigned int)))) {
         launch_ok();

@@ -109,6 +109,19 @@ def test_time_of_event_columns_above_one_list(cuda):
   assert us(1_250_000) < 1.25 * us(1_200_000)
 
 
+def test_time_of_event_columns_of_few_connections(cuda):
+  """A stream of less than one connection is walked by one lane, into short outputs as into longer ones."""
+  x = torch.rand(4_000_000, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4)) < 0.1
+  short, longer = (_device_us(lambda: _call(x, 'normal', 5e-5, (n_row, x.shape[0]), False, True)) for n_row in (3000, 4200))
+  assert short < 1.25 * longer
+
+
+@pytest.mark.parametrize('kind', sorted(KINDS))
+@pytest.mark.parametrize('prob', [0.0019, 0.0021])        # 3.9 and 4.3 connections per stream: by one lane, by eight
+def test_event_columns_around_the_line_of_connections(cuda, prob, kind):
+  test_event_columns_by_chunks(cuda, (2048, 40_009), prob, 0.3, 0, torch.bool, kind)
+
+
 # the largest number of columns; the first whose last chunk ends less than a round of loads before 2^32
 @pytest.mark.parametrize('n_col', [(1 << 32) - 1, (1 << 32) - 16_383])
 def test_event_columns_up_to_32_bits(cuda, n_col):
