@@ -415,6 +415,44 @@ def test_time_of_a_product_with_a_long_row(cuda, n_row, n_col, op, bound):
   assert _device_us(call) < bound
 
 
+@pytest.mark.parametrize('events', [False, True])
+def test_time_of_few_equal_rows(cuda, events):
+  """Rows that are longer than a warp's share of all entries, because there are fewer rows than warps, but no longer than the
+  others: as fast as a few more rows of as many entries in all (cut and walked twice: 2.0 times the time)."""
+  def us(n_row, length, n_col=20_000):
+    data, indices, indptr = _skewed(n_row, n_col, np.full(n_row, length), torch.float32, cuda)
+    x = torch.rand(n_col, device=cuda)
+    fires = x < 0.05
+    if events:
+      return _device_us(lambda: bpl.event_csr_matvec(data, indices, indptr, fires, shape=(n_row, n_col), transpose=False), 30)
+    return _device_us(lambda: bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col)), 30)
+  assert us(2000, 6000) < 1.2 * us(2400, 5000)
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('n_row,mean', [(30, 3000), (1700, 3000), (2000, 3000), (4800, 1500)])
+def test_products_of_few_rows(cuda, n_row, mean, dtype):
+  """Rows around the line from which they are cut: twice the mean, one entry less and more, far longer, empty.  Small whole numbers: the
+  sums are exact."""
+  n_col = 12_001
+  rng = np.random.default_rng(mean + n_row)
+  lengths = rng.poisson(mean, n_row)
+  lengths[[0, 3, 9, 14, n_row // 2, n_row - 1]] = 2 * mean, 2 * mean + 1, 2 * mean - 1, 0, 11_000, 4 * mean
+  data, indices, indptr = _skewed(n_row, n_col, lengths, dtype, cuda)
+  data = torch.randint(-8, 9, data.shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(1)).to(dtype)
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  for transpose in (False, True):
+    src, dst = (row, col) if transpose else (col, row)
+    n_in, n_out = (n_row, n_col) if transpose else (n_col, n_row)
+    x = torch.randint(-4, 5, (n_in,), device=cuda, generator=torch.Generator(device=cuda).manual_seed(2)).to(dtype)
+    for w in (data, data[:1]):
+      want = torch.zeros(n_out, dtype=torch.float64, device=cuda).index_add_(0, dst, w.double() * x.double()[src])
+      assert torch.equal(bpl.csr_matvec(w, indices, indptr, x, shape=(n_row, n_col), transpose=transpose).double(), want)
+      want = torch.zeros(n_out, dtype=torch.float64, device=cuda).index_add_(0, dst, w.double() * (x > 0).double()[src])
+      got = bpl.event_csr_matvec(w, indices, indptr, x > 0, shape=(n_row, n_col), transpose=transpose)
+      assert torch.equal(got.double(), want)
+
+
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 @pytest.mark.parametrize('transpose', [False, True])
 # vector in shared memory with rows cut for warps and blocks, swept in bands by one lane and by several, neither; aligned or not
