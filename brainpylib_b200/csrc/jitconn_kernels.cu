@@ -62,6 +62,7 @@ jit_rows_dense_v1_kernel(const T *__restrict__ vector, const unsigned int seed, 
 //   FROM_MASK    events as one bit each in shared memory (1e6 inputs = 125 KB): truthiness is all that is needed.  A hit
 //                leaves its raw draws in a queue of its thread (shared memory); the weights are computed when a queue is
 //                full, by all threads of the warp together, instead of by one thread at a time where it hits
+//   FROM_MASK_SHORT   the same with fewer connections per batch, which need shorter queues: beside long masks
 //   FROM_BYTES   the same with one byte per event where they fit beside the queues: three instructions fewer per connection
 //   FROM_TILES   the vector in shared memory, in as few tiles as fit (58,000 floats each).  Positions ascend along a
 //                stream, so all streams of a block cross one tile together; a batch that straddles the end of a tile is
@@ -82,7 +83,7 @@ __device__ __forceinline__ void push_pair_if(const bool second, const uint32_t h
                      : "+r"(next), "+r"(seconds) : "r"(hit), "r"(x), "r"(y), "r"(step) : "memory");
 }
 
-enum { FROM_GLOBAL = 0, FROM_MASK = 1, FROM_TILES = 2, FROM_BYTES = 3 };
+enum { FROM_GLOBAL = 0, FROM_MASK = 1, FROM_TILES = 2, FROM_BYTES = 3, FROM_MASK_SHORT = 4 };
 
 constexpr int WALK_THREADS = 1024;                          // per block with shared memory, one block per SM
 constexpr int GATHER_THREADS = 256;                         // at most, per block without
@@ -91,7 +92,11 @@ constexpr unsigned int MASK_MAX_BITS = 200u * 1024u * 8u;   // the rest of it: t
 
 // Connections that a walk over truths takes at a time.  (Uniform weights, 1e9 connections: 1517 us with 5, 1392 with 8, 1420
 // with 10, where the registers of 1024 threads run out; normal 1669 with 4, 1530 with 8.)
-constexpr int TRUTH_BATCH = 8;
+// A queue has one slot more than a batch at least.  Pairs of draws (normal) are 8 bytes, and from 1.26e6 events on the mask leaves
+// room for fewer than 1024 threads with nine slots: batches of 4 with six.  (Normal weights, p = 0.0005, 2 % of the events, batches of
+// 8 and of 4: 300,000 rows, 1.28e6 events 458, 375 us; 1.47e6 592, 480; 1.64e6 761, 600; 1e6 rows, 1.35e6 events 1283, 1222; 1.64e6
+// 2138, 1816.  With five slots instead of six: 1e6 rows, 1.54e6 events, 1545 and 1461.)
+constexpr int TRUTH_BATCH = 8, TRUTH_BATCH_SHORT = 4, SLOTS_SHORT = 6;
 // and a walk over tiles (homogeneous weights, 100,000 streams of 400: 155 us with 5, 149 with 8; uniform and normal: 2 % and 1 %
 // faster with 6 than with 5 and 4)
 template<int KIND> constexpr int TILE_BATCH = KIND == W_HOMO ? 8 : 6;
@@ -146,18 +151,18 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
                 const T scale, T *__restrict__ out) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     uint32_t *mask = reinterpret_cast<uint32_t *>(walk_smem);
-    constexpr bool BYTES = FROM == FROM_BYTES, TRUTH = FROM == FROM_MASK || BYTES;
+    constexpr bool BYTES = FROM == FROM_BYTES, BITS = FROM == FROM_MASK || FROM == FROM_MASK_SHORT, TRUTH = BITS || BYTES;
     // the queue of hits of this thread behind the events: slots of 4 (normal: 8) bytes, `queue_step` apart
     constexpr uint32_t SLOT = queue_slot_bytes(KIND);
     const uint32_t queue_step = SLOT * blockDim.x;
     const uint32_t queue = static_cast<uint32_t>(__cvta_generic_to_shared(walk_smem)) + truth_bytes(num_col, BYTES) + SLOT * threadIdx.x;
     E *tile = reinterpret_cast<E *>(walk_smem);
     constexpr bool SUMS = TRUTH || FROM == FROM_TILES;
-    constexpr int N = TRUTH ? TRUTH_BATCH : FROM == FROM_TILES ? TILE_BATCH<KIND> : Batch<KIND, QUICK>::N;
+    constexpr int N = FROM == FROM_MASK_SHORT ? TRUTH_BATCH_SHORT : TRUTH ? TRUTH_BATCH : FROM == FROM_TILES ? TILE_BATCH<KIND> : Batch<KIND, QUICK>::N;
     const Share share(num_row);
     const bool one_tile = tile_len >= num_col;
 
-    if (FROM == FROM_MASK) {
+    if (BITS) {
         pack_event_mask(in, num_col, mask);
         __syncthreads();
         // the first event of a word in its top bit: one shift by the position brings an event into the sign bit
@@ -248,7 +253,7 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
                 if (KIND != W_HOMO && __any_sync(FULL_MASK, next >= full)) drain();
             };
             auto draw = [&]() {
-                b.template draw<FROM == FROM_MASK>(s, at, num_col, gp);
+                b.template draw<BITS>(s, at, num_col, gp);
                 if (BYTES) at = min(at, num_col);
             };
             draw();
@@ -661,6 +666,13 @@ struct WalkGrid {
         waves = blocks_for(per_block, WALK_THREADS);
         threads = std::max(blocks_for(blocks_for(per_block, waves), 32) * 32u, at_least);
     }
+    // no more threads than `most` (a multiple of 32)
+    void at_most(unsigned int n, unsigned int most) {
+        if (threads <= most) return;
+        const unsigned int per_block = blocks_for(n, blocks);
+        waves = blocks_for(per_block, most);
+        threads = std::min(most, std::max(512u, blocks_for(blocks_for(per_block, waves), 32) * 32u));
+    }
 };
 
 // Tiles of equal length, a multiple of 32 elements, as few as fit.
@@ -705,27 +717,30 @@ void jit_rows(const JitCall<T, E> &c) {
     WalkGrid g(a.n_row, 512);
     if constexpr (TRUTH_ONLY) {
         // Bytes where they leave room for queues of 12 (normal: 10) hits of 1024 threads; then bits, whose walk keeps positions
-        // in 24 bits (a batch runs TRUTH_BATCH gaps, each below 23 mean ones, behind the end).
+        // in 24 bits (a batch runs TRUTH_BATCH gaps, each below 23 mean ones, behind the end).  Matrices beyond are gathered from global
+        // memory, which is faster for them (normal, 1e6 rows, 1.6e6 events, p = 1.2e-5, as bits in batches of 4: 236 us; gathered: 107).
         const unsigned int room = KIND == W_HOMO ? 0u : (KIND == W_UNIFORM ? 48u : 80u) * 1024u;
         const bool bytes = truth_bytes(a.n_col, true) <= WALK_SMEM - room && a.n_col <= WALK_SMEM;
         const bool bits = a.n_col <= MASK_MAX_BITS && a.n_col - TRUTH_BATCH * 23.0 / a.log_p < 16777216.0;
         if (gp.quick && (bytes || bits) && gathers > static_cast<double>(a.n_col) * sizeof(E) / 56 + 2000) {
             constexpr auto byte_kernel = jit_rows_kernel<T, E, KIND, EVENT, FROM_BYTES, true>;
             constexpr auto bit_kernel = jit_rows_kernel<T, E, KIND, EVENT, FROM_MASK, true>;
-            if (!(bytes ? allow_shared<byte_kernel>(WALK_SMEM) : allow_shared<bit_kernel>(WALK_SMEM))) {
+            constexpr auto short_kernel = jit_rows_kernel<T, E, KIND, EVENT, KIND == W_NORMAL ? FROM_MASK_SHORT : FROM_MASK, true>;
+            // what the events leave holds the queues of hits, up to 16 slots per thread (`seconds` has 32 bits); where they do not
+            // fit for all threads, for fewer, in equal waves again
+            const unsigned int taken = truth_bytes(a.n_col, bytes), left = WALK_SMEM - taken, slot_bytes = queue_slot_bytes(KIND);
+            unsigned int slots = 0;
+            bool in_short = false;
+            if (KIND != W_HOMO) {
+                in_short = KIND == W_NORMAL && left < slot_bytes * (TRUTH_BATCH + 1) * g.threads;
+                g.at_most(a.n_row, left / (slot_bytes * (in_short ? SLOTS_SHORT : TRUTH_BATCH + 1)) & ~31u);
+                slots = std::min(16u, left / (slot_bytes * g.threads));
+            }
+            if (!(bytes ? allow_shared<byte_kernel>(WALK_SMEM) : in_short ? allow_shared<short_kernel>(WALK_SMEM) : allow_shared<bit_kernel>(WALK_SMEM))) {
                 launch_ok();
                 return;
             }
-            // what the events leave holds the queues of hits, up to 16 slots per thread (`seconds` has 32 bits), and one more
-            // than a batch at least: beside a mask of the largest size only those of some threads fit
-            const unsigned int taken = truth_bytes(a.n_col, bytes), slot_bytes = queue_slot_bytes(KIND);
-            unsigned int slots = 0;
-            if (KIND != W_HOMO) {
-                const unsigned int fit = (WALK_SMEM - taken) / (slot_bytes * (TRUTH_BATCH + 1));
-                g.threads = std::min(g.threads, fit & ~31u);
-                slots = std::min(16u, (WALK_SMEM - taken) / (slot_bytes * g.threads));
-            }
-            (bytes ? byte_kernel : bit_kernel)<<<g.blocks, g.threads, static_cast<size_t>(taken) + slots * slot_bytes * g.threads, c.stream>>>(
+            (bytes ? byte_kernel : in_short ? short_kernel : bit_kernel)<<<g.blocks, g.threads, static_cast<size_t>(taken) + slots * slot_bytes * g.threads, c.stream>>>(
                 c.in, a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, 0, slots, c.scale, c.out);
             launch_ok();
             return;

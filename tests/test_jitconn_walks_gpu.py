@@ -202,6 +202,24 @@ def test_events_as_bytes_and_as_bits(cuda, kind, most, more):
   _compare(cuda, x, kind, 0.001, (9001, most + more), True, True)
 
 
+@pytest.mark.parametrize('n_row', [12_001, 160_001])       # 512 threads, 1024
+@pytest.mark.parametrize('n_col', [1_269_760, 1_269_761, 1_466_369, 1_638_400])
+def test_queues_beside_long_masks(cuda, n_row, n_col):
+  """The longest mask beside which 1024 threads have queues for batches of eight, and longer ones with queues of six for 1024 and
+  for fewer threads; half of the vector fires, so that they fill."""
+  x = np.random.default_rng(10).random(n_col) < 0.05
+  x[:n_col // 2] = True
+  _compare(cuda, x, 'normal', 1.2e-4 if n_row < 100_000 else 4e-5, (n_row, n_col), True, True)
+
+
+def test_time_of_event_rows_beside_long_masks(cuda):
+  """The masks that leave too little for queues of batches of eight cost no wave of rows (1.05 times the time; with it, 1.25)."""
+  def us(n_col):
+    x = torch.rand(n_col, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4)) < 0.02
+    return _device_us(lambda: _call(x, 'normal', 0.001, (300_000, n_col), True, True))
+  assert us(1_300_000) < 1.15 * us(1_250_000)
+
+
 @pytest.mark.parametrize('prob', [1.22e-5, 1.2e-5])      # the last mean gap whose positions bits keep in 24 bits; one beyond
 def test_events_as_bits_far_apart(cuda, prob):
   n = 1_638_400
