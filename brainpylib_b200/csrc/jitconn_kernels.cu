@@ -34,8 +34,8 @@ jit_rows_dense_v1_kernel(const T *__restrict__ vector, const unsigned int seed, 
     curandState state;
     curand_init(seed + row_i, 0, 0, &state);
     T sum = 0;
-    for (unsigned int c0 = 0; c0 < num_col; c0 += JIT_THREADS) {
-        const unsigned int n_tile = min(static_cast<unsigned int>(JIT_THREADS), num_col - c0);
+    for (unsigned int c0 = 0, n_tile; c0 < num_col; c0 += n_tile) {
+        n_tile = min(static_cast<unsigned int>(JIT_THREADS), num_col - c0);
         if (idx < n_tile) tile[idx] = vector[c0 + idx];
         __syncthreads();
         for (unsigned int sh_i = 0; sh_i < n_tile; ++sh_i) {
@@ -104,12 +104,13 @@ __host__ __device__ constexpr unsigned int queue_slot_bytes(int kind) { return k
 // shared memory of the events, as bits or bytes
 __host__ __device__ constexpr unsigned int truth_bytes(unsigned int n, bool bytes) { return ((bytes ? n : (n + 7u) >> 3) + 7u) & ~7u; }
 
-// The rows (columns) of a block: equal shares, so that no SM is left with a last wave of its own.
+// The rows (columns) of a block: equal shares, so that no SM is left with a last wave of its own.  They are counted from the
+// first: their numbers go up to 2^32 - 1, where a step of a block's threads would wrap.
 struct Share {
-    unsigned int begin, end;
+    unsigned int begin, count;
     __device__ __forceinline__ explicit Share(unsigned int n) {
         begin = static_cast<unsigned int>(static_cast<unsigned long long>(n) * blockIdx.x / gridDim.x);
-        end = static_cast<unsigned int>(static_cast<unsigned long long>(n) * (blockIdx.x + 1ull) / gridDim.x);
+        count = static_cast<unsigned int>(static_cast<unsigned long long>(n) * (blockIdx.x + 1ull) / gridDim.x) - begin;
     }
 };
 
@@ -175,9 +176,9 @@ jit_rows_kernel(const E *__restrict__ in, const unsigned int seed, const GapPara
         load_tile(tile, in, 0, num_col);
         __syncthreads();
     }
-    for (unsigned int row0 = share.begin; row0 < share.end; row0 += blockDim.x) {
-        const unsigned int row = row0 + threadIdx.x;
-        const bool live = row < share.end;
+    for (unsigned int from = 0; from < share.count; from += blockDim.x) {
+        const unsigned int row = share.begin + from + threadIdx.x;
+        const bool live = from + threadIdx.x < share.count;
         if (FROM == FROM_GLOBAL && !live) break;
         if (TRUTH && !__any_sync(FULL_MASK, live)) break;
         Xorwow s;
@@ -359,9 +360,9 @@ jit_cols_kernel(const T *__restrict__ vector, const unsigned int seed, const Gap
     T *tile = reinterpret_cast<T *>(walk_smem);
     constexpr int N = TILES ? TILE_BATCH<KIND> : Batch<KIND, QUICK>::N;
     const Share share(num_col);
-    for (unsigned int col0 = share.begin; col0 < share.end; col0 += blockDim.x) {
-        const unsigned int col = col0 + threadIdx.x;
-        const bool live = col < share.end;
+    for (unsigned int from = 0; from < share.count; from += blockDim.x) {
+        const unsigned int col = share.begin + from + threadIdx.x;
+        const bool live = from + threadIdx.x < share.count;
         if (!TILES && !live) break;
         Xorwow s;
         s.seed(seed + col);

@@ -136,6 +136,30 @@ def test_event_columns_up_to_32_bits(cuda, n_col):
     torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-6)
 
 
+def _ends(n):
+  return [*range(3), *range(n // 148 - 2, n // 148 + 2), n // 2, *range(n - 1030, n - 1020), *range(n - 3, n)]
+
+
+@pytest.mark.parametrize('kind,event,prob', [('homo', True, 0.3), ('uniform', True, 0.3), ('uniform', False, 0.3), ('homo', False, 1e-6)])
+def test_rows_up_to_32_bits(cuda, kind, event, prob):
+  """The largest number of rows, by events in shared memory, by tiles, by gathers: single rows against calls with each of them alone."""
+  n_row, n_col = (1 << 32) - 1, 11
+  x = torch.arange(n_col, device=cuda) % 2 == 0 if event else torch.arange(1., n_col + 1., device=cuda)
+  got = _call(x, kind, prob, (n_row, n_col), True, event)
+  for row in _ends(n_row):
+    torch.testing.assert_close(got[row:row + 1], _call(x, kind, prob, (1, n_col), True, event, seed=(77 + row) % (1 << 32)))
+
+
+@pytest.mark.parametrize('n_row,prob', [(11, 0.02), (11, 1e-6)])        # by tiles, by reductions
+def test_columns_up_to_32_bits(cuda, n_row, prob):
+  n_col = (1 << 32) - 1
+  x = torch.zeros(n_col, device=cuda)
+  x[_ends(n_col)] = torch.arange(1., len(_ends(n_col)) + 1., device=cuda)
+  got = _call(x, 'uniform', prob, (n_row, n_col), False, False)
+  want = sum(_call(x[c:c + 1].clone(), 'uniform', prob, (n_row, 1), False, False, seed=(77 + c) % (1 << 32)) for c in _ends(n_col))
+  torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize('kind', sorted(KINDS))
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 def test_one_lane_per_stream_in_tiles(cuda, dtype, kind):
