@@ -37,8 +37,8 @@ struct GapParams {
 };
 
 // The gap is (int) ceil(log(u) / log_p): float logarithm, double division.  With L = lg2.approx(u), over all 2^32 draws (on the
-// hardware; bpl_jit_gap_mismatches does it again for any log_p)
-//     |L ln2 - log(u)| <= LOG_ABS + LOG_REL |ln(u)|,
+// hardware: a test takes the largest share of it, RATIO)
+//     |L ln2 - log(u)| <= LOG_ABS + LOG_REL |L ln2|,
 // the error of the float logarithm included, so that the reference's quotient lies between the two ends
 //     L ln2 / log_p (1 -+ LOG_REL) -+ LOG_ABS / |log_p|,
 // whose roundings go outwards.  Adding 2^23 with rounding up leaves 2^23 + ceil() in the mantissa; where both ends agree that is

@@ -1,14 +1,12 @@
 """The ways a just-in-time product reads its input and gathers its sums (global memory, event bits, tiles of the vector,
 tiles of the output) against the CPU oracle, at sizes around the edges of tiles and of the rules that choose.  The
 oracle's logarithm may move single connections (it counts them); so many outputs may differ."""
-import ctypes
-
 import numpy as np
 import pytest
 import torch
 
 import brainpylib_b200 as bpl
-from oracle import cpu
+from oracle import cpu, draws
 from test_native_path_gpu import _device_us
 
 pytestmark = pytest.mark.gpu
@@ -285,9 +283,19 @@ def test_matmat_at_the_edges_of_tiles(cuda, k, dtype):
 @pytest.mark.parametrize('prob', [0.3, 0.01, 0.001, 5.7e-6])
 def test_gaps_of_all_draws(cuda, prob):
   """The two-sided test of a gap rests on measured errors of the logarithms: over all 2^32 draws it gives the reference's gap."""
-  from brainpylib_b200 import _lib
-  fn = _lib.lib().bpl_jit_gap_mismatches
-  fn.argtypes, fn.restype = [ctypes.c_void_p, ctypes.c_double, ctypes.c_void_p], ctypes.c_int
-  wrong = torch.zeros(1, dtype=torch.int64, device=cuda)
-  assert fn(torch.cuda.current_stream().cuda_stream, float(np.float32(np.log1p(-prob))), wrong.data_ptr()) == 1
-  assert int(wrong) == 0
+  assert draws.gap_mismatches(float(np.float32(np.log1p(-prob)))) == 0
+
+
+def test_errors_of_the_logarithms(cuda):
+  """The bound that the ends of a gap take, over all 2^32 draws: for every probability."""
+  assert 0.5 < draws.log_error() < 1
+
+
+@pytest.mark.parametrize('kind', [0, 1, 2])               # homogeneous, uniform, normal
+# batches of event walks (bits: positions in 24 bits, and bytes), of tiles, of the others
+@pytest.mark.parametrize('per_batch,sums,low24', [(8, True, True), (8, True, False), (4, True, True), (6, True, False), (4, False, False)])
+@pytest.mark.parametrize('prob,n', [(0.9, 3000), (0.01, 40_000), (0.001, 1_638_400), (1.22e-5, 1_638_400)])
+def test_batches_of_a_stream(cuda, prob, n, per_batch, sums, low24, kind):
+  """Positions and raw draws of batches, bit for bit, against one connection at a time by the reference's expression."""
+  connections, wrong = draws.batch_mismatches(kind, per_batch, sums, low24, float(np.float32(np.log1p(-prob))), 77, 20_000, n)
+  assert wrong == 0 and connections > 0.8 * 20_000 * n * prob
