@@ -37,7 +37,7 @@ struct GapParams {
 };
 
 // The gap is (int) ceil(log(u) / log_p): float logarithm, double division.  With L = lg2.approx(u), over all 2^32 draws (on the
-// hardware: a test takes the largest share of it, RATIO)
+// hardware: a test takes the largest share of it, 0.78)
 //     |L ln2 - log(u)| <= LOG_ABS + LOG_REL |L ln2|,
 // the error of the float logarithm included, so that the reference's quotient lies between the two ends
 //     L ln2 / log_p (1 -+ LOG_REL) -+ LOG_ABS / |log_p|,
