@@ -684,14 +684,15 @@ struct OuterVisit {
     __device__ __forceinline__ void put(uint32_t, Sum) const {}
 };
 
-// (`zero`: n_zero elements to clear for the launch behind this one)
+// (`zero`: n_zero elements to clear for the launch behind this one, which may then start early.  Without it the launch behind may be
+// any, also a dependent one that reads g as weights through the read-only path, and starts when this one has finished.)
 template<typename T, int U, uint32_t W, uint32_t LANES>
 __global__ void __launch_bounds__(W * 32, 1)
 outer_shared_kernel(const uint32_t *__restrict__ indices, const uint32_t *__restrict__ indptr,
                     const T *__restrict__ row_vector, const T *__restrict__ col_vector, T *__restrict__ g, T *__restrict__ zero,
                     const uint32_t n_zero, const uint32_t n_row, const uint32_t nse, const uint32_t n_col, const uint32_t long_from) {
     extern __shared__ __align__(16) unsigned char shared_vector[];
-    pdl_launch_dependents();
+    if (zero != nullptr) pdl_launch_dependents();
     for (uint32_t i = blockIdx.x * (W * 32u) + threadIdx.x; i < n_zero; i += gridDim.x * (W * 32u)) zero[i] = T(0);
     T *xs = reinterpret_cast<T *>(shared_vector);
     constexpr Deal<W, LANES> deal;

@@ -415,6 +415,29 @@ def test_time_of_a_product_with_a_long_row(cuda, n_row, n_col, op, bound):
   assert _device_us(call) < bound
 
 
+def test_a_list_product_right_behind_the_gradient_of_its_weights(cuda):
+  """The list product is a launch that may start early: behind the gradient of the weights alone, which it reads as constants, it
+  starts when that has finished."""
+  n_row, n_col = 40_000, 9001
+  data, indices, indptr = _skewed(n_row, n_col, np.random.default_rng(4).poisson(90, n_row), torch.float32, cuda)
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  p = bpl.LifExpParams(dt=0.1, tau_syn=[5.0], E_rev=[0.0])
+  zeros, V = torch.zeros(n_row, device=cuda), torch.full((n_row,), -40., device=cuda)
+  fired, spikes = bpl.lif_exp_step(zeros.clone(), zeros.clone(), V, torch.full_like(V, -1e7), p, 0.0)
+  assert bool((fired > 0).all())
+  data.requires_grad_(True)
+  for turn in range(5):
+    g = torch.Generator(device=cuda).manual_seed(turn)
+    x, ct = torch.rand(n_col, device=cuda, generator=g), torch.rand(n_row, device=cuda, generator=g)
+    y = bpl.csr_matvec(data, indices, indptr, x, shape=(n_row, n_col))
+    out, junk = torch.zeros(n_col, device=cuda), torch.full_like(data, float('nan'))
+    del junk                             # its memory is the gradient's
+    weights, = torch.autograd.grad(y, data, ct)
+    got = bpl.event_csr_matvec_from_list(weights, indices, indptr, spikes, out, shape=(n_row, n_col))
+    want = torch.zeros(n_col, dtype=torch.float64, device=cuda).index_add_(0, col, ct.double()[row] * x.double()[col])
+    torch.testing.assert_close(got.double(), want, rtol=1e-4, atol=1e-4)
+
+
 @pytest.mark.parametrize('events', [False, True])
 def test_time_of_few_equal_rows(cuda, events):
   """Rows that are longer than a warp's share of all entries, because there are fewer rows than warps, but no longer than the
