@@ -805,9 +805,11 @@ void jit_cols(const JitCall<T, T> &c) {
 template<typename T, typename E, int KIND>
 void jit_cols_event(const JitCall<T, E> &c) {
     const JitArgs &a = c.a;
+    if (a.n_col == 0) {                                    // (the clearing kernel lets the launch behind it start early: only with one of its own there)
+        if (cudaMemsetAsync(c.out, 0, sizeof(T) * static_cast<size_t>(a.n_row), c.stream) != cudaSuccess) launch_ok();
+        return;
+    }
     const unsigned int sms = static_cast<unsigned int>(sm_count());
-    jit_clear_kernel<T><<<std::min(blocks_for(a.n_row, 1024), 8 * sms), 256, 0, c.stream>>>(c.out, a.n_row);
-    if (!launch_ok() || a.n_col == 0) return;
     const GapParams gp = gap_params(a.log_p, a.n_row);
     const unsigned int waves = blocks_for(a.n_col, sms * COL_CHUNK);
     const unsigned int chunk = blocks_for(blocks_for(a.n_col, sms * waves), 16) * 16u, blocks = blocks_for(a.n_col, chunk);
@@ -824,6 +826,8 @@ void jit_cols_event(const JitCall<T, E> &c) {
         launch_ok();
         return;
     }
+    jit_clear_kernel<T><<<std::min(blocks_for(a.n_row, 1024), 8 * sms), 256, 0, c.stream>>>(c.out, a.n_row);
+    if (!launch_ok()) return;
     const cudaError_t e = launch_dependent(gp.quick ? quick : any, dim3(blocks), dim3(threads), chunk * sizeof(unsigned int), c.stream, c.in,
                                            a.seed, gp, a.w1, a.w2, a.n_row, a.n_col, chunk, few, c.out);
     if (e != cudaSuccess) set_status(BPL_ERR_CUDA, cudaGetErrorString(e));

@@ -99,6 +99,13 @@ def test_event_columns_by_chunks(cuda, shape, prob, rate, offset, dtype, kind):
   torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * max(float(want.abs().max()), 1e-3))
 
 
+def test_event_columns_of_a_matrix_without_columns(cuda):
+  x = torch.zeros(0, dtype=torch.bool, device=cuda)
+  junk = torch.full((501,), float('nan'), device=cuda)
+  del junk                                                # its memory is the output's
+  assert torch.equal(_call(x, 'uniform', 0.2, (501, 0), False, True), torch.zeros(501, device=cuda))
+
+
 def test_time_of_event_columns_above_one_list(cuda):
   """A few more columns than lists of 8192 on 148 SMs: no second wave of blocks (1.05 times the time; with it, 1.55)."""
   def us(n_col):
