@@ -849,11 +849,12 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     // clock).  The alternative gathers events through L1 and L2, 1.1 clocks each where they miss.
     const double per = static_cast<double>(m.nse) / sm_count(), gather = m.n_col * sizeof(E) > 200000u ? 1.0 : 0.6;
     const bool pack = m.n_col * sizeof(E) > 32768u;
-    // Few events, which L1 serves by broadcast: rows of one or two of the walk's steps, half of them empty, take it longer than
-    // the plain kernel (1e8 entries, rows of 121, 1037 columns: 106 us and 88; rows of 30: 35 and 41; of 700: 31 and 32).
-    // The lines lie between these three; where exactly both take the same was not measured.
+    // Few events, which L1 serves by broadcast, and one weight: with the entries of doubles taken one quad at a time, this walk is
+    // the slower one for rows of medium length (3001 columns, 1e8 entries, rows of 64, 121, 300, 512: plain kernel 113, 105, 119, 99
+    // us, here 119, 129, 121, 116; rows of 700, here 114).  Floats take two quads, and are faster here throughout (plain 113,
+    // 105, 121, 99; here 113, 86, 80, 79; with float events the same).  The lines lie where the plain kernel was measured to win.
     const double mean_row = static_cast<double>(m.nse) / m.n_row;
-    if (HOMO && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
+    if (HOMO && sizeof(T) == 8 && m.n_col * sizeof(E) <= 8192u && mean_row >= 64 && mean_row <= 512) return false;
     if (per * (gather - 0.25) < 2500 + (pack ? 2500 + bytes / 56.0 : m.n_col * sizeof(E) / 34.0)) return false;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     // Bytes take the vector's own length from L1, which streams the entries: 200 KB of them 157 us for 1e8 entries, bits 143.

@@ -157,7 +157,7 @@ def test_event_gather_over_bits(cuda, n_row, n_col, mean, homo, dtype, bool_even
 
 @pytest.mark.parametrize('homo', [True, False])
 @pytest.mark.parametrize('bool_events', [True, False])
-# events as bytes in shared memory: ragged ends, the most of them, one more (bits); few events with rows around the line
+# events as bytes in shared memory: ragged ends, the most of them, one more (bits); few events
 @pytest.mark.parametrize('n_row,n_col,mean', [(40_000, 8203, 60), (30_000, 131_072, 90), (30_000, 131_073, 90),
                                               (60_000, 2003, 64), (60_000, 2003, 63)])
 def test_event_gather_over_bytes(cuda, n_row, n_col, mean, homo, bool_events):
