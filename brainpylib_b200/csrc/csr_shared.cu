@@ -94,6 +94,11 @@ __host__ __device__ constexpr int from_quad(const uint32_t position, const uint3
 static_assert(from_quad(0x80000001u, 0x7ffffffcu) == 5 && from_quad(0x7ffffffdu, 0x80000000u) == -3, "");
 constexpr uint32_t MOST_ENTRIES = 0x7fffffffu;
 
+// Rows have 32 bits as well, and a walk asks for up to 256 rows per warp behind the last one: with at most so many rows, and 65536
+// blocks, their numbers stay below 2^32, where one would wrap and the walk begin again.
+constexpr uint32_t MOST_ROWS = 0x7fffffffu;
+static_assert(MOST_ROWS + 256ull * MANY_WARPS * 65536u < 1ull << 32, "the rows that a walk asks for");
+
 // `visit` has
 //   fetch(row)                            what is needed of a row besides its entries (requested one row ahead)
 //   quad<FULL>(base, c[4], w[4], lo, hi)  entries base .. base + 3, of which lo <= e < hi belong to the row (FULL: all)
@@ -777,7 +782,7 @@ struct Plan {
 
 template<typename T>
 bool usable(const CsrMatrix<T> &m, const bool weights) {
-    return m.n_row != 0 && m.n_col != 0 && m.nse != 0 && m.nse <= MOST_ENTRIES && m.n_col <= SHARED_SMEM / sizeof(T) && aligned16(m.indices) &&
+    return m.n_row != 0 && m.n_row <= MOST_ROWS && m.n_col != 0 && m.nse != 0 && m.nse <= MOST_ENTRIES && m.n_col <= SHARED_SMEM / sizeof(T) && aligned16(m.indices) &&
            (!weights || aligned16(m.data));
 }
 
@@ -842,7 +847,7 @@ bool gather_events_impl(cudaStream_t stream, const CsrMatrix<T> &m, const E *eve
     constexpr int U = sizeof(T) == 8 ? 1 : 2;
     using Sum = std::conditional_t<HOMO, uint32_t, T>;
     const uint32_t bytes = (m.n_col + 31u) / 32u * 4u;
-    if (m.n_row == 0 || m.n_col == 0 || m.nse == 0 || m.nse > MOST_ENTRIES || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
+    if (m.n_row == 0 || m.n_row > MOST_ROWS || m.n_col == 0 || m.nse == 0 || m.nse > MOST_ENTRIES || m.n_col > 8u * SHARED_SMEM || !aligned16(m.indices) ||
         (!HOMO && !aligned16(m.data)))
         return false;
     // The bits are packed by a launch of their own where the events are more than a block reads in its time (34 bytes per
