@@ -1,4 +1,4 @@
-// Whole-matrix CSR products with a vector in shared memory (csr_shared.cu).  Each function returns false, having done
+// Whole-matrix CSR products with a vector in shared memory (csr_shared.cuh).  Each function returns false, having done
 // nothing, where the plain kernels are faster or the operands do not fit; nse is the number of stored entries.
 #ifndef BPL_CSRC_CSR_SHARED_H_
 #define BPL_CSRC_CSR_SHARED_H_
@@ -25,9 +25,11 @@ bool gather_events(cudaStream_t stream, const CsrMatrix<T> &m, const E *events, 
 // y = A^T x; y need not be zero
 bool scatter_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *x, float *y);
 bool scatter_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *x, double *y);
-// g[e] = row_vector[row of e] * col_vector[indices[e]]; m.data is not read
-bool outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *row_vector, const float *col_vector, float *g);
-bool outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *row_vector, const double *col_vector, double *g);
+// g[e] = row_vector[row of e] * col_vector[indices[e]]; m.data is not read.  `zero`: n_zero elements to clear for the launch behind
+bool outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *row_vector, const float *col_vector, float *g,
+                  float *zero = nullptr, uint32_t n_zero = 0);
+bool outer_shared(cudaStream_t stream, const CsrMatrix<double> &m, const double *row_vector, const double *col_vector, double *g,
+                  double *zero = nullptr, uint32_t n_zero = 0);
 // g as above and y[row] = sum of data * col_vector[column] (the gradients of a transposed product), or y[column] = sum of
 // data * row_vector[row] (of the other one); y need not be zero
 bool gather_outer_shared(cudaStream_t stream, const CsrMatrix<float> &m, const float *row_vector, const float *col_vector, float *g, float *y);
