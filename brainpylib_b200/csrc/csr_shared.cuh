@@ -59,7 +59,8 @@ constexpr uint32_t LONG_ROWS = 128, BLOCK_ROW = 4096;
 // by 4, 8, 16 and 32 lanes, us: events, rows of 40 (one weight) 18.5, 22.5, 28.8, 50.6; of 64 20.1, 18.5, 21.3, 26.1; of 150 18.6, 16.4,
 // 17.6, 18.3; of 300 17.9, 17.3, 15.9, 17.7; products, rows of 64 20.0, 17.2, 20.5, 25.1; of 100 20.0, 17.4, 16.5, 19.0; of 300 17.0, 16.3,
 // 15.9, 15.9; of 900 32.4, 26.5, 15.6, 14.0.  4e6 double: products, rows of 100 20.9, 17.9, 16.0, 16.5; transposed, rows of 64 31.7, 32.0,
-// 30.8, 32.3, of 100 36.0, 31.7, 30.2, 28.7.  (The lanes that finish a mean row in one step, which is what all of them had: events, rows
+// 30.8, 32.3, of 100 36.0, 31.7, 30.2, 28.7.  Transposed floats, 1.2e7 entries, by 16 and 32 lanes: rows of 300, 1700 columns 39.0, 36.9,
+// 12,000 columns 34.9 both, 40,000 37.1, 38.9; of 396 40.8, 36.9; 34.9, 32.8; 37.1, 36.7.  (The lanes that finish a mean row in one step, which is what all of them had: events, rows
 // of 150 by 32 lanes 20.6.)  The lanes are constants of the kernels: as numbers they cost 3 to 10 % (rows of 300, 16 lanes, 16.9 us
 // and 15.9).  Products with outer values store what they read, and keep the lanes of one step.
 // Where few rows leave most warps with one group, or with none, the longest chain counts: a warp's groups, times the steps of `step`
@@ -68,7 +69,7 @@ constexpr uint32_t LONG_ROWS = 128, BLOCK_ROW = 4096;
 // uneven lengths count for more: by 16 lanes 15.6, by 32 14.0.)
 struct LaneRule { uint32_t four, eight, sixteen, step; };
 template<typename T> constexpr LaneRule PRODUCT_LANES = sizeof(T) == 8 ? LaneRule{32, 80, 200, 4} : LaneRule{48, 80, 400, 8};
-template<typename T> constexpr LaneRule SCATTER_LANES = sizeof(T) == 8 ? LaneRule{16, 40, 80, 4} : LaneRule{48, 80, 400, 8};
+template<typename T> constexpr LaneRule SCATTER_LANES = sizeof(T) == 8 ? LaneRule{16, 40, 80, 4} : LaneRule{48, 80, 280, 8};
 template<typename T> constexpr LaneRule EVENT_LANES = sizeof(T) == 8 ? LaneRule{80, 120, 400, 16} : LaneRule{48, 192, 400, 8};
 template<int U> constexpr LaneRule STEP_LANES{16u * U, 32u * U, 64u * U, 4u * U};
 inline uint32_t lanes_per_row(const uint32_t nse, const uint32_t n_row, const uint32_t warps, const LaneRule &rule) {
