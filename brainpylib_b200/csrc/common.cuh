@@ -138,12 +138,6 @@ __device__ __forceinline__ void zero_outside_rows(T *__restrict__ g, const uint3
     for (uint64_t i = from + me; i < nse; i += step) g[i] = T(0);
 }
 
-// *p = v in shared memory where `yes` is not zero, without a branch
-__device__ __forceinline__ void store_shared_if(const uint32_t yes, uint32_t *p, const uint32_t v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.shared.u32 [%1], %2; }"
-                 :: "r"(yes), "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(v) : "memory");
-}
-
 // 4 consecutive values to a 16-byte aligned address
 __device__ __forceinline__ void store_quad(float *p, float a, float b, float c, float d) {
     *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);

@@ -5,12 +5,13 @@
 //
 // What bounds the plain kernels (csr_kernels.cu): a gather of x through L1 takes one clock per entry and SM whatever it
 // hits (1e7 entries: 35 us, three times their memory time), a scattered reduction into L2 1.8 clocks (more on few
-// columns: 1.9e7 entries into 2185 sums took 853 us, here 46).  A lookup in shared memory takes a tenth of a clock, an
+// columns: 1.9e7 entries into 2185 sums took 853 us, here 52).  A lookup in shared memory takes a tenth of a clock, an
 // addition there 0.3.  So one block per SM holds the whole vector.
 //
-// Longer vectors are gathered through L1 (bands_kernel, csr_shared_gather.cu) or scattered into L2 (csr_kernels.cu).  What shared memory takes from
-// the 256 KB of an SM is missing for the entries in flight, which pass through L1: 1e7 float entries, 80 MB, take 18.6 us with up to 132 KB of x, 19.9 with
-// 160 KB, 23 with 195 KB, 31 with 226 KB.  For that reason neither the first 160 KB of a longer vector here and the rest
+// Longer vectors are gathered through L1 (bands_kernel, csr_shared_gather.cu) or scattered into L2 (csr_kernels.cu).  What
+// shared memory takes from the 256 KB of an SM is missing for the entries in flight, which pass through L1: 1e7 float entries, 80 MB,
+// rows of 100, take 18.5 us with up to 131 KB of x, 19.3 with 132 (24 warps), 19.8 with 160 KB, 30 with 195 KB; rows of 1000 17.8 with
+// 160 KB, 21.9 with 195 KB, 31.4 with 226 KB.  For that reason neither the first 160 KB of a longer vector here and the rest
 // by the plain ways (100,000 columns: gather 44 us against 39, scatter 78 against 65), nor slices of it in several blocks
 // that read the same rows side by side (58 us) paid; and reading a neighbour's slice out of its shared memory moves 0.33
 // random words per clock and SM.
