@@ -70,7 +70,7 @@ constexpr uint32_t LONG_ROWS = 128, BLOCK_ROW = 4096;
 // uneven lengths count for more: by 16 lanes 15.6, by 32 14.0.)
 struct LaneRule { uint32_t four, eight, sixteen, step; };
 template<typename T> constexpr LaneRule PRODUCT_LANES = sizeof(T) == 8 ? LaneRule{32, 80, 200, 4} : LaneRule{48, 80, 400, 8};
-template<typename T> constexpr LaneRule SCATTER_LANES = sizeof(T) == 8 ? LaneRule{16, 40, 80, 4} : LaneRule{48, 80, 280, 8};
+template<typename T> constexpr LaneRule SCATTER_LANES = sizeof(T) == 8 ? LaneRule{16, 40, 80, 4} : LaneRule{48, 80, 340, 8};
 template<typename T> constexpr LaneRule EVENT_LANES = sizeof(T) == 8 ? LaneRule{80, 120, 400, 16} : LaneRule{48, 192, 400, 8};
 template<int U> constexpr LaneRule STEP_LANES{16u * U, 32u * U, 64u * U, 4u * U};
 inline uint32_t lanes_per_row(const uint32_t nse, const uint32_t n_row, const uint32_t warps, const LaneRule &rule) {

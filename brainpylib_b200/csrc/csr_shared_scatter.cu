@@ -79,8 +79,12 @@ bool scatter_impl(cudaStream_t stream, const CsrMatrix<T> &m, const T *x, T *y, 
     // columns 20.5, 22.6; 1.2e7, of 500, 34.8, 36.8; 2e7, of 450, 51.3, 52.8; of 900 the same.  (Of 1500, 1.2e7, 34.8 and 32.8; doubles of
     // 1500 41.9 and 34.5, of 396, 1.5e6, 17.8 and 15.2.)
     const uint32_t mean = m.nse / m.n_row;
-    if (sizeof(T) == 4 && mean > 400u && mean <= 1000u) with_lanes<FEW_WARPS>(m.nse, m.n_row, SCATTER_LANES<T>, launch);
-    else with_block(m, m.n_col * sizeof(T), SCATTER_LANES<T>, launch);
+    LaneRule rule = SCATTER_LANES<T>;
+    // Few columns: the 32 lanes sooner.  By 16 and 32, rows of 300: 1.2e7 entries, 1700 columns 39.0, 36.9, 8000 columns 35.7, 33.8,
+    // 40,000 columns 35.9, 38.0; 2e7, 16,000 columns 47.5, 50.3, 40,000 columns 50.3, 52.3.
+    if (sizeof(T) == 4 && m.n_col <= 8192u) rule.sixteen = 280u;
+    if (sizeof(T) == 4 && mean > 400u && mean <= 1000u) with_lanes<FEW_WARPS>(m.nse, m.n_row, rule, launch);
+    else with_block(m, m.n_col * sizeof(T), rule, launch);
     return true;
 }
 
