@@ -367,11 +367,17 @@ bool usable(const CsrMatrix<T> &m, const bool weights) {
 // columns from which the bands are faster than x in shared memory (200 KB of floats; of doubles, 164 KB)
 template<typename T> constexpr uint32_t BANDS_FROM = sizeof(T) == 4 ? 51200u : 21000u;
 
+// Where a row is cut: see LONG_ROWS.  No farther than any row reaches, so that a row's start and this stay below 2^32.
+constexpr uint32_t cut_from(const uint32_t nse, const uint32_t n_row, const uint32_t warps, const uint32_t lanes) {
+    return std::min(std::max(std::max(64u, nse / warps / 16u) * lanes, 2u * (nse / n_row)), MOST_ENTRIES);
+}
+static_assert(MOST_ENTRIES + static_cast<uint64_t>(cut_from(MOST_ENTRIES, 1u, FEW_WARPS, 32u)) < 1ull << 32, "where the longest row is cut");
+
 // go(warps of a block, lanes of a row, where rows are cut): the first two are constants
 template<uint32_t W, typename Go>
 void with_lanes(const uint32_t nse, const uint32_t n_row, const LaneRule &rule, Go go) {
     const uint32_t warps = static_cast<uint32_t>(sm_count()) * W, lanes = lanes_per_row(nse, n_row, warps, rule);
-    const uint32_t long_from = std::max(std::max(64u, nse / warps / 16u) * lanes, 2u * (nse / n_row));
+    const uint32_t long_from = cut_from(nse, n_row, warps, lanes);
     constexpr std::integral_constant<uint32_t, W> w;
     if (lanes == 4u) go(w, std::integral_constant<uint32_t, 4>(), long_from);
     else if (lanes == 8u) go(w, std::integral_constant<uint32_t, 8>(), long_from);
