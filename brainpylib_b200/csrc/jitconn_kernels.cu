@@ -616,6 +616,17 @@ jit_matmat_kernel(const T *__restrict__ X, const unsigned int seed, const GapPar
     }
 }
 
+// Tests: how many of all 2^32 draws have another gap than the reference's expression gives.
+__global__ void __launch_bounds__(256) jit_gap_mismatches_kernel(const GapParams g, unsigned long long *__restrict__ count) {
+    unsigned long long wrong = 0;
+    for (unsigned long long x = blockIdx.x * 256ull + threadIdx.x; x < 1ull << 32; x += gridDim.x * 256ull) {
+        const float u = _curand_uniform(static_cast<uint32_t>(x));
+        wrong += gap_of(static_cast<uint32_t>(x), g) != static_cast<int>(ceil(log(u) / g.log_p));
+    }
+    for (int o = 16; o > 0; o >>= 1) wrong += __shfl_xor_sync(FULL_MASK, wrong, o);
+    if ((threadIdx.x & 31u) == 0 && wrong != 0) atomicAdd(count, wrong);
+}
+
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
@@ -938,6 +949,14 @@ void bpl_jit_matvec(bpl_stream_t stream, const void *in, void *out, int in_type,
     const JitArgs a{n_row, n_col, seed, log_p, kind == W_HOMO ? 0.0 : static_cast<double>(w1),
                     kind == W_HOMO ? 0.0 : static_cast<double>(w2)};
     (events ? event[in_type] : dense[in_type - 1])[kind](stream, in, out, a, rows != 0, scale);
+}
+
+// Tests only: adds to *count (device memory) the draws whose gap the quick test gets wrong; 0 where log_p is outside its range.
+int bpl_jit_gap_mismatches(bpl_stream_t stream, double log_p, unsigned long long *count) {
+    const GapParams g = gap_params(log_p, 1u);
+    if (!g.quick) return 0;
+    jit_gap_mismatches_kernel<<<16 * sm_count(), 256, 0, stream>>>(g, count);
+    return launch_ok() ? 1 : 0;
 }
 
 #define JIT_MATVEC(name, T, KIND, ROWS) \

@@ -88,6 +88,9 @@ size_t bpl_workspace_bytes(const char *target_name, const char *opaque, size_t o
  * the *_v1_ws matmat targets (0 restores the computed ones), so that a small matrix overflows its lists (the
  * recomputation pass runs) or is walked in several chunks. */
 void bpl_matmat_list_limits_for_tests(uint32_t cap, size_t budget_bytes);
+/* Tests only: adds to *count (device memory) how many of all 2^32 draws the quick test of the just-in-time walks gives another
+ * gap than (int) ceil(log(u) / log_p); returns 0, having done nothing, for a log_p outside its range. */
+int bpl_jit_gap_mismatches(bpl_stream_t stream, double log_p, unsigned long long *count);
 
 /* ---- profiling hook (no counterpart in the reference) -------------------------------------
  * When both are non-NULL cudaEvent_t handles, every later event_csr_matvec_* call with

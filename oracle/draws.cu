@@ -17,17 +17,6 @@ __global__ void __launch_bounds__(256) log_error_kernel(unsigned long long *__re
     if ((threadIdx.x & 31u) == 0) atomicMax(most, static_cast<unsigned long long>(__double_as_longlong(worst)));      // (not negative)
 }
 
-// How many of all 2^32 draws have another gap than the reference's expression gives.
-__global__ void __launch_bounds__(256) gap_mismatches_kernel(const GapParams g, unsigned long long *__restrict__ count) {
-    unsigned long long wrong = 0;
-    for (unsigned long long x = blockIdx.x * 256ull + threadIdx.x; x < 1ull << 32; x += gridDim.x * 256ull) {
-        const float u = _curand_uniform(static_cast<uint32_t>(x));
-        wrong += gap_of(static_cast<uint32_t>(x), g) != static_cast<int>(ceil(log(u) / g.log_p));
-    }
-    for (int o = 16; o > 0; o >>= 1) wrong += __shfl_xor_sync(0xffffffffu, wrong, o);
-    if ((threadIdx.x & 31u) == 0 && wrong != 0) atomicAdd(count, wrong);
-}
-
 // Streams seed .. seed + n_streams - 1 in batches, and one connection at a time by the reference's expression: count[0] the
 // connections inside the range, count[1] those whose position or raw draws differ.
 template<int KIND, int COUNT, bool SUMS, bool LOW24>
@@ -83,13 +72,6 @@ extern "C" {
 // All write to device memory that the caller has cleared, and return 0 or a CUDA error; -1 for a log_p outside the quick test's range.
 int draws_log_error(double *most, cudaStream_t stream) {
     log_error_kernel<<<148 * 8, 256, 0, stream>>>(reinterpret_cast<unsigned long long *>(most));
-    return cudaGetLastError();
-}
-
-int draws_gap_mismatches(double log_p, unsigned long long *count, cudaStream_t stream) {
-    const GapParams g = gap_params(log_p, 1u);
-    if (!g.quick) return -1;
-    gap_mismatches_kernel<<<148 * 8, 256, 0, stream>>>(g, count);
     return cudaGetLastError();
 }
 

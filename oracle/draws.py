@@ -36,14 +36,6 @@ def log_error():
   return float(out)
 
 
-def gap_mismatches(log_p):
-  """How many of all 2^32 draws get another gap than ``(int) ceil(log(u) / log_p)``."""
-  import torch
-  out = torch.zeros(1, dtype=torch.int64, device='cuda')
-  _call('gap_mismatches', ctypes.c_double(log_p), ctypes.c_void_p(out.data_ptr()))
-  return int(out)
-
-
 def batch_mismatches(kind, per_batch, sums, low24, log_p, seed, n_streams, n):
   """``(connections, wrong ones)`` of the streams ``seed ..`` over ``n`` positions, in batches against one connection at a time."""
   import torch

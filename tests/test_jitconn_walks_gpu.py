@@ -1,6 +1,8 @@
 """The ways a just-in-time product reads its input and gathers its sums (global memory, event bits, tiles of the vector,
 tiles of the output) against the CPU oracle, at sizes around the edges of tiles and of the rules that choose.  The
 oracle's logarithm may move single connections (it counts them); so many outputs may differ."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -290,7 +292,12 @@ def test_matmat_at_the_edges_of_tiles(cuda, k, dtype):
 @pytest.mark.parametrize('prob', [0.3, 0.01, 0.001, 5.7e-6])
 def test_gaps_of_all_draws(cuda, prob):
   """The two-sided test of a gap rests on measured errors of the logarithms: over all 2^32 draws it gives the reference's gap."""
-  assert draws.gap_mismatches(float(np.float32(np.log1p(-prob)))) == 0
+  from brainpylib_b200 import _lib
+  fn = _lib.lib().bpl_jit_gap_mismatches
+  fn.argtypes, fn.restype = [ctypes.c_void_p, ctypes.c_double, ctypes.c_void_p], ctypes.c_int
+  wrong = torch.zeros(1, dtype=torch.int64, device=cuda)
+  assert fn(torch.cuda.current_stream().cuda_stream, float(np.float32(np.log1p(-prob))), wrong.data_ptr()) == 1
+  assert int(wrong) == 0
 
 
 def test_errors_of_the_logarithms(cuda):
