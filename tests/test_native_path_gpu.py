@@ -502,11 +502,16 @@ def test_both_gradients_at_once(cuda, kind, front, transpose, dtype):
   torch.testing.assert_close(g_x.double(), want_x, **tol)
 
 
-# One weight and few events: rows of 64 to 512 go to the plain kernel; 9001 events are too many for that.
-@pytest.mark.parametrize('homo,n_col', [(False, 3001), (True, 3001), (True, 9001)])
+@pytest.mark.parametrize('homo', [True, False])
 @pytest.mark.parametrize('mean', [60, 100, 200, 300, 500])         # 4, 8, 16, 16 and 32 lanes per row
-def test_event_gather_of_doubles(cuda, mean, homo, n_col):
-  test_event_gather_over_bits(cuda, 30_000, n_col, mean, homo, np.float64, True)
+def test_event_gather_of_doubles(cuda, mean, homo):
+  test_event_gather_over_bits(cuda, 30_000, 3001, mean, homo, np.float64, True)
+
+
+# One weight and few events: rows of 64 to 512 go to the plain kernel; 9001 events are too many for that.
+@pytest.mark.parametrize('mean', [60, 100, 200, 300, 500])         # 4, 8, 16, 16 and 32 lanes per row
+def test_event_gather_of_doubles_with_one_weight(cuda, mean):
+  test_event_gather_over_bits(cuda, 30_000, 9001, mean, True, np.float64, True)
 
 
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
@@ -532,6 +537,29 @@ def test_products_by_more_and_fewer_warps(cuda, more, dtype):
 @pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
 @pytest.mark.parametrize('n_row,mean', [(60_000, 12), (40_000, 30), (30_000, 60), (30_000, 90), (15_000, 300), (9_000, 600), (2_000, 300)])
 def test_products_by_lanes_per_row(cuda, n_row, mean, dtype):
+  n_col = 3001
+  rng = np.random.default_rng(mean)
+  lengths = rng.poisson(mean, n_row)
+  lengths[rng.integers(0, n_row, n_row // 50)] = 0
+  lengths[[1, n_row // 2, n_row - 1]] = 70 * mean, 30_000, 65 * 32          # cut: for the warp, for the block, the last row
+  data, indices, indptr = _skewed(n_row, n_col, lengths, dtype, cuda)
+  row, col = sparse_ops.csr_to_coo(indices, indptr)
+  g = torch.Generator(device=cuda).manual_seed(9)
+  eps = torch.finfo(dtype).eps
+  for transpose in (False, True):
+    src, dst = (row, col) if transpose else (col, row)
+    x = torch.randn(n_row if transpose else n_col, dtype=dtype, device=cuda, generator=g)
+    for w in (data, data[:1]):
+      y = bpl.csr_matvec(w, indices, indptr, x, shape=(n_row, n_col), transpose=transpose)
+      terms = w.double() * x.double()[src]
+      want, size = (torch.zeros_like(y, dtype=torch.float64).index_add_(0, dst, t) for t in (terms, terms.abs()))
+      steps = torch.bincount(dst, minlength=y.shape[0]) + 1
+      assert bool(((y.double() - want).abs() <= eps * steps * size).all())          # each term takes part in at most so many sums
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('n_row,mean', [(60_000, 12), (40_000, 30), (30_000, 60), (30_000, 90), (15_000, 300), (9_000, 600), (2_000, 300)])
+def test_exact_products_by_lanes_per_row(cuda, n_row, mean, dtype):
   n_col = 3001
   rng = np.random.default_rng(mean)
   lengths = rng.poisson(mean, n_row)
